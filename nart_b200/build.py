@@ -1,5 +1,5 @@
-"""In-tree build of ``libnart_b200.so`` (CUDA kernels + C-ABI) and, where the art runtime headers
-are available, of the art plugin ``libart_module_b200.so``.
+"""In-tree build of ``libnart_b200.so`` (CUDA kernels + C-ABI), of ``_py_ops.so`` (the native call path of
+``nart_b200.ops``) and, where the art runtime headers are available, of the art plugin ``libart_module_b200.so``.
 
     python -m nart_b200.build            # build what is stale
     python -m nart_b200.build --force
@@ -23,6 +23,7 @@ MODSRC = os.path.join(PKG, "module")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libnart_b200.so")
 MODULE_LIB = os.path.join(PKG, "libart_module_b200.so")
+PY_OPS = os.path.join(PKG, "_py_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -80,6 +81,28 @@ def build_library(force: bool = False) -> str:
     return LIB
 
 
+def build_py_ops(force: bool = False) -> str:
+    """The native call path of ``nart_b200.ops`` (CPython + torch headers, linked to libnart_b200.so)."""
+    src = os.path.join(CSRC, "py_ops.cpp")
+    if force or _stale(PY_OPS, [src, os.path.join(ROOT, "include", "nart_b200.h")]):
+        import sysconfig
+
+        import torch
+        base = os.path.dirname(torch.__file__)
+        incs = [os.path.join(ROOT, "include"), os.path.join(base, "include"),
+                os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+                os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+        cmd += ["-I" + d for d in incs[:1]] + ["-isystem" + d for d in incs[1:]] + [src, "-o", PY_OPS]
+        cmd += ["-L" + PKG, "-lnart_b200", "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu",
+                "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError("py_ops build failed:\n" + res.stdout + res.stderr)
+    return PY_OPS
+
+
 def art_include_dirs() -> list[str] | None:
     """Include directories of the art runtime (the plugin's ABI headers).  They belong to the
     reference project and are used where they lie; ``NART_ART_ROOT`` names its ``art`` folder (default:
@@ -130,6 +153,7 @@ def main(argv=None) -> int:
     ap.add_argument("--ptxas", action="store_true", help="print the ptxas -v report")
     a = ap.parse_args(argv)
     print(build_library(a.force))
+    print(build_py_ops(a.force))
     print(build_module(a.force))
     if a.ptxas:
         print(ptxas_report())

@@ -4,7 +4,8 @@ Names and argument meaning follow the art ``quant`` module's ops (conv_2d, ip, q
 dequantize, eltwise, add, relu, pool -- art/modules/quant/src/quant_module.c:49-66 of
 ModelTC/NART) and their ``SETTING_QUANT_*`` settings (ialpha/izp, walpha/wzp, oalpha/ozp/obits).
 torch is used only to own device memory and to name the current stream; all compute goes through
-``libnart_b200.so``.  Device activations are uint8 NHWC ``[N, H, W, C]`` tensors.
+``libnart_b200.so``.  The calls of a forward pass cross into it through ``_py_ops.so`` (csrc/py_ops.cpp), which checks
+the tensors, allocates the output and launches natively; like the library it has no fallback.  Device activations are uint8 NHWC ``[N, H, W, C]`` tensors.
 """
 from __future__ import annotations
 
@@ -14,6 +15,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from . import _py_ops
 from ._lib import ACT_S8, ACT_U8, ALGO_AUTO, ALGO_DIRECT, ALGO_IGEMM, POOL_AVE, POOL_MAX, ConvParams, check, lib
 
 
@@ -80,17 +82,16 @@ class Conv2d:
         self.algo = lib.b200_conv2d_algo(self._h)
 
     def __call__(self, x: torch.Tensor, return_acc: bool = False):
+        if not return_acc:
+            return _py_ops.conv_run(self._h.value or 0, x, self.signed, *self.in_hw, self.c, *self.out_hw, self.k)
         _dev_s8(x) if self.signed else _dev_u8(x)
         n, h, w, c = x.shape
         if (h, w) != self.in_hw or c != self.c:
             raise ValueError("input %s does not match the prepared plan" % (tuple(x.shape),))
         y = torch.empty((n, self.out_hw[0], self.out_hw[1], self.k), dtype=x.dtype, device=x.device)
-        if return_acc:
-            acc = torch.empty(y.shape, dtype=torch.int32, device=x.device)
-            check(lib.b200_conv2d_run_acc(self._h, x.data_ptr(), n, y.data_ptr(), acc.data_ptr(), _stream()))
-            return y, acc
-        check(lib.b200_conv2d_run(self._h, x.data_ptr(), n, y.data_ptr(), _stream()))
-        return y
+        acc = torch.empty(y.shape, dtype=torch.int32, device=x.device)
+        check(lib.b200_conv2d_run_acc(self._h, x.data_ptr(), n, y.data_ptr(), acc.data_ptr(), _stream()))
+        return y, acc
 
     def describe(self) -> str:
         buf = C.create_string_buffer(256)
@@ -168,46 +169,22 @@ class InnerProductS8(Conv2d):
 
 def quantize_s8(x: torch.Tensor, oalpha: float, obits: int = 8, nhwc: bool = True):
     """quantize with qtype SYMMETRIC: float32 NCHW -> int8 (NHWC by default)."""
-    if not (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and x.dim() == 4):
-        raise ValueError("expected a contiguous float32 NCHW CUDA tensor")
-    n, c, h, w = x.shape
-    y = torch.empty((n, h, w, c) if nhwc else (n, c, h, w), dtype=torch.int8, device=x.device)
-    check(lib.b200_quantize_s8(x.data_ptr(), y.data_ptr(), n, c, h, w, oalpha, obits, int(nhwc), _stream()))
-    return y
+    return _py_ops.quantize(x, oalpha, 0, obits, nhwc, True)
 
 
 def dequantize_s8(x: torch.Tensor, ialpha: float, nhwc: bool = True):
     """dequantize of an int8 tensor (NHWC by default) -> float32 NCHW."""
-    _dev_s8(x)
-    if nhwc:
-        n, h, w, c = x.shape
-    else:
-        n, c, h, w = x.shape
-    y = torch.empty((n, c, h, w), dtype=torch.float32, device=x.device)
-    check(lib.b200_dequantize_s8(x.data_ptr(), y.data_ptr(), n, c, h, w, ialpha, int(nhwc), _stream()))
-    return y
+    return _py_ops.dequantize(x, ialpha, 0, nhwc, True)
 
 
 def quantize(x: torch.Tensor, oalpha: float, ozp: int, obits: int = 8, nhwc: bool = True):
     """quantize: float32 NCHW -> uint8 (NHWC by default, the device layout)."""
-    if not (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and x.dim() == 4):
-        raise ValueError("expected a contiguous float32 NCHW CUDA tensor")
-    n, c, h, w = x.shape
-    y = torch.empty((n, h, w, c) if nhwc else (n, c, h, w), dtype=torch.uint8, device=x.device)
-    check(lib.b200_quantize_u8(x.data_ptr(), y.data_ptr(), n, c, h, w, oalpha, ozp, obits, int(nhwc), _stream()))
-    return y
+    return _py_ops.quantize(x, oalpha, ozp, obits, nhwc, False)
 
 
 def dequantize(x: torch.Tensor, ialpha: float, izp: int, nhwc: bool = True):
     """dequantize: uint8 (NHWC by default) -> float32 NCHW."""
-    _dev_u8(x)
-    if nhwc:
-        n, h, w, c = x.shape
-    else:
-        n, c, h, w = x.shape
-    y = torch.empty((n, c, h, w), dtype=torch.float32, device=x.device)
-    check(lib.b200_dequantize_u8(x.data_ptr(), y.data_ptr(), n, c, h, w, ialpha, izp, int(nhwc), _stream()))
-    return y
+    return _py_ops.dequantize(x, ialpha, izp, nhwc, False)
 
 
 def nchw_to_nhwc(x: torch.Tensor, c_pad: int | None = None, fill: int = 0):
@@ -230,16 +207,7 @@ def nhwc_to_nchw(x: torch.Tensor, c: int | None = None):
 
 def eltwise_sum(xs, ialpha, izp, oalpha, ozp, obits: int = 8, coeff=None, relu: bool = False):
     """eltwise SUM / add of the quant module on same-shaped uint8 tensors."""
-    xs = [_dev_u8(t) for t in xs]
-    n = len(xs)
-    ptrs = (C.c_void_p * n)(*[t.data_ptr() for t in xs])
-    ia = (C.c_float * n)(*[float(a) for a in ialpha])
-    iz = (C.c_uint8 * n)(*[int(z) for z in izp])
-    cf = None if coeff is None else (C.c_float * n)(*[float(v) for v in coeff])
-    y = torch.empty_like(xs[0])
-    check(lib.b200_eltwise_sum_u8(ptrs, n, xs[0].numel(), ia, iz, cf, oalpha, ozp, obits, int(relu),
-                                  y.data_ptr(), _stream()))
-    return y
+    return _py_ops.eltwise_sum(list(xs), list(ialpha), list(izp), None if coeff is None else list(coeff), oalpha, ozp, obits, relu)
 
 
 def add(x0, x1, ialpha, izp, oalpha, ozp, obits: int = 8):
@@ -248,10 +216,7 @@ def add(x0, x1, ialpha, izp, oalpha, ozp, obits: int = 8):
 
 
 def relu(x: torch.Tensor, ialpha, izp, oalpha, ozp, obits: int = 8):
-    _dev_u8(x)
-    y = torch.empty_like(x)
-    check(lib.b200_relu_u8(x.data_ptr(), x.numel(), ialpha, izp, oalpha, ozp, obits, y.data_ptr(), _stream()))
-    return y
+    return _py_ops.relu(x, ialpha, izp, oalpha, ozp, obits)
 
 
 def pool_out_dims(h, w, kernel, pad, stride, ceil_mode):
@@ -264,14 +229,8 @@ def pool_out_dims(h, w, kernel, pad, stride, ceil_mode):
 def pool(x: torch.Tensor, method: int, kernel, pad, stride, ceil_mode, ialpha, izp, oalpha, ozp,
          obits: int = 8):
     """pool of the quant module (method POOL_MAX / POOL_AVE) on a uint8 NHWC tensor."""
-    _dev_u8(x)
-    n, h, w, c = x.shape
-    oh, ow = pool_out_dims(h, w, kernel, pad, stride, ceil_mode)
-    y = torch.empty((n, oh, ow, c), dtype=torch.uint8, device=x.device)
-    check(lib.b200_pool_u8(x.data_ptr(), n, c, h, w, method, kernel[0], kernel[1], pad[0], pad[1],
-                           stride[0], stride[1], int(ceil_mode), ialpha, izp, oalpha, ozp, obits,
-                           y.data_ptr(), _stream()))
-    return y
+    return _py_ops.pool(x, method, kernel[0], kernel[1], pad[0], pad[1], stride[0], stride[1], ceil_mode, ialpha, izp, oalpha,
+                        ozp, obits)
 
 
 def device_status() -> int:
