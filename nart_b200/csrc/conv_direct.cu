@@ -62,6 +62,8 @@ __global__ void __launch_bounds__(256) conv_direct_kernel(
     const uint32_t x_flip = g.act_signed ? 0x80808080u : 0u;   // int8 bytes seen as uint8 with zero point 128
     const uint8_t *ximg = x + (size_t)img * g.h * g.w * g.c + (size_t)grp * cg;
 
+    pdl_wait();
+    pdl_trigger();
     int acc[4] = { 0, 0, 0, 0 };
     // wzp != 128: sum of the bytes the products see (out-of-image taps read izp, like the products),
     // with the bytes past the group's last channel masked out of the last word
@@ -153,6 +155,8 @@ __global__ void __launch_bounds__(256) conv_depthwise_kernel(
     const int32_t *__restrict__ bias_fold, const uint32_t *__restrict__ mult,
     const int32_t *__restrict__ shift, uint8_t *__restrict__ y, int n)
 {
+    pdl_wait();
+    pdl_trigger();
     const int cv = g.c / 16;
     const size_t total = (size_t)n * g.oh * g.ow * cv;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -243,6 +247,8 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_kernel(
     ConvGeom g, const uint32_t *__restrict__ x, const uint4 *__restrict__ w3, const int4 *__restrict__ q3,
     uint32_t *__restrict__ y, int n)
 {
+    pdl_wait();
+    pdl_trigger();
     const uint32_t cq = (uint32_t)g.c / 4;
     const uint32_t total = (uint32_t)n * g.oh * g.ow * cq;      // the launcher checks that it fits 32 bits
     const uint32_t izp4 = (uint32_t)g.izp * 0x01010101u;
@@ -316,6 +322,8 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_pair_kernel(
     uint32_t *__restrict__ y, int n)
 {
     constexpr int IN_ROWS = 3 + (ROWS - 1) * S, IN_COLS = 3 + S, NV = S == 2 ? 3 : 2;
+    pdl_wait();
+    pdl_trigger();
     const uint32_t cq = (uint32_t)g.c / 4;
     const uint32_t owp = ((uint32_t)g.ow + 1) / 2, ohp = ((uint32_t)g.oh + ROWS - 1) / ROWS;
     const uint32_t total = (uint32_t)n * ohp * owp * cq;      // the launcher checks that it fits 32 bits
@@ -406,10 +414,11 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_pair_kernel(
 }
 
 template <int ROWS, int S>
-static void depthwise3x3_pair_launch(const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st)
+static int depthwise3x3_pair_launch(const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st)
 {
     const size_t total = (size_t)n * ((g.oh + ROWS - 1) / ROWS) * ((g.ow + 1) / 2) * (g.c / 4);
-    conv_depthwise3x3_pair_kernel<ROWS, S><<<resident_grid<conv_depthwise3x3_pair_kernel<ROWS, S>, 256>((total + 255) / 256), 256, 0, st>>>(
+    return launch_kernel(
+        conv_depthwise3x3_pair_kernel<ROWS, S>, dim3(resident_grid<conv_depthwise3x3_pair_kernel<ROWS, S>, 256>((total + 255) / 256)), dim3(256), 0, st, (size_t)n * g.c * (g.h * g.w + g.oh * g.ow), 1,
         g, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint4 *>(p.w_dw3p_dev), p.q_dw3_dev,
         reinterpret_cast<uint32_t *>(y), n);
 }
@@ -423,6 +432,8 @@ __global__ void __launch_bounds__(256) conv_lower_rows_kernel(
     const uint32_t *__restrict__ x, uint4 *__restrict__ out, int n, int h, int w, int ow, int stride_w, int pad_w,
     uint32_t izp4)
 {
+    pdl_wait();
+    pdl_trigger();
     const size_t total = (size_t)n * h * ow;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -451,11 +462,10 @@ int conv_lower_rows_launch(const ConvGeom &g, const uint8_t *x, int n, uint8_t *
         return fail(B200_ERR_INVALID, "conv(lower): needs a 4-channel, word-aligned input");
     const size_t total = (size_t)n * g.h * g.ow;
     const int blocks = resident_grid<conv_lower_rows_kernel, 256>((total + 255) / 256);
-    conv_lower_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>(
+    return launch_kernel(
+        conv_lower_rows_kernel, dim3((unsigned)blocks), dim3(256), 0, st, total * (kLowerWindow * 4), 1,
         reinterpret_cast<const uint32_t *>(x), reinterpret_cast<uint4 *>(out), n, g.h, g.w, g.ow, g.stride_w, g.pad_w,
         (uint32_t)g.izp * 0x01010101u);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -466,6 +476,8 @@ int conv_lower_rows_launch(const ConvGeom &g, const uint8_t *x, int n, uint8_t *
 __global__ void __launch_bounds__(256) conv_channel_sum_kernel(
     const uint8_t *__restrict__ x, int32_t *__restrict__ csum, size_t pixels, int c)
 {
+    pdl_wait();
+    pdl_trigger();
     // a quarter warp per pixel: 8 lanes stride over the pixel's 16-byte (or 4-byte, or single) pieces
     const size_t pix = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const int sub = threadIdx.x & 7;
@@ -498,6 +510,8 @@ __global__ void __launch_bounds__(256) conv_channel_sum_kernel(
 __global__ void __launch_bounds__(256) conv_window_sum_kernel(
     ConvGeom g, const int32_t *__restrict__ csum, int32_t *__restrict__ wsum, size_t total)
 {
+    pdl_wait();
+    pdl_trigger();
     for (size_t pix = (size_t)blockIdx.x * blockDim.x + threadIdx.x; pix < total; pix += (size_t)gridDim.x * blockDim.x) {
         const int ox = (int)(pix % g.ow);
         const int oy = (int)((pix / g.ow) % g.oh);
@@ -528,11 +542,9 @@ int conv_window_sum_launch(const ConvGeom &g, const uint8_t *x, int n, int32_t *
     const size_t blocks = (in_pix * 8 + 255) / 256;
     if (blocks > 0x7fffffffull)
         return fail(B200_ERR_UNSUPPORTED, "conv(window sum): too many pixels");
-    conv_channel_sum_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, csum, in_pix, g.c);
-    conv_window_sum_kernel<<<resident_grid<conv_window_sum_kernel, 256>((out_pix + 255) / 256), 256, 0, st>>>(
-        g, csum, wsum, out_pix);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
+    B200_TRY(launch_kernel(conv_channel_sum_kernel, dim3((unsigned)blocks), dim3(256), 0, st, in_pix * (g.c + 4), 1, x, csum, in_pix, g.c));
+    return launch_kernel(conv_window_sum_kernel, dim3((resident_grid<conv_window_sum_kernel, 256>((out_pix + 255) / 256))), dim3(256), 0, st, (in_pix + out_pix) * 4, 1,
+                         g, csum, wsum, out_pix);
 }
 
 int conv_direct_launch(
@@ -543,20 +555,21 @@ int conv_direct_launch(
         return B200_OK;
     const size_t npix = (size_t)n * g.oh * g.ow;
     const int kg = g.k / g.group, cg = g.c / g.group;
+    const size_t bytes = (size_t)n * g.h * g.w * g.c + npix * g.k;
     const bool depthwise = p.w_dw_dev && !acc_out && !g.act_signed && ((((uintptr_t)x | (uintptr_t)y) & 15) == 0);
     const bool dw3 = depthwise && p.w_dw3_dev && p.q_dw3_dev && npix * (size_t)(g.c / 4) < 0xffffffffull
         && (size_t)n * g.h * g.w * (size_t)(g.c / 4) < 0xffffffffull;
     if (dw3 && p.w_dw3p_dev && (g.stride_w == 1 || g.stride_w == 2)) {
         // two output rows per thread where the vertical stride equals the horizontal one
-        if (g.stride_w == 1 && g.stride_h == 1) depthwise3x3_pair_launch<2, 1>(g, p, x, n, y, st);
-        else if (g.stride_w == 1) depthwise3x3_pair_launch<1, 1>(g, p, x, n, y, st);
-        else if (g.stride_h == 2) depthwise3x3_pair_launch<2, 2>(g, p, x, n, y, st);
-        else depthwise3x3_pair_launch<1, 2>(g, p, x, n, y, st);
+        if (g.stride_w == 1 && g.stride_h == 1) return depthwise3x3_pair_launch<2, 1>(g, p, x, n, y, st);
+        if (g.stride_w == 1) return depthwise3x3_pair_launch<1, 1>(g, p, x, n, y, st);
+        if (g.stride_h == 2) return depthwise3x3_pair_launch<2, 2>(g, p, x, n, y, st);
+        return depthwise3x3_pair_launch<1, 2>(g, p, x, n, y, st);
     } else if (dw3) {
         const size_t total = npix * (g.c / 4);
         const int grid = resident_grid<conv_depthwise3x3_kernel, 256>((total + 255) / 256);
-        conv_depthwise3x3_kernel<<<grid, 256, 0, st>>>(
-            g, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint4 *>(p.w_dw3_dev), p.q_dw3_dev,
+        return launch_kernel(
+            conv_depthwise3x3_kernel, dim3(grid), dim3(256), 0, st, bytes, 1, g, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint4 *>(p.w_dw3_dev), p.q_dw3_dev,
             reinterpret_cast<uint32_t *>(y), n);
     } else if (depthwise) {
         size_t total = npix * (g.c / 16);
@@ -564,9 +577,8 @@ int conv_direct_launch(
         size_t cap = (size_t)sm_count() * 8;
         int grid = (int)(blocks < cap ? blocks : cap);
         if (g.wzp_d != 0)
-            conv_depthwise_kernel<true><<<grid, 256, 0, st>>>(g, x, p.w_dw_dev, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, n);
-        else
-            conv_depthwise_kernel<false><<<grid, 256, 0, st>>>(g, x, p.w_dw_dev, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, n);
+            return launch_kernel(conv_depthwise_kernel<true>, dim3(grid), dim3(256), 0, st, bytes, 1, g, x, p.w_dw_dev, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, n);
+        return launch_kernel(conv_depthwise_kernel<false>, dim3(grid), dim3(256), 0, st, bytes, 1, g, x, p.w_dw_dev, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, n);
     } else {
         const int ktiles = (kg + DK - 1) / DK;
         size_t gx = (npix + DP - 1) / DP;
@@ -576,14 +588,11 @@ int conv_direct_launch(
         const bool word = (g.c % 4 == 0) && (cg % 4 == 0) && (((uintptr_t)x & 3) == 0);
         const uint32_t *wq = reinterpret_cast<const uint32_t *>(p.w_dev);
         if (word)
-            conv_direct_kernel<true><<<grid, 256, 0, st>>>(
-                g, p.cg4, x, wq, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, acc_out, n);
-        else
-            conv_direct_kernel<false><<<grid, 256, 0, st>>>(
-                g, p.cg4, x, wq, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, acc_out, n);
+            return launch_kernel(
+                conv_direct_kernel<true>, grid, dim3(256), 0, st, bytes, 1, g, p.cg4, x, wq, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, acc_out, n);
+        return launch_kernel(
+            conv_direct_kernel<false>, grid, dim3(256), 0, st, bytes, 1, g, p.cg4, x, wq, p.bias_fold_dev, p.mult_dev, p.shift_dev, y, acc_out, n);
     }
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
 }
 
 }  // namespace b200

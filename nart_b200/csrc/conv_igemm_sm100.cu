@@ -814,6 +814,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
             // a CTA pair: the leading CTA's barrier counts the bytes of both CTAs
             const uint32_t tx_bytes = (a_tile_bytes + (g.b_resident ? 0u : (uint32_t)bnl * g.bk)) * (uint32_t)g.kgroup * (PAIR ? 2u : 1u);
             const uint32_t fb_lead = PAIR ? cluster_addr(fb, 0) : fb;
+            // weights are written once, at preparation: they need not wait for the launch before this one
             if (g.b_resident && lane == 0) {
                 // one channel tile and weights that fit: every k-block of B is loaded once and stays
                 mbar_expect_tx(bres_bar, (uint32_t)kblocks * g.bn * g.bk);
@@ -831,6 +832,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
                 tw.advance(g);
             }
             uint32_t phase = 0;
+            pdl_wait();
             // Every pass of the loop each lane polls its own stage once (without suspending: a blocked
             // lane would hold back the ready ones); a lane whose stage is free issues its loads and
             // moves on to its next k-block, the others poll again in the next pass.  No lane ever waits
@@ -902,6 +904,9 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
                 }
             }
         }
+        // every load is on its way: the next launch's blocks may come (a block per SM that waits for longer
+        // would keep the SM from the launches of other streams)
+        pdl_trigger();
     } else if (warp == 1 || ((MODE == 1 || MODE == 2) && warp == kMma2Warp)) {
         // ================= MMA issuer =================
         // The whole warp walks the loop (uniform control flow); lane 0 alone issues.  Descriptors of
@@ -1054,6 +1059,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
         const int own_sh = g.ob_sh > 5 ? g.ob_sh : 5;           // ownership granule: a sub-tile, at least one chunk
         const int p0 = quarter * 32;                            // first pixel of this warp's rows inside a tile
         const int qlw = p0 & (g.tw - 1), qlh = (p0 >> g.tw_sh) & (g.th - 1), qln = p0 >> (g.tw_sh + g.th_sh);
+        pdl_wait();            // the output may be what the launch before this one still reads
         bool failed = false;   // a wait ran out: skip the work of the remaining tiles, keep meeting the group barriers
 
         TileWalker tw;
@@ -2100,30 +2106,18 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
     // the window sums live in the caller's scratch, not in the launch cache's key: set them per launch
     p->args.wsum = wsum;
     p->args.wzp_d = p->g.wzp_d;
+    const size_t bytes = (size_t)n * ((size_t)p->g.h * p->g.w * p->g.c + (size_t)p->g.oh * p->g.ow * p->g.k) + p->w_bytes;
     if (res != nullptr)
-        conv_igemm_i8_kernel<true><<<p->grid, kThreads, p->smem, st>>>(p->maps, p->args, p->tab);
-    else if (wsum != nullptr)
-        conv_igemm_i8_kernel<false, true><<<p->grid, kThreads, p->smem, st>>>(p->maps, p->args, p->tab);
-    else if (p->cta_pair) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.gridDim = p->grid;
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = p->smem;
-        cfg.stream = st;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, conv_igemm_i8_kernel<false, false, 3>, p->maps, p->args, p->tab));
-    } else if (p->pair)
-        conv_igemm_i8_kernel<false, false, 2><<<p->grid, kThreads2, p->smem, st>>>(p->maps, p->args, p->tab);
-    else if (p->mma_warps == 2)
-        conv_igemm_i8_kernel<false, false, 1><<<p->grid, kThreads2, p->smem, st>>>(p->maps, p->args, p->tab);
-    else
-        conv_igemm_i8_kernel<false><<<p->grid, kThreads, p->smem, st>>>(p->maps, p->args, p->tab);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
+        return launch_kernel(conv_igemm_i8_kernel<true>, p->grid, dim3(kThreads), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
+    if (wsum != nullptr)
+        return launch_kernel(conv_igemm_i8_kernel<false, true>, p->grid, dim3(kThreads), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
+    if (p->cta_pair)
+        return launch_kernel(conv_igemm_i8_kernel<false, false, 3>, p->grid, dim3(kThreads), p->smem, st, bytes, 2, p->maps, p->args, p->tab);
+    if (p->pair)
+        return launch_kernel(conv_igemm_i8_kernel<false, false, 2>, p->grid, dim3(kThreads2), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
+    if (p->mma_warps == 2)
+        return launch_kernel(conv_igemm_i8_kernel<false, false, 1>, p->grid, dim3(kThreads2), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
+    return launch_kernel(conv_igemm_i8_kernel<false>, p->grid, dim3(kThreads), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
 }
 
 // Everything the first launch of any plan would otherwise do once per process or device: the driver

@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(TP) nchw_to_nhwc_kernel(
     const int p = p0 + t;
     const TIn *src = in + ((size_t)n * C) * P;
     const int cend = min(TC, c_pad - c0);
+    pdl_wait();
+    pdl_trigger();
 #pragma unroll 4
     for (int c = 0; c < cend; ++c) {
         uint8_t v = (uint8_t)fill;
@@ -128,6 +130,8 @@ __global__ void __launch_bounds__(TP) nhwc_to_nchw_kernel(
     const int t = threadIdx.x;
     const int p = p0 + t;
     const int cend = min(TC, C - c0);
+    pdl_wait();
+    pdl_trigger();
     if (p < P) {
         const uint8_t *src = in + ((size_t)n * P + p) * c_pad + c0;
         if (c0 + TC <= c_pad && (c_pad & 15) == 0) {
@@ -158,6 +162,8 @@ __global__ void __launch_bounds__(TP) nhwc_to_nchw_kernel(
 template <typename Fn>
 __global__ void quantize_flat_kernel(const float *__restrict__ in, uint8_t *__restrict__ out, size_t count, Fn fn)
 {
+    pdl_wait();
+    pdl_trigger();
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i + 4 <= count) {
         float4 v = *reinterpret_cast<const float4 *>(in + i);
@@ -171,6 +177,8 @@ __global__ void quantize_flat_kernel(const float *__restrict__ in, uint8_t *__re
 template <typename Fn>
 __global__ void dequantize_flat_kernel(const uint8_t *__restrict__ in, float *__restrict__ out, size_t count, Fn fn)
 {
+    pdl_wait();
+    pdl_trigger();
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i + 4 <= count) {
         uint32_t q = *reinterpret_cast<const uint32_t *>(in + i);
@@ -203,6 +211,8 @@ template <int N_IN, bool FAST, bool PLAIN = false, bool REV = false>
 __global__ void __launch_bounds__(256) eltwise_sum_kernel(EltwiseArgs a, uint8_t *__restrict__ y, size_t count)
 {
     constexpr int VPT = 4;   // 16-byte vectors per input per thread (2: 0.80 ms, 4: 0.78 ms, 8: 0.79 ms for the 16 adds of ResNet-50)
+    pdl_wait();
+    pdl_trigger();
     const size_t nvec = count / 16;
     // a block works on tiles of 256 * VPT vectors; vector u of a thread lies 256 vectors after vector
     // u - 1, so that every load and store instruction of a warp covers 512 contiguous bytes
@@ -258,8 +268,10 @@ __global__ void __launch_bounds__(256) lut_u8_kernel(
     const uint8_t *__restrict__ x, uint8_t *__restrict__ y, size_t count, const uint8_t *__restrict__ lut_g)
 {
     __shared__ uint8_t lut[256];
-    lut[threadIdx.x] = lut_g[threadIdx.x];
+    lut[threadIdx.x] = lut_g[threadIdx.x];   // written once, at preparation
     __syncthreads();
+    pdl_wait();
+    pdl_trigger();
     const size_t nvec = count / 16;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += stride) {
@@ -306,9 +318,7 @@ int lut_u8_launch(const uint8_t *x, uint8_t *y, size_t count, const uint8_t *lut
     if (count == 0)
         return B200_OK;
     const int grid = resident_grid<lut_u8_kernel, 256>((count / 16 + 1 + 255) / 256);
-    lut_u8_kernel<<<grid, 256, 0, st>>>(x, y, count, lut_dev);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
+    return launch_kernel(lut_u8_kernel, dim3(grid), dim3(256), 0, st, 2 * count, 1, x, y, count, lut_dev);
 }
 
 }  // namespace b200
@@ -400,6 +410,8 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_c4_kernel(
     const uint8_t *__restrict__ x, uint4 *__restrict__ y, int c, uint32_t quads_per_image, uint32_t total, uint8_t fill)
 {
     constexpr int UNR = 4;
+    pdl_wait();
+    pdl_trigger();
     const uint32_t fill4 = (uint32_t)fill * 0x01010101u;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t idx0 = blockIdx.x * blockDim.x + threadIdx.x; idx0 < total; idx0 += UNR * stride) {
@@ -449,13 +461,12 @@ int b200_quantize_u8(
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
         dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        nchw_to_nhwc_kernel<float, QuantizeFn><<<grid, TP, 0, as_stream(stream)>>>(x, y, c, P, c, 0, fn);
+        B200_TRY((launch_kernel(nchw_to_nhwc_kernel<float, QuantizeFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, 0, fn)));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
-        quantize_flat_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(x, y, count, fn);
+        B200_TRY((launch_kernel(quantize_flat_kernel<QuantizeFn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
     }
-    B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
 
@@ -473,13 +484,12 @@ int b200_dequantize_u8(
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
         dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        nhwc_to_nchw_kernel<float, DequantizeFn><<<grid, TP, 0, as_stream(stream)>>>(x, y, c, P, c, fn);
+        B200_TRY((launch_kernel(nhwc_to_nchw_kernel<float, DequantizeFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, fn)));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
-        dequantize_flat_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(x, y, count, fn);
+        B200_TRY((launch_kernel(dequantize_flat_kernel<DequantizeFn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
     }
-    B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
 
@@ -500,13 +510,12 @@ int b200_quantize_s8(
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
         dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        nchw_to_nhwc_kernel<float, QuantizeS8Fn><<<grid, TP, 0, as_stream(stream)>>>(x, y, c, P, c, 0, fn);
+        B200_TRY((launch_kernel(nchw_to_nhwc_kernel<float, QuantizeS8Fn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, 0, fn)));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
-        quantize_flat_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(x, y, count, fn);
+        B200_TRY((launch_kernel(quantize_flat_kernel<QuantizeS8Fn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
     }
-    B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
 
@@ -524,13 +533,12 @@ int b200_dequantize_s8(
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
         dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        nhwc_to_nchw_kernel<float, DequantizeS8Fn><<<grid, TP, 0, as_stream(stream)>>>(x, y, c, P, c, fn);
+        B200_TRY((launch_kernel(nhwc_to_nchw_kernel<float, DequantizeS8Fn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, fn)));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
-        dequantize_flat_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(x, y, count, fn);
+        B200_TRY((launch_kernel(dequantize_flat_kernel<DequantizeS8Fn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
     }
-    B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
 
@@ -547,13 +555,11 @@ int b200_nchw_to_nhwc_u8(
         && (size_t)n * (P / 4) < 0xf0000000ull) {   // 32-bit indices, with room for the unrolled rounds past the end
         const uint32_t quads = (uint32_t)(P / 4), total = (uint32_t)n * quads;
         const int blocks = resident_grid<nchw_to_nhwc_c4_kernel, 256>(((size_t)total + 1023) / 1024);   // four quads per thread and round
-        nchw_to_nhwc_c4_kernel<<<blocks, 256, 0, as_stream(stream)>>>(x, reinterpret_cast<uint4 *>(y), c, quads, total, fill);
-        B200_CUDA_TRY(cudaGetLastError());
-        return B200_OK;
+        B200_TRY((launch_kernel(nchw_to_nhwc_c4_kernel, dim3(blocks), dim3(256), 0, as_stream(stream), (size_t)total * 28, 1, x, reinterpret_cast<uint4 *>(y), c, quads, total, fill)));
+            return B200_OK;
     }
     dim3 grid((P + TP - 1) / TP, (c_pad + TC - 1) / TC, n);
-    nchw_to_nhwc_kernel<uint8_t, IdentityFn><<<grid, TP, 0, as_stream(stream)>>>(x, y, c, P, c_pad, fill, IdentityFn());
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_TRY((launch_kernel(nchw_to_nhwc_kernel<uint8_t, IdentityFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * (c + c_pad) * P, 1, x, y, c, P, c_pad, fill, IdentityFn())));
     return B200_OK;
 }
 
@@ -567,8 +573,7 @@ int b200_nhwc_to_nchw_u8(
         return B200_OK;
     const int P = h * w;
     dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-    nhwc_to_nchw_kernel<uint8_t, IdentityFn><<<grid, TP, 0, as_stream(stream)>>>(x, y, c, P, c_pad, IdentityFn());
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_TRY((launch_kernel(nhwc_to_nchw_kernel<uint8_t, IdentityFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * (c + c_pad) * P, 1, x, y, c, P, c_pad, IdentityFn())));
     return B200_OK;
 }
 
@@ -606,7 +611,7 @@ int eltwise_launch(const EltwiseArgs &prepared, bool fast, const uint8_t *const 
         return B200_OK;
     const size_t want = count / (256 * 64) + 1;   // tiles of 256 threads x 64 bytes
 #define B200_ELT_LAUNCH(...) \
-    eltwise_sum_kernel<__VA_ARGS__><<<resident_grid<eltwise_sum_kernel<__VA_ARGS__>, 256>(want), 256, 0, st>>>(a, y, count)
+    B200_TRY((launch_kernel(eltwise_sum_kernel<__VA_ARGS__>, dim3(resident_grid<eltwise_sum_kernel<__VA_ARGS__>, 256>(want)), dim3(256), 0, st, (n_in + 1) * count, 1, a, y, count)))
     if (fast) {
         switch (n_in) {
         case 1: B200_ELT_LAUNCH(1, true); break;
@@ -630,7 +635,6 @@ int eltwise_launch(const EltwiseArgs &prepared, bool fast, const uint8_t *const 
         }
     }
 #undef B200_ELT_LAUNCH
-    B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
 

@@ -64,8 +64,10 @@ __global__ void __launch_bounds__(256) pool_max_kernel(
     const uint8_t *__restrict__ x, uint8_t *__restrict__ y, PoolGeom g, const uint8_t *__restrict__ lut_g)
 {
     __shared__ uint8_t lut[256];
-    lut[threadIdx.x] = lut_g[threadIdx.x];
+    lut[threadIdx.x] = lut_g[threadIdx.x];   // written once, at preparation
     __syncthreads();
+    pdl_wait();
+    pdl_trigger();
     constexpr int W = (VEC + 3) / 4;
     const int cv = g.c / VEC;
     const size_t total = (size_t)g.n * g.oh * g.ow * cv;
@@ -124,6 +126,8 @@ __global__ void __launch_bounds__(256) pool_max_pair_kernel(
         lut[threadIdx.x] = lut_g[threadIdx.x];
         __syncthreads();
     }
+    pdl_wait();
+    pdl_trigger();
     constexpr int UW = KW + SW;   // columns of the union of the two windows
     const uint32_t cv = (uint32_t)g.c >> 4, owp = (uint32_t)g.ow >> 1;
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
@@ -190,13 +194,10 @@ int pool_max_pair_launch(const uint8_t *x, uint8_t *y, const PoolGeom &g, const 
     const uint4 *x4 = reinterpret_cast<const uint4 *>(x);
     uint4 *y4 = reinterpret_cast<uint4 *>(y);
     if (g.lut_identity)
-        pool_max_pair_kernel<KH, KW, SW, true><<<resident_grid<pool_max_pair_kernel<KH, KW, SW, true>, 256>(blocks), 256, 0, st>>>(
-            x4, y4, g, lut_dev, (uint32_t)pairs);
-    else
-        pool_max_pair_kernel<KH, KW, SW, false><<<resident_grid<pool_max_pair_kernel<KH, KW, SW, false>, 256>(blocks), 256, 0, st>>>(
-            x4, y4, g, lut_dev, (uint32_t)pairs);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
+        return launch_kernel(pool_max_pair_kernel<KH, KW, SW, true>, dim3(resident_grid<pool_max_pair_kernel<KH, KW, SW, true>, 256>(blocks)), dim3(256), 0, st, (size_t)g.n * g.c * (g.h * g.w + g.oh * g.ow), 1,
+                             x4, y4, g, lut_dev, (uint32_t)pairs);
+    return launch_kernel(pool_max_pair_kernel<KH, KW, SW, false>, dim3(resident_grid<pool_max_pair_kernel<KH, KW, SW, false>, 256>(blocks)), dim3(256), 0, st, (size_t)g.n * g.c * (g.h * g.w + g.oh * g.ow), 1,
+                             x4, y4, g, lut_dev, (uint32_t)pairs);
 }
 
 // AVE: sum of (x - izp) over the in-image part of the window; the multiplier and shift depend on
@@ -206,6 +207,8 @@ template <int VEC>
 __global__ void __launch_bounds__(256) pool_avg_kernel(
     const uint8_t *__restrict__ x, uint8_t *__restrict__ y, PoolGeom g, PoolAvgTab tab)
 {
+    pdl_wait();
+    pdl_trigger();
     constexpr int W = (VEC + 3) / 4;
     const int cv = g.c / VEC;
     const size_t total = (size_t)g.n * g.oh * g.ow * cv;
@@ -370,6 +373,7 @@ int pool_launch(
     size_t total = (size_t)n * g.oh * g.ow * (c / vec);
     const size_t blocks = (total + 255) / 256;
     const size_t cv16 = (size_t)c / 16;
+    const size_t bytes = (size_t)n * c * (g.h * g.w + g.oh * g.ow);
     if (method == 0 && vec == 16 && g.ow % 2 == 0 && (size_t)n * g.h * g.w * cv16 < 0xffffffffull) {
         // two outputs per thread, unrolled window, 32-bit indices: the common window shapes
         const size_t pairs = (size_t)n * g.oh * (g.ow / 2) * cv16;
@@ -383,16 +387,14 @@ int pool_launch(
         }
     }
     if (method == 0) {
-        if (vec == 16) pool_max_kernel<16><<<resident_grid<pool_max_kernel<16>, 256>(blocks), 256, 0, st>>>(x, y, g, lut_dev);
-        else if (vec == 4) pool_max_kernel<4><<<resident_grid<pool_max_kernel<4>, 256>(blocks), 256, 0, st>>>(x, y, g, lut_dev);
-        else pool_max_kernel<1><<<resident_grid<pool_max_kernel<1>, 256>(blocks), 256, 0, st>>>(x, y, g, lut_dev);
+        if (vec == 16) return launch_kernel(pool_max_kernel<16>, dim3(resident_grid<pool_max_kernel<16>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
+        if (vec == 4) return launch_kernel(pool_max_kernel<4>, dim3(resident_grid<pool_max_kernel<4>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
+        return launch_kernel(pool_max_kernel<1>, dim3(resident_grid<pool_max_kernel<1>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
     } else {
-        if (vec == 16) pool_avg_kernel<16><<<resident_grid<pool_avg_kernel<16>, 256>(blocks), 256, 0, st>>>(x, y, g, tab);
-        else if (vec == 4) pool_avg_kernel<4><<<resident_grid<pool_avg_kernel<4>, 256>(blocks), 256, 0, st>>>(x, y, g, tab);
-        else pool_avg_kernel<1><<<resident_grid<pool_avg_kernel<1>, 256>(blocks), 256, 0, st>>>(x, y, g, tab);
+        if (vec == 16) return launch_kernel(pool_avg_kernel<16>, dim3(resident_grid<pool_avg_kernel<16>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
+        if (vec == 4) return launch_kernel(pool_avg_kernel<4>, dim3(resident_grid<pool_avg_kernel<4>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
+        return launch_kernel(pool_avg_kernel<1>, dim3(resident_grid<pool_avg_kernel<1>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
     }
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
 }
 
 }  // namespace b200
