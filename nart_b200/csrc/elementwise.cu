@@ -8,13 +8,14 @@
 namespace b200 {
 
 // ---------------------------------------------------------------------------------------------
-// Tiled transpose between [N][C][P] (P = H*W, the reference's NCHW) and [N][P][Cpad] (NHWC).
-// One block moves a tile of 32 channels x 256 pixels through shared memory so that both the
-// global read and the global write are contiguous.  The element conversion (quantize,
-// dequantize or none) happens on the way.
+// [N][C][P] (P = H*W, the reference's NCHW) to and from [N][P][Cpad] (NHWC), the element conversion
+// (quantize, dequantize or none) on the way.  A thread owns 32 channels of one pixel: on the NCHW side
+// neighbouring threads read or write neighbouring elements of every channel plane, whatever P is, and
+// on the NHWC side a thread's 32 bytes are one sector.  Nothing passes through shared memory.  Pixels
+// are numbered through all images of the batch, so that small maps fill their blocks too.
 // ---------------------------------------------------------------------------------------------
-constexpr int TC = 32;    // channels per tile
-constexpr int TP = 256;   // pixels per tile (= threads per block)
+constexpr int TC = 32;          // channels per thread
+constexpr int kLayoutThreads = 256;
 
 struct QuantizeFn {
     // op_quantize_run_u8 (quantize.c:145-157) with saturate_float_by_bits (quant_helper.h:38-41):
@@ -23,6 +24,12 @@ struct QuantizeFn {
     // fp32.  __fsub_rn/__fdiv_rn keep the two roundings separate (no contraction).
     float alpha, beta;
     int qmax;
+    // The divide bounds the op (1.9 TB/s at 25.7 M elements).  u = x * inv + (zp + 0.5) differs from
+    // t + 0.5 by less than 2^-13 for t in -1 .. 256: the roundings of inv, beta, x - beta, t and of the
+    // multiply-add are at most 2^-24 of numbers below 512 each.  So floor(u) is the answer unless u lies
+    // within 2^-12 of an integer, and only those (one element in 2000 of evenly spread data) are divided.
+    float inv, half_zp;
+    bool fast;                  // alpha is far from the ends of the fp32 range (else inv and u mean nothing)
     __device__ __forceinline__ uint8_t operator()(float x) const
     {
         float t = __fdiv_rn(__fsub_rn(x, beta), alpha);
@@ -35,6 +42,27 @@ struct QuantizeFn {
         float f = floorf(t);
         int v = (int)f + ((t - f) >= 0.5f ? 1 : 0);
         return (uint8_t)v;
+    }
+    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d) const
+    {
+        const float x[4] = { a, b, c, d };
+        uint32_t r[4];
+        bool sure = fast;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            // (maximum and minimum return the number where one operand is NaN: 0 comes out, as above)
+            const float u = fminf(fmaxf(__fmaf_rn(x[i], inv, half_zp), 0.5f), (float)qmax + 0.5f);
+            const float big = __fadd_rz(u, 8388608.f);          // 2^23 + floor(u): the integer in the low bits
+            const float centre = __fsub_rn(big, 8388607.5f);    // floor(u) + 0.5
+            sure = sure && fabsf(__fsub_rn(u, centre)) < 0.5f - 0x1p-12f;
+            r[i] = __float_as_uint(big);
+        }
+        if (!sure) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                r[i] = (*this)(x[i]);
+        }
+        return __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
     }
 };
 
@@ -62,6 +90,10 @@ struct QuantizeS8Fn {
         const int v = (int)fminf(fmaxf(r, (float)-l), (float)l);
         return (uint8_t)(int8_t)v;
     }
+    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d) const
+    {
+        return pack4((*this)(a), (*this)(b), (*this)(c), (*this)(d));
+    }
 };
 
 struct DequantizeS8Fn {
@@ -72,90 +104,160 @@ struct DequantizeS8Fn {
 
 struct IdentityFn {
     __device__ __forceinline__ uint8_t operator()(uint8_t q) const { return q; }
+    __device__ __forceinline__ uint32_t word(uint8_t a, uint8_t b, uint8_t c, uint8_t d) const { return pack4(a, b, c, d); }
 };
 
 // in: [N][C][P] of TIn  ->  out: [N][P][c_pad] of uint8; channels c..c_pad-1 are written `fill`.
-template <typename TIn, typename Fn>
-__global__ void __launch_bounds__(TP) nchw_to_nhwc_kernel(
-    const TIn *__restrict__ in, uint8_t *__restrict__ out, int C, int P, int c_pad, int fill, Fn fn)
+// STORE: bytes per store (16 or 4, which divide c_pad and the address, or 1).
+template <typename TIn, typename Fn, int STORE>
+__global__ void __launch_bounds__(kLayoutThreads) nchw_to_nhwc_kernel(
+    const TIn *__restrict__ in, uint8_t *__restrict__ out, int C, uint32_t P, int c_pad, int fill, uint32_t pixels, uint32_t groups, Fn fn)
 {
-    __shared__ uint8_t tile[TC][TP + 4];
-    const int n = blockIdx.z;
-    const int c0 = blockIdx.y * TC;
-    const int p0 = blockIdx.x * TP;
-    const int t = threadIdx.x;
-    const int p = p0 + t;
-    const TIn *src = in + ((size_t)n * C) * P;
-    const int cend = min(TC, c_pad - c0);
     pdl_wait();
     pdl_trigger();
-#pragma unroll 4
-    for (int c = 0; c < cend; ++c) {
-        uint8_t v = (uint8_t)fill;
-        if (c0 + c < C && p < P)
-            v = fn(src[(size_t)(c0 + c) * P + p]);
-        tile[c][t] = v;
-    }
-    __syncthreads();
-    if (p >= P)
+    // the channel groups of a pixel block are neighbouring blocks: they share the NHWC side's lines
+    const uint32_t block = blockIdx.x / groups, gp = block * kLayoutThreads + threadIdx.x;
+    if (gp >= pixels)
         return;
-    uint8_t *dst = out + ((size_t)n * P + p) * c_pad + c0;
-    if (cend == TC && (c_pad & 15) == 0) {
-        uint32_t wv[8];
+    const int c0 = (int)(blockIdx.x - block * groups) * TC;
+    const uint32_t img = gp / P, p = gp - img * P;
+    const TIn *src = in + ((size_t)img * C + c0) * P + p;
+    uint8_t *dst = out + (size_t)gp * c_pad + c0;
+    if (c0 + TC <= C && STORE != 1) {
+        TIn v[TC];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            wv[j] = pack4(tile[4 * j][t], tile[4 * j + 1][t], tile[4 * j + 2][t], tile[4 * j + 3][t]);
-        uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-        d4[0] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-        d4[1] = make_uint4(wv[4], wv[5], wv[6], wv[7]);
-    } else if ((c_pad & 3) == 0 && (cend & 3) == 0) {
-        for (int j = 0; j < cend / 4; ++j)
-            reinterpret_cast<uint32_t *>(dst)[j]
-                = pack4(tile[4 * j][t], tile[4 * j + 1][t], tile[4 * j + 2][t], tile[4 * j + 3][t]);
-    } else {
-        for (int c = 0; c < cend; ++c)
-            dst[c] = tile[c][t];
+        for (int c = 0; c < TC; ++c)
+            v[c] = __ldg(src + (size_t)c * P);
+        uint32_t wv[TC / 4];
+#pragma unroll
+        for (int j = 0; j < TC / 4; ++j)
+            wv[j] = fn.word(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        if (STORE == 16) {
+            reinterpret_cast<uint4 *>(dst)[0] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+            reinterpret_cast<uint4 *>(dst)[1] = make_uint4(wv[4], wv[5], wv[6], wv[7]);
+        } else {
+            // rows at word addresses only: the words change hands inside the warp, so that eight lanes write the
+            // 32 bytes of one pixel and not 32 lanes a word each of 32 pixels (16 M elements of 236 channels: 27.5 us so)
+            __shared__ uint32_t tile[kLayoutThreads / 32][32][TC / 4 + 1];
+            uint32_t (*t)[TC / 4 + 1] = tile[threadIdx.x / 32];
+            const unsigned lane = threadIdx.x & 31, active = __activemask();
+#pragma unroll
+            for (int j = 0; j < TC / 4; ++j)
+                t[lane][j] = wv[j];
+            __syncwarp(active);
+            uint8_t *first = out + (size_t)(gp - lane) * c_pad + c0;      // the warp's first pixel
+            const unsigned live = __popc(active);                         // lanes below `pixels`: a prefix of the warp
+            for (unsigned i = lane; i < live * (TC / 4); i += live)
+                *reinterpret_cast<uint32_t *>(first + (size_t)(i / (TC / 4)) * c_pad + (i % (TC / 4)) * 4) = t[i / (TC / 4)][i % (TC / 4)];
+        }
+        return;
+    }
+    // the last, narrower group of channels, and rows that no word store fits
+    const int cend = min(TC, c_pad - c0);
+#pragma unroll 4
+    for (int c = 0; c < cend; c += 4) {
+        TIn v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            v[i] = c0 + c + i < C ? __ldg(src + (size_t)(c + i) * P) : TIn(0);
+        uint32_t wv = fn.word(v[0], v[1], v[2], v[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c0 + c + i >= C)
+                wv = (wv & ~(0xffu << (8 * i))) | ((uint32_t)fill << (8 * i));
+        if (STORE != 1) {
+            *reinterpret_cast<uint32_t *>(dst + c) = wv;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c + i < cend)
+                    dst[c + i] = (uint8_t)(wv >> (8 * i));
+        }
     }
 }
 
 // in: [N][P][c_pad] uint8 -> out: [N][C][P] of TOut (channels >= C are dropped).
-template <typename TOut, typename Fn>
-__global__ void __launch_bounds__(TP) nhwc_to_nchw_kernel(
-    const uint8_t *__restrict__ in, TOut *__restrict__ out, int C, int P, int c_pad, Fn fn)
+// LOAD: bytes per load, as STORE above.
+template <typename TOut, typename Fn, int LOAD>
+__global__ void __launch_bounds__(kLayoutThreads) nhwc_to_nchw_kernel(
+    const uint8_t *__restrict__ in, TOut *__restrict__ out, int C, uint32_t P, int c_pad, uint32_t pixels, uint32_t groups, Fn fn)
 {
-    __shared__ uint8_t tile[TC][TP + 4];
-    const int n = blockIdx.z;
-    const int c0 = blockIdx.y * TC;
-    const int p0 = blockIdx.x * TP;
-    const int t = threadIdx.x;
-    const int p = p0 + t;
-    const int cend = min(TC, C - c0);
     pdl_wait();
     pdl_trigger();
-    if (p < P) {
-        const uint8_t *src = in + ((size_t)n * P + p) * c_pad + c0;
-        if (c0 + TC <= c_pad && (c_pad & 15) == 0) {
-            const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
-            uint4 a = s4[0], b = s4[1];
-            uint32_t wv[8] = { a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w };
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                tile[4 * j + 0][t] = (uint8_t)(wv[j]);
-                tile[4 * j + 1][t] = (uint8_t)(wv[j] >> 8);
-                tile[4 * j + 2][t] = (uint8_t)(wv[j] >> 16);
-                tile[4 * j + 3][t] = (uint8_t)(wv[j] >> 24);
-            }
-        } else {
-            for (int c = 0; c < cend; ++c)
-                tile[c][t] = src[c];
-        }
-    }
-    __syncthreads();
-    if (p >= P)
+    // the channel groups of a pixel block are neighbouring blocks: they share the NHWC side's lines
+    const uint32_t block = blockIdx.x / groups, gp = block * kLayoutThreads + threadIdx.x;
+    if (gp >= pixels)
         return;
-    TOut *dst = out + ((size_t)n * C) * P;
-    for (int c = 0; c < cend; ++c)
-        dst[(size_t)(c0 + c) * P + p] = fn(tile[c][t]);
+    const int c0 = (int)(blockIdx.x - block * groups) * TC;
+    const uint32_t img = gp / P, p = gp - img * P;
+    const uint8_t *src = in + (size_t)gp * c_pad + c0;
+    TOut *dst = out + ((size_t)img * C + c0) * P + p;
+    if (c0 + TC <= C && LOAD != 1) {
+        uint32_t wv[TC / 4];
+        if (LOAD == 16) {
+            const uint4 a = __ldg(reinterpret_cast<const uint4 *>(src)), b = __ldg(reinterpret_cast<const uint4 *>(src) + 1);
+            wv[0] = a.x; wv[1] = a.y; wv[2] = a.z; wv[3] = a.w; wv[4] = b.x; wv[5] = b.y; wv[6] = b.z; wv[7] = b.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < TC / 4; ++j)
+                wv[j] = __ldg(reinterpret_cast<const uint32_t *>(src) + j);
+        }
+#pragma unroll
+        for (int c = 0; c < TC; ++c)
+            dst[(size_t)c * P] = fn((uint8_t)(wv[c / 4] >> (8 * (c % 4))));
+        return;
+    }
+    const int cend = min(TC, C - c0);
+#pragma unroll 4
+    for (int c = 0; c < cend; c += 4) {
+        uint32_t wv = 0;
+        if (LOAD != 1) {
+            wv = __ldg(reinterpret_cast<const uint32_t *>(src + c));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c + i < cend)
+                    wv |= (uint32_t)__ldg(src + c + i) << (8 * i);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c + i < cend)
+                dst[(size_t)(c + i) * P] = fn((uint8_t)(wv >> (8 * i)));
+    }
+}
+
+template <typename TIn, typename Fn>
+static int nchw_to_nhwc_launch(const TIn *x, uint8_t *y, int n, int c, int P, int c_pad, int fill, Fn fn, cudaStream_t st)
+{
+    const size_t pixels = (size_t)n * P;
+    const size_t groups = ((size_t)c_pad + TC - 1) / TC, blocks = (pixels + kLayoutThreads - 1) / kLayoutThreads * groups;
+    if (pixels > 0xffffff00ull || blocks > 0x7fffffffull)
+        return fail(B200_ERR_UNSUPPORTED, "layout: more than 2^32 pixels or 2^31 blocks");
+    const dim3 grid((unsigned)blocks);
+    const size_t bytes = pixels * (c * sizeof(TIn) + c_pad);
+    const bool a16 = c_pad % 16 == 0 && ((uintptr_t)y & 15) == 0, a4 = c_pad % 4 == 0 && ((uintptr_t)y & 3) == 0;
+    if (a16)
+        return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 16>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+    if (a4)
+        return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 4>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+    return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 1>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+}
+
+template <typename TOut, typename Fn>
+static int nhwc_to_nchw_launch(const uint8_t *x, TOut *y, int n, int c, int P, int c_pad, Fn fn, cudaStream_t st)
+{
+    const size_t pixels = (size_t)n * P;
+    const size_t groups = ((size_t)c + TC - 1) / TC, blocks = (pixels + kLayoutThreads - 1) / kLayoutThreads * groups;
+    if (pixels > 0xffffff00ull || blocks > 0x7fffffffull)
+        return fail(B200_ERR_UNSUPPORTED, "layout: more than 2^32 pixels or 2^31 blocks");
+    const dim3 grid((unsigned)blocks);
+    const size_t bytes = pixels * (c * sizeof(TOut) + c_pad);
+    const bool a16 = c_pad % 16 == 0 && ((uintptr_t)x & 15) == 0, a4 = c_pad % 4 == 0 && ((uintptr_t)x & 3) == 0;
+    if (a16)
+        return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 16>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
+    if (a4)
+        return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 4>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
+    return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 1>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
 }
 
 // Flat variants (no layout change): 4 elements per thread.
@@ -167,7 +269,7 @@ __global__ void quantize_flat_kernel(const float *__restrict__ in, uint8_t *__re
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i + 4 <= count) {
         float4 v = *reinterpret_cast<const float4 *>(in + i);
-        *reinterpret_cast<uint32_t *>(out + i) = pack4(fn(v.x), fn(v.y), fn(v.z), fn(v.w));
+        *reinterpret_cast<uint32_t *>(out + i) = fn.word(v.x, v.y, v.z, v.w);
     } else {
         for (; i < count; ++i)
             out[i] = fn(in[i]);
@@ -207,30 +309,27 @@ __device__ __forceinline__ int elt_finish(int t, const EltwiseArgs &a)
 // the host, exact because it is a multiple of 2^b[0]); then y = sat_u8(max((t >> s0) + ozp, relu_lo))
 // and the saturation comes with the pack.  64 bytes per input per thread and iteration.
 // PLAIN (with FAST): ozp == 0 and no floor above 0, so y = sat_u8(t >> s0) and the pack does the rest.
-template <int N_IN, bool FAST, bool PLAIN = false, bool REV = false>
+// VPT: 16-byte vectors per input and thread (2: 0.80 ms, 4: 0.78 ms, 8: 0.79 ms for the 16 adds of ResNet-50 at
+// batch 256).  One where four would leave SMs without a block: the time is then one thread's.
+template <int N_IN, bool FAST, bool PLAIN = false, bool REV = false, int VPT = 4>
 __global__ void __launch_bounds__(256) eltwise_sum_kernel(EltwiseArgs a, uint8_t *__restrict__ y, size_t count)
 {
-    constexpr int VPT = 4;   // 16-byte vectors per input per thread (2: 0.80 ms, 4: 0.78 ms, 8: 0.79 ms for the 16 adds of ResNet-50)
     pdl_wait();
     pdl_trigger();
     const size_t nvec = count / 16;
     // a block works on tiles of 256 * VPT vectors; vector u of a thread lies 256 vectors after vector
     // u - 1, so that every load and store instruction of a warp covers 512 contiguous bytes
-    const size_t ntile = nvec / (256 * VPT);
-    for (size_t tile_i = blockIdx.x; tile_i < ntile; tile_i += gridDim.x) {
-        const size_t tile = REV ? ntile - 1 - tile_i : tile_i;   // REV: from the last tile to the first
-        const size_t v0 = tile * (256 * VPT) + threadIdx.x;
-        uint32_t xin[N_IN][4 * VPT];
+    auto load = [&](uint32_t (&xin)[N_IN][4], size_t v) {
 #pragma unroll
-        for (int i = 0; i < N_IN; ++i)
+        for (int i = 0; i < N_IN; ++i) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(a.x[i]) + v);
+            xin[i][0] = q.x; xin[i][1] = q.y; xin[i][2] = q.z; xin[i][3] = q.w;
+        }
+    };
+    auto sum = [&](const uint32_t (&xin)[N_IN][4]) {
+        uint32_t o[4];
 #pragma unroll
-            for (int u = 0; u < VPT; ++u) {
-                uint4 q = __ldg(reinterpret_cast<const uint4 *>(a.x[i]) + v0 + u * 256);
-                xin[i][4 * u + 0] = q.x; xin[i][4 * u + 1] = q.y; xin[i][4 * u + 2] = q.z; xin[i][4 * u + 3] = q.w;
-            }
-        uint32_t o[4 * VPT];
-#pragma unroll
-        for (int wd = 0; wd < 4 * VPT; ++wd) {
+        for (int wd = 0; wd < 4; ++wd) {
             int r[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -244,20 +343,39 @@ __global__ void __launch_bounds__(256) eltwise_sum_kernel(EltwiseArgs a, uint8_t
             }
             o[wd] = FAST ? pack_sat_u8x4(r[0], r[1], r[2], r[3]) : pack4(r[0], r[1], r[2], r[3]);
         }
+        return make_uint4(o[0], o[1], o[2], o[3]);
+    };
+    const size_t ntile = nvec / (256 * VPT);
+    for (size_t tile_i = blockIdx.x; tile_i < ntile; tile_i += gridDim.x) {
+        const size_t tile = REV ? ntile - 1 - tile_i : tile_i;   // REV: from the last tile to the first
+        const size_t v0 = tile * (256 * VPT) + threadIdx.x;
+        uint32_t xin[VPT][N_IN][4];
 #pragma unroll
         for (int u = 0; u < VPT; ++u)
-            reinterpret_cast<uint4 *>(y)[v0 + u * 256] = make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
-    }
-    // tail (what is left after whole tiles: less than 256 * VPT * 16 bytes)
-    if (blockIdx.x == 0) {
-        for (size_t e = ntile * (256 * VPT * 16) + threadIdx.x; e < count; e += blockDim.x) {
-            int t = 0;
+            load(xin[u], v0 + u * 256);
+        uint4 o[VPT];
 #pragma unroll
-            for (int i = 0; i < N_IN; ++i)
-                t += ((int)a.x[i][e] * a.m[i] + a.add[i]) >> a.b[i];
-            int v = FAST ? min(max((t >> a.s0) + a.ozp, 0), 255) : elt_finish(t, a);
-            y[e] = (uint8_t)(FAST ? max(v, a.relu_lo) : v);
-        }
+        for (int u = 0; u < VPT; ++u)
+            o[u] = sum(xin[u]);
+#pragma unroll
+        for (int u = 0; u < VPT; ++u)
+            reinterpret_cast<uint4 *>(y)[v0 + u * 256] = o[u];
+    }
+    // the vectors behind the last whole tile: fewer than 256 * VPT, over as many blocks as they fill
+    for (size_t v = ntile * (256 * VPT) + (size_t)blockIdx.x * 256 + threadIdx.x; v < nvec; v += (size_t)gridDim.x * 256) {
+        uint32_t xin[N_IN][4];
+        load(xin, v);
+        reinterpret_cast<uint4 *>(y)[v] = sum(xin);
+    }
+    // the last, incomplete vector: fewer than 16 bytes
+    if (blockIdx.x == 0 && threadIdx.x < count - nvec * 16) {
+        const size_t e = nvec * 16 + threadIdx.x;
+        int t = 0;
+#pragma unroll
+        for (int i = 0; i < N_IN; ++i)
+            t += ((int)a.x[i][e] * a.m[i] + a.add[i]) >> a.b[i];
+        int v = FAST ? min(max((t >> a.s0) + a.ozp, 0), 255) : elt_finish(t, a);
+        y[e] = (uint8_t)(FAST ? max(v, a.relu_lo) : v);
     }
 }
 
@@ -458,10 +576,12 @@ int b200_quantize_u8(
     fn.alpha = oalpha;
     fn.beta = -(oalpha * (float)ozp);
     fn.qmax = (1 << obits) - 1;
+    fn.inv = 1.f / oalpha;
+    fn.half_zp = (float)ozp + 0.5f;
+    fn.fast = oalpha > 1e-30f && oalpha < 1e30f;
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
-        dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        B200_TRY((launch_kernel(nchw_to_nhwc_kernel<float, QuantizeFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, 0, fn)));
+        return nchw_to_nhwc_launch(x, y, n, c, P, c, 0, fn, as_stream(stream));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
@@ -483,8 +603,7 @@ int b200_dequantize_u8(
     fn.zp = izp;
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
-        dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        B200_TRY((launch_kernel(nhwc_to_nchw_kernel<float, DequantizeFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, fn)));
+        return nhwc_to_nchw_launch(x, y, n, c, P, c, fn, as_stream(stream));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
@@ -509,8 +628,7 @@ int b200_quantize_s8(
     fn.l = (1 << (obits - 1)) - 1;
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
-        dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        B200_TRY((launch_kernel(nchw_to_nhwc_kernel<float, QuantizeS8Fn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, 0, fn)));
+        return nchw_to_nhwc_launch(x, y, n, c, P, c, 0, fn, as_stream(stream));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
@@ -532,8 +650,7 @@ int b200_dequantize_s8(
     fn.alpha = ialpha;
     const int P = h * w;
     if (nhwc && !(c == 1 || P == 1)) {
-        dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-        B200_TRY((launch_kernel(nhwc_to_nchw_kernel<float, DequantizeS8Fn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * c * P * 5, 1, x, y, c, P, c, fn)));
+        return nhwc_to_nchw_launch(x, y, n, c, P, c, fn, as_stream(stream));
     } else {
         size_t count = (size_t)n * c * P;
         size_t threads = (count + 3) / 4;
@@ -558,9 +675,7 @@ int b200_nchw_to_nhwc_u8(
         B200_TRY((launch_kernel(nchw_to_nhwc_c4_kernel, dim3(blocks), dim3(256), 0, as_stream(stream), (size_t)total * 28, 1, x, reinterpret_cast<uint4 *>(y), c, quads, total, fill)));
             return B200_OK;
     }
-    dim3 grid((P + TP - 1) / TP, (c_pad + TC - 1) / TC, n);
-    B200_TRY((launch_kernel(nchw_to_nhwc_kernel<uint8_t, IdentityFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * (c + c_pad) * P, 1, x, y, c, P, c_pad, fill, IdentityFn())));
-    return B200_OK;
+    return nchw_to_nhwc_launch(x, y, n, c, P, c_pad, fill, IdentityFn(), as_stream(stream));
 }
 
 int b200_nhwc_to_nchw_u8(
@@ -572,9 +687,7 @@ int b200_nhwc_to_nchw_u8(
     if (n == 0)
         return B200_OK;
     const int P = h * w;
-    dim3 grid((P + TP - 1) / TP, (c + TC - 1) / TC, n);
-    B200_TRY((launch_kernel(nhwc_to_nchw_kernel<uint8_t, IdentityFn>, dim3(grid), dim3(TP), 0, as_stream(stream), (size_t)n * (c + c_pad) * P, 1, x, y, c, P, c_pad, IdentityFn())));
-    return B200_OK;
+    return nhwc_to_nchw_launch(x, y, n, c, P, c_pad, IdentityFn(), as_stream(stream));
 }
 
 int b200_eltwise_sum_u8(
@@ -609,33 +722,33 @@ int eltwise_launch(const EltwiseArgs &prepared, bool fast, const uint8_t *const 
         return fail(B200_ERR_INVALID, "eltwise: output is not 16-byte aligned");
     if (count == 0)
         return B200_OK;
-    const size_t want = count / (256 * 64) + 1;   // tiles of 256 threads x 64 bytes
+    const bool few = count < (size_t)sm_count() * (256 * 64);
+    const size_t tile = few ? 256 * 16 : 256 * 64;    // bytes per block and round
+    const size_t want = (count + tile - 1) / tile;
 #define B200_ELT_LAUNCH(...) \
-    B200_TRY((launch_kernel(eltwise_sum_kernel<__VA_ARGS__>, dim3(resident_grid<eltwise_sum_kernel<__VA_ARGS__>, 256>(want)), dim3(256), 0, st, (n_in + 1) * count, 1, a, y, count)))
+    return launch_kernel(eltwise_sum_kernel<__VA_ARGS__>, dim3(resident_grid<eltwise_sum_kernel<__VA_ARGS__>, 256>(want)), dim3(256), 0, st, (n_in + 1) * count, 1, a, y, count)
+    if (fast && n_in == 2 && few)
+        B200_ELT_LAUNCH(2, true, false, false, 1);
     if (fast) {
         switch (n_in) {
-        case 1: B200_ELT_LAUNCH(1, true); break;
+        case 1: B200_ELT_LAUNCH(1, true);
         case 2:
             if (a.ozp == 0 && a.relu_lo <= 0)
                 B200_ELT_LAUNCH(2, true, true);
-            else if (a.rev)
+            if (a.rev)
                 B200_ELT_LAUNCH(2, true, false, true);
-            else
-                B200_ELT_LAUNCH(2, true);
-            break;
-        case 3: B200_ELT_LAUNCH(3, true); break;
-        default: B200_ELT_LAUNCH(4, true); break;
-        }
-    } else {
-        switch (n_in) {
-        case 1: B200_ELT_LAUNCH(1, false); break;
-        case 2: B200_ELT_LAUNCH(2, false); break;
-        case 3: B200_ELT_LAUNCH(3, false); break;
-        default: B200_ELT_LAUNCH(4, false); break;
+            B200_ELT_LAUNCH(2, true);
+        case 3: B200_ELT_LAUNCH(3, true);
+        default: B200_ELT_LAUNCH(4, true);
         }
     }
+    switch (n_in) {
+    case 1: B200_ELT_LAUNCH(1, false);
+    case 2: B200_ELT_LAUNCH(2, false);
+    case 3: B200_ELT_LAUNCH(3, false);
+    default: B200_ELT_LAUNCH(4, false);
+    }
 #undef B200_ELT_LAUNCH
-    return B200_OK;
 }
 
 }  // namespace b200

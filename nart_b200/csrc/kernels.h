@@ -18,6 +18,7 @@ struct PoolGeom {
     int kernel_h, kernel_w, pad_h, pad_w, stride_h, stride_w;
     int izp, ozp, qmax;
     int lut_identity;   // MAX: the requantize table maps every byte to itself (equal scales and zero points)
+    int avg32;          // AVE: multiplier * sum and its rounding term fit 32 bits
 };
 struct PoolAvgTab {
     static constexpr int kMax = 4;

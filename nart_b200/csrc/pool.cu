@@ -111,25 +111,53 @@ __global__ void __launch_bounds__(256) pool_max_kernel(
     }
 }
 
-// MAX on 16-channel vectors for a compile-time window KH x KW and horizontal stride SW, with 32-bit
-// index arithmetic: one thread owns 16 channels of TWO output pixels side by side and loads the
-// union of their windows (KH x (KW + SW) vectors) in one unrolled batch, so that all of a thread's
-// loads are in flight together and the columns the two windows share are loaded once.  Taps
-// outside the image read as 0, the value the running maximum starts from.  IDENT skips the table
-// (it maps every byte to itself).  Results equal pool_max_kernel<16>.
-template <int KH, int KW, int SW, bool IDENT>
-__global__ void __launch_bounds__(256) pool_max_pair_kernel(
-    const uint4 *__restrict__ x, uint4 *__restrict__ y, PoolGeom g, const uint8_t *__restrict__ lut_g, uint32_t total)
+// Small windows of a compile-time size KH x KW and horizontal stride SW, with 32-bit index arithmetic: one
+// thread owns 4 * W channels of TWO output pixels side by side and loads the union of their windows
+// (KH x (KW + SW) vectors) in one unrolled batch, so that all of a thread's loads are in flight together
+// and the columns the two windows share are loaded, and reduced, once.  Taps outside the image read as 0:
+// the value the running maximum starts from, and nothing to a sum.  Reductions run on 16-bit lanes down
+// each column first, then across the columns of each output.
+//   MAX        the maximum goes through the 256-entry table (IDENT: it maps every byte to itself)
+//   AVE        at most 9 bytes a lane; the requantize of pool_avg_kernel in 32 bits (pool_launch checks that
+//              its terms fit).  3x3 stride 2 on 64 channels of 112 x 112, batch 32: 33.6 us a pixel per thread.
+// W = 4 where channels and addresses allow 16-byte vectors, else 1.
+enum PoolPairOp { kPairMaxIdent, kPairMaxLut, kPairAve };
+
+template <int W>
+__device__ __forceinline__ void load_vec(const uint32_t *p, uint32_t (&v)[W])
+{
+    if constexpr (W == 4) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+        v[0] = __ldg(p);
+    }
+}
+
+template <int KH, int KW, int SW, PoolPairOp OP, int W>
+__global__ void __launch_bounds__(256) pool_pair_kernel(
+    const uint32_t *__restrict__ x, uint32_t *__restrict__ y, PoolGeom g, const uint8_t *__restrict__ lut_g, PoolAvgTab tab,
+    uint32_t total)
 {
     __shared__ uint8_t lut[256];
-    if (!IDENT) {
+    __shared__ int2 mult_shift[PoolAvgTab::kMax][PoolAvgTab::kMax];   // indexed at run time: not as parameters
+    if (OP == kPairMaxLut) {
         lut[threadIdx.x] = lut_g[threadIdx.x];
+        __syncthreads();
+    }
+    if (OP == kPairAve) {
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int i = 0; i < PoolAvgTab::kMax * PoolAvgTab::kMax; ++i)
+                mult_shift[i / PoolAvgTab::kMax][i % PoolAvgTab::kMax]
+                    = make_int2(tab.mult[i / PoolAvgTab::kMax][i % PoolAvgTab::kMax], tab.shift[i / PoolAvgTab::kMax][i % PoolAvgTab::kMax]);
+        }
         __syncthreads();
     }
     pdl_wait();
     pdl_trigger();
     constexpr int UW = KW + SW;   // columns of the union of the two windows
-    const uint32_t cv = (uint32_t)g.c >> 4, owp = (uint32_t)g.ow >> 1;
+    const uint32_t cw = (uint32_t)g.c >> 2, cv = cw / W, owp = ((uint32_t)g.ow + 1) >> 1;
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
         const uint32_t ci = idx % cv;
         uint32_t pix = idx / cv;
@@ -138,71 +166,115 @@ __global__ void __launch_bounds__(256) pool_max_pair_kernel(
         const uint32_t oy = pix % (uint32_t)g.oh, n = pix / (uint32_t)g.oh;
         const int hs = (int)oy * g.stride_h - g.pad_h;
         const int ws = (int)oxp * 2 * SW - g.pad_w;
-        const uint4 *img = x + (size_t)n * (uint32_t)g.h * (uint32_t)g.w * cv + ci;
-        uint4 q[KH][UW];
+        const uint32_t *img = x + (size_t)n * (uint32_t)g.h * (uint32_t)g.w * cw + ci * W;
+        uint32_t q[KH][UW][W];
 #pragma unroll
         for (int r = 0; r < KH; ++r)
 #pragma unroll
             for (int j = 0; j < UW; ++j) {
                 const int iy = hs + r, ix = ws + j;
-                q[r][j] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    q[r][j][i] = 0;
                 if ((unsigned)iy < (unsigned)g.h && (unsigned)ix < (unsigned)g.w)
-                    q[r][j] = __ldg(img + ((uint32_t)iy * (uint32_t)g.w + (uint32_t)ix) * cv);
+                    load_vec<W>(img + ((uint32_t)iy * (uint32_t)g.w + (uint32_t)ix) * cw, q[r][j]);
             }
-        // separable: the maximum down each of the UW columns first, then across the KW columns of each
-        // output; the columns the two windows share are reduced once
-        U16x4 col[UW][4];
+        auto join = [](const U16x4 &a, const U16x4 &b) {
+            if constexpr (OP == kPairAve)
+                return U16x4{ a.lo + b.lo, a.hi + b.hi };       // no carry between the lanes: sums stay below 2^16
+            else
+                return max_u16x4(a, b);
+        };
+        U16x4 s0[W], s1[W];
 #pragma unroll
-        for (int j = 0; j < UW; ++j) {
-            col[j][0] = spread_bytes(q[0][j].x); col[j][1] = spread_bytes(q[0][j].y);
-            col[j][2] = spread_bytes(q[0][j].z); col[j][3] = spread_bytes(q[0][j].w);
+        for (int i = 0; i < W; ++i) {
+            U16x4 col[UW];
 #pragma unroll
-            for (int r = 1; r < KH; ++r) {
-                col[j][0] = max_u16x4(col[j][0], spread_bytes(q[r][j].x)); col[j][1] = max_u16x4(col[j][1], spread_bytes(q[r][j].y));
-                col[j][2] = max_u16x4(col[j][2], spread_bytes(q[r][j].z)); col[j][3] = max_u16x4(col[j][3], spread_bytes(q[r][j].w));
+            for (int j = 0; j < UW; ++j) {
+                col[j] = spread_bytes(q[0][j][i]);
+#pragma unroll
+                for (int r = 1; r < KH; ++r)
+                    col[j] = join(col[j], spread_bytes(q[r][j][i]));
             }
-        }
-        uint32_t m0[4], m1[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            U16x4 a = col[0][i], b = col[SW][i];
+            s0[i] = col[0];
+            s1[i] = col[SW];
 #pragma unroll
             for (int j = 1; j < KW; ++j) {
-                a = max_u16x4(a, col[j][i]);
-                b = max_u16x4(b, col[SW + j][i]);
+                s0[i] = join(s0[i], col[j]);
+                s1[i] = join(s1[i], col[SW + j]);
             }
-            m0[i] = pack_bytes(a);
-            m1[i] = pack_bytes(b);
         }
-        if (!IDENT) {
+        uint32_t m0[W], m1[W];
+        if constexpr (OP == kPairAve) {
+            // valid taps, and the multiplier and shift of the window as the far edge (with its padding) cuts it
+            const int vh = min(hs + KH, g.h) - max(hs, 0), dh = max(hs + KH - (g.h + g.pad_h), 0);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                m0[j] = pack4(lut[m0[j] & 0xff], lut[(m0[j] >> 8) & 0xff], lut[(m0[j] >> 16) & 0xff], lut[m0[j] >> 24]);
-                m1[j] = pack4(lut[m1[j] & 0xff], lut[(m1[j] >> 8) & 0xff], lut[(m1[j] >> 16) & 0xff], lut[m1[j] >> 24]);
+            for (int o = 0; o < 2; ++o) {
+                const int wo = ws + o * SW;
+                const int vw = min(wo + KW, g.w) - max(wo, 0), dw = min(max(wo + KW - (g.w + g.pad_w), 0), PoolAvgTab::kMax - 1);
+                const int mult = mult_shift[dh][dw].x, sh = mult_shift[dh][dw].y;
+                const int add = (1 << (sh - 1)) - mult * (max(vh, 0) * max(vw, 0) * g.izp);
+#pragma unroll
+                for (int i = 0; i < W; ++i) {
+                    const U16x4 &s = o ? s1[i] : s0[i];
+                    const int r0 = ((mult * (int)(s.lo & 0xffff) + add) >> sh) + g.ozp, r1 = ((mult * (int)(s.lo >> 16) + add) >> sh) + g.ozp;
+                    const int r2 = ((mult * (int)(s.hi & 0xffff) + add) >> sh) + g.ozp, r3 = ((mult * (int)(s.hi >> 16) + add) >> sh) + g.ozp;
+                    (o ? m1[i] : m0[i]) = pack_sat_u8x4(min(r0, g.qmax), min(r1, g.qmax), min(r2, g.qmax), min(r3, g.qmax));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                m0[i] = pack_bytes(s0[i]);
+                m1[i] = pack_bytes(s1[i]);
+                if (OP == kPairMaxLut) {
+                    m0[i] = pack4(lut[m0[i] & 0xff], lut[(m0[i] >> 8) & 0xff], lut[(m0[i] >> 16) & 0xff], lut[m0[i] >> 24]);
+                    m1[i] = pack4(lut[m1[i] & 0xff], lut[(m1[i] >> 8) & 0xff], lut[(m1[i] >> 16) & 0xff], lut[m1[i] >> 24]);
+                }
             }
         }
-        uint4 *out = y + ((n * (uint32_t)g.oh + oy) * (uint32_t)g.ow + oxp * 2) * cv + ci;
-        out[0] = make_uint4(m0[0], m0[1], m0[2], m0[3]);
-        out[cv] = make_uint4(m1[0], m1[1], m1[2], m1[3]);
+        uint32_t *out = y + ((n * (uint32_t)g.oh + oy) * (uint32_t)g.ow + oxp * 2) * cw + ci * W;
+        const bool second = oxp * 2 + 1 < (uint32_t)g.ow;
+        if constexpr (W == 4) {
+            *reinterpret_cast<uint4 *>(out) = make_uint4(m0[0], m0[1], m0[2], m0[3]);
+            if (second)
+                *reinterpret_cast<uint4 *>(out + cw) = make_uint4(m1[0], m1[1], m1[2], m1[3]);
+        } else {
+            out[0] = m0[0];
+            if (second)
+                out[cw] = m1[0];
+        }
     }
 }
 
-template <int KH, int KW, int SW>
-int pool_max_pair_launch(const uint8_t *x, uint8_t *y, const PoolGeom &g, const uint8_t *lut_dev, size_t pairs, cudaStream_t st)
+template <int KH, int KW, int SW, PoolPairOp OP, int W>
+static int pool_pair_launch(const uint8_t *x, uint8_t *y, const PoolGeom &g, const uint8_t *lut_dev, const PoolAvgTab &tab, size_t bytes,
+                            cudaStream_t st)
 {
-    const size_t blocks = (pairs + 255) / 256;
-    const uint4 *x4 = reinterpret_cast<const uint4 *>(x);
-    uint4 *y4 = reinterpret_cast<uint4 *>(y);
+    const size_t total = (size_t)g.n * g.oh * ((g.ow + 1) / 2) * (g.c / (4 * W));
+    return launch_kernel(pool_pair_kernel<KH, KW, SW, OP, W>, dim3(resident_grid<pool_pair_kernel<KH, KW, SW, OP, W>, 256>((total + 255) / 256)),
+                         dim3(256), 0, st, bytes, 1, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<uint32_t *>(y), g, lut_dev, tab,
+                         (uint32_t)total);
+}
+
+template <int KH, int KW, int SW>
+static int pool_pair_pick(int method, int vec, const uint8_t *x, uint8_t *y, const PoolGeom &g, const uint8_t *lut_dev, const PoolAvgTab &tab,
+                          size_t bytes, cudaStream_t st)
+{
+#define B200_PAIR(OP) return vec == 16 ? pool_pair_launch<KH, KW, SW, OP, 4>(x, y, g, lut_dev, tab, bytes, st) \
+                                       : pool_pair_launch<KH, KW, SW, OP, 1>(x, y, g, lut_dev, tab, bytes, st)
+    if (method == 1)
+        B200_PAIR(kPairAve);
     if (g.lut_identity)
-        return launch_kernel(pool_max_pair_kernel<KH, KW, SW, true>, dim3(resident_grid<pool_max_pair_kernel<KH, KW, SW, true>, 256>(blocks)), dim3(256), 0, st, (size_t)g.n * g.c * (g.h * g.w + g.oh * g.ow), 1,
-                             x4, y4, g, lut_dev, (uint32_t)pairs);
-    return launch_kernel(pool_max_pair_kernel<KH, KW, SW, false>, dim3(resident_grid<pool_max_pair_kernel<KH, KW, SW, false>, 256>(blocks)), dim3(256), 0, st, (size_t)g.n * g.c * (g.h * g.w + g.oh * g.ow), 1,
-                             x4, y4, g, lut_dev, (uint32_t)pairs);
+        B200_PAIR(kPairMaxIdent);
+    B200_PAIR(kPairMaxLut);
+#undef B200_PAIR
 }
 
 // AVE: sum of (x - izp) over the in-image part of the window; the multiplier and shift depend on
 // the padded window size (pool.c:217-221) and come from a small host-built table indexed by how
-// many rows / columns the window loses at the far edge.
+// many rows / columns the window loses at the far edge.  The sums run on 16-bit lanes: pool_prepare
+// admits at most 257 taps, 65535 a lane.
 template <int VEC>
 __global__ void __launch_bounds__(256) pool_avg_kernel(
     const uint8_t *__restrict__ x, uint8_t *__restrict__ y, PoolGeom g, PoolAvgTab tab)
@@ -210,7 +282,7 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
     pdl_wait();
     pdl_trigger();
     constexpr int W = (VEC + 3) / 4;
-    const int cv = g.c / VEC;
+    const uint32_t cv = (uint32_t)(g.c / VEC);
     const size_t total = (size_t)g.n * g.oh * g.ow * cv;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -227,32 +299,39 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
         ws = max(ws, 0);
         he = min(he, g.h);
         we = min(we, g.w);
-        int sum[VEC];
+        U16x4 sum[W];
 #pragma unroll
-        for (int j = 0; j < VEC; ++j)
-            sum[j] = 0;
-        const int cnt = max(he - hs, 0) * max(we - ws, 0);
-        // eight taps per round, loaded before any is used, so that a large window (the global average
-        // of a 7x7 map is 49 taps per thread) keeps several loads in flight
+        for (int j = 0; j < W; ++j)
+            sum[j] = { 0u, 0u };
+        const int wd = max(we - ws, 0), cnt = max(he - hs, 0) * wd;
+        // the window's taps as one sequence, eight per round, loaded before any is used: a large window (the
+        // global average of a 7x7 map is 49 taps) keeps several loads in flight
         constexpr int UNR = 8;
-        for (int iy = hs; iy < he; ++iy) {
-            const uint8_t *row = x + (((size_t)n * g.h + iy) * g.w) * g.c + (size_t)ci * VEC;
-            for (int ix = ws; ix < we; ix += UNR) {
-                uint32_t v[UNR][W];
+        const uint8_t *base = x + (((size_t)n * g.h + hs) * g.w + ws) * g.c + (size_t)ci * VEC;
+        int ty = 0, tx = 0;
+        for (int t = 0; t < cnt; t += UNR) {
+            uint32_t v[UNR][W];
 #pragma unroll
-                for (int u = 0; u < UNR; ++u) {
+            for (int u = 0; u < UNR; ++u) {
 #pragma unroll
-                    for (int j = 0; j < W; ++j)
-                        v[u][j] = 0;
-                    if (ix + u < we)
-                        load_words<VEC>(row + (size_t)(ix + u) * g.c, v[u]);
+                for (int j = 0; j < W; ++j)
+                    v[u][j] = 0;
+                if (t + u < cnt) {
+                    load_words<VEC>(base + (size_t)(ty * g.w + tx) * g.c, v[u]);
+                    if (++tx == wd) {
+                        tx = 0;
+                        ++ty;
+                    }
                 }
-#pragma unroll
-                for (int u = 0; u < UNR; ++u)
-#pragma unroll
-                    for (int j = 0; j < VEC; ++j)
-                        sum[j] += (int)((v[u][j / 4] >> (8 * (j % 4))) & 0xff);
             }
+#pragma unroll
+            for (int u = 0; u < UNR; ++u)
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    const U16x4 b = spread_bytes(v[u][j]);
+                    sum[j].lo += b.lo;
+                    sum[j].hi += b.hi;
+                }
         }
         uint32_t o[W];
 #pragma unroll
@@ -260,7 +339,8 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
             o[j] = 0;
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
-            int s = sum[j] - cnt * g.izp;
+            const uint32_t lanes = j % 4 < 2 ? sum[j / 4].lo : sum[j / 4].hi;
+            int s = (int)((lanes >> (16 * (j % 2))) & 0xffff) - cnt * g.izp;
             // (int32)mult * sum is an int32 product in the reference; rshift_rn then runs on the
             // sign-extended value.
             long long p = (long long)(mult * s);
@@ -303,6 +383,7 @@ int pool_prepare(
     g->stride_h = stride_h; g->stride_w = stride_w;
     g->izp = izp; g->ozp = ozp; g->qmax = (1 << obits) - 1;
     g->lut_identity = 0;
+    g->avg32 = 1;
     const int qmax = g->qmax;
     if (method == 0) {
         uint32_t m16;
@@ -353,6 +434,8 @@ int pool_prepare(
                     return fail(B200_ERR_UNSUPPORTED, "pool: shift %d outside 1..62", (int)sh);
                 tab->mult[dh][dw] = (int)m;
                 tab->shift[dh][dw] = sh;
+                if (sh > 30 || (long long)kernel_h * kernel_w * 255 * m + (1ll << (sh - 1)) >= (1ll << 31))
+                    g->avg32 = 0;
             }
     }
     return B200_OK;
@@ -370,22 +453,22 @@ int pool_launch(
     int vec = (c % 16 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) ? 16
         : (c % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) & 3) == 0)       ? 4
                                                                            : 1;
-    size_t total = (size_t)n * g.oh * g.ow * (c / vec);
-    const size_t blocks = (total + 255) / 256;
-    const size_t cv16 = (size_t)c / 16;
     const size_t bytes = (size_t)n * c * (g.h * g.w + g.oh * g.ow);
-    if (method == 0 && vec == 16 && g.ow % 2 == 0 && (size_t)n * g.h * g.w * cv16 < 0xffffffffull) {
-        // two outputs per thread, unrolled window, 32-bit indices: the common window shapes
-        const size_t pairs = (size_t)n * g.oh * (g.ow / 2) * cv16;
-        if (pairs < 0xffffffffull - 256ull * 65536ull) {
-            if (g.kernel_h == 3 && g.kernel_w == 3 && g.stride_w == 2)
-                return pool_max_pair_launch<3, 3, 2>(x, y, g, lut_dev, pairs, st);
-            if (g.kernel_h == 3 && g.kernel_w == 3 && g.stride_w == 1)
-                return pool_max_pair_launch<3, 3, 1>(x, y, g, lut_dev, pairs, st);
-            if (g.kernel_h == 2 && g.kernel_w == 2 && g.stride_w == 2)
-                return pool_max_pair_launch<2, 2, 2>(x, y, g, lut_dev, pairs, st);
-        }
+    // two outputs per thread, unrolled window, 32-bit indices: the common window shapes
+    if (vec >= 4 && (size_t)n * g.h * g.w * (c / 4) < 0xffffffffull && (size_t)n * g.oh * ((g.ow + 1) / 2) * (c / vec) < 0xffffffffull - 256ull * 65536ull
+        && (method == 0 || g.avg32)) {
+        if (g.kernel_h == 3 && g.kernel_w == 3 && g.stride_w == 2)
+            return pool_pair_pick<3, 3, 2>(method, vec, x, y, g, lut_dev, tab, bytes, st);
+        if (g.kernel_h == 3 && g.kernel_w == 3 && g.stride_w == 1)
+            return pool_pair_pick<3, 3, 1>(method, vec, x, y, g, lut_dev, tab, bytes, st);
+        if (g.kernel_h == 2 && g.kernel_w == 2 && g.stride_w == 2)
+            return pool_pair_pick<2, 2, 2>(method, vec, x, y, g, lut_dev, tab, bytes, st);
     }
+    // an average whose 16-byte vectors would not give every SM a few warps goes by words: four times the threads, and
+    // the loop over the window is a chain of loads (2048 channels of 7x7, batch 256)
+    if (method == 1 && vec == 16 && (size_t)n * g.oh * g.ow * (c / 16) < (size_t)sm_count() * 1024)
+        vec = 4;
+    const size_t blocks = ((size_t)n * g.oh * g.ow * (c / vec) + 255) / 256;
     if (method == 0) {
         if (vec == 16) return launch_kernel(pool_max_kernel<16>, dim3(resident_grid<pool_max_kernel<16>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
         if (vec == 4) return launch_kernel(pool_max_kernel<4>, dim3(resident_grid<pool_max_kernel<4>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);

@@ -256,6 +256,30 @@ def test_pool(ops, port):
     assert_same(to_host_nchw(ops.pool(to_dev_nhwc(x), 1, (7, 7), (0, 0), (1, 1), 0, 0.05, 3, 0.02, 0)), want, "resnet gap")
 
 
+@pytest.mark.parametrize("n,c,h,w", [(1, 32, 1, 3), (2, 64, 5, 51), (3, 36, 16, 16), (2, 20, 9, 7), (1, 67, 8, 9), (5, 100, 3, 5), (2, 16, 40, 13)])
+def test_memory_bound_ops_at_ragged_sizes(ops, port, n, c, h, w):
+    """Layout changes at the edges of a thread's 32 channels and a block's 256 pixels (whole, ragged, shared
+    between images), sums at every remainder of 16 bytes, two-outputs-per-thread pools at odd widths and by words."""
+    import torch
+    rng = np.random.default_rng(c * h + w)
+    x = (rng.standard_normal((n, c, h, w)) * 3).astype(np.float32)
+    x.reshape(-1)[::7] = np.float32(0.03) * (np.arange(x.reshape(-1)[::7].size) % 300 - 140 + np.float32(0.5))     # near ties
+    for obits in (8, 5):
+        q = ops.quantize(torch.from_numpy(x).cuda(), 0.03, 97, obits)
+        assert_same(to_host_nchw(q), port.quantize_u8(x, 0.03, 97, obits), "quantize obits=%d" % obits)
+    u = port.quantize_u8(x, 0.03, 97)
+    d = ops.dequantize(to_dev_nhwc(u), 0.03, 97)
+    assert_same(d.cpu().numpy().view(np.uint32), port.dequantize_u8(u, 0.03, 97).view(np.uint32), "dequantize")
+    v = rng.integers(0, 256, u.shape, dtype=np.uint8)
+    got = ops.add(torch.from_numpy(u).cuda(), torch.from_numpy(v).cuda(), [0.03, 0.05], [97, 40], 0.06, 110)
+    assert_same(got.cpu().numpy(), port.eltwise_sum_u8([u, v], [0.03, 0.05], [97, 40], 0.06, 110), "add")
+    for m in (0, 1):
+        for kern, pad, stride, cm in (((3, 3), (1, 1), (2, 2), 0), ((3, 3), (1, 1), (2, 2), 1), ((3, 3), (1, 1), (1, 1), 0), ((2, 2), (1, 1), (2, 2), 1)):
+            want = port.pool_u8(u, m, kern, pad, stride, cm, 0.03, 97, 0.04, 31)
+            got = ops.pool(to_dev_nhwc(u), m, kern, pad, stride, cm, 0.03, 97, 0.04, 31)
+            assert_same(to_host_nchw(got), want, "pool m=%d %s %s ceil=%d" % (m, kern, stride, cm))
+
+
 @pytest.mark.parametrize("k,ks,st,pd,h,w", [(64, 7, 2, 3, 33, 35), (32, 3, 2, 1, 20, 22), (16, 3, 1, 1, 9, 8),
                                              (48, 5, 1, 0, 12, 17), (64, 7, 2, 3, 224, 224)])
 def test_conv_four_channel_image_row_lowering(ops, port, k, ks, st, pd, h, w):
