@@ -124,6 +124,7 @@ B200_API void b200_get_quant_scale(float x, int bits, uint32_t *mult, int8_t *sh
  *   B200_IGEMM_MMA_WARPS=<1|2>               MMA-issuing warps
  *   B200_IGEMM_PAIR=0                        never pair tiles on one weight tile
  *   B200_IGEMM_CTA_PAIR=<0|1>                never / wherever possible run on CTA pairs (tcgen05 cta_group::2)
+ *   B200_IGEMM_SMALL=0                       never one tile per CTA or cluster (launches that leave SMs without a tile)
  *   B200_IGEMM_EPI_CONST=0                   never use the uniform-shift epilogue (per-channel constants as kernel parameters)
  * and by b200_case_prepare:
  *   B200_CASE_ZIGZAG=0                       every op walks its tiles first to last (default: each op walks against the
@@ -154,8 +155,8 @@ typedef struct b200_conv_params {
     float ialpha;           /* SETTING_QUANT_IALPHA[0]                                        */
     uint8_t izp;            /* SETTING_QUANT_IZERO_POINT[0]                                   */
     uint8_t wzp;            /* SETTING_QUANT_WZERO_POINT[0]; 128 = int8 weights stored as value + 128.
-                             * Other values cost one extra pass over the activations on the
-                             * tensor-core path (window sums of x) and rule out the fused residual add */
+                             * Other values cost the tensor-core path 16 more columns per MMA (the window
+                             * sum of x) and rule out the fused residual add */
     uint8_t ozp;            /* SETTING_QUANT_OZERO_POINT[0]                                   */
     uint8_t obits;          /* SETTING_QUANT_OBITS[0], 1..8                                   */
     float oalpha;           /* SETTING_QUANT_OALPHA[0]                                        */
@@ -179,7 +180,7 @@ B200_API int b200_conv2d_algo(const b200_conv_t *conv);
 /* One line of text naming the kernel variant and tiling the plan resolved to (for logs and tuning). */
 B200_API int b200_conv2d_describe(const b200_conv_t *conv, char *buf, size_t len);
 /* x: device NHWC [n][h][w][c]; y: device NHWC [n][oh][ow][k].  Plans with a scratch tensor (the
- * row-lowered 4-channel stem; window sums for wzp != 128) grow it, with a device synchronization,
+ * row-lowered 4-channel stem) grow it, with a device synchronization,
  * the first time a larger batch arrives; the old tensor is freed then. */
 B200_API int b200_conv2d_run(
     b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, b200_stream_t stream);

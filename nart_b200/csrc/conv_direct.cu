@@ -468,85 +468,6 @@ int conv_lower_rows_launch(const ConvGeom &g, const uint8_t *x, int n, uint8_t *
         (uint32_t)g.izp * 0x01010101u);
 }
 
-// ---------------------------------------------------------------------------------------------
-// Window sums for the tensor-core path when wzp != 128 (see ConvGeom::wzp_d).  Two small passes:
-// the channel sum of every input pixel (one read of the activations), then the sum of those over
-// each output pixel's in-image taps, less izp for every byte summed.
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) conv_channel_sum_kernel(
-    const uint8_t *__restrict__ x, int32_t *__restrict__ csum, size_t pixels, int c)
-{
-    pdl_wait();
-    pdl_trigger();
-    // a quarter warp per pixel: 8 lanes stride over the pixel's 16-byte (or 4-byte, or single) pieces
-    const size_t pix = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    const int sub = threadIdx.x & 7;
-    unsigned sum = 0;
-    if (pix < pixels) {
-        const uint8_t *px = x + pix * (size_t)c;
-        if ((c & 15) == 0 && (((uintptr_t)x) & 15) == 0) {
-            for (int i = sub; i < c / 16; i += 8) {
-                const uint4 q = __ldg(reinterpret_cast<const uint4 *>(px) + i);
-                sum = __dp4a(q.x, 0x01010101u, sum);
-                sum = __dp4a(q.y, 0x01010101u, sum);
-                sum = __dp4a(q.z, 0x01010101u, sum);
-                sum = __dp4a(q.w, 0x01010101u, sum);
-            }
-        } else if ((c & 3) == 0 && (((uintptr_t)x) & 3) == 0) {
-            for (int i = sub; i < c / 4; i += 8)
-                sum = __dp4a(__ldg(reinterpret_cast<const uint32_t *>(px) + i), 0x01010101u, sum);
-        } else {
-            for (int i = sub; i < c; i += 8)
-                sum += __ldg(px + i);
-        }
-    }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-    if (pix < pixels && sub == 0)
-        csum[pix] = (int32_t)sum;
-}
-
-__global__ void __launch_bounds__(256) conv_window_sum_kernel(
-    ConvGeom g, const int32_t *__restrict__ csum, int32_t *__restrict__ wsum, size_t total)
-{
-    pdl_wait();
-    pdl_trigger();
-    for (size_t pix = (size_t)blockIdx.x * blockDim.x + threadIdx.x; pix < total; pix += (size_t)gridDim.x * blockDim.x) {
-        const int ox = (int)(pix % g.ow);
-        const int oy = (int)((pix / g.ow) % g.oh);
-        const size_t img = pix / ((size_t)g.ow * g.oh);
-        const int iy0 = oy * g.stride_h - g.pad_h, ix0 = ox * g.stride_w - g.pad_w;
-        int sum = 0, taps = 0;
-        for (int rr = 0; rr < g.r; ++rr) {
-            const int iy = iy0 + rr;
-            if (iy < 0 || iy >= g.h)
-                continue;
-            for (int ss = 0; ss < g.s; ++ss) {
-                const int ix = ix0 + ss;
-                if (ix < 0 || ix >= g.w)
-                    continue;
-                sum += __ldg(csum + (img * g.h + iy) * g.w + ix);
-                ++taps;
-            }
-        }
-        wsum[pix] = sum - g.izp * g.c * taps;
-    }
-}
-
-int conv_window_sum_launch(const ConvGeom &g, const uint8_t *x, int n, int32_t *csum, int32_t *wsum, cudaStream_t st)
-{
-    if (n == 0)
-        return B200_OK;
-    const size_t in_pix = (size_t)n * g.h * g.w, out_pix = (size_t)n * g.oh * g.ow;
-    const size_t blocks = (in_pix * 8 + 255) / 256;
-    if (blocks > 0x7fffffffull)
-        return fail(B200_ERR_UNSUPPORTED, "conv(window sum): too many pixels");
-    B200_TRY(launch_kernel(conv_channel_sum_kernel, dim3((unsigned)blocks), dim3(256), 0, st, in_pix * (g.c + 4), 1, x, csum, in_pix, g.c));
-    return launch_kernel(conv_window_sum_kernel, dim3((resident_grid<conv_window_sum_kernel, 256>((out_pix + 255) / 256))), dim3(256), 0, st, (in_pix + out_pix) * 4, 1,
-                         g, csum, wsum, out_pix);
-}
-
 int conv_direct_launch(
     const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, int32_t *acc_out,
     cudaStream_t st)

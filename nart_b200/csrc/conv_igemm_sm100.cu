@@ -42,7 +42,9 @@
 #include <vector>
 
 #include "common.cuh"
+#include "conv_small.h"
 #include "kernels.h"
+#include "sm100_ptx.cuh"
 
 namespace b200 {
 
@@ -60,7 +62,6 @@ constexpr int kTileM = 128;
 constexpr int kMaxStages = 8;
 constexpr int kGroupBytes = 32 * 1024;        // target size of one pipeline stage (a group of k-blocks)
 constexpr int kMaxGroup = 10;                 // three stages of a group must fit the producer's 32 lanes
-constexpr long long kWaitCycles = 4000000000ll;   // ~2 s at 1.9 GHz
 
 // device status codes (which wait gave up)
 constexpr int kErrProducerWait = 0x101;
@@ -73,6 +74,7 @@ struct alignas(64) IgemmMaps {
     CUtensorMap a[4];   // activations, one per (row parity, column parity) of a strided conv
     CUtensorMap b;      // weights [Cout][R*S*C]
     CUtensorMap y;      // output NHWC
+    CUtensorMap ones;   // 16 rows, the first all ones (HAS_WZP)
 };
 
 struct IgemmArgs {
@@ -114,9 +116,8 @@ struct IgemmArgs {
     const uint8_t *res;
     int r_m[2], r_add[2], r_b[2];
     int r_s0, r_ozp, r_lo;
-    // weight zero point other than 128: acc -= wzp_d * wsum[pixel] before the requantize, wsum = window
-    // sums of (x - izp) per output pixel [n][oh][ow] (conv_window_sum_launch); nullptr: off
-    const int32_t *wsum;
+    // weight zero point other than 128 (HAS_WZP): acc -= wzp_d * sum of x over the pixel's window before the
+    // requantize; the MMA forms that sum in a 17th..32nd column behind the tile's channels (weight row of ones)
     int wzp_d;
     // Uniform-shift epilogue (epi_const != 0): every channel's shift was brought to the layer's smallest
     // one, S, by dropping low zero bits of its multiplier, so that
@@ -208,247 +209,6 @@ struct TileWalker {
     __device__ __forceinline__ int ni(const IgemmArgs &g) const { return (g.rev && tni < g.tiles_n) ? g.tiles_n - 1 - tni : tni; }
 };
 
-// ---- PTX wrappers --------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Non-blocking form: the producer lanes poll many barriers from one warp, where a try_wait that
-// suspends on one lane's barrier would hold back the lanes whose barrier is ready.
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: returns false when the barrier did not flip within kWaitCycles or another role
-// has already given up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, long long limit = kWaitCycles)
-{
-    if (mbar_try_wait(bar, parity))
-        return true;
-    const long long t0 = clock64();
-    int spins = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if ((++spins & 255) == 0) {
-            if (*abort_flag != 0 || clock64() - t0 > limit)
-                return false;
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
-        : "memory");
-}
-// Loads of a CTA pair: the data lands in this CTA's shared memory, the bytes are counted on the mbarrier of
-// the pair's leading CTA (`bar` is a shared::cluster address).  Plain tiled loads -- every CTA fetches its own box.
-__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
-        : "memory");
-}
-// The shared::cluster address of `addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank)
-{
-    uint32_t out;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
-    return out;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, uint32_t src, int c0, int c1, int c2, int c3)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-        ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// all but the most recent store group have finished reading their shared-memory source
-__device__ __forceinline__ void tma_store_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void prefetch_map(const CUtensorMap *map)
-{
-    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols)
-{
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish()
-{
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-// The same three for a CTA pair: one warp of each CTA of the pair issues them.
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols)
-{
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair()
-{
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-// One MMA over both CTAs of a pair (M = 256): rows 0..127 of A and D live in the leading CTA, rows 128..255 in
-// its peer, each CTA holds half of B's rows; the descriptors are this (the leading) CTA's shared addresses.
-__device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
-                                            uint32_t accumulate, uint32_t issue)
-{
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "mov.b64 da, {%1, %3};\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(issue)
-        : "memory");
-}
-// Arrival on `bar` (a shared::cluster address, this CTA's or the peer's) when every MMA of the pair issued so
-// far has completed.  One such commit per CTA that has to hear of it: no multicast form is used.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint32_t issue)
-{
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(bar), "r"(issue)
-        : "memory");
-}
-// D[tmem] (+)= A[smem] * B[smem]^T, 8-bit integer operands, int32 accumulate.  The descriptors
-// come as low words plus the high word both share; `issue` predicates the instruction.
-__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
-                                       uint32_t accumulate, uint32_t issue)
-{
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "mov.b64 da, {%1, %3};\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(issue)
-        : "memory");
-}
-// The barrier gets one arrival when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint32_t bar, uint32_t issue)
-{
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(bar), "r"(issue)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Named barriers of one epilogue group (ids 1 + 2g and 2 + 2g for group g).
 __device__ __forceinline__ void epi_bar_sync(int group, int group_threads)
 {
@@ -468,21 +228,6 @@ __device__ __forceinline__ bool epi_bar_all(int group, int group_threads, bool p
         : "r"((uint32_t)pred), "r"(group_threads), "r"(2 + 2 * group)
         : "memory");
     return out != 0;
-}
-
-// Shared-memory matrix descriptor of a K-major operand tile whose rows are `bk` bytes
-// (bk = 128 / 64 / 32 selects the 128B / 64B / 32B swizzle both TMA and the MMA use); eight rows
-// form one swizzle atom, atoms follow each other every 8*bk bytes (the stride byte offset).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, int bk)
-{
-    const uint64_t layout = bk == 128 ? 2ull : (bk == 64 ? 4ull : 6ull);
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);          // start address, 16-byte units
-    d |= (uint64_t)1 << 16;                           // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)((8 * bk) >> 4) << 32;             // stride byte offset
-    d |= (uint64_t)1 << 46;                           // descriptor version of sm_100
-    d |= layout << 61;
-    return d;
 }
 
 // ---- epilogue arithmetic ------------------------------------------------------------------------
@@ -709,7 +454,8 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
     if (PAIR)
         asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
     const bool leader = !PAIR || cta_rank == 0;
-    const int bnl = PAIR ? g.bn >> 1 : g.bn;     // rows of B this CTA holds
+    constexpr int kOnes = HAS_WZP ? 16 : 0;      // rows of B, and accumulator columns, behind the tile's channels
+    const int bnl = PAIR ? g.bn >> 1 : g.bn + kOnes;     // rows of B this CTA holds
     const SmemLayout L = smem_layout(MODE == 2 ? 2 * slots : slots, g.b_resident ? kblocks_all : slots, g.bk, g.bn, g.groups, bnl);
 
     const int warp = threadIdx.x >> 5;
@@ -817,9 +563,12 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
             // weights are written once, at preparation: they need not wait for the launch before this one
             if (g.b_resident && lane == 0) {
                 // one channel tile and weights that fit: every k-block of B is loaded once and stays
-                mbar_expect_tx(bres_bar, (uint32_t)kblocks * g.bn * g.bk);
-                for (int kb = 0; kb < kblocks; ++kb)
+                mbar_expect_tx(bres_bar, (uint32_t)kblocks * bnl * g.bk);
+                for (int kb = 0; kb < kblocks; ++kb) {
                     tma_load_2d(base + L.b + kb * b_tile_bytes, &maps.b, bres_bar, kb * g.bk, 0);
+                    if (HAS_WZP)
+                        tma_load_2d(base + L.b + kb * b_tile_bytes + g.bn * g.bk, &maps.ones, bres_bar, kb * g.bk, 0);
+                }
             }
             const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;   // strides are 1 or 2
             // this lane's first k-block
@@ -882,8 +631,11 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
                         else
                             tma_load_4d(a_dst, amap, fb, cc, xw, yh, n0);
                         }
-                        if (!g.b_resident && !PAIR)
+                        if (!g.b_resident && !PAIR) {
                             tma_load_2d(b_dst, &maps.b, fb, kb * g.bk, tw.nt * g.bn);
+                            if (HAS_WZP)
+                                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, fb, kb * g.bk, 0);
+                        }
                         phase ^= 1;
                         kb += ring_slots;
                         while (kb >= kblocks) {
@@ -955,7 +707,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(as * g.bn);
+                const uint32_t d_tmem = tmem_base + (uint32_t)(as * (g.bn + kOnes));
                 uint32_t accumulate = 0;
                 for (int grp = 0; grp < groups; ++grp) {
                     if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
@@ -1082,10 +834,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
             const uint8_t *res_row = g.res;
             if ((HAS_RES && g.res != nullptr) && pix_valid)
                 res_row += (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
-            // wzp != 128: this pixel's correction, the same for every channel
-            int wz_t = 0;
-            if (HAS_WZP && pix_valid)
-                wz_t = -g.wzp_d * __ldg(g.wsum + ((size_t)img * g.oh + oh) * g.ow + ow);
+            int wz_t = 0;       // wzp != 128: this pixel's correction, the same for every channel
             const long long *off_row = g.off + k0;
             if (!single_class)
                 off_row += (size_t)((int)g.row_cls[min(oh, g.oh - 1)] * g.n_col_cls + (int)g.col_cls[min(ow, g.ow - 1)]) * g.kpad;
@@ -1121,7 +870,13 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
             }
             if (!failed) {
                 tc_fence_after();
-                const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * g.bn);
+                const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * (g.bn + kOnes));
+                if (HAS_WZP) {
+                    uint32_t xs;
+                    tmem_ld1(t_row + g.bn, xs);
+                    tmem_ld_wait();
+                    wz_t = -g.wzp_d * (int)xs;
+                }
                 if (!HAS_RES && g.epi_const) {
                 const long long rnd = ((long long)g.rnd_hi << 32) | (unsigned long long)(uint32_t)g.rnd_lo;
                 const int32_t *off_row32 = g.off32;
@@ -1427,7 +1182,6 @@ struct ConvIgemmPlan {
     // wins 3-6 % once every cluster walks many tiles and loses a little on short launches (cluster launch,
     // two cluster-wide syncs), so the plan carries both configurations and build_launch picks.
     int pair_ok = 0, pair_want = -1, stages_pair = 0;
-    int cta_pair = 0;               // the configuration of the current launch
     int max_clusters = 0;           // co-resident CTA pairs of that kernel on this device
     int n_row_cls = 0, n_col_cls = 0;
     int generic_requant = 0;
@@ -1449,33 +1203,31 @@ struct ConvIgemmPlan {
     bool has_res = false;
     int r_m[2] = { 0, 0 }, r_add[2] = { 0, 0 }, r_b[2] = { 1, 1 };
     int r_s0 = 1, r_ozp = 0, r_lo = 0;
-    // tensor maps of the last (x, y, n) seen
-    const uint8_t *last_res = nullptr;
-    const uint8_t *last_x = nullptr;
-    uint8_t *last_y = nullptr;
-    int last_n = -1;
-    int *last_status = nullptr;
-    IgemmMaps maps;
-    IgemmArgs args;
-    dim3 grid;
-    size_t smem = 0;
+    bool small_ok = true;           // one tile per CTA where a launch leaves SMs without a tile
+    int8_t *ones_dev = nullptr;     // wzp != 128: [16][r][s][c], the first row ones where the window has a channel
     bool attr_set = false;
-    // a few earlier launch configurations (callers that rotate through a handful of buffers)
-    struct Saved {
+    // Launch configurations by buffers and batch (callers that rotate through a handful of buffers): found again
+    // without encoding tensor maps.
+    struct Launch {
         const uint8_t *x;
         const uint8_t *res;
         uint8_t *y;
         int n;
         int *status;
-        IgemmMaps maps;
-        IgemmArgs args;
+        bool small;                 // the one-tile-per-CTA kernel (conv_small_sm100.cu): smaps, sargs, m_tiles
+        int cta_pair;
+        int m_tiles;
         dim3 grid;
         size_t smem;
-        int cta_pair;
+        SmallMaps smaps;
+        SmallArgs sargs;
+        IgemmMaps maps;
+        IgemmArgs args;
     };
     static constexpr size_t kMaxSaved = 8;
-    std::vector<Saved> saved;
-    size_t next_saved = 0;
+    std::vector<Launch> saved;
+    size_t next_saved = 0, last = 0;
+    const Launch *last_launch() const { return last < saved.size() ? &saved[last] : nullptr; }
 };
 
 int conv_igemm_supported(const ConvGeom &g, char *why, size_t why_len)
@@ -1523,7 +1275,7 @@ static void tap_classes(int out, int in, int kernel, int pad, int stride, std::v
 
 int conv_igemm_create(
     const ConvGeom &g, const std::vector<int8_t> &w_s8, const int32_t *bias, const uint32_t *mult,
-    const int32_t *shift, ConvIgemmPlan **out, bool a_row_swizzled)
+    const int32_t *shift, ConvIgemmPlan **out, bool a_row_swizzled, int window)
 {
     if (a_row_swizzled && !(g.c == 32 && g.s == 1 && g.stride_w == 1 && g.pad_w == 0 && g.w == g.ow))
         return fail(B200_ERR_INVALID, "conv(igemm): pre-swizzled rows need 32 channels and an r x 1 kernel");
@@ -1545,6 +1297,7 @@ int conv_igemm_create(
     }
     ConvIgemmPlan *p = new ConvIgemmPlan();
     p->g = g;
+    p->small_ok = !(getenv("B200_IGEMM_SMALL") && atoi(getenv("B200_IGEMM_SMALL")) == 0);   // tuning aid
     p->saved.reserve(ConvIgemmPlan::kMaxSaved);   // launches never grow it: a later run touches no heap
     p->a_wide = a_row_swizzled ? 1 : 0;
     // K of an 8-bit MMA is 32 bytes: the channel count is rounded up to a multiple of 32 in the
@@ -1552,14 +1305,16 @@ int conv_igemm_create(
     // channel extent and reads zeros there
     p->cpad = (g.c + 31) / 32 * 32;
     p->bk = p->cpad % 128 == 0 ? 128 : (p->cpad % 64 == 0 ? 64 : 32);
+    const int ones = g.wzp_d ? 16 : 0;      // rows of B and accumulator columns behind a tile's channels (window sums)
     // output-channel tile: a multiple of 16 up to 256 that wastes little of Cout
     {
         const int k16 = (g.k + 15) / 16 * 16;
-        if (k16 <= 256) {
+        const int widest = 256 - ones;
+        if (k16 <= widest) {
             p->bn = k16;
         } else {
-            int best = 256, best_waste = 1 << 30;
-            for (int bn = 256; bn >= 128; bn -= 16) {
+            int best = widest, best_waste = 1 << 30;
+            for (int bn = widest; bn >= 128; bn -= 16) {
                 int tiles = (g.k + bn - 1) / bn;
                 int waste = tiles * bn - g.k;
                 if (waste < best_waste) {
@@ -1577,7 +1332,7 @@ int conv_igemm_create(
         p->bn = 32;
     if (const char *e = getenv("B200_IGEMM_BN")) {   // tuning aid: channel-tile width, a multiple of 16 up to 256
         int v = atoi(e);
-        if (v >= 16 && v <= 256 && v % 16 == 0 && v <= (g.k + 15) / 16 * 16)
+        if (v >= 16 && v <= 256 - ones && v % 16 == 0 && v <= (g.k + 15) / 16 * 16)
             p->bn = v;
     }
     const int n_tiles_n = (g.k + p->bn - 1) / p->bn;
@@ -1588,10 +1343,10 @@ int conv_igemm_create(
         // weights resident when there is one channel tile and they leave room for >= 3 A stages
         // four epilogue groups (four tiles in flight behind the mainloop) when the tiles are narrow:
         // their per-tile latency chain, not their arithmetic, sets the epilogue rate
-        p->groups = (p->bn <= 64 || (p->bn <= 128 && kblocks * p->bk <= 256)) ? 4 : 2;
+        p->groups = (p->bn <= 64 || (p->bn <= 128 - ones && kblocks * p->bk <= 256)) ? 4 : 2;
         if (const char *e = getenv("B200_IGEMM_GROUPS")) {   // tuning aid: 2, or 4 when four accumulators fit
             int v = atoi(e);
-            if (v == 2 || (v == 4 && 4 * p->bn <= 512))
+            if (v == 2 || (v == 4 && 4 * (p->bn + ones) <= 512))
                 p->groups = v;
         }
         // staging sub-tile width: the largest of 128/64/32/16 that divides bn and, where possible,
@@ -1605,16 +1360,16 @@ int conv_igemm_create(
             if (!p->ob)
                 p->ob = p->bn % 128 == 0 ? 128 : (p->bn % 64 == 0 ? 64 : (p->bn % 32 == 0 ? 32 : 16));
         }
-        p->acc_stages = 4 * p->bn <= 512 ? 4 : p->groups;
+        p->acc_stages = 4 * (p->bn + ones) <= 512 ? 4 : p->groups;
         if (const char *e = getenv("B200_IGEMM_ACC")) {
             int v = atoi(e);
-            if ((v == 2 || v == 4) && v * p->bn <= 512 && v >= p->groups)
+            if ((v == 2 || v == 4) && v * (p->bn + ones) <= 512 && v >= p->groups)
                 p->acc_stages = v;
         }
-        p->b_resident = n_tiles_n == 1 && smem_layout(3, kblocks, p->bk, p->bn, p->groups).total + 1024 <= 227 * 1024;
+        p->b_resident = n_tiles_n == 1 && smem_layout(3, kblocks, p->bk, p->bn, p->groups, p->bn + ones).total + 1024 <= 227 * 1024;
         // Narrow k-blocks (few bytes per barrier round trip) travel in groups: the largest divisor of
         // the tile's k-blocks that keeps a stage at or under kGroupBytes.
-        const int kb_bytes = kTileM * p->bk + (p->b_resident ? 0 : p->bn * p->bk);
+        const int kb_bytes = kTileM * p->bk + (p->b_resident ? 0 : (p->bn + ones) * p->bk);
         int kgroup = 1;
         for (int d = 1; d <= kblocks; ++d)
             if (kblocks % d == 0 && d * kb_bytes <= kGroupBytes && d <= kMaxGroup)
@@ -1626,7 +1381,7 @@ int conv_igemm_create(
         }
         int stages = kMaxStages;
         auto fits = [&](int st, int kg) {
-            return smem_layout(st * kg, p->b_resident ? kblocks : st * kg, p->bk, p->bn, p->groups).total + 1024 <= 227 * 1024;
+            return smem_layout(st * kg, p->b_resident ? kblocks : st * kg, p->bk, p->bn, p->groups, p->bn + ones).total + 1024 <= 227 * 1024;
         };
         while (kgroup > 1 && !fits(3, kgroup)) {   // keep at least three stages in flight
             int d = kgroup - 1;
@@ -1641,10 +1396,10 @@ int conv_igemm_create(
         // ~100 cycles whatever their size: two issuing warps, each on its own half of the ring and on
         // every second tile, keep the tensor pipe fed (3x3 64-channel layer: 0.082 -> 0.061 ms; 256-wide
         // tiles gain nothing).
-        p->mma_warps = (p->bn <= 128 && stages >= 4) ? 2 : 1;
+        p->mma_warps = (p->bn <= 128 && stages >= 4 && !ones) ? 2 : 1;
         if (const char *e = getenv("B200_IGEMM_MMA_WARPS")) {   // tuning aid: 1, or 2 when the ring has four stages or more
             int v = atoi(e);
-            if (v == 1 || (v == 2 && stages >= 4))
+            if (v == 1 || (v == 2 && stages >= 4 && !ones))
                 p->mma_warps = v;
         }
         if (p->mma_warps == 2)
@@ -1654,7 +1409,7 @@ int conv_igemm_create(
         // (3x3 128-channel layer 0.047 -> 0.043 ms.  256-wide tiles lose: their two accumulators fill the
         // tensor memory, so the next pair's mainloop cannot overlap this pair's epilogue: 0.039 -> 0.044 ms.)
         const bool pair_off = getenv("B200_IGEMM_PAIR") && atoi(getenv("B200_IGEMM_PAIR")) == 0;   // tuning aid
-        if (!pair_off && !p->b_resident && kgroup == 1 && !p->a_wide && n_tiles_n == 1 && p->bn <= 128) {
+        if (!pair_off && !ones && !p->b_resident && kgroup == 1 && !p->a_wide && n_tiles_n == 1 && p->bn <= 128) {
             int st = kMaxStages;
             auto fits2 = [&](int n) { return smem_layout(2 * n, n, p->bk, p->bn, p->groups).total + 1024 <= 227 * 1024; };
             while (st > 2 && !fits2(st))
@@ -1691,7 +1446,7 @@ int conv_igemm_create(
         p->stages = stages;
         p->kgroup = kgroup;
     }
-    if (smem_layout((p->pair ? 2 : 1) * p->stages * p->kgroup, p->b_resident ? g.r * g.s * (p->cpad / p->bk) : p->stages * p->kgroup, p->bk, p->bn, p->groups).total + 1024 > 227 * 1024) {
+    if (smem_layout((p->pair ? 2 : 1) * p->stages * p->kgroup, p->b_resident ? g.r * g.s * (p->cpad / p->bk) : p->stages * p->kgroup, p->bk, p->bn, p->groups, p->bn + ones).total + 1024 > 227 * 1024) {
         delete p;
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): tile does not fit shared memory");
     }
@@ -1734,6 +1489,14 @@ int conv_igemm_create(
                 long long v = (long long)(bias ? bias[k] : 0) - (long long)(g.act_signed ? 0 : g.izp) * sum;
                 // the int32 accumulator offset, folded with the multiplier, the rounding term and the
                 // output zero point into the 64-bit addend of the epilogue's multiply-add
+                if (ones) {
+                    // the window-sum column holds the raw bytes: sum (x - izp) over the in-image taps is that less izp for each
+                    int taps_in = 0;
+                    for (int rr = 0; rr < g.r; ++rr)
+                        for (int ss = 0; ss < g.s; ++ss)
+                            taps_in += row_valid[rc][rr] && col_valid[cc][ss] ? 1 : 0;
+                    v += (long long)g.wzp_d * g.izp * taps_in * (window ? window * 4 : g.c);
+                }
                 const long long off32 = (long long)(int32_t)(uint32_t)(unsigned long long)v;
                 off32_all[((size_t)rc * p->n_col_cls + cc) * p->kpad + k] = (int32_t)off32;
                 off[((size_t)rc * p->n_col_cls + cc) * p->kpad + k]
@@ -1792,8 +1555,16 @@ int conv_igemm_create(
         B200_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
         return B200_OK;
     };
+    std::vector<int8_t> one_row;
+    if (ones) {
+        one_row.assign((size_t)16 * taps * p->cpad, 0);
+        for (int t = 0; t < taps; ++t)
+            for (int c = 0; c < (window ? window * 4 : g.c); ++c)
+                one_row[(size_t)t * p->cpad + c] = 1;
+    }
     p->w_bytes = wp.size();
     int rc = up(wp.data(), wp.size(), (void **)&p->w_dev);
+    if (rc == B200_OK && ones) rc = up(one_row.data(), one_row.size(), (void **)&p->ones_dev);
     if (rc == B200_OK) rc = up(off.data(), off.size() * 8, (void **)&p->off_dev);
     if (rc == B200_OK) rc = up(off32_all.data(), off32_all.size() * 4, (void **)&p->off32_dev);
     if (rc == B200_OK) rc = up(multp.data(), multp.size() * 4, (void **)&p->mult_dev);
@@ -1813,6 +1584,7 @@ void conv_igemm_destroy(ConvIgemmPlan *p)
     if (!p)
         return;
     cudaFree(p->w_dev);
+    cudaFree(p->ones_dev);
     cudaFree(p->off_dev);
     cudaFree(p->off32_dev);
     cudaFree(p->mult_dev);
@@ -1842,12 +1614,19 @@ static void choose_tile(int ow, int oh, int n, int *tw, int *th, int *tn, int mi
 
 void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
 {
-    const char *mode = p->cta_pair ? "cta-pair (cta_group::2, M=256)" : p->pair ? "tile pairs on one weight tile"
+    const ConvIgemmPlan::Launch *l = p->last_launch();      // the tiling depends on the batch of the run
+    if (l && l->small) {
+        snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d slots=%d split=%d one tile per %s", l->sargs.bn, p->bk, l->sargs.slots, l->sargs.split,
+                 l->sargs.split > 1 ? "cluster" : "CTA");
+        return;
+    }
+    const bool cta_pair = l && l->cta_pair;
+    const char *mode = cta_pair ? "cta-pair (cta_group::2, M=256)" : p->pair ? "tile pairs on one weight tile"
         : p->pair_ok ? "one issuing warp (cta pairs on long launches)"
         : p->mma_warps == 2 ? "two issuing warps" : "one issuing warp";
     snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d stages=%d kgroup=%d groups=%d acc_stages=%d %s%s%s%s", p->bn, p->bk,
-             p->cta_pair ? p->stages_pair : p->stages, p->kgroup, p->groups, p->acc_stages, mode, p->b_resident ? ", weights resident" : "",
-             (p->epi_const && !p->cta_pair) ? ", uniform-shift epilogue" : (p->generic_requant ? ", generic requantize" : ""),
+             cta_pair ? p->stages_pair : p->stages, p->kgroup, p->groups, p->acc_stages, mode, p->b_resident ? ", weights resident" : "",
+             (p->epi_const && !cta_pair) ? ", uniform-shift epilogue" : (p->generic_requant ? ", generic requantize" : ""),
              p->rev ? ", reversed" : "");
 }
 
@@ -1855,8 +1634,7 @@ void conv_igemm_set_reverse(ConvIgemmPlan *p, int reverse)
 {
     if (p->rev != (reverse ? 1 : 0)) {
         p->rev = reverse ? 1 : 0;
-        p->last_n = -1;        // cached launch configurations carry the old direction
-        p->saved.clear();
+        p->saved.clear();      // they carry the old direction
     }
 }
 
@@ -1875,7 +1653,6 @@ void conv_igemm_set_next_readonly(ConvIgemmPlan *p, const uint8_t *ptr, size_t b
     if (p->next_ro != ptr || p->next_ro_bytes != b) {
         p->next_ro = ptr;
         p->next_ro_bytes = b;
-        p->last_n = -1;
         p->saved.clear();
     }
 }
@@ -1894,20 +1671,113 @@ int conv_igemm_set_residual(ConvIgemmPlan *p, const EltwiseArgs &e, int conv_inp
     p->r_m[1] = e.m[other]; p->r_add[1] = e.add[other]; p->r_b[1] = e.b[other];
     p->r_s0 = e.s0; p->r_ozp = e.ozp; p->r_lo = e.relu_lo;
     p->has_res = true;
-    p->last_n = -1;        // cached launch configurations carry the old constants
-    p->saved.clear();
+    p->saved.clear();      // they carry the old constants
     return B200_OK;
 }
 
-static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status_word, const uint8_t *res)
+// Tensor maps of the activations for M tiles of tw x th x tn pixels.
+static int encode_activations(const ConvIgemmPlan *p, const uint8_t *x, int n, int tw, int th, int tn, CUtensorMap (&maps)[4])
+{
+    const ConvGeom &g = p->g;
+    for (int ph = 0; ph < g.stride_h; ++ph)
+        for (int pw = 0; pw < g.stride_w; ++pw) {
+            // input pixels (ph + stride_h * i, pw + stride_w * j): a dense 4-D tensor (c, j, i, image)
+            if (ph >= g.h || pw >= g.w) {
+                maps[ph * 2 + pw] = maps[0];
+                continue;
+            }
+            if (p->a_wide) {
+                // rows of this parity as a 3-D tensor (ow * 32 bytes in 8-byte elements, row, image);
+                // no swizzle: the bytes are already laid out as the MMA's 32-byte swizzle wants them
+                cuuint64_t dims[3] = { (cuuint64_t)g.w * 4, (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
+                cuuint64_t strides[2] = { (cuuint64_t)g.stride_h * g.w * 32, (cuuint64_t)g.h * g.w * 32 };
+                cuuint32_t box[3] = { (cuuint32_t)tw * 4, (cuuint32_t)th, (cuuint32_t)tn };
+                void *base = (void *)(x + (size_t)ph * g.w * 32);
+                B200_TRY(encode(&maps[ph * 2 + pw], base, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_DATA_TYPE_UINT64));
+                continue;
+            }
+            cuuint64_t dims[4] = { (cuuint64_t)g.c, (cuuint64_t)((g.w - pw + g.stride_w - 1) / g.stride_w),
+                                   (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
+            cuuint64_t strides[3] = { (cuuint64_t)g.stride_w * g.c, (cuuint64_t)g.stride_h * g.w * g.c,
+                                      (cuuint64_t)g.h * g.w * g.c };
+            cuuint32_t box[4] = { (cuuint32_t)p->bk, (cuuint32_t)tw, (cuuint32_t)th, (cuuint32_t)tn };
+            void *base = (void *)(x + ((size_t)ph * g.w + pw) * g.c);
+            B200_TRY(encode(&maps[ph * 2 + pw], base, 4, dims, strides, box, swizzle_for(p->bk)));
+        }
+    for (int i = 0; i < 4; ++i)
+        if (i / 2 >= g.stride_h || i % 2 >= g.stride_w)
+            maps[i] = maps[0];
+    return B200_OK;
+}
+
+// Tensor map of [rows][r*s*c] weights in boxes of `box_rows` rows and one k-block.
+static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int box_rows, CUtensorMap *map)
+{
+    const int ktot = p->g.r * p->g.s * p->cpad;
+    cuuint64_t dims[2] = { (cuuint64_t)ktot, (cuuint64_t)rows };
+    cuuint64_t strides[1] = { (cuuint64_t)ktot };
+    cuuint32_t box[2] = { (cuuint32_t)p->bk, (cuuint32_t)box_rows };
+    return encode(map, const_cast<int8_t *>(w), 2, dims, strides, box, swizzle_for(p->bk));
+}
+
+// Fills l.smaps / l.sargs if the launch leaves SMs without a tile; l.small says so.
+static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status, int tw, int th, int tn, ConvIgemmPlan::Launch &l)
+{
+    const ConvGeom &g = p->g;
+    SmallArgs &a = l.sargs;
+    memset(&a, 0, sizeof(a));
+    a.tiles_w = (g.ow + tw - 1) / tw;
+    a.tiles_h = (g.oh + th - 1) / th;
+    const int m_tiles = a.tiles_w * a.tiles_h * ((n + tn - 1) / tn);
+    a.cchunks = p->cpad / p->bk;
+    a.kblocks = g.r * g.s * a.cchunks;
+    a.bk = p->bk;
+    if (!conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, &a.bn, &a.split))
+        return B200_OK;
+    a.n = n; a.oh = g.oh; a.ow = g.ow; a.cout = g.k;
+    a.r = g.r; a.s = g.s; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
+    for (a.tw_sh = 0; (1 << a.tw_sh) < tw; ++a.tw_sh) {}
+    for (a.th_sh = 0; (1 << a.th_sh) < th; ++a.th_sh) {}
+    a.tn = tn;
+    a.n_tiles_n = (g.k + a.bn - 1) / a.bn;
+    a.a_wide = p->a_wide;
+    a.off32 = p->off32_dev; a.mult = p->mult_dev; a.shift = p->shift_dev;
+    a.row_cls = p->row_cls_dev; a.col_cls = p->col_cls_dev;
+    a.n_col_cls = p->n_col_cls; a.n_cls = p->n_row_cls * p->n_col_cls; a.kpad = p->kpad;
+    a.ozp = g.ozp; a.qmax = g.qmax; a.relu_lo = g.relu_lo; a.out_flip = g.act_signed ? 0x80 : 0;
+    a.wzp_d = g.wzp_d;
+    a.y = y;
+    a.status = status;
+    a.next_ro = p->next_ro; a.next_ro_bytes = p->next_ro_bytes;
+    const size_t smem = conv_small_smem(a, g.act_signed != 0);
+    if (smem > 227 * 1024)
+        return B200_OK;
+    B200_TRY(encode_activations(p, x, n, tw, th, tn, l.smaps.a));
+    B200_TRY(encode_weights(p, p->w_dev, p->kpad, a.bn, &l.smaps.b));
+    l.smaps.ones = l.smaps.b;
+    if (p->ones_dev)
+        B200_TRY(encode_weights(p, p->ones_dev, 16, 16, &l.smaps.ones));
+    l.smem = smem;
+    l.m_tiles = m_tiles;
+    l.small = true;
+    return B200_OK;
+}
+
+static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status_word, const uint8_t *res, ConvIgemmPlan::Launch &l)
 {
     const ConvGeom &g = p->g;
     if ((((uintptr_t)x | (uintptr_t)y) & 15) != 0)
         return fail(B200_ERR_INVALID, "conv(igemm): x and y must be 16-byte aligned");
-    IgemmArgs &a = p->args;
+    l.x = x; l.res = res; l.y = y; l.n = n; l.status = status_word;
+    l.small = false;
+    l.cta_pair = 0;
+    IgemmArgs &a = l.args;
     memset(&a, 0, sizeof(a));
+    if (status_word)
+        a.status = status_word;       // caller-provided word (the allocation-free entry point)
+    else
+        B200_TRY(status_word_ptr(&a.status));
     a.n = n; a.oh = g.oh; a.ow = g.ow; a.cout = g.k;
-    p->cta_pair = 0;
     a.r = g.r; a.s = g.s; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
     a.c = p->cpad;
     if (p->a_wide)   // whole swizzle atoms (8 pixels) per row segment, at most 256 8-byte elements
@@ -1922,6 +1792,11 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     if (!p->attr_set) {
         B200_TRY(conv_igemm_warm());
         p->attr_set = true;
+    }
+    if (!res && p->small_ok && !(p->pair_ok && p->pair_want == 1)) {
+        B200_TRY(build_small(p, x, n, y, a.status, a.tw, a.th, a.tn, l));
+        if (l.small)
+            return B200_OK;
     }
     if (p->pair_ok) {
         if (p->max_clusters == 0) {
@@ -1943,9 +1818,9 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         }
         const int pair_tiles = (a.tiles_w * a.tiles_h * a.tiles_n + 1) / 2 * (p->kpad / p->bn);
         // long launches only: at least six pair tiles for every cluster
-        p->cta_pair = (p->pair_want == 1 || pair_tiles >= 6 * p->max_clusters) ? 1 : 0;
+        l.cta_pair = (p->pair_want == 1 || pair_tiles >= 6 * p->max_clusters) ? 1 : 0;
     }
-    a.bk = p->bk; a.bn = p->bn; a.stages = p->cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
+    a.bk = p->bk; a.bn = p->bn; a.stages = l.cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
     a.rcp_cchunks = (uint32_t)(((1ull << 30) + (uint64_t)(p->cpad / p->bk) - 1) / (uint64_t)(p->cpad / p->bk));
     a.rcp_s = (uint32_t)(((1ull << 30) + (uint64_t)g.s - 1) / (uint64_t)g.s); a.ob = p->ob; a.b_resident = p->b_resident; a.a_wide = p->a_wide;
     for (a.tw_sh = 0; (1 << a.tw_sh) < a.tw; ++a.tw_sh) {}
@@ -1953,10 +1828,11 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     for (a.ob_sh = 0; (1 << a.ob_sh) < a.ob; ++a.ob_sh) {}
     // instruction descriptor: D = S32 (2 at bit 4), A = unsigned 8-bit (0 at bit 7), B = signed 8-bit
     // (1 at bit 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-    a.idesc = (2u << 4) | ((g.act_signed ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(p->bn >> 3) << 17)
-        | ((uint32_t)((p->cta_pair ? 2 * kTileM : kTileM) >> 4) << 24);
+    a.idesc = (2u << 4) | ((g.act_signed ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)((p->bn + (g.wzp_d ? 16 : 0)) >> 3) << 17)
+        | ((uint32_t)((l.cta_pair ? 2 * kTileM : kTileM) >> 4) << 24);
     uint32_t cols = 32;
-    while (cols < (uint32_t)(p->acc_stages * p->bn))
+    const int ones = g.wzp_d ? 16 : 0;       // accumulator columns behind the channels
+    while (cols < (uint32_t)(p->acc_stages * (p->bn + ones)))
         cols <<= 1;
     a.tmem_cols = cols;
     a.off = p->off_dev; a.mult = p->mult_dev; a.shift = p->shift_dev;
@@ -1965,7 +1841,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     a.ozp = g.ozp; a.qmax = g.qmax; a.relu_lo = g.relu_lo;
     a.generic_requant = p->generic_requant;
     a.out_flip = g.act_signed ? 0x80808080u : 0u;
-    a.epi_const = p->cta_pair ? 0 : p->epi_const; a.ushift = p->ushift;
+    a.epi_const = l.cta_pair ? 0 : p->epi_const; a.ushift = p->ushift;
     a.rnd_lo = (int)(uint32_t)(unsigned long long)p->rnd; a.rnd_hi = (int)(p->rnd >> 32);
     a.off32 = p->off32_dev;
     a.rev = p->rev;
@@ -1977,51 +1853,14 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         a.r_m[i] = p->r_m[i]; a.r_add[i] = p->r_add[i]; a.r_b[i] = p->r_b[i];
     }
     a.r_s0 = p->r_s0; a.r_ozp = p->r_ozp; a.r_lo = p->r_lo;
-    if (status_word)
-        a.status = status_word;       // caller-provided word (the allocation-free entry point)
-    else
-        B200_TRY(status_word_ptr(&a.status));
+    a.wzp_d = g.wzp_d;
 
     // ---- tensor maps -------------------------------------------------------------------------------
-    const CUtensorMapSwizzle sw_ab = swizzle_for(p->bk);
-    for (int ph = 0; ph < g.stride_h; ++ph)
-        for (int pw = 0; pw < g.stride_w; ++pw) {
-            // input pixels (ph + stride_h * i, pw + stride_w * j): a dense 4-D tensor (c, j, i, image)
-            if (ph >= g.h || pw >= g.w) {
-                p->maps.a[ph * 2 + pw] = p->maps.a[0];
-                continue;
-            }
-            if (p->a_wide) {
-                // rows of this parity as a 3-D tensor (ow * 32 bytes in 8-byte elements, row, image);
-                // no swizzle: the bytes are already laid out as the MMA's 32-byte swizzle wants them
-                cuuint64_t dims[3] = { (cuuint64_t)g.w * 4, (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
-                cuuint64_t strides[2] = { (cuuint64_t)g.stride_h * g.w * 32, (cuuint64_t)g.h * g.w * 32 };
-                cuuint32_t box[3] = { (cuuint32_t)a.tw * 4, (cuuint32_t)a.th, (cuuint32_t)a.tn };
-                void *base = (void *)(x + (size_t)ph * g.w * 32);
-                B200_TRY(encode(&p->maps.a[ph * 2 + pw], base, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                CU_TENSOR_MAP_DATA_TYPE_UINT64));
-                continue;
-            }
-            cuuint64_t dims[4] = { (cuuint64_t)g.c, (cuuint64_t)((g.w - pw + g.stride_w - 1) / g.stride_w),
-                                   (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
-            cuuint64_t strides[3] = { (cuuint64_t)g.stride_w * g.c, (cuuint64_t)g.stride_h * g.w * g.c,
-                                      (cuuint64_t)g.h * g.w * g.c };
-            cuuint32_t box[4] = { (cuuint32_t)p->bk, (cuuint32_t)a.tw, (cuuint32_t)a.th, (cuuint32_t)a.tn };
-            void *base = (void *)(x + ((size_t)ph * g.w + pw) * g.c);
-            B200_TRY(encode(&p->maps.a[ph * 2 + pw], base, 4, dims, strides, box, sw_ab));
-        }
-    for (int i = 0; i < 4; ++i) {
-        int ph = i / 2, pw = i % 2;
-        if (ph >= g.stride_h || pw >= g.stride_w)
-            p->maps.a[i] = p->maps.a[0];
-    }
-    {
-        const int ktot = g.r * g.s * p->cpad;
-        cuuint64_t dims[2] = { (cuuint64_t)ktot, (cuuint64_t)p->kpad };
-        cuuint64_t strides[1] = { (cuuint64_t)ktot };
-        cuuint32_t box[2] = { (cuuint32_t)p->bk, (cuuint32_t)(p->cta_pair ? p->bn / 2 : p->bn) };   // a CTA of a pair loads half the rows
-        B200_TRY(encode(&p->maps.b, p->w_dev, 2, dims, strides, box, sw_ab));
-    }
+    B200_TRY(encode_activations(p, x, n, a.tw, a.th, a.tn, l.maps.a));
+    B200_TRY(encode_weights(p, p->w_dev, p->kpad, l.cta_pair ? p->bn / 2 : p->bn, &l.maps.b));   // a CTA of a pair loads half the rows
+    l.maps.ones = l.maps.b;
+    if (p->ones_dev)
+        B200_TRY(encode_weights(p, p->ones_dev, 16, 16, &l.maps.ones));
     if (a.use_tma_store) {
         cuuint64_t dims[4] = { (cuuint64_t)g.k, (cuuint64_t)g.ow, (cuuint64_t)g.oh, (cuuint64_t)n };
         cuuint64_t strides[3] = { (cuuint64_t)g.k, (cuuint64_t)g.ow * g.k, (cuuint64_t)g.oh * g.ow * g.k };
@@ -2030,25 +1869,25 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         cuuint32_t qh = a.tw >= 32 ? 1 : (a.tw * a.th >= 32 ? 32 / a.tw : a.th);
         cuuint32_t qn = a.tw * a.th >= 32 ? 1 : 32 / (a.tw * a.th);
         cuuint32_t box[4] = { (cuuint32_t)p->ob, qw, qh, qn };
-        B200_TRY(encode(&p->maps.y, y, 4, dims, strides, box, swizzle_for(p->ob)));
+        B200_TRY(encode(&l.maps.y, y, 4, dims, strides, box, swizzle_for(p->ob)));
     } else {
-        p->maps.y = p->maps.b;
+        l.maps.y = l.maps.b;
     }
     const int total_tiles = a.tiles_w * a.tiles_h * a.tiles_n * a.n_tiles_n;
-    p->grid = dim3((unsigned)(total_tiles < sms ? total_tiles : sms));
-    p->smem = smem_layout((p->pair ? 2 : 1) * a.stages * p->kgroup, p->b_resident ? g.r * g.s * (p->cpad / p->bk) : a.stages * p->kgroup, p->bk, p->bn, p->groups,
-                          p->cta_pair ? p->bn / 2 : 0).total + 1024;
-    if (p->cta_pair) {
+    l.grid = dim3((unsigned)(total_tiles < sms ? total_tiles : sms));
+    l.smem = smem_layout((p->pair ? 2 : 1) * a.stages * p->kgroup, p->b_resident ? g.r * g.s * (p->cpad / p->bk) : a.stages * p->kgroup, p->bk, p->bn, p->groups,
+                         l.cta_pair ? p->bn / 2 : p->bn + ones).total + 1024;
+    if (l.cta_pair) {
         // pair tiles (two neighbouring M tiles, one channel tile) over the CTA pairs that fit the device at once
         a.pm_tiles = (a.tiles_w * a.tiles_h * a.tiles_n + 1) / 2;
         const int pair_tiles = a.pm_tiles * a.n_tiles_n;
         const int clusters = pair_tiles < p->max_clusters ? pair_tiles : p->max_clusters;
-        p->grid = dim3((unsigned)(2 * clusters));
+        l.grid = dim3((unsigned)(2 * clusters));
         a.step_nt = clusters % a.n_tiles_n;
         a.step_pm = clusters / a.n_tiles_n;
     } else
     {
-        int gsz = (int)p->grid.x;
+        int gsz = (int)l.grid.x;
         a.step_nt = gsz % a.n_tiles_n;
         gsz /= a.n_tiles_n;
         a.step_w = gsz % a.tiles_w;
@@ -2056,22 +1895,14 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         a.step_h = gsz % a.tiles_h;
         a.step_n = gsz / a.tiles_h;
     }
-    p->last_x = x;
-    p->last_res = res;
-    p->last_y = y;
-    p->last_n = n;
-    p->last_status = status_word;
     return B200_OK;
 }
 
-int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st, int *status_word,
-                      const uint8_t *res, const int32_t *wsum)
+int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st, int *status_word, const uint8_t *res)
 {
     if (n == 0)
         return B200_OK;
-    if ((p->g.wzp_d != 0) != (wsum != nullptr))
-        return fail(B200_ERR_INVALID, "conv(igemm): window sums are needed exactly when the weight zero point is not 128");
-    if (wsum != nullptr && res != nullptr)
+    if (p->g.wzp_d != 0 && res != nullptr)
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): a fused residual add and a weight zero point other than 128 do not combine");
     if (res != nullptr && !p->has_res)
         return fail(B200_ERR_INVALID, "conv(igemm): a residual tensor was given but no residual add is set");
@@ -2079,45 +1910,39 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
         return fail(B200_ERR_INVALID, "conv(igemm): this conv was fused with a residual add and needs the residual tensor");
     if (res != nullptr && (((uintptr_t)res) & 15) != 0)
         return fail(B200_ERR_INVALID, "conv(igemm): the residual tensor must be 16-byte aligned");
-    if (p->last_x != x || p->last_y != y || p->last_n != n || p->last_status != status_word || p->last_res != res) {
-        bool hit = false;
-        for (const auto &sv : p->saved)
-            if (sv.x == x && sv.y == y && sv.n == n && sv.status == status_word && sv.res == res) {
-                p->maps = sv.maps;
-                p->args = sv.args;
-                p->grid = sv.grid;
-                p->smem = sv.smem;
-                p->cta_pair = sv.cta_pair;
-                p->last_x = x; p->last_y = y; p->last_n = n; p->last_status = status_word; p->last_res = res;
-                hit = true;
-                break;
-            }
-        if (!hit) {
-            B200_TRY(build_launch(p, x, n, y, status_word, res));
-            ConvIgemmPlan::Saved sv = { x, res, y, n, status_word, p->maps, p->args, p->grid, p->smem, p->cta_pair };
+    auto matches = [&](const ConvIgemmPlan::Launch &l) { return l.x == x && l.y == y && l.n == n && l.status == status_word && l.res == res; };
+    if (p->last >= p->saved.size() || !matches(p->saved[p->last])) {
+        size_t i = 0;
+        while (i < p->saved.size() && !matches(p->saved[i]))
+            ++i;
+        if (i == p->saved.size()) {
+            ConvIgemmPlan::Launch l;
+            B200_TRY(build_launch(p, x, n, y, status_word, res, l));
             if (p->saved.size() < ConvIgemmPlan::kMaxSaved) {
-                p->saved.push_back(sv);
+                p->saved.push_back(l);
             } else {
-                p->saved[p->next_saved] = sv;
-                p->next_saved = (p->next_saved + 1) % ConvIgemmPlan::kMaxSaved;
+                i = p->next_saved;
+                p->saved[i] = l;
+                p->next_saved = (i + 1) % ConvIgemmPlan::kMaxSaved;
             }
         }
+        p->last = i;
     }
-    // the window sums live in the caller's scratch, not in the launch cache's key: set them per launch
-    p->args.wsum = wsum;
-    p->args.wzp_d = p->g.wzp_d;
+    const ConvIgemmPlan::Launch &l = p->saved[p->last];
     const size_t bytes = (size_t)n * ((size_t)p->g.h * p->g.w * p->g.c + (size_t)p->g.oh * p->g.ow * p->g.k) + p->w_bytes;
+    if (l.small)
+        return conv_small_launch(l.smaps, l.sargs, l.m_tiles, l.smem, bytes, st);
     if (res != nullptr)
-        return launch_kernel(conv_igemm_i8_kernel<true>, p->grid, dim3(kThreads), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
-    if (wsum != nullptr)
-        return launch_kernel(conv_igemm_i8_kernel<false, true>, p->grid, dim3(kThreads), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
-    if (p->cta_pair)
-        return launch_kernel(conv_igemm_i8_kernel<false, false, 3>, p->grid, dim3(kThreads), p->smem, st, bytes, 2, p->maps, p->args, p->tab);
+        return launch_kernel(conv_igemm_i8_kernel<true>, l.grid, dim3(kThreads), l.smem, st, bytes, 1, l.maps, l.args, p->tab);
+    if (p->g.wzp_d != 0)
+        return launch_kernel(conv_igemm_i8_kernel<false, true>, l.grid, dim3(kThreads), l.smem, st, bytes, 1, l.maps, l.args, p->tab);
+    if (l.cta_pair)
+        return launch_kernel(conv_igemm_i8_kernel<false, false, 3>, l.grid, dim3(kThreads), l.smem, st, bytes, 2, l.maps, l.args, p->tab);
     if (p->pair)
-        return launch_kernel(conv_igemm_i8_kernel<false, false, 2>, p->grid, dim3(kThreads2), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
+        return launch_kernel(conv_igemm_i8_kernel<false, false, 2>, l.grid, dim3(kThreads2), l.smem, st, bytes, 1, l.maps, l.args, p->tab);
     if (p->mma_warps == 2)
-        return launch_kernel(conv_igemm_i8_kernel<false, false, 1>, p->grid, dim3(kThreads2), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
-    return launch_kernel(conv_igemm_i8_kernel<false>, p->grid, dim3(kThreads), p->smem, st, bytes, 1, p->maps, p->args, p->tab);
+        return launch_kernel(conv_igemm_i8_kernel<false, false, 1>, l.grid, dim3(kThreads2), l.smem, st, bytes, 1, l.maps, l.args, p->tab);
+    return launch_kernel(conv_igemm_i8_kernel<false>, l.grid, dim3(kThreads), l.smem, st, bytes, 1, l.maps, l.args, p->tab);
 }
 
 // Everything the first launch of any plan would otherwise do once per process or device: the driver
@@ -2127,6 +1952,7 @@ int conv_igemm_warm()
 {
     if (!encode_fn())
         return fail(B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    B200_TRY(conv_small_warm());
     B200_CUDA_TRY(cudaFuncSetAttribute(conv_igemm_i8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     B200_CUDA_TRY(cudaFuncSetAttribute(conv_igemm_i8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     B200_CUDA_TRY((cudaFuncSetAttribute(conv_igemm_i8_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)));

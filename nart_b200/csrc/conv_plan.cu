@@ -40,7 +40,6 @@ void destroy_conv(b200_conv *cv)
     if (cv->igemm)
         conv_igemm_destroy(cv->igemm);
     cudaFree(cv->scratch);
-    cudaFree(cv->sums);
     delete cv;
 }
 
@@ -236,7 +235,7 @@ int b200_conv2d_create(
                 for (int rr = 0; rr < g.r; ++rr)
                     for (int j = 0; j < g.s; ++j)
                         w_low[((size_t)k * gl.c + j * 4 + c) * g.r + rr] = w_s8[(((size_t)k * 4 + c) * g.r + rr) * g.s + j];
-        rc = conv_igemm_create(gl, w_low, bias, mult.data(), shift.data(), &cv->igemm, true);
+        rc = conv_igemm_create(gl, w_low, bias, mult.data(), shift.data(), &cv->igemm, true, g.s);
         if (rc == B200_OK) {
             cv->algo = B200_CONV_ALGO_IGEMM;
             cv->lowered = true;
@@ -335,18 +334,12 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
         return fail(B200_ERR_INVALID, "conv: this plan has a residual add, run it with b200_conv2d_run_residual");
     B200_TRY(b200_conv2d_reserve(conv, n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
     const ConvGeom &g = conv->g;
-    const int32_t *wsum = nullptr;
-    if (conv->algo == B200_CONV_ALGO_IGEMM && g.wzp_d != 0) {
-        int32_t *w = conv->sums + conv->sums_images * g.h * g.w;
-        B200_TRY(conv_window_sum_launch(g, x, n, conv->sums, w, as_stream(stream)));
-        wsum = w;
-    }
     if (conv->lowered) {
         B200_TRY(conv_lower_rows_launch(g, x, n, conv->scratch, as_stream(stream)));
-        return conv_igemm_launch(conv->igemm, conv->scratch, n, y, as_stream(stream), nullptr, nullptr, wsum);
+        return conv_igemm_launch(conv->igemm, conv->scratch, n, y, as_stream(stream));
     }
     if (conv->algo == B200_CONV_ALGO_IGEMM)
-        return conv_igemm_launch(conv->igemm, x, n, y, as_stream(stream), nullptr, nullptr, wsum);
+        return conv_igemm_launch(conv->igemm, x, n, y, as_stream(stream));
     return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, as_stream(stream));
 }
 
@@ -364,13 +357,6 @@ int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
             B200_TRY(b200_malloc((void **)&conv->scratch, need));
             conv->scratch_bytes = need;
         }
-    }
-    if (conv->algo == B200_CONV_ALGO_IGEMM && g.wzp_d != 0 && (size_t)n > conv->sums_images) {
-        B200_CUDA_TRY(cudaFree(conv->sums));
-        conv->sums = nullptr;
-        conv->sums_images = 0;
-        B200_TRY(b200_malloc((void **)&conv->sums, (size_t)n * ((size_t)g.h * g.w + (size_t)g.oh * g.ow) * sizeof(int32_t)));
-        conv->sums_images = (size_t)n;
     }
     return B200_OK;
 }

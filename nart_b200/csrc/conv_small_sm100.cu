@@ -1,0 +1,407 @@
+// Implicit-GEMM int8 convolution for launches that do not fill the GPU: a batch of one or a few images, the
+// last stages of a network at a serving batch, an inner product.  Same arithmetic and operands as the persistent
+// kernel (conv_igemm_sm100.cu); what differs is what bounds it.  There the tensor pipe and the epilogue set the
+// pace; here a launch is one chain -- launch, first TMA round trip, MMAs, accumulator, store -- and its length is the
+// time.  On one image the persistent kernel walked all k-blocks of 256 channels x 3x3 on two CTAs (14.4 us) and of
+// 512 channels on two (22.8 us): 72 and 144 MMAs one after the other at 64 cycles or more each, 3 to 6 stages of
+// operands in flight.  So:
+//   * one tile per CTA, narrow channel tiles, and the k-blocks of a tile split over a cluster of up to eight CTAs
+//     (int32 sums: any order gives the same bits).  The partial accumulators meet in a reduce-scatter over distributed
+//     shared memory: CTA r of the cluster receives and finishes channels [r * bn / split, (r + 1) * bn / split);
+//   * every k-block of a CTA has a slot of its own where they fit, the weights' loads are issued before
+//     griddepcontrol.wait, and constants reach shared memory while the operands are on their way;
+//   * 192 threads and as little shared memory as that needs, so that the next launch's CTAs are resident beside these.
+// Roles: warp 0 TMA (one lane per slot), warp 1 tensor memory and MMAs, warps 2-5 epilogue.
+#include <stdlib.h>
+
+#include "common.cuh"
+#include "conv_small.h"
+#include "kernels.h"
+#include "sm100_ptx.cuh"
+
+namespace b200 {
+
+namespace {
+
+constexpr int kSmallThreads = 192;
+constexpr int kSmallM = 128;            // pixels per tile
+constexpr int kSmallSlots = 16;
+constexpr int kSmallClsCols = 4096;     // border classes x channels that are staged in shared memory; more are read in place
+
+constexpr int kErrSmallProducer = 0x201, kErrSmallFull = 0x202, kErrSmallEpilogue = 0x203;
+
+struct SmallLayout {
+    uint32_t b, b_tile, red, xred, mult, shift, off, bars, tmem_slot, abort_flag, total;
+};
+__host__ __device__ inline SmallLayout small_layout(const SmallArgs &g)
+{
+    SmallLayout L;
+    uint32_t o = (uint32_t)g.slots * kSmallM * g.bk;
+    L.b = o;
+    L.b_tile = ((uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk + 1023u) & ~1023u;
+    o += g.slots * L.b_tile;
+    L.red = o;                                              // [split][bn / split][128] partial accumulators
+    o += g.split > 1 ? (uint32_t)g.bn * kSmallM * 4 : 0;
+    L.xred = o;                                             // [split][128] partial window sums
+    o += g.split > 1 && g.wzp_d ? (uint32_t)g.split * kSmallM * 4 : 0;
+    L.mult = o;
+    o += g.bn * 4;
+    L.shift = o;
+    o += g.bn * 4;
+    L.off = o;
+    o += g.n_cls * g.bn <= kSmallClsCols ? (uint32_t)g.n_cls * g.bn * 4 : 0;
+    o = (o + 15u) & ~15u;
+    L.bars = o;                                             // full[slots], empty[slots], accumulator
+    o += (2 * kSmallSlots + 1) * 8;
+    L.tmem_slot = o;
+    o += 8;
+    L.abort_flag = o;
+    o += 8;
+    L.total = o + 1024;                                     // the base is aligned to 1024
+    return L;
+}
+
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// N channels from accumulators `acc` (one pixel): requantized, packed, stored at `dst`; k: the first channel.
+template <int N>
+__device__ __forceinline__ void store_channels(const int (&acc)[N], const SmallArgs &g, const int *s_mult, const int *s_shift, const int32_t *off,
+                                               int xcorr, int j, int k, uint8_t *dst)
+{
+    uint32_t w[N / 4];
+#pragma unroll
+    for (int q = 0; q < N / 4; ++q) {
+        int v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = 4 * q + e;
+            v[e] = sat_relu(requant_raw(acc[i] + off[j + i] + xcorr, (uint32_t)s_mult[j + i], s_shift[j + i], g.ozp), g.qmax, g.relu_lo) ^ g.out_flip;
+        }
+        w[q] = pack4(v[0], v[1], v[2], v[3]);
+    }
+    if (k + N <= g.cout && (g.cout & (N - 1)) == 0) {
+        if constexpr (N == 16)
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        else
+            *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (k + i < g.cout)
+                dst[i] = (uint8_t)(w[i / 4] >> (8 * (i % 4)));
+    }
+}
+
+__global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_constant__ SmallMaps maps, const __grid_constant__ SmallArgs g)
+{
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;
+    uint8_t *smem = smem_raw + (base - raw_addr);
+    const SmallLayout L = small_layout(g);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t bars = base + L.bars;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (kSmallSlots + s); };
+    const uint32_t acc_bar = bars + 8u * (2 * kSmallSlots);
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + L.tmem_slot);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.abort_flag);
+
+    const int split = g.split;
+    const int rank = split > 1 ? (int)(blockIdx.x % (unsigned)split) : 0;    // clusters are consecutive blocks
+    const int tile = (int)(blockIdx.x / (unsigned)split);
+    const int nt = tile % g.n_tiles_n;
+    int mt = tile / g.n_tiles_n;
+    const int twi = mt % g.tiles_w;
+    mt /= g.tiles_w;
+    const int thi = mt % g.tiles_h, tni = mt / g.tiles_h;
+    const int kb0 = rank * g.kblocks / split, kb1 = (rank + 1) * g.kblocks / split;
+    const int k0 = nt * g.bn;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.slots; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(acc_bar, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x == 64) {
+        prefetch_map(&maps.a[0]);
+        prefetch_map(&maps.b);
+    }
+    if (warp == 1) {
+        tmem_alloc(base + L.tmem_slot, g.tmem_cols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (split > 1)
+        cluster_sync_all();         // the peers run: their shared memory may be written
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t a_tile = (uint32_t)kSmallM * g.bk;
+
+    if (warp == 0) {
+        // ================= TMA =================
+        const uint32_t tx = a_tile + (uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk;
+        const uint32_t a_dst = base + lane * a_tile, b_dst = base + L.b + lane * L.b_tile;
+        const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;
+        auto load_b = [&](int kb) {
+            mbar_expect_tx(full_bar(lane), tx);
+            tma_load_2d(b_dst, &maps.b, full_bar(lane), kb * g.bk, k0);
+            if (g.wzp_d)
+                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(lane), kb * g.bk, 0);
+        };
+        int kb = kb0 + lane;
+        bool active = lane < g.slots && kb < kb1;
+        if (active)
+            load_b(kb);             // weights are constant: the launch before this one does not matter to them
+        pdl_wait();
+        bool first = true;
+        uint32_t phase = 0;
+        long long t0 = clock64();
+        int spins = 0;
+        while (__any_sync(0xffffffffu, active)) {
+            if (active) {
+                if (first || mbar_test_wait(empty_bar(lane), phase ^ 1)) {
+                    if (!first)
+                        load_b(kb);
+                    const int tap = kb / g.cchunks, cc = (kb - tap * g.cchunks) * g.bk;
+                    const int rr = tap / g.s, ss = tap - rr * g.s;
+                    // see the producer of conv_igemm_i8_kernel
+                    const int dh = rr - g.pad_h, ph = dh & sh_h, dw = ss - g.pad_w, pw = dw & sh_w;
+                    const int yh = (thi << g.th_sh) + ((dh - ph) >> sh_h), xw = (twi << g.tw_sh) + ((dw - pw) >> sh_w), n0 = tni * g.tn;
+                    const CUtensorMap *amap = &maps.a[ph * 2 + pw];
+                    if (g.a_wide)
+                        tma_load_3d(a_dst, amap, full_bar(lane), xw << 2, yh, n0);
+                    else
+                        tma_load_4d(a_dst, amap, full_bar(lane), cc, xw, yh, n0);
+                    first = false;
+                    phase ^= 1;
+                    kb += g.slots;
+                    active = kb < kb1;
+                    t0 = clock64();
+                    spins = 0;
+                } else if ((++spins & 255) == 0 && (*abort_flag != 0 || clock64() - t0 > kWaitCycles)) {
+                    atomicCAS(g.status, 0, kErrSmallProducer);
+                    *abort_flag = 1;
+                    active = false;
+                }
+            }
+        }
+        pdl_trigger();
+    } else if (warp == 1) {
+        // ================= MMA =================
+        const uint32_t lead = lane == 0 ? 1u : 0u;
+        const uint64_t adesc0 = make_smem_desc(base, g.bk), bdesc0 = make_smem_desc(base + L.b, g.bk);
+        const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);
+        const int ksteps = g.bk / 32;
+        int slot = 0;
+        uint32_t phase = 0, accumulate = 0;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            if (!mbar_wait(full_bar(slot), phase, abort_flag)) {
+                if (lead)
+                    atomicCAS(g.status, 0, kErrSmallFull);
+                *abort_flag = 1;
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t a_lo = (uint32_t)adesc0 + slot * (a_tile >> 4), b_lo = (uint32_t)bdesc0 + slot * (L.b_tile >> 4);
+            for (int j = 0; j < ksteps; ++j) {
+                mma_i8(tmem_base, a_lo + 2 * j, b_lo + 2 * j, desc_hi, g.idesc, accumulate, lead);
+                accumulate = 1;
+            }
+            if (kb + g.slots < kb1)
+                mma_commit(empty_bar(slot), lead);
+            if (++slot == g.slots) {
+                slot = 0;
+                phase ^= 1;
+            }
+        }
+        if (ok)
+            mma_commit(acc_bar, lead);
+    }
+
+    // ================= epilogue (warps 2..5) =================
+    const int quarter = warp & 3;                       // tensor-memory lanes of this warp
+    const int row = quarter * 32 + lane;
+    const int bnl = g.bn / split;                       // channels this CTA finishes
+    int *s_mult = reinterpret_cast<int *>(smem + L.mult), *s_shift = reinterpret_cast<int *>(smem + L.shift);
+    int32_t *s_off = reinterpret_cast<int32_t *>(smem + L.off);
+    const bool off_staged = g.n_cls * g.bn <= kSmallClsCols;
+    const int lw = row & ((1 << g.tw_sh) - 1), lh = (row >> g.tw_sh) & ((1 << g.th_sh) - 1), ln = row >> (g.tw_sh + g.th_sh);
+    const int ow = (twi << g.tw_sh) + lw, oh = (thi << g.th_sh) + lh, img = tni * g.tn + ln;
+    const bool pix_valid = ow < g.ow && oh < g.oh && img < g.n;
+    uint8_t *dst = g.y + (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
+    const int32_t *off = nullptr;
+    const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    bool ok = true;
+    if (warp >= 2) {
+        const int et = threadIdx.x - 64;
+        if (et == 0 && g.next_ro_bytes != 0) {
+            const uint32_t granules = g.next_ro_bytes >> 4, per = (granules + gridDim.x - 1) / gridDim.x, from = blockIdx.x * per;
+            if (from < granules)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g.next_ro + ((size_t)from << 4)), "r"(min(per, granules - from) << 4) : "memory");
+        }
+        for (int j = et; j < g.bn; j += 128) {
+            const bool in = k0 + j < g.kpad;
+            s_mult[j] = in ? (int)__ldg(g.mult + k0 + j) : 0;
+            s_shift[j] = in ? __ldg(g.shift + k0 + j) : 33;
+        }
+        if (off_staged)
+            for (int i = et; i < g.n_cls * g.bn; i += 128) {
+                const int c = i / g.bn, j = i - c * g.bn;
+                s_off[i] = k0 + j < g.kpad ? __ldg(g.off32 + (size_t)c * g.kpad + k0 + j) : 0;
+            }
+        const int cls = (int)__ldg(g.row_cls + min(oh, g.oh - 1)) * g.n_col_cls + (int)__ldg(g.col_cls + min(ow, g.ow - 1));
+        off = off_staged ? s_off + cls * g.bn : g.off32 + (size_t)cls * g.kpad + k0;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        ok = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag));
+        if (!ok && lane == 0) {
+            atomicCAS(g.status, 0, kErrSmallEpilogue);
+            *abort_flag = 1;
+        }
+        tc_fence_after();
+        pdl_wait();                                     // the output may be what the launch before this one still reads
+        if (ok && split == 1) {
+            int xcorr = 0;
+            if (g.wzp_d) {
+                uint32_t xs;
+                tmem_ld1(t_row + g.bn, xs);
+                tmem_ld_wait();
+                xcorr = -g.wzp_d * (int)xs;
+            }
+            for (int c0 = 0; c0 < g.bn && k0 + c0 < g.cout; c0 += 16) {
+                uint32_t v[16];
+                tmem_ld16(t_row + c0, v);
+                tmem_ld_wait();
+                int acc[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    acc[i] = (int)v[i];
+                if (pix_valid)
+                    store_channels<16>(acc, g, s_mult, s_shift, off, xcorr, c0, k0 + c0, dst + c0);
+                __syncwarp();
+            }
+        } else if (ok) {
+            // this CTA's partial sums to the CTAs that finish them: [source rank][channel][pixel]
+            for (int c0 = 0; c0 < g.bn; c0 += 16) {
+                uint32_t v[16];
+                tmem_ld16(t_row + c0, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int h = 0; h < 16; h += 8) {       // bn / split is a multiple of 8
+                    const int owner = (c0 + h) / bnl, j = (c0 + h) - owner * bnl;
+                    const uint32_t to = cluster_addr(base + L.red + (uint32_t)((rank * bnl + j) * kSmallM + row) * 4, (uint32_t)owner);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        st_cluster(to + i * (kSmallM * 4), v[h + i]);
+                }
+            }
+            if (g.wzp_d) {
+                uint32_t xs;
+                tmem_ld1(t_row + g.bn, xs);
+                tmem_ld_wait();
+                for (int o = 0; o < split; ++o)
+                    st_cluster(cluster_addr(base + L.xred + (uint32_t)(rank * kSmallM + row) * 4, (uint32_t)o), xs);
+            }
+        }
+    }
+    if (split > 1) {
+        __syncthreads();
+        cluster_sync_all();
+        if (warp >= 2 && ok && pix_valid) {
+            const int *red = reinterpret_cast<const int *>(smem + L.red);
+            int xcorr = 0;
+            if (g.wzp_d) {
+                const int *xred = reinterpret_cast<const int *>(smem + L.xred);
+                for (int s = 0; s < split; ++s)
+                    xcorr -= xred[s * kSmallM + row];
+                xcorr *= g.wzp_d;
+            }
+            const int c1 = rank * bnl;                  // first channel of this CTA's share
+            for (int j = 0; j < bnl && k0 + c1 + j < g.cout; j += 8) {
+                int acc[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    acc[i] = red[(j + i) * kSmallM + row];
+                for (int s = 1; s < split; ++s)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        acc[i] += red[(s * bnl + j + i) * kSmallM + row];
+                store_channels<8>(acc, g, s_mult, s_shift, off, xcorr, c1 + j, k0 + c1 + j, dst + c1 + j);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, g.tmem_cols);
+    }
+}
+
+}  // namespace
+
+bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int *bn_out, int *split_out)
+{
+    const int sms = sm_count();
+    const int k16 = (k + 15) / 16 * 16;
+    double best = 1e30;
+    for (int bn = 16; bn <= 128; bn *= 2) {
+        if (bn > k16 && bn != 16 && bn / 2 >= k16)
+            break;
+        const int tiles = m_tiles * ((k + bn - 1) / bn);
+        for (int split = 1; split <= 8 && split <= kblocks; split *= 2) {
+            if (tiles * split > sms || bn / split < 8)
+                continue;
+            // nanoseconds on this GPU: the operands of a CTA's k-blocks through its memory port, its MMAs one
+            // after the other, the reduction, the share of the epilogue that follows the last MMA
+            const int kb = (kblocks + split - 1) / split;
+            const double load = kb * (double)(kSmallM + bn + (wzp ? 16 : 0)) * bk / 110.0;
+            const double mma = kb * (bk / 32) * (bn + (wzp ? 16 : 0) > 128 ? 38.0 : 34.0);
+            const double cost = (load > mma ? load : mma) + (split > 1 ? 900.0 + bn * 4.0 : 0.0) + bn / split * 10.0;
+            if (cost < best) {
+                best = cost;
+                *bn_out = bn;
+                *split_out = split;
+            }
+        }
+    }
+    return best < 1e30;
+}
+
+size_t conv_small_smem(SmallArgs &a, bool act_signed)
+{
+    const int kb = (a.kblocks + a.split - 1) / a.split, n = a.bn + (a.wzp_d ? 16 : 0);
+    a.idesc = (2u << 4) | ((act_signed ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
+    a.tmem_cols = 32;
+    while (a.tmem_cols < (uint32_t)n)
+        a.tmem_cols <<= 1;
+    a.slots = kb < kSmallSlots ? kb : kSmallSlots;
+    while (a.slots > 4 && small_layout(a).total > 110 * 1024)       // two CTAs per SM: this launch's and the next one's
+        --a.slots;
+    while (a.slots > 1 && small_layout(a).total > 227 * 1024)
+        --a.slots;
+    return small_layout(a).total;
+}
+
+int conv_small_launch(const SmallMaps &maps, const SmallArgs &a, int m_tiles, size_t smem, size_t bytes, cudaStream_t st)
+{
+    return launch_kernel(conv_small_kernel, dim3((unsigned)(m_tiles * a.n_tiles_n * a.split)), dim3(kSmallThreads), smem, st, bytes, a.split, maps, a);
+}
+
+int conv_small_warm()
+{
+    B200_CUDA_TRY(cudaFuncSetAttribute(conv_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    return B200_OK;
+}
+
+}  // namespace b200
