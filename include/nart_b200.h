@@ -146,7 +146,8 @@ B200_API void b200_get_quant_scale(float x, int bits, uint32_t *mult, int8_t *sh
 
 #define B200_CONV_ALGO_AUTO 0
 #define B200_CONV_ALGO_DIRECT 1 /* CUDA-core dp4a kernel: any group, any channel count   */
-#define B200_CONV_ALGO_IGEMM 2  /* tcgen05 kind::i8 implicit GEMM: group 1, c % 16 == 0, k % 16 == 0 */
+#define B200_CONV_ALGO_IGEMM 2  /* tcgen05 kind::i8 implicit GEMM: group 1, k >= 16; asked for by name, c % 16 == 0 or a
+                                   4-channel image (AUTO also pads other channel counts to it) */
 
 typedef struct b200_conv_params {
     int32_t c, h, w;        /* input channels and spatial size (batch is a run-time argument) */
@@ -180,7 +181,7 @@ B200_API int b200_conv2d_algo(const b200_conv_t *conv);
 /* One line of text naming the kernel variant and tiling the plan resolved to (for logs and tuning). */
 B200_API int b200_conv2d_describe(const b200_conv_t *conv, char *buf, size_t len);
 /* x: device NHWC [n][h][w][c]; y: device NHWC [n][oh][ow][k].  Plans with a scratch tensor (the
- * row-lowered 4-channel stem) grow it, with a device synchronization,
+ * row-lowered 4-channel stem; channel counts that are no multiple of 16, copied into padded tensors) grow it, with a device synchronization,
  * the first time a larger batch arrives; the old tensor is freed then. */
 B200_API int b200_conv2d_run(
     b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, b200_stream_t stream);

@@ -42,6 +42,24 @@ int status_word_ptr(int **dev_ptr);
 // and cached for the life of the process (runtime.cu).
 int lut_cache_get(const uint8_t lut[256], const uint8_t **dev_ptr);
 
+// Division of 32-bit numbers below 2^31 by a launch constant: one high multiplication, one shift (the multiplier is
+// rounded up, 2^(31 + l) / d with 2^(l-1) < d <= 2^l, whose error stays below one part in 2^31).
+struct FastDiv {
+    uint32_t d = 1, mul = 0x80000000u, shift = 0;
+    FastDiv() = default;
+    explicit FastDiv(uint32_t divisor) : d(divisor)
+    {
+        uint32_t l = 0;
+        while ((1ull << l) < divisor)
+            ++l;
+        mul = (uint32_t)(((1ull << (31 + l)) + divisor - 1) / divisor);
+        shift = l;
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t div(uint32_t n) const { return (uint32_t)(((uint64_t)n * mul) >> 31) >> shift; }
+#endif
+};
+
 // Number of SMs of the current device (cached).
 int sm_count();
 

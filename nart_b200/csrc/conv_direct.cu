@@ -306,121 +306,168 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------
-// Depthwise 3x3 with horizontal stride S (1 or 2): a thread computes two output pixels side by
-// side, in ROWS (1 or 2) output rows.  The two windows of a row cover 3 + S neighbouring input
+// Depthwise 3x3 with stride S (1 or 2) both ways: a thread computes two output pixels side by
+// side, in ROWS output rows, for four channels.  The two windows of a row cover 3 + S neighbouring input
 // pixels per kernel row.  One transpose of the first four of those words gives, per channel, a
 // word (x0, x1, x2, x3) that serves both pixels: dp4a against (w0, w1, w2, 0) is the left pixel's
 // kernel row; the right pixel's is (0, w0, w1, w2) for S == 1, and for S == 2 (0, 0, w0, w1) plus
-// the fifth word against w2 placed at the channel's own byte (no extraction).  With ROWS == 2 (the
-// vertical stride is S as well) the output rows share 3 - S of their input rows.  The per-channel
-// weights and requantize constants are read once per thread.  Arithmetic and results equal
-// conv_depthwise3x3_kernel.  Weight table: [c/4][3 kernel rows][2 + (S == 2)][4 channels] words.
+// the fifth word against w2 placed at the channel's own byte (no extraction).  Neighbouring output rows
+// share 3 - S of their input rows.
+//
+// Instruction issue bounds it, and the dp4a pipe (one per two cycles): with 2 x 2 outputs per thread, 64-bit
+// divisions and a wide integer requantize it took 24 instructions per output byte (144 channels of 56 x 56,
+// batch 64: 35.7 us, 1.6 TB/s).  So weights and constants are read once for ROWS rows, indices are divided by
+// multiplication, and the requantize is fp32, exactly, two values per instruction: the accumulator starts at
+// bits(1.5 * 2^23) + bias, which makes its bits the float 1.5 * 2^23 + acc (|acc| < 2^22, checked when the table
+// is built); mult * 2^-shift is a float m (24 significant bits); acc * m + (zero point + 1/2) is formed by one
+// multiply-add rounded toward zero, which never crosses an integer, and 2^23 is added, again toward zero: the low
+// bits are then floor(acc * m + 1/2) + zero point for every result of 0 or more, and for every negative one the
+// low 16 bits are a negative 16-bit number (results stay below 2^13 in magnitude, checked as well).  Floor and
+// ceiling run on pairs of those.
+// (A thread that walks whole columns, every input row loaded and transposed once, is no faster: its accumulators in
+// flight and weights leave 16 to 20 warps per SM, and its row loop's bookkeeping costs what the shared rows save.)
+// Weight table: [c/4][3 kernel rows][2 + (S == 2)][4 channels] words.  Requantize table: [c/4] 4 start values, 4 floats.
 // ---------------------------------------------------------------------------------------------
+struct DwArgs {
+    int c4, h, w, oh, ow, pad_h, pad_w;
+    FastDiv by_c4, by_pairs, by_strips;         // channel words, pixel pairs of a row, strips of ROWS rows
+    uint32_t total, izp4;
+    float add;                                  // zero point + 1/2
+    uint32_t lo2;                               // floor, twice
+};
+
+// The bits of 2^23 + floor(((a0, a1) - 1.5 * 2^23) * (m0, m1) + add): their low halves in one word
+__device__ __forceinline__ uint32_t requant_pair(int a0, int a1, float m0, float m1, float add)
+{
+    uint32_t q0, q1;
+    asm("{\n\t.reg .b64 a, m, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 c, {%6, %6};\n\t"
+        "add.rn.f32x2 a, a, c;\n\t"
+        "mov.b64 m, {%4, %5};\n\t"
+        "mov.b64 d, {%7, %7};\n\t"
+        "fma.rz.f32x2 a, a, m, d;\n\t"
+        "mov.b64 c, {%8, %8};\n\t"
+        "add.rz.f32x2 a, a, c;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "=r"(q0), "=r"(q1)
+        : "r"(a0), "r"(a1), "f"(m0), "f"(m1), "f"(-12582912.f), "f"(add), "f"(8388608.f));
+    return __byte_perm(q0, q1, 0x5410);
+}
+__device__ __forceinline__ uint32_t clamp_s16x2(uint32_t v, uint32_t lo2)
+{
+    uint32_t d;
+    asm("max.s16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(lo2));
+    asm("min.s16x2 %0, %0, %1;" : "+r"(d) : "r"(0x00ff00ffu));
+    return d;
+}
+
 template <int ROWS, int S>
-__global__ void __launch_bounds__(256) conv_depthwise3x3_pair_kernel(
-    ConvGeom g, const uint32_t *__restrict__ x, const uint4 *__restrict__ w3p, const int4 *__restrict__ q3,
-    uint32_t *__restrict__ y, int n)
+__global__ void __launch_bounds__(128) conv_depthwise3x3_strip_kernel(
+    const __grid_constant__ DwArgs g, const uint32_t *__restrict__ x, const uint4 *__restrict__ w3p, const uint4 *__restrict__ qf,
+    uint32_t *__restrict__ y)
 {
     constexpr int IN_ROWS = 3 + (ROWS - 1) * S, IN_COLS = 3 + S, NV = S == 2 ? 3 : 2;
+    const uint32_t idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= g.total) {
+        pdl_wait();
+        return;
+    }
+    const uint32_t pp = g.by_c4.div(idx), ci = idx - pp * g.c4;
+    const uint32_t rowi = g.by_pairs.div(pp), oxp = pp - rowi * g.by_pairs.d;
+    const uint32_t img = g.by_strips.div(rowi), strip = rowi - img * g.by_strips.d;
+    const int ox = (int)oxp * 2, oy = (int)strip * ROWS;
+    uint4 wv[3][NV];
+#pragma unroll
+    for (int rr = 0; rr < 3; ++rr)
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            wv[rr][v] = __ldg(w3p + ((size_t)ci * 3 + rr) * NV + v);
+    const uint4 start = __ldg(qf + ci * 2), mb = __ldg(qf + ci * 2 + 1);
     pdl_wait();
     pdl_trigger();
-    const uint32_t cq = (uint32_t)g.c / 4;
-    const uint32_t owp = ((uint32_t)g.ow + 1) / 2, ohp = ((uint32_t)g.oh + ROWS - 1) / ROWS;
-    const uint32_t total = (uint32_t)n * ohp * owp * cq;      // the launcher checks that it fits 32 bits
-    const uint32_t izp4 = (uint32_t)g.izp * 0x01010101u;
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-        const uint32_t ci = idx % cq;
-        const uint32_t pp = idx / cq;
-        const int ox = (int)(pp % owp) * 2;
-        const uint32_t rowi = pp / owp;
-        const int oy = (int)(rowi % ohp) * ROWS;
-        const uint32_t img = rowi / ohp;
-        const int iy0 = oy * g.stride_h - g.pad_h, ix0 = ox * S - g.pad_w;   // ROWS == 2 only with stride_h == S
-        const uint32_t row_pitch = (uint32_t)g.w * cq;
-        const uint32_t *xc = x + (img * (uint32_t)g.h * row_pitch + ci);
-        uint32_t t[IN_ROWS][IN_COLS];
-        if (iy0 >= 0 && iy0 + IN_ROWS - 1 < g.h && ix0 >= 0 && ix0 + IN_COLS - 1 < g.w) {
-            const uint32_t *p0 = xc + ((uint32_t)iy0 * row_pitch + (uint32_t)ix0 * cq);
+    const int iy0 = oy * S - g.pad_h, ix0 = ox * S - g.pad_w;
+    // byte offsets of 32 bits from the tensor's start (the launcher checks that it ends below 4 GB)
+    auto at = [&](uint32_t off) { return __ldg(reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(x) + off)); };
+    const uint32_t col_pitch = (uint32_t)g.c4 * 4, row_pitch = (uint32_t)g.w * col_pitch;
+    const uint32_t x0 = (img * (uint32_t)g.h + (uint32_t)iy0) * row_pitch + (uint32_t)ix0 * col_pitch + ci * 4;   // modulo 2^32
+    uint32_t t[IN_ROWS][IN_COLS];
+    if (iy0 >= 0 && iy0 + IN_ROWS - 1 < g.h && ix0 >= 0 && ix0 + IN_COLS - 1 < g.w) {
 #pragma unroll
-            for (int rr = 0; rr < IN_ROWS; ++rr)
+        for (int rr = 0; rr < IN_ROWS; ++rr)
 #pragma unroll
-                for (int ss = 0; ss < IN_COLS; ++ss)
-                    t[rr][ss] = __ldg(p0 + (rr * row_pitch + ss * cq));
-        } else {
+            for (int ss = 0; ss < IN_COLS; ++ss)
+                t[rr][ss] = at(x0 + rr * row_pitch + ss * col_pitch);
+    } else {
 #pragma unroll
-            for (int rr = 0; rr < IN_ROWS; ++rr)
+        for (int rr = 0; rr < IN_ROWS; ++rr)
 #pragma unroll
-                for (int ss = 0; ss < IN_COLS; ++ss) {
-                    const int iy = iy0 + rr, ix = ix0 + ss;
-                    t[rr][ss] = (iy >= 0 && iy < g.h && ix >= 0 && ix < g.w)
-                        ? __ldg(xc + ((uint32_t)iy * row_pitch + (uint32_t)ix * cq)) : izp4;
-                }
-        }
-        uint4 wv[3][NV];
-#pragma unroll
-        for (int rr = 0; rr < 3; ++rr)
-#pragma unroll
-            for (int v = 0; v < NV; ++v)
-                wv[rr][v] = __ldg(w3p + ((size_t)ci * 3 + rr) * NV + v);
-        int acc[ROWS][2][4];
-#pragma unroll
-        for (int o = 0; o < ROWS; ++o)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                acc[o][0][j] = acc[o][1][j] = 0;
-#pragma unroll
-        for (int ir = 0; ir < IN_ROWS; ++ir) {
-            uint32_t ch[4];
-            transpose4x4(t[ir][0], t[ir][1], t[ir][2], t[ir][3], ch);
-#pragma unroll
-            for (int o = 0; o < ROWS; ++o) {
-                const int kr = ir - o * S;     // kernel row this input row meets in output row o
-                if (kr < 0 || kr > 2)
-                    continue;
-                const uint4 w0 = wv[kr][0], w1 = wv[kr][1];
-                acc[o][0][0] = dp4a_us(ch[0], w0.x, acc[o][0][0]); acc[o][0][1] = dp4a_us(ch[1], w0.y, acc[o][0][1]);
-                acc[o][0][2] = dp4a_us(ch[2], w0.z, acc[o][0][2]); acc[o][0][3] = dp4a_us(ch[3], w0.w, acc[o][0][3]);
-                acc[o][1][0] = dp4a_us(ch[0], w1.x, acc[o][1][0]); acc[o][1][1] = dp4a_us(ch[1], w1.y, acc[o][1][1]);
-                acc[o][1][2] = dp4a_us(ch[2], w1.z, acc[o][1][2]); acc[o][1][3] = dp4a_us(ch[3], w1.w, acc[o][1][3]);
-                if (S == 2) {
-                    const uint4 w2 = wv[kr][NV - 1];
-                    const uint32_t x4 = t[ir][IN_COLS - 1];
-                    acc[o][1][0] = dp4a_us(x4, w2.x, acc[o][1][0]); acc[o][1][1] = dp4a_us(x4, w2.y, acc[o][1][1]);
-                    acc[o][1][2] = dp4a_us(x4, w2.z, acc[o][1][2]); acc[o][1][3] = dp4a_us(x4, w2.w, acc[o][1][3]);
-                }
+            for (int ss = 0; ss < IN_COLS; ++ss) {
+                const int iy = iy0 + rr, ix = ix0 + ss;
+                t[rr][ss] = (iy >= 0 && iy < g.h && ix >= 0 && ix < g.w) ? at(x0 + rr * row_pitch + ss * col_pitch) : g.izp4;
             }
+    }
+    int acc[ROWS][2][4];
+#pragma unroll
+    for (int o = 0; o < ROWS; ++o)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            acc[o][p][0] = (int)start.x; acc[o][p][1] = (int)start.y; acc[o][p][2] = (int)start.z; acc[o][p][3] = (int)start.w;
         }
-        int q[ROWS][2][4];
+    const float m0 = __uint_as_float(mb.x), m1 = __uint_as_float(mb.y), m2 = __uint_as_float(mb.z), m3 = __uint_as_float(mb.w);
+    const uint32_t out_row = (uint32_t)g.ow * col_pitch;
+    const uint32_t out = ((img * (uint32_t)g.oh + (uint32_t)oy) * (uint32_t)g.ow + (uint32_t)ox) * col_pitch + ci * 4;
+    const bool second = ox + 1 < g.ow;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int4 c4 = __ldg(q3 + (size_t)ci * 4 + j);
-            const long long off = (long long)(((unsigned long long)(uint32_t)c4.y << 32) | (uint32_t)c4.x);
-#pragma unroll
-            for (int o = 0; o < ROWS; ++o)
-#pragma unroll
-                for (int p = 0; p < 2; ++p)
-                    q[o][p][j] = max((int)(((long long)acc[o][p][j] * c4.z + off) >> 32) >> c4.w, g.relu_lo);
-        }
+    for (int ir = 0; ir < IN_ROWS; ++ir) {
+        uint32_t ch[4];
+        transpose4x4(t[ir][0], t[ir][1], t[ir][2], t[ir][3], ch);
 #pragma unroll
         for (int o = 0; o < ROWS; ++o) {
-            if (oy + o >= g.oh)
-                break;
-            uint32_t *out = y + (((img * (uint32_t)g.oh + (uint32_t)(oy + o)) * (uint32_t)g.ow + (uint32_t)ox) * cq + ci);
-            out[0] = pack_sat_u8x4(q[o][0][0], q[o][0][1], q[o][0][2], q[o][0][3]);
-            if (ox + 1 < g.ow)
-                out[cq] = pack_sat_u8x4(q[o][1][0], q[o][1][1], q[o][1][2], q[o][1][3]);
+            const int kr = ir - o * S;     // kernel row this input row meets in output row o
+            if (kr < 0 || kr > 2)
+                continue;
+            const uint4 w0 = wv[kr][0], w1 = wv[kr][1];
+            acc[o][0][0] = dp4a_us(ch[0], w0.x, acc[o][0][0]); acc[o][0][1] = dp4a_us(ch[1], w0.y, acc[o][0][1]);
+            acc[o][0][2] = dp4a_us(ch[2], w0.z, acc[o][0][2]); acc[o][0][3] = dp4a_us(ch[3], w0.w, acc[o][0][3]);
+            acc[o][1][0] = dp4a_us(ch[0], w1.x, acc[o][1][0]); acc[o][1][1] = dp4a_us(ch[1], w1.y, acc[o][1][1]);
+            acc[o][1][2] = dp4a_us(ch[2], w1.z, acc[o][1][2]); acc[o][1][3] = dp4a_us(ch[3], w1.w, acc[o][1][3]);
+            if (S == 2) {
+                const uint4 w2 = wv[kr][NV - 1];
+                const uint32_t x4 = t[ir][IN_COLS - 1];
+                acc[o][1][0] = dp4a_us(x4, w2.x, acc[o][1][0]); acc[o][1][1] = dp4a_us(x4, w2.y, acc[o][1][1]);
+                acc[o][1][2] = dp4a_us(x4, w2.z, acc[o][1][2]); acc[o][1][3] = dp4a_us(x4, w2.w, acc[o][1][3]);
+            }
+            if (kr == 2 && (o == 0 || oy + o < g.oh)) {
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const uint32_t lo = clamp_s16x2(requant_pair(acc[o][p][0], acc[o][p][1], m0, m1, g.add), g.lo2);
+                    const uint32_t hi = clamp_s16x2(requant_pair(acc[o][p][2], acc[o][p][3], m2, m3, g.add), g.lo2);
+                    if (p == 0 || second)
+                        *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(y) + out + o * out_row + p * col_pitch) = __byte_perm(lo, hi, 0x6420);
+                }
+            }
         }
     }
 }
 
 template <int ROWS, int S>
-static int depthwise3x3_pair_launch(const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st)
+static int depthwise3x3_strip_launch(const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st)
 {
-    const size_t total = (size_t)n * ((g.oh + ROWS - 1) / ROWS) * ((g.ow + 1) / 2) * (g.c / 4);
+    DwArgs a;
+    a.c4 = g.c / 4; a.h = g.h; a.w = g.w; a.oh = g.oh; a.ow = g.ow; a.pad_h = g.pad_h; a.pad_w = g.pad_w;
+    const uint32_t pairs = (uint32_t)(g.ow + 1) / 2, strips = (uint32_t)(g.oh + ROWS - 1) / ROWS;
+    a.by_c4 = FastDiv((uint32_t)a.c4);
+    a.by_pairs = FastDiv(pairs);
+    a.by_strips = FastDiv(strips);
+    a.total = (uint32_t)n * strips * pairs * (uint32_t)a.c4;
+    a.izp4 = (uint32_t)g.izp * 0x01010101u;
+    a.add = (float)g.ozp + 0.5f;
+    a.lo2 = (uint32_t)(g.relu_lo > 0 ? g.relu_lo : 0) * 0x00010001u;
     return launch_kernel(
-        conv_depthwise3x3_pair_kernel<ROWS, S>, dim3(resident_grid<conv_depthwise3x3_pair_kernel<ROWS, S>, 256>((total + 255) / 256)), dim3(256), 0, st, (size_t)n * g.c * (g.h * g.w + g.oh * g.ow), 1,
-        g, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint4 *>(p.w_dw3p_dev), p.q_dw3_dev,
-        reinterpret_cast<uint32_t *>(y), n);
+        conv_depthwise3x3_strip_kernel<ROWS, S>, dim3((a.total + 127) / 128), dim3(128), 0, st, (size_t)n * g.c * (g.h * g.w + g.oh * g.ow), 1,
+        a, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint4 *>(p.w_dw3p_dev), reinterpret_cast<const uint4 *>(p.q_dw3p_dev),
+        reinterpret_cast<uint32_t *>(y));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -468,6 +515,59 @@ int conv_lower_rows_launch(const ConvGeom &g, const uint8_t *x, int n, uint8_t *
         (uint32_t)g.izp * 0x01010101u);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Channel padding ahead of the tensor-core path.  One thread builds 16 bytes (or the 4 of a pixel of four
+// channels) of one pixel; where a pixel is no whole number of words, they come out of two neighbouring
+// aligned words each, and only words that hold a valid byte are read.
+// ---------------------------------------------------------------------------------------------
+template <int WORDS>
+__global__ void __launch_bounds__(256) conv_pad_channels_kernel(
+    const uint8_t *__restrict__ x, uint32_t *__restrict__ y, int c, FastDiv by_vecs, uint32_t total, uint32_t fill4)
+{
+    const uint32_t idx = blockIdx.x * 256 + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    if (idx >= total)
+        return;
+    const uint32_t pix = by_vecs.div(idx), c0 = (idx - pix * by_vecs.d) * (WORDS * 4);
+    const uint8_t *src = x + (size_t)pix * c + c0;
+    const int valid = min(WORDS * 4, c - (int)c0);       // at least one: the padding is less than a vector
+    const int skew = (int)((uintptr_t)src & 3);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(src - skew);
+    uint32_t in[WORDS + 1];
+#pragma unroll
+    for (int i = 0; i <= WORDS; ++i)
+        in[i] = i * 4 < skew + valid ? __ldg(w + i) : 0;
+    uint32_t o[WORDS];
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        o[i] = __funnelshift_r(in[i], in[i + 1], 8 * skew);
+        const int left = valid - 4 * i;                 // bytes of this word that exist
+        if (left < 4) {
+            const uint32_t keep = left <= 0 ? 0u : 0xffffffffu >> (32 - 8 * left);
+            o[i] = (o[i] & keep) | (fill4 & ~keep);
+        }
+    }
+    if constexpr (WORDS == 4)
+        reinterpret_cast<uint4 *>(y)[idx] = make_uint4(o[0], o[1], o[2], o[3]);
+    else
+        y[idx] = o[0];
+}
+
+int conv_pad_channels_launch(const uint8_t *x, uint8_t *y, size_t pixels, int c, int c_pad, uint8_t fill, cudaStream_t st)
+{
+    const int vecs = c_pad == 4 ? 1 : c_pad / 16;
+    const size_t total = pixels * vecs;
+    if (total >= 0x7fffff00ull)
+        return fail(B200_ERR_UNSUPPORTED, "conv(pad): tensor too large");
+    const dim3 grid((unsigned)((total + 255) / 256));
+    const uint32_t fill4 = (uint32_t)fill * 0x01010101u;
+    const size_t bytes = pixels * (c + c_pad);
+    if (c_pad == 4)
+        return launch_kernel(conv_pad_channels_kernel<1>, grid, dim3(256), 0, st, bytes, 1, x, reinterpret_cast<uint32_t *>(y), c, FastDiv(vecs), (uint32_t)total, fill4);
+    return launch_kernel(conv_pad_channels_kernel<4>, grid, dim3(256), 0, st, bytes, 1, x, reinterpret_cast<uint32_t *>(y), c, FastDiv(vecs), (uint32_t)total, fill4);
+}
+
 int conv_direct_launch(
     const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, int32_t *acc_out,
     cudaStream_t st)
@@ -480,12 +580,24 @@ int conv_direct_launch(
     const bool depthwise = p.w_dw_dev && !acc_out && !g.act_signed && ((((uintptr_t)x | (uintptr_t)y) & 15) == 0);
     const bool dw3 = depthwise && p.w_dw3_dev && p.q_dw3_dev && npix * (size_t)(g.c / 4) < 0xffffffffull
         && (size_t)n * g.h * g.w * (size_t)(g.c / 4) < 0xffffffffull;
-    if (dw3 && p.w_dw3p_dev && (g.stride_w == 1 || g.stride_w == 2)) {
-        // two output rows per thread where the vertical stride equals the horizontal one
-        if (g.stride_w == 1 && g.stride_h == 1) return depthwise3x3_pair_launch<2, 1>(g, p, x, n, y, st);
-        if (g.stride_w == 1) return depthwise3x3_pair_launch<1, 1>(g, p, x, n, y, st);
-        if (g.stride_h == 2) return depthwise3x3_pair_launch<2, 2>(g, p, x, n, y, st);
-        return depthwise3x3_pair_launch<1, 2>(g, p, x, n, y, st);
+    if (dw3 && p.w_dw3p_dev && npix * (size_t)g.c < 0xffffff00ull && (size_t)n * g.h * g.w * g.c < 0xffffff00ull) {
+        // Rows per thread: as many as leave every SM about a thousand threads, of the heights that fit the map
+        // (144 channels of 56 x 56, batch 256: 80.6 us with 4 rows, 71.2 with 7, 60.3 with 14; 960 of 7 x 7: 10.3 with 7,
+        // 13.1 with 14; stride 2 to 28 x 28: 41.4 with 2, 34.4 with 4, 35.0 with 7).
+        const size_t per_row = (size_t)n * ((g.ow + 1) / 2) * (g.c / 4), few = (size_t)sm_count() * 1024;
+        auto strips = [&](int rows) { return (size_t)((g.oh + rows - 1) / rows); };
+        if (g.stride_w == 1) {
+            if (strips(14) * 14 * 7 <= strips(7) * 7 * 8 && per_row * strips(14) >= few)
+                return depthwise3x3_strip_launch<14, 1>(g, p, x, n, y, st);
+            if (per_row * strips(7) >= few)
+                return depthwise3x3_strip_launch<7, 1>(g, p, x, n, y, st);
+            return depthwise3x3_strip_launch<2, 1>(g, p, x, n, y, st);
+        }
+        if (g.oh <= 7 && per_row >= few)
+            return depthwise3x3_strip_launch<7, 2>(g, p, x, n, y, st);
+        if (per_row * strips(4) >= few)
+            return depthwise3x3_strip_launch<4, 2>(g, p, x, n, y, st);
+        return depthwise3x3_strip_launch<1, 2>(g, p, x, n, y, st);
     } else if (dw3) {
         const size_t total = npix * (g.c / 4);
         const int grid = resident_grid<conv_depthwise3x3_kernel, 256>((total + 255) / 256);

@@ -987,18 +987,25 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
                     }
                     store_pending = true;
                 } else {
-                    // plain stores for channel counts the TMA store cannot address (Cout % 16 != 0):
-                    // every thread copies the columns its warp computed for its pixel
+                    // plain stores for channel counts the TMA store cannot address (Cout % 16 != 0): pixel by pixel, the
+                    // lanes side by side along the channels the warp computed, by words where Cout allows
                     __syncwarp();
-                    if (pix_valid) {
-                        uint8_t *dst = g.y + (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
-                        const int nvalid = min(g.bn, g.cout - k0);
-                        for (int j = 0; j < nvalid; ++j) {
+                    const int nvalid = min(g.bn, g.cout - k0), unit = (g.cout & 3) == 0 ? 4 : 1;
+                    for (int pr = 0; pr < 32; ++pr) {
+                        if (!__shfl_sync(0xffffffffu, (int)pix_valid, pr))
+                            continue;
+                        const int prow = p0 + pr, psw = (prow >> sw_shift) & sw_mask;
+                        const int plw = prow & (g.tw - 1), plh = (prow >> g.tw_sh) & (g.th - 1), pln = prow >> (g.tw_sh + g.th_sh);
+                        uint8_t *dst = g.y + (((size_t)(n0 + pln) * g.oh + (oh0 + plh)) * g.ow + (ow0 + plw)) * g.cout + k0;
+                        for (int j = lane * unit; j < nvalid; j += 32 * unit) {
                             if (((j >> own_sh) & (wpq - 1)) != sub_warp)
                                 continue;
                             const int sub = j >> g.ob_sh, cin = j & (g.ob - 1);
-                            const int chunk = cin >> 4;
-                            dst[j] = s_out[(((size_t)sub * kTileM + row) << g.ob_sh) + ((chunk ^ sw) << 4) + (cin & 15)];
+                            const uint8_t *src = s_out + (((size_t)sub * kTileM + prow) << g.ob_sh) + (((cin >> 4) ^ psw) << 4) + (cin & 15);
+                            if (unit == 4)
+                                *reinterpret_cast<uint32_t *>(dst + j) = *reinterpret_cast<const uint32_t *>(src);
+                            else
+                                dst[j] = *src;
                         }
                     }
                     __syncwarp();

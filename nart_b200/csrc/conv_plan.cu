@@ -3,6 +3,8 @@
 // (art/modules/quant/src/op/conv_2d.c:95-147, conv_2d_uint8_impl.c:61-124 of ModelTC/NART) --
 // done once here: weights repacked for the kernels, per-channel (mult, shift) tables, folded
 // bias.  b200_conv2d_run then only launches.
+#include <cmath>
+#include <cstdlib>
 #include <string.h>
 
 #include <vector>
@@ -34,12 +36,14 @@ void destroy_conv(b200_conv *cv)
     cudaFree(cv->direct.w_dw3_dev);
     cudaFree(cv->direct.w_dw3p_dev);
     cudaFree(cv->direct.q_dw3_dev);
+    cudaFree(cv->direct.q_dw3p_dev);
     cudaFree(cv->direct.bias_fold_dev);
     cudaFree(cv->direct.mult_dev);
     cudaFree(cv->direct.shift_dev);
     if (cv->igemm)
         conv_igemm_destroy(cv->igemm);
     cudaFree(cv->scratch);
+    cudaFree(cv->padded);
     delete cv;
 }
 
@@ -184,8 +188,13 @@ int b200_conv2d_create(
             }
             rc = upload(w3, &cv->direct.w_dw3_dev);
             if (rc == B200_OK) rc = upload(q3, &cv->direct.q_dw3_dev);
-            if (rc == B200_OK && (g.stride_w == 1 || g.stride_w == 2)) {
-                // one kernel row against 3 + stride_w neighbouring input pixels (conv_depthwise3x3_pair_kernel)
+            // its fp32 requantize: every accumulator (9 products of at most 255 * 128) below 2^22, every result below 2^13
+            bool strip = g.stride_w == g.stride_h && (g.stride_w == 1 || g.stride_w == 2);
+            for (int k = 0; k < g.k; ++k)
+                strip = strip && std::abs((long long)bias_fold[k]) < (1 << 22) - 9 * 255 * 128
+                    && ldexp((std::abs((double)bias_fold[k]) + 9 * 255 * 128) * mult[k], -shift[k]) < 8000.0;
+            if (rc == B200_OK && strip) {
+                // one kernel row against 3 + stride_w neighbouring input pixels (conv_depthwise3x3_strip_kernel)
                 const int nv = g.stride_w == 2 ? 3 : 2;
                 std::vector<uint32_t> w3p((size_t)(g.c / 4) * 3 * nv * 4, 0);
                 for (int c = 0; c < g.c; ++c)
@@ -203,6 +212,13 @@ int b200_conv2d_create(
                         }
                     }
                 rc = upload(w3p, &cv->direct.w_dw3p_dev);
+                std::vector<uint32_t> qf((size_t)g.c * 2);
+                for (int c = 0; c < g.c; ++c) {
+                    const float m = ldexpf((float)mult[c], -shift[c]);      // exact: mult has 24 significant bits
+                    qf[(size_t)(c / 4) * 8 + c % 4] = 0x4B400000u + (uint32_t)bias_fold[c];
+                    memcpy(&qf[(size_t)(c / 4) * 8 + 4 + c % 4], &m, 4);
+                }
+                if (rc == B200_OK) rc = upload(qf, &cv->direct.q_dw3p_dev);
             }
         }
     }
@@ -214,16 +230,42 @@ int b200_conv2d_create(
     // ---- tensor-core plan ---------------------------------------------------------------------
     char why[256] = "";
     const bool ig_ok = conv_igemm_supported(g, why, sizeof(why)) != 0 && !g.s8_wrap;
+    // Channel counts that are no multiple of 16 (the pixel stride of a TMA map) run on a copy padded to one, or to
+    // the four channels of the row lowering below: the copy costs a pass over the input, the CUDA-core kernel
+    // twenty (1x1 24 -> 144 channels on 56 x 56, batch 32: 129 us against 9).  Padding channels have zero weights and
+    // hold the byte izp, so that their (x - izp) is zero in the window sums of a weight zero point as well.
+    ConvGeom gt = g;                        // what the tensor cores see
+    const std::vector<int8_t> *wt = &w_s8;
+    std::vector<int8_t> w_pad;
+    auto can_lower = [](const ConvGeom &q) {
+        return q.group == 1 && q.c == 4 && q.s <= kLowerWindow && q.k >= 16 && q.stride_h <= 2 && q.h >= q.stride_h && !q.act_signed;
+    };
+    bool tc_ok = ig_ok;
+    if (!ig_ok && !can_lower(g) && g.group == 1 && g.c % 16 != 0 && !g.s8_wrap && p->algo == B200_CONV_ALGO_AUTO) {
+        gt.c = 4;
+        if (g.c >= 4 || !can_lower(gt))
+            gt.c = (g.c + 15) / 16 * 16;
+        if (gt.c != 4)
+            tc_ok = conv_igemm_supported(gt, why, sizeof(why)) != 0;
+        if (gt.c == 4 || tc_ok) {
+            cv->pad_c = gt.c;
+            cv->g_pad = gt;
+            w_pad.assign((size_t)g.k * gt.c * taps, 0);
+            for (int k = 0; k < g.k; ++k)
+                memcpy(&w_pad[(size_t)k * gt.c * taps], &w_s8[(size_t)k * g.c * taps], (size_t)g.c * taps);
+            wt = &w_pad;
+        }
+    }
     // A 4-channel image with a short kernel row is no contraction the tensor cores can take as it
     // is (4 bytes per tap).  Gathering, for every input row and output column, the 8-pixel window
     // the kernel row slides over gives a 32-channel tensor [n][h][ow][8 pixels x 4 channels] on
     // which the same conv is an r x 1 kernel with stride (stride_h, 1): that is dense enough.
     // Window cells outside the image hold the byte izp, whose contribution the epilogue's
     // zero-point term removes exactly; cells past the kernel width get zero weights.
-    const bool low_ok = g.group == 1 && g.c == 4 && g.s <= kLowerWindow && g.k >= 16 && g.stride_h <= 2
-        && g.h >= g.stride_h && !g.act_signed;
-    if (!ig_ok && low_ok && p->algo != B200_CONV_ALGO_DIRECT) {
-        ConvGeom gl = g;
+    rc = B200_ERR_UNSUPPORTED;
+    if (p->algo == B200_CONV_ALGO_DIRECT) {
+    } else if (!tc_ok && can_lower(gt)) {
+        ConvGeom gl = gt;
         gl.c = kLowerWindow * 4;
         gl.w = g.ow;
         gl.s = 1;
@@ -234,10 +276,9 @@ int b200_conv2d_create(
             for (int c = 0; c < 4; ++c)
                 for (int rr = 0; rr < g.r; ++rr)
                     for (int j = 0; j < g.s; ++j)
-                        w_low[((size_t)k * gl.c + j * 4 + c) * g.r + rr] = w_s8[(((size_t)k * 4 + c) * g.r + rr) * g.s + j];
+                        w_low[((size_t)k * gl.c + j * 4 + c) * g.r + rr] = (*wt)[(((size_t)k * 4 + c) * g.r + rr) * g.s + j];
         rc = conv_igemm_create(gl, w_low, bias, mult.data(), shift.data(), &cv->igemm, true, g.s);
         if (rc == B200_OK) {
-            cv->algo = B200_CONV_ALGO_IGEMM;
             cv->lowered = true;
             cv->g_low = gl;
             // for callers of b200_conv2d_run_static_scratch: everything that entry point would otherwise do
@@ -245,19 +286,17 @@ int b200_conv2d_create(
             // allowed; a failure only matters to that entry point, which reports it itself
             if (conv_igemm_warm() != B200_OK || conv_static_scratch_prepare() != B200_OK)
                 cudaGetLastError();
-        } else if (rc != B200_ERR_UNSUPPORTED || p->algo == B200_CONV_ALGO_IGEMM) {
-            destroy_conv(cv);
-            return rc;
         }
-    } else if (p->algo == B200_CONV_ALGO_IGEMM && !ig_ok) {
-        destroy_conv(cv);
-        return fail(B200_ERR_UNSUPPORTED, "conv: implicit-GEMM path declined: %s", why);
+    } else if (tc_ok) {
+        rc = conv_igemm_create(gt, *wt, bias, mult.data(), shift.data(), &cv->igemm);
+    } else if (p->algo == B200_CONV_ALGO_IGEMM) {
+        rc = fail(B200_ERR_UNSUPPORTED, "conv: implicit-GEMM path declined: %s", why);
     }
-    if (ig_ok && p->algo != B200_CONV_ALGO_DIRECT) {
-        rc = conv_igemm_create(g, w_s8, bias, mult.data(), shift.data(), &cv->igemm);
-        if (rc == B200_OK) {
-            cv->algo = B200_CONV_ALGO_IGEMM;
-        } else if (rc != B200_ERR_UNSUPPORTED || p->algo == B200_CONV_ALGO_IGEMM) {
+    if (rc == B200_OK) {
+        cv->algo = B200_CONV_ALGO_IGEMM;
+    } else {
+        cv->pad_c = 0;
+        if (rc != B200_ERR_UNSUPPORTED || p->algo == B200_CONV_ALGO_IGEMM) {
             destroy_conv(cv);
             return rc;
         }   // declined under AUTO: the CUDA-core kernel runs it
@@ -318,6 +357,10 @@ int b200_conv2d_describe(const b200_conv_t *conv, char *buf, size_t len)
             size_t used = strlen(buf);
             snprintf(buf + used, len - used, ", on the row-lowered image");
         }
+        if (conv->pad_c) {
+            size_t used = strlen(buf);
+            snprintf(buf + used, len - used, ", channels padded to %d", conv->pad_c);
+        }
     } else {
         snprintf(buf, len, "CUDA cores (dp4a)%s", conv->g.group == conv->g.c && conv->g.group == conv->g.k ? ", depthwise" : "");
     }
@@ -333,7 +376,11 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
     if (conv->fused_residual)
         return fail(B200_ERR_INVALID, "conv: this plan has a residual add, run it with b200_conv2d_run_residual");
     B200_TRY(b200_conv2d_reserve(conv, n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
-    const ConvGeom &g = conv->g;
+    const ConvGeom &g = conv->pad_c ? conv->g_pad : conv->g;
+    if (conv->pad_c) {
+        B200_TRY(conv_pad_channels_launch(x, conv->padded, (size_t)n * g.h * g.w, conv->g.c, conv->pad_c, (uint8_t)g.izp, as_stream(stream)));
+        x = conv->padded;
+    }
     if (conv->lowered) {
         B200_TRY(conv_lower_rows_launch(g, x, n, conv->scratch, as_stream(stream)));
         return conv_igemm_launch(conv->igemm, conv->scratch, n, y, as_stream(stream));
@@ -348,16 +395,20 @@ int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
     if (!conv || n < 0)
         return fail(B200_ERR_INVALID, "conv(reserve): bad argument");
     const ConvGeom &g = conv->g;
-    if (conv->lowered) {
-        const size_t need = (size_t)n * g.h * g.ow * (kLowerWindow * 4);
-        if (need > conv->scratch_bytes) {
-            B200_CUDA_TRY(cudaFree(conv->scratch));
-            conv->scratch = nullptr;
-            conv->scratch_bytes = 0;
-            B200_TRY(b200_malloc((void **)&conv->scratch, need));
-            conv->scratch_bytes = need;
-        }
-    }
+    auto grow = [](uint8_t *&buf, size_t &have, size_t need) -> int {
+        if (need <= have)
+            return B200_OK;
+        B200_CUDA_TRY(cudaFree(buf));
+        buf = nullptr;
+        have = 0;
+        B200_TRY(b200_malloc((void **)&buf, need));
+        have = need;
+        return B200_OK;
+    };
+    if (conv->lowered)
+        B200_TRY(grow(conv->scratch, conv->scratch_bytes, (size_t)n * g.h * g.ow * (kLowerWindow * 4)));
+    if (conv->pad_c)
+        B200_TRY(grow(conv->padded, conv->padded_bytes, (size_t)n * g.h * g.w * conv->pad_c));
     return B200_OK;
 }
 
@@ -367,7 +418,7 @@ int b200_conv2d_fuse_residual_add(
 {
     if (!conv || !ialpha || !izp || conv_input < 0 || conv_input > 1)
         return fail(B200_ERR_INVALID, "conv(fuse): bad argument");
-    if (conv->algo != B200_CONV_ALGO_IGEMM || conv->lowered || !conv->igemm)
+    if (conv->algo != B200_CONV_ALGO_IGEMM || conv->lowered || conv->pad_c || !conv->igemm)
         return fail(B200_ERR_UNSUPPORTED, "conv(fuse): only plans on the tensor-core path take a residual add");
     if (conv->g.wzp_d != 0)
         return fail(B200_ERR_UNSUPPORTED, "conv(fuse): a weight zero point other than 128 and a fused residual add do not combine");

@@ -87,6 +87,11 @@ __device__ __forceinline__ void store_channels(const int (&acc)[N], const SmallA
             *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
         else
             *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
+    } else if ((g.cout & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < N / 4; ++q)
+            if (k + 4 * q < g.cout)
+                reinterpret_cast<uint32_t *>(dst)[q] = w[q];
     } else {
 #pragma unroll
         for (int i = 0; i < N; ++i)

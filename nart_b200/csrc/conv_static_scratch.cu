@@ -81,7 +81,7 @@ extern "C" int b200_conv2d_run_static_scratch(
     using namespace b200;
     if (!conv || n < 0 || (n > 0 && (!x || !y)))
         return fail(B200_ERR_INVALID, "conv(static scratch): bad argument");
-    if (!conv->lowered)
+    if (!conv->lowered || conv->pad_c)
         return fail(
             B200_ERR_INVALID,
             "conv(static scratch): this plan uses no scratch tensor (only row-lowered 4-channel convs do); "

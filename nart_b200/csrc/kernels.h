@@ -93,9 +93,11 @@ struct ConvDirectPlan {
     // {folded 64-bit addend, mult, shift - 32}
     uint32_t *w_dw3_dev = nullptr;
     int4 *q_dw3_dev = nullptr;
-    // the same for two output pixels side by side (stride_w 1 or 2), see conv_depthwise3x3_pair_kernel:
-    // [c/4][3 kernel rows][2 or 3][4 channels] words of one kernel row against 3 + stride_w input pixels
+    // the same for two output pixels side by side (stride 1 or 2 both ways), see conv_depthwise3x3_strip_kernel:
+    // [c/4][3 kernel rows][2 or 3][4 channels] words of one kernel row against 3 + stride_w input pixels, and
+    // [c/4] of four accumulator start values and four fp32 multipliers
     uint32_t *w_dw3p_dev = nullptr;
+    uint32_t *q_dw3p_dev = nullptr;
     int32_t *bias_fold_dev = nullptr;
     uint32_t *mult_dev = nullptr;
     int32_t *shift_dev = nullptr;
@@ -112,6 +114,9 @@ int conv_direct_launch(
 // rows of pixels with wide unswizzled copies (see conv_igemm_create, a_row_swizzled).
 constexpr int kLowerWindow = 8;
 int conv_lower_rows_launch(const ConvGeom &g, const uint8_t *x, int n, uint8_t *out, cudaStream_t st);
+
+// NHWC tensor of `pixels` x c bytes into one of c_pad channels (4 or a multiple of 16), the rest `fill`.
+int conv_pad_channels_launch(const uint8_t *x, uint8_t *y, size_t pixels, int c, int c_pad, uint8_t fill, cudaStream_t st);
 
 // Implicit-GEMM (tcgen05) convolution plan; defined in conv_igemm_sm100.cu.
 struct ConvIgemmPlan;
@@ -168,6 +173,12 @@ struct b200_conv {
     b200::ConvGeom g_low;
     uint8_t *scratch = nullptr;     // [n][h][ow][32]
     size_t scratch_bytes = 0;
+    // Channel counts the tensor-core path does not take (no multiple of 16): every run copies the activations into
+    // a scratch tensor of pad_c channels, and the igemm plan (g_pad, or g_low on it) has zero weights there.
+    int pad_c = 0;
+    b200::ConvGeom g_pad;
+    uint8_t *padded = nullptr;      // [n][h][w][pad_c]
+    size_t padded_bytes = 0;
     float oalpha = 0.f;             // output scale, kept for b200_conv2d_fuse_residual_add
     bool fused_residual = false;    // the plan computes eltwise_sum(conv(x), res)
 };

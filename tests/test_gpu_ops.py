@@ -336,6 +336,58 @@ def test_depthwise3x3_two_pixels_per_thread(ops, port, c, h, w, sh, sw, pd):
     assert len(np.unique(want)) > 16
 
 
+@pytest.mark.parametrize("c,h,w,st", [(64, 29, 15, 1), (48, 14, 33, 1), (96, 7, 9, 1), (64, 15, 16, 1), (64, 31, 30, 2), (96, 14, 13, 2)])
+def test_depthwise3x3_long_strips(ops, port, c, h, w, st):
+    """Launches large enough for threads that own 14, 7 or 4 output rows: heights that fill their last strip and not."""
+    n = 148 * 1024 * 14 // (c // 4 * ((w // st + 1) // 2) * 7) + 1
+    rng = np.random.default_rng(c + h)
+    x = rng.integers(0, 256, (n, c, h, w), dtype=np.uint8)
+    wt = (rng.integers(-127, 128, (c, 1, 3, 3)) + 128).astype(np.uint8)
+    bias = rng.integers(-4096, 4097, c).astype(np.int32)
+    q = dict(ialpha=0.04, izp=77, walpha=rng.uniform(0.001, 0.01, c).astype(np.float32), wzp=128, oalpha=0.12, ozp=90)
+    pick = [0, n // 2, n - 1]
+    for relu in (False, True):
+        conv = ops.Conv2d(wt, bias, in_hw=(h, w), stride=(st, st), pad=(1, 1), group=c, relu=relu, **q)
+        want = port.conv2d_u8(x[pick], wt, bias, (st, st), (1, 1), c, relu=relu, **q)
+        assert_same(to_host_nchw(conv(to_dev_nhwc(x)))[pick], want, "c=%d %dx%d relu=%d" % (c, h, w, relu))
+
+
+# (n, c, k, h, w, kernel, stride, wzp, signed): launches below and above one tile per SM (the one-tile kernel with and
+# without split sums, the persistent one), channel counts that are padded to the tensor cores' 16 or 4 and output
+# counts no TMA store takes, window sums beside both
+TILING_SHAPES = [(1, 512, 512, 7, 7, 3, 1, 128, False), (1, 256, 64, 14, 13, 3, 2, 90, False), (2, 2048, 1000, 1, 1, 1, 1, 128, False),
+                 (1, 1024, 256, 5, 6, 1, 1, 140, False), (3, 64, 40, 30, 31, 3, 1, 128, True), (40, 64, 272, 30, 31, 1, 1, 101, False),
+                 (50, 128, 256, 28, 29, 1, 1, 101, False), (40, 32, 64, 33, 30, 3, 1, 128, True), (40, 24, 100, 30, 31, 1, 1, 128, False),
+                 (2, 24, 100, 9, 8, 3, 1, 77, False), (40, 20, 18, 30, 31, 3, 1, 131, False), (2, 7, 33, 12, 11, 3, 2, 128, True),
+                 (2, 3, 32, 33, 35, 7, 2, 60, False), (30, 3, 24, 40, 41, 3, 2, 128, False), (1, 1, 16, 9, 9, 3, 1, 128, False)]
+
+
+@pytest.mark.parametrize("n,c,k,h,w,ks,st,wzp,signed", TILING_SHAPES)
+def test_conv_tilings_and_ragged_channels(ops, port, n, c, k, h, w, ks, st, wzp, signed):
+    rng = np.random.default_rng(c + 3 * k + n)
+    pick = [0, n // 2, n - 1] if n > 3 else list(range(n))
+    bias = rng.integers(-4096, 4097, k).astype(np.int32)
+    walpha = rng.uniform(0.001, 0.01, k).astype(np.float32)
+    oalpha = float(np.float32(0.02 * 74 * 0.0055 * 73 * np.sqrt(c * ks * ks) / (20 if signed else 45)))
+    pad = ks // 2
+    if signed:
+        x = rng.integers(-127, 128, (n, c, h, w)).astype(np.int8)
+        wt = rng.integers(-127, 128, (k, c, ks, ks)).astype(np.int8)
+        want = port.conv2d_i8(x[pick], wt, bias, (st, st), (pad, pad), 1, 0.02, walpha, oalpha, 7)
+        q = dict(ialpha=0.02, walpha=walpha, oalpha=oalpha, obits=7)
+    else:
+        x = rng.integers(0, 256, (n, c, h, w), dtype=np.uint8)
+        wt = rng.integers(0, 256, (k, c, ks, ks), dtype=np.uint8)
+        q = dict(ialpha=0.02, izp=117, wzp=wzp, walpha=walpha, oalpha=oalpha, ozp=99)
+        want = port.conv2d_u8(x[pick], wt, bias, (st, st), (pad, pad), 1, relu=True, **q)
+    conv = ops.Conv2d(wt, bias, in_hw=(h, w), stride=(st, st), pad=(pad, pad), relu=not signed, signed=signed, **q)
+    assert conv.algo == ops.ALGO_IGEMM
+    assert len(np.unique(want)) > 16
+    got = to_host_nchw(conv(to_dev_nhwc(x)))
+    assert ops.device_status() == 0
+    assert_same(got[pick], want, conv.describe())
+
+
 # (c, k, kernel, stride, pad, group, h, w, algo name): every kernel that forms products
 WZP_SHAPES = [(64, 64, 3, 1, 1, 1, 13, 11, "igemm"), (32, 48, 1, 1, 0, 1, 9, 9, "igemm"), (128, 32, 3, 2, 1, 1, 12, 12, "igemm"),
               (256, 272, 1, 1, 0, 1, 7, 7, "igemm"), (4, 64, 7, 2, 3, 1, 30, 34, "igemm"), (64, 64, 3, 1, 1, 1, 13, 11, "direct"),
