@@ -1,0 +1,957 @@
+// Implicit-GEMM int8 convolution on the 5th-generation tensor cores (sm_100a):
+//   D[pixels, Cout] (int32, TMEM) += A[pixels, R*S*C] (uint8 activations) x B[Cout, R*S*C]^T (int8)
+// with tcgen05.mma kind::i8, operands staged by TMA into swizzled shared memory, accumulators in
+// tensor memory, and the reference's zero-point correction, bias, requantize and ReLU clamp
+// fused into the epilogue (art/modules/quant/src/op/conv_2d_uint8_impl.c:107-164 of ModelTC/NART).
+//
+// GEMM view.  An M tile is 128 output pixels arranged as a TW x TH x TN box of
+// (ow, oh, image); for filter tap (r, s) and a BK-channel slice the A operand is the box of input
+// pixels one tiled TMA load fetches from the NHWC tensor (coordinates may run outside the image:
+// TMA fills zeros).  Strided convs address the input through one tensor map per (row, column)
+// parity so that every load stays a plain dense box.  B is the weight matrix repacked once to
+// [Cout][R][S][C] int8.  K is walked tap by tap, BK channels at a time.
+//
+// Zero point.  The MMA multiplies the raw uint8 activation, and TMA pads with the byte 0, whereas
+// the reference pads with the real value 0, i.e. the byte izp.  With
+//   raw = sum_{valid taps} x * w      true = sum_{valid taps} (x - izp) * w = raw - izp * sum_{valid} w
+// the correction depends only on which taps are inside the image, i.e. on the output pixel's
+// border class.  The host builds off[class][k] = bias[k] - izp * sum_{taps valid in class} w[k].
+//
+// Warp roles (576 threads, one CTA per SM, persistent over tiles):
+//   warp 0      TMA producer (one lane per pipeline slot)
+//   warp 1      tensor-memory allocation, MMA issue (one elected lane)
+//   warps 2..17 epilogue, two groups of 8 warps (two per tensor-memory lane quarter) or, for narrow
+//               channel tiles with a short mainloop, four groups of 4 warps; group i
+//               owns accumulator stage i: tcgen05.ld -> requantize -> pack -> swizzled smem -> TMA store
+//   warp 18     a second MMA-issuing warp in the instantiations for narrow tiles (MODE 1, 2)
+// One accumulator stage per group in tensor memory lets the epilogue of tile i overlap the mainloop
+// of the next tiles and their epilogues (the other groups).  MODE 3 runs on clusters of two CTAs that
+// share every MMA (tcgen05 cta_group::2, M = 256), each CTA loading its own operands with plain TMA
+// loads; the other instantiations launch without clusters.  No load is multicast.  Every wait is bounded:
+// when one runs out the kernel records a code in the status word, all roles leave their loops,
+// tensor memory is freed and the kernel returns.
+#pragma once
+
+#include <cuda.h>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "sm100_ptx.cuh"
+
+namespace b200 {
+
+constexpr int kMaxAccStages = 4;              // accumulator stages in tensor memory = epilogue groups: 2 or 4
+#ifndef B200_EPI_WARPS
+#define B200_EPI_WARPS 16
+#endif
+constexpr int kEpiWarps = B200_EPI_WARPS;     // split into 2 groups of 8 warps or 4 groups of 4
+constexpr int kMma2Warp = 2 + kEpiWarps;        // the second MMA-issuing warp, behind the epilogue warps
+constexpr int kThreads = 64 + kEpiWarps * 32;
+constexpr int kThreads2 = kThreads + 32;         // with the second MMA-issuing warp
+constexpr int kTileM = 128;
+constexpr int kMaxStages = 8;
+constexpr int kGroupBytes = 32 * 1024;        // target size of one pipeline stage (a group of k-blocks)
+constexpr int kMaxGroup = 10;                 // three stages of a group must fit the producer's 32 lanes
+
+// device status codes (which wait gave up)
+constexpr int kErrProducerWait = 0x101;
+constexpr int kErrMmaFullWait = 0x102;
+constexpr int kErrMmaTmemWait = 0x103;
+constexpr int kErrEpilogueWait = 0x104;
+
+struct alignas(64) IgemmMaps {
+    CUtensorMap a[4];   // activations, one per (row parity, column parity) of a strided conv
+    CUtensorMap b;      // weights [Cout][R*S*C]
+    CUtensorMap y[2];   // output NHWC, one per column segment of the staging buffer
+    CUtensorMap ones;   // 16 rows, the first all ones (HAS_WZP)
+};
+
+struct IgemmArgs {
+    // problem
+    int n, oh, ow, cout;
+    int r, s, pad_h, pad_w, stride_h, stride_w;
+    int c;               // input channels, rounded up to a multiple of 32: the weights' pitch per tap
+    int cchunks;         // k-blocks per tap
+    int last_steps;      // 32-byte steps of a tap's last k-block that hold channels (the rest of its box is padding)
+    // tiling
+    int tw, th, tn;      // M-tile box (ow, oh, image), tw*th*tn == 128, each a power of two
+    int tw_sh, th_sh;    // log2(tw), log2(th)
+    int tiles_w, tiles_h, tiles_n, n_tiles_n;   // tile counts along ow, oh, image and Cout
+    int step_nt, step_w, step_h, step_n;        // mixed-radix digits of the grid size (see TileWalker)
+    int bk;              // channels per k-block (32, 64, 128) == swizzle span of the operands
+    int bn;              // output channels per tile (multiple of 16, <= 256)
+    int stages;          // smem pipeline depth
+    int groups;          // epilogue groups (2 or 4); group i takes every groups-th tile of the CTA
+    int acc_stages;      // accumulator stages in tensor memory (a multiple of groups, at most 4)
+    int kgroup;          // k-blocks per pipeline stage (divides the k-blocks of a tile): one barrier round trip per group
+    uint32_t rcp_cchunks, rcp_s;   // ceil(2^30 / (c / bk)), ceil(2^30 / s): k-block index -> tap, tap -> row
+    int b_resident;      // 1: all k-blocks of B stay in shared memory (one channel tile, weights fit)
+    int a_wide;          // 1: 32-channel rows stored pre-swizzled; A is fetched as whole rows of pixels
+    int seg_w[2];        // column segments of a tile: widths in bytes (the second may be 0), see epilogue_segments
+    uint32_t idesc;      // tcgen05 instruction descriptor
+    uint32_t tmem_cols;  // columns to allocate (power of two >= 2*bn)
+    // epilogue (see EpiForm)
+    const int32_t *off32;    // [n_cls][kpad] accumulator offsets (form kEpiFp: plus the bits of 1.5 * 2^23)
+    const int32_t *mul;      // [kpad] fp32 bits, uniform-shift multiplier or multiplier, by form
+    const int32_t *shift;    // [kpad] (form kEpiGeneric)
+    const uint8_t *row_cls;  // [oh]
+    const uint8_t *col_cls;  // [ow]
+    int n_col_cls, n_cls, kpad;
+    int ozp, qmax, relu_lo;
+    uint32_t out_flip;       // 0x80808080 for int8 outputs, else 0
+    int ushift, rnd_hi;      // form kEpiInt: S - 32; high word of 2^(S-1) + (ozp << S) (the low one is 0)
+    int use_tma_store;       // 0: plain stores (Cout not a multiple of 16)
+    uint8_t *y;
+    int *status;
+    // fused residual add (eltwise SUM of this conv's output and `res`, see EltwiseArgs): index 0 is
+    // the conv's own output, index 1 the residual tensor (NHWC, the dims of y); res == nullptr: off
+    const uint8_t *res;
+    int r_m[2], r_add[2], r_b[2];
+    int r_s0, r_ozp, r_lo;
+    // weight zero point other than 128 (HAS_WZP): acc -= wzp_d * sum of x over the pixel's window before the
+    // requantize; the MMA forms that sum in a 17th..32nd column behind the tile's channels (weight row of ones)
+    int wzp_d;
+    // 1: the M tiles are visited from the last image / row / column tile down to the first, so that a layer
+    // starts on the part of its input that the layer before wrote last (and that still sits in L2)
+    int rev;
+    // Read-only bytes the launch after this one starts on (the next layer's repacked weights): every CTA asks
+    // for its slice to be brought into L2 while this layer runs, so that the next launch's first weight loads
+    // do not all miss at once.  nullptr / 0: none.
+    const uint8_t *next_ro;
+    uint32_t next_ro_bytes;
+    // CTA pair (MODE 3): two CTAs of a cluster share every MMA (tcgen05 cta_group::2, M = 256): CTA r of the
+    // pair owns M tile 2 * pm + r of pair tile pm and loads that tile's activations and half r of the
+    // weight tile; the pair tiles are walked as (nt fastest, pm) with the digits step_nt, step_pm of the
+    // number of clusters.
+    int pm_tiles;            // pair tiles along M: ceil(m_tiles / 2)
+    int step_pm;
+};
+
+// How accumulators become output bytes.  For the reference's  y = sat(rshift_rn((acc + off) * mult, shift) + ozp)
+//   kEpiFp       floor((acc + off) * m + 1/2) + ozp with m = mult * 2^-shift, exactly, in fp32 (off32 carries the bits of
+//                1.5 * 2^23, so that one integer add makes the float; see conv_depthwise3x3_strip_kernel for the rest).
+//                For layers whose accumulators stay below 2^22 whatever the input: reductions of a few hundred bytes, where
+//                the epilogue sets the pace.  Two values per fp32 instruction.
+//   kEpiInt      every channel's shift brought to the layer's smallest one, S, by dropping low zero bits of its
+//                multiplier (an fp32 scale leaves at least 7): ((acc + off) * mult_u + 2^(S-1) + (ozp << S)) >> S
+//   kEpiGeneric  64-bit shifts per channel, for shifts below 33 and layers no single shift serves
+// The constants of a tile's channels sit in shared memory, two per channel, read four at a time; the offsets of
+// layers with several border classes are read through L1 from the class's row.
+// (64 -> 256 channels 1x1 on 56 x 56, batch 256: 95.3 us with the two integer constants as kernel parameters, 78.4 fp32;
+// 128 -> 512 on 28 x 28: 54.7 us with a 64-bit addend and a shift per channel in shared memory, 41.1 fp32.)
+enum EpiForm { kEpiFp, kEpiInt, kEpiGeneric };
+// One kernel per form and kind of offsets and clamp: side by side in one kernel they spill (96 registers a thread).
+//   One / Many  one border class (offsets in shared memory) or several
+//   Full        floor, ceiling below 255 and output flip; else the floor relu_lo and the pack's own ceiling
+enum EpiVariant { kEpiFpOne, kEpiFpOneFull, kEpiFpMany, kEpiFpManyFull, kEpiIntOne, kEpiIntOneFull, kEpiIntMany, kEpiIntManyFull, kEpiAny, kEpiVariants };
+
+// Tile index -> (Cout tile, ow tile, oh tile, image tile), Cout tile fastest.  A persistent CTA
+// visits tiles blockIdx.x, blockIdx.x + gridDim.x, ...: the digits advance by the mixed-radix
+// digits of gridDim.x (computed on the host) with carries, so no role divides inside its loop.
+struct TileWalker {
+    int nt, twi, thi, tni;
+    int pm = 0, rank = -1;   // CTA-pair mode (rank >= 0): pair tile index along M and this CTA's rank in its pair
+    __device__ __forceinline__ void decode_pair(const IgemmArgs &g)
+    {
+        int mt = 2 * pm + rank;          // an M tile past the last one decodes to an image index past the batch
+        twi = mt % g.tiles_w;
+        mt /= g.tiles_w;
+        thi = mt % g.tiles_h;
+        tni = mt / g.tiles_h;
+    }
+    __device__ __forceinline__ void init_pair(const IgemmArgs &g, int pair_tile, int cta_rank)
+    {
+        rank = cta_rank;
+        nt = pair_tile % g.n_tiles_n;
+        pm = pair_tile / g.n_tiles_n;
+        decode_pair(g);
+    }
+    __device__ __forceinline__ void init(const IgemmArgs &g, int tile)
+    {
+        nt = tile % g.n_tiles_n;
+        int mt = tile / g.n_tiles_n;
+        twi = mt % g.tiles_w;
+        mt /= g.tiles_w;
+        thi = mt % g.tiles_h;
+        tni = mt / g.tiles_h;
+    }
+    __device__ __forceinline__ void advance(const IgemmArgs &g)
+    {
+        if (rank >= 0) {
+            nt += g.step_nt;
+            int carry = 0;
+            if (nt >= g.n_tiles_n) { nt -= g.n_tiles_n; carry = 1; }
+            pm += g.step_pm + carry;
+            decode_pair(g);
+            return;
+        }
+        nt += g.step_nt;
+        int carry = 0;
+        if (nt >= g.n_tiles_n) { nt -= g.n_tiles_n; carry = 1; }
+        twi += g.step_w + carry;
+        carry = 0;
+        if (twi >= g.tiles_w) { twi -= g.tiles_w; carry = 1; }
+        thi += g.step_h + carry;
+        carry = 0;
+        if (thi >= g.tiles_h) { thi -= g.tiles_h; carry = 1; }
+        tni += g.step_n + carry;
+    }
+    // tile coordinates as the roles use them (reversed traversal mirrors every M digit)
+    __device__ __forceinline__ int wi(const IgemmArgs &g) const { return g.rev ? g.tiles_w - 1 - twi : twi; }
+    __device__ __forceinline__ int hi(const IgemmArgs &g) const { return g.rev ? g.tiles_h - 1 - thi : thi; }
+    // (an M tile past the end -- the odd tail of a CTA pair -- keeps its out-of-range image index)
+    __device__ __forceinline__ int ni(const IgemmArgs &g) const { return (g.rev && tni < g.tiles_n) ? g.tiles_n - 1 - tni : tni; }
+};
+
+// Named barriers of one epilogue group (ids 1 + 2g and 2 + 2g for group g).
+__device__ __forceinline__ void epi_bar_sync(int group, int group_threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + 2 * group), "r"(group_threads) : "memory");
+}
+// AND-reduction of a predicate over the threads of one epilogue group: every thread gets
+// the same answer, so all of them leave the tile loop together.
+__device__ __forceinline__ bool epi_bar_all(int group, int group_threads, bool pred)
+{
+    uint32_t out;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, %3, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(out)
+        : "r"((uint32_t)pred), "r"(group_threads), "r"(2 + 2 * group)
+        : "memory");
+    return out != 0;
+}
+
+// ---- epilogue arithmetic ------------------------------------------------------------------------
+struct EpiConsts {
+    int ozp, qmax, relu_lo, ushift, rnd_hi;
+    float add;                 // ozp + 1/2
+    uint32_t out_flip;
+    int r_m0, r_add0, r_b0, r_m1, r_add1, r_b1, r_s0, r_ozp, r_lo;   // fused residual add
+};
+
+constexpr int kFpMagic = 0x4B400000;    // bits of 1.5 * 2^23
+constexpr int kFpOne = 0x4B000000;      // bits of 2^23
+
+// The bits of 2^23 + floor(((a0, a1) - 1.5 * 2^23) * (m0, m1) + add)
+__device__ __forceinline__ void fp_requant_pair(int a0, int a1, int m0, int m1, float add, int &q0, int &q1)
+{
+    asm("{\n\t.reg .b64 a, m, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 c, {%6, %6};\n\t"
+        "add.rn.f32x2 a, a, c;\n\t"
+        "mov.b64 m, {%4, %5};\n\t"
+        "mov.b64 d, {%7, %7};\n\t"
+        "fma.rz.f32x2 a, a, m, d;\n\t"
+        "mov.b64 c, {%8, %8};\n\t"
+        "add.rz.f32x2 a, a, c;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "=r"(q0), "=r"(q1)
+        : "r"(a0), "r"(a1), "r"(m0), "r"(m1), "f"(-12582912.f), "f"(add), "f"(8388608.f));
+}
+
+// (volatile: the constants of later columns are not loaded ahead, there are no registers for them)
+__device__ __forceinline__ int4 lds4(uint32_t addr)
+{
+    int4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts4(uint32_t addr, uint4 v)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+// Sixteen accumulator columns of this thread's row, requantized and packed.  tab: shared address of the columns' offsets,
+// multipliers and shifts, `pitch` bytes apart; off: the border class's offsets in global memory where the layer has
+// several (ONE false); rv: the residual's bytes (RES).
+template <int FORM, bool ONE, bool FULL, bool WZP, bool RES>
+__device__ __forceinline__ uint4 epi_half(const uint32_t (&v)[16], const uint32_t tab, const uint32_t pitch, const int32_t *off,
+                                          const EpiConsts &ec, const int wz, const uint4 rv)
+{
+    uint32_t packed[4];
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) {
+        const int4 o = ONE ? lds4(tab + q4 * 16) : __ldg(reinterpret_cast<const int4 *>(off + q4 * 4));
+        const int4 m = lds4(tab + pitch + q4 * 16);
+        int a[4] = { (int)v[q4 * 4] + o.x, (int)v[q4 * 4 + 1] + o.y, (int)v[q4 * 4 + 2] + o.z, (int)v[q4 * 4 + 3] + o.w };
+        const int mm[4] = { m.x, m.y, m.z, m.w };
+        if (WZP) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                a[i] += wz;
+        }
+        int q[4];
+        if constexpr (FORM == kEpiFp) {
+            fp_requant_pair(a[0], a[1], mm[0], mm[1], ec.add, q[0], q[1]);
+            fp_requant_pair(a[2], a[3], mm[2], mm[3], ec.add, q[2], q[3]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                q[i] = FULL ? q[i] - kFpOne : __viaddmax_s32(q[i], -kFpOne, ec.relu_lo);
+        } else if constexpr (FORM == kEpiInt) {
+            const long long rnd = (long long)((unsigned long long)(uint32_t)ec.rnd_hi << 32);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                q[i] = (int)(((long long)a[i] * mm[i] + rnd) >> 32) >> ec.ushift;
+                if (!FULL)
+                    q[i] = max(q[i], ec.relu_lo);
+            }
+        } else {
+            const int4 sh = lds4(tab + 2 * pitch + q4 * 16);
+            const int ss[4] = { sh.x, sh.y, sh.z, sh.w };
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                // narrowed to int32 as the reference narrows before saturating
+                q[i] = (int)(((long long)a[i] * mm[i] + (1ll << (ss[i] - 1)) + ((long long)ec.ozp << ss[i])) >> ss[i]);
+            }
+        }
+        if (FULL) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                q[i] = max(min(q[i], ec.qmax), ec.relu_lo);
+        }
+        if (RES) {
+            // fused eltwise SUM with the residual bytes rv: the conv's own value is first saturated as
+            // it would have been stored (floor, then 0..255), then both inputs go through
+            // (x * m + add) >> b, the sum through >> s0 plus the output zero point and floor
+            const uint32_t rw = q4 == 0 ? rv.x : q4 == 1 ? rv.y : q4 == 2 ? rv.z : rv.w;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int y = min(max(q[i], ec.relu_lo), 255), x = (int)__byte_perm(rw, 0, 0x4440 | i);
+                const int t = ((y * ec.r_m0 + ec.r_add0) >> ec.r_b0) + ((x * ec.r_m1 + ec.r_add1) >> ec.r_b1);
+                q[i] = max((t >> ec.r_s0) + ec.r_ozp, ec.r_lo);
+            }
+        }
+        packed[q4] = pack_sat_u8x4(q[0], q[1], q[2], q[3]);
+        if (FULL)
+            packed[q4] ^= ec.out_flip;
+    }
+    return make_uint4(packed[0], packed[1], packed[2], packed[3]);
+}
+
+// The n16 groups of sixteen columns of one segment for this thread's row: the tensor-memory read of the next group is in
+// flight while one is requantized (two register sets).  row_out: shared address of the row in the staging buffer, whose
+// 16-byte chunks lie XOR-swizzled with sw16 / 16 as the TMA store's swizzle mode expects.  The accumulator stage goes back to
+// the MMA warp (tempty: 0 = not yet) after the last read.
+template <int FORM, bool ONE, bool FULL, bool WZP, bool RES>
+__device__ __forceinline__ void epi_segment(uint32_t t_col, const int n16, uint32_t tab, const uint32_t pitch, const int32_t *off,
+                                            const EpiConsts &ec, const int wz, const uint8_t *res, const uint32_t row_out, const uint32_t sw16,
+                                            const uint32_t tempty, const bool remote)
+{
+    uint32_t va[16], vb[16];
+    auto residual = [&](int h) { return RES && res ? __ldg(reinterpret_cast<const uint4 *>(res) + h) : make_uint4(0, 0, 0, 0); };
+    auto drained = [&]() {
+        if (tempty != 0) {
+            tc_fence_before();
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) {
+                if (remote)
+                    mbar_arrive_cluster(tempty);
+                else
+                    mbar_arrive(tempty);
+            }
+        }
+    };
+    tmem_ld16(t_col, va);
+#pragma unroll 1
+    for (int h = 0; h < n16; h += 2, tab += 128) {
+        const uint4 ra = residual(h);
+        tmem_ld_wait();
+        if (h + 1 < n16)
+            tmem_ld16(t_col + (h + 1) * 16, vb);
+        else
+            drained();
+        sts4(row_out + ((uint32_t)(h << 4) ^ sw16), epi_half<FORM, ONE, FULL, WZP, RES>(va, tab, pitch, off + h * 16, ec, wz, ra));
+        if (h + 1 < n16) {
+            const uint4 rb = residual(h + 1);
+            tmem_ld_wait();
+            if (h + 2 < n16)
+                tmem_ld16(t_col + (h + 2) * 16, va);
+            else
+                drained();
+            sts4(row_out + ((uint32_t)((h + 1) << 4) ^ sw16), epi_half<FORM, ONE, FULL, WZP, RES>(vb, tab + 64, pitch, off + h * 16 + 16, ec, wz, rb));
+        }
+    }
+}
+
+// ---- shared memory layout (dynamic, base aligned to 1024) ---------------------------------------
+//   [stages x A tile (128 x bk)] [stages x B tile (bn x bk)] [2 x output staging 128 x bn]
+//   [per epilogue group: offsets, multipliers, shifts, bn x 4 each] [barriers][tmem address][abort flag]
+struct SmemLayout {
+    uint32_t a, b, out, tables, bars, tmem_slot, abort_flag, total;
+};
+// b_slots: B tiles held in shared memory -- one per pipeline stage, or every k-block of the layer
+// when the weights stay resident.
+__host__ __device__ inline SmemLayout smem_layout(int a_slots, int b_slots, int bk, int bn, int groups, int bn_b = 0)
+{
+    if (bn_b == 0)
+        bn_b = bn;      // rows of a B tile in this CTA's shared memory (half of bn in a CTA pair)
+    SmemLayout L;
+    uint32_t o = 0;
+    L.a = o;
+    o += (uint32_t)a_slots * kTileM * bk;
+    L.b = o;
+    uint32_t b_tile = ((uint32_t)bn_b * bk + 1023u) & ~1023u;
+    o += (uint32_t)b_slots * b_tile;
+    L.out = o;
+    o += (uint32_t)groups * kTileM * bn;   // one output staging buffer per epilogue group
+    o = (o + 1023u) & ~1023u;
+    L.tables = o;                      // per epilogue group: off[bn], mul[bn], shift[bn] (int32)
+    o += (uint32_t)groups * bn * 12;
+    o = (o + 15u) & ~15u;
+    L.bars = o;
+    o += (2 * kMaxStages + 2 * kMaxAccStages + 1) * 8;
+    L.tmem_slot = o;
+    o += 8;
+    L.abort_flag = o;
+    o += 8;
+    L.total = o;
+    return L;
+}
+
+// HAS_RES: the instantiation whose epilogue can add a residual tensor; plans without a fused add run the
+// other one, which carries none of that code.
+// MODE 0: one MMA-issuing warp.  MODE 1 and 2 add a second one (one more warp in the block):
+//   1: the CTA's tiles alternate between the two warps, each on its own half of the stage ring;
+//   2: the CTA's tiles go in pairs that share every weight k-block: a stage holds the activation
+//      tiles of both and ONE weight tile, each warp issues the MMAs of its own tile of the pair.
+template <int EPI, bool HAS_RES, bool HAS_WZP, int MODE>
+__global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ IgemmArgs g)
+{
+    extern __shared__ uint8_t smem_raw[];
+    // the swizzle patterns are functions of the absolute shared address: align the base to 1024
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;
+    uint8_t *smem = smem_raw + (base - raw_addr);
+    const int kblocks_all = g.r * g.s * g.cchunks;
+    const int slots = g.stages * g.kgroup;
+    constexpr bool PAIR = MODE == 3;
+    uint32_t cta_rank = 0;
+    if (PAIR)
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
+    const bool leader = !PAIR || cta_rank == 0;
+    constexpr int kOnes = HAS_WZP ? 16 : 0;      // rows of B, and accumulator columns, behind the tile's channels
+    const int bnl = PAIR ? g.bn >> 1 : g.bn + kOnes;     // rows of B this CTA holds
+    const SmemLayout L = smem_layout(MODE == 2 ? 2 * slots : slots, g.b_resident ? kblocks_all : slots, g.bk, g.bn, g.groups, bnl);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t a_tile_bytes = (uint32_t)kTileM * g.bk;
+    const uint32_t b_tile_bytes = ((uint32_t)bnl * g.bk + 1023u) & ~1023u;
+    const uint32_t bar0 = base + L.bars;
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
+    auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kMaxStages + s); };
+    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kMaxStages + kMaxAccStages + s); };
+    const uint32_t bres_bar = bar0 + 8u * (2 * kMaxStages + 2 * kMaxAccStages);   // resident weights have landed
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + L.tmem_slot);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.abort_flag);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), MODE == 2 ? 2 : 1);   // pair mode: both issuing warps release a stage
+        }
+        mbar_init(bres_bar, 1);
+        for (int s = 0; s < g.acc_stages; ++s) {
+            mbar_init(tfull_bar(s), 1);
+            // one arrival per warp of the stage's epilogue group (of both CTAs of a pair: the leading CTA's
+            // barrier tells its MMA warp that the accumulator halves of both are free)
+            mbar_init(tempty_bar(s), (kEpiWarps / g.groups) * (PAIR ? 2 : 1));
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_map(&maps.a[0]);
+        prefetch_map(&maps.b);
+        prefetch_map(&maps.y[0]);
+    }
+    if (warp == 1) {
+        if (PAIR) {
+            tmem_alloc_pair(base + L.tmem_slot, g.tmem_cols);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(base + L.tmem_slot, g.tmem_cols);
+            tmem_relinquish();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (PAIR)
+        cluster_sync_all();     // the peer's barriers are initialised before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (threadIdx.x == 2 * 32 && g.next_ro_bytes != 0) {
+        // this CTA's slice of the next launch's read-only operand, in 16-byte granules
+        const uint32_t granules = g.next_ro_bytes >> 4;
+        const uint32_t per = (granules + gridDim.x - 1) / gridDim.x;
+        const uint32_t first = blockIdx.x * per;
+        if (first < granules) {
+            const uint32_t cnt = min(per, granules - first);
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g.next_ro + ((size_t)first << 4)), "r"(cnt << 4) : "memory");
+        }
+    }
+
+    const int m_tiles = g.tiles_w * g.tiles_h * g.tiles_n;
+    // the tile sequence of this CTA: tile0, tile0 + tstride, ...  (a CTA pair walks pair tiles together)
+    const int total_tiles = PAIR ? g.pm_tiles * g.n_tiles_n : m_tiles * g.n_tiles_n;
+    const int tile0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+    const int tstride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    auto walker_init = [&](TileWalker &w) {
+        if (PAIR)
+            w.init_pair(g, tile0, (int)cta_rank);
+        else
+            w.init(g, tile0);
+    };
+    const int cchunks = g.cchunks;
+    const int kblocks = g.r * g.s * cchunks;
+
+    if (warp == 0) {
+        // ================= TMA producer =================
+        // The pipeline's k-blocks form one sequence over this CTA's tiles; slot l = q mod slots
+        // (slots = stages * kgroup <= 32) holds k-block q.  Lane l owns slot l for the whole kernel and
+        // issues the loads of k-blocks l, l + slots, ...: the lanes work side by side, so the latency
+        // of one lane's bookkeeping (decode the k-block, wait for the stage, issue) is shared by
+        // `slots` k-blocks.  The first lane of a group posts the group's byte count; a load of another
+        // lane may complete before that (the transaction count is signed), the phase cannot, because
+        // the arrival is still pending.
+        //
+        // With two MMA-issuing warps the ring is split in two halves, one per warp: the lanes of half
+        // r load the k-blocks of the CTA's tiles r, r + 2, ... only, so that every stage barrier has
+        // one consumer that meets its phases in order.
+        const int slots = g.stages * g.kgroup;
+        //
+        // Pair mode: one ring; slot l holds, for k-block q of the PAIR sequence, the activation tiles of
+        // the pair's two tiles and the one weight tile both use (the host has checked that the two
+        // tiles share their channel tile).
+        constexpr int rings = MODE == 1 ? 2 : 1;
+        constexpr int tiles_per_step = (MODE == 0 || MODE == 3) ? 1 : 2;   // tiles a lane moves on by when its k-block wraps
+        const int ring_slots = slots / rings;
+        if (lane < slots && tile0 < total_tiles) {
+            const int stage = lane / g.kgroup;
+            const int ring = lane / ring_slots, rl = lane - ring * ring_slots;
+            const bool first = lane == stage * g.kgroup;
+            const uint32_t fb = full_bar(stage), eb = empty_bar(stage);
+            const uint32_t a_dst = base + L.a + lane * a_tile_bytes * (MODE == 2 ? 2 : 1), b_dst = base + L.b + lane * b_tile_bytes;
+            // a CTA pair: the leading CTA's barrier counts the bytes of both CTAs
+            const uint32_t tx_bytes = (a_tile_bytes + (g.b_resident ? 0u : (uint32_t)bnl * g.bk)) * (uint32_t)g.kgroup * (PAIR ? 2u : 1u);
+            const uint32_t fb_lead = PAIR ? cluster_addr(fb, 0) : fb;
+            // weights are written once, at preparation: they need not wait for the launch before this one
+            if (g.b_resident && lane == 0) {
+                // one channel tile and weights that fit: every k-block of B is loaded once and stays
+                mbar_expect_tx(bres_bar, (uint32_t)kblocks * bnl * g.bk);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    const int tap = kb / cchunks, kc = tap * g.c + (kb - tap * cchunks) * g.bk;
+                    tma_load_2d(base + L.b + kb * b_tile_bytes, &maps.b, bres_bar, kc, 0);
+                    if (HAS_WZP)
+                        tma_load_2d(base + L.b + kb * b_tile_bytes + g.bn * g.bk, &maps.ones, bres_bar, kc, 0);
+                }
+            }
+            const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;   // strides are 1 or 2
+            // this lane's first k-block
+            int kb = rl % kblocks;
+            int tile = tile0;
+            TileWalker tw;
+            walker_init(tw);
+            for (int i = (rl / kblocks) * tiles_per_step + ring; i > 0; --i) {
+                tile += tstride;
+                tw.advance(g);
+            }
+            uint32_t phase = 0;
+            pdl_wait();
+            // Every pass of the loop each lane polls its own stage once (without suspending: a blocked
+            // lane would hold back the ready ones); a lane whose stage is free issues its loads and
+            // moves on to its next k-block, the others poll again in the next pass.  No lane ever waits
+            // for another lane's stage.
+            const unsigned lanes_mask = slots >= 32 ? 0xffffffffu : ((1u << slots) - 1u);
+            bool active = tile < total_tiles;
+            long long t0 = clock64();
+            int spins = 0;
+            while (__any_sync(lanes_mask, active)) {
+                if (active) {
+                    if (mbar_test_wait(eb, phase ^ 1)) {
+                        // k-block -> (tap row, tap column, channel chunk); the divisions are multiplications
+                        // by reciprocals the host rounded up (exact for operands below 2^15)
+                        const int tap = (int)(((uint64_t)(uint32_t)kb * g.rcp_cchunks) >> 30);
+                        const int cc = (kb - tap * cchunks) * g.bk;
+                        const int rr = (int)(((uint64_t)(uint32_t)tap * g.rcp_s) >> 30);
+                        const int ss = tap - rr * g.s;
+                        // input row of output row oh for this tap: ih = oh*stride + d, d = rr - pad
+                        //   = stride * (oh + (d - p) / stride) + p with p = d mod stride (0 <= p < stride)
+                        const int dh = rr - g.pad_h, ph = dh & sh_h;
+                        const int dw = ss - g.pad_w, pw = dw & sh_w;
+                        const int yh = (tw.hi(g) << g.th_sh) + ((dh - ph) >> sh_h);
+                        const int xw = (tw.wi(g) << g.tw_sh) + ((dw - pw) >> sh_w);
+                        const int n0 = tw.ni(g) * g.tn;
+                        const CUtensorMap *amap = &maps.a[ph * 2 + pw];
+                        if (PAIR) {
+                            if (first && leader)
+                                mbar_expect_tx(fb, tx_bytes);
+                            tma_load_4d_pair(a_dst, amap, fb_lead, cc, xw, yh, n0);
+                            tma_load_2d_pair(b_dst, &maps.b, fb_lead, tap * g.c + cc, tw.nt * g.bn + (int)cta_rank * bnl);
+                        } else if (MODE == 2) {
+                            // the pair's second tile (absent behind an odd number of tiles): same tap, its own pixels
+                            const bool second = tile + (int)gridDim.x < total_tiles;
+                            mbar_expect_tx(fb, tx_bytes + (second ? a_tile_bytes : 0u));
+                            tma_load_4d(a_dst, amap, fb, cc, xw, yh, n0);
+                            if (second) {
+                                TileWalker t2 = tw;
+                                t2.advance(g);
+                                tma_load_4d(a_dst + a_tile_bytes, amap, fb, cc, (t2.wi(g) << g.tw_sh) + ((dw - pw) >> sh_w),
+                                            (t2.hi(g) << g.th_sh) + ((dh - ph) >> sh_h), t2.ni(g) * g.tn);
+                            }
+                        } else {
+                        if (first)
+                            mbar_expect_tx(fb, tx_bytes);
+                        if (g.a_wide)   // rows of tw pixels x 32 bytes, in 8-byte elements
+                            tma_load_3d(a_dst, amap, fb, xw << 2, yh, n0);
+                        else
+                            tma_load_4d(a_dst, amap, fb, cc, xw, yh, n0);
+                        }
+                        if (!g.b_resident && !PAIR) {
+                            tma_load_2d(b_dst, &maps.b, fb, tap * g.c + cc, tw.nt * g.bn);
+                            if (HAS_WZP)
+                                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, fb, tap * g.c + cc, 0);
+                        }
+                        phase ^= 1;
+                        kb += ring_slots;
+                        while (kb >= kblocks) {
+                            kb -= kblocks;
+                            for (int i = 0; i < tiles_per_step; ++i) {
+                                tile += tstride;
+                                tw.advance(g);
+                            }
+                        }
+                        active = tile < total_tiles;
+                        t0 = clock64();
+                        spins = 0;
+                    } else if ((++spins & 255) == 0 && (*abort_flag != 0 || clock64() - t0 > kWaitCycles)) {
+                        atomicCAS(g.status, 0, kErrProducerWait);
+                        *abort_flag = 1;
+                        active = false;
+                    }
+                }
+            }
+        }
+        // every load is on its way: the next launch's blocks may come (a block per SM that waits for longer
+        // would keep the SM from the launches of other streams)
+        pdl_trigger();
+    } else if (warp == 1 || ((MODE == 1 || MODE == 2) && warp == kMma2Warp)) {
+        // ================= MMA issuer =================
+        // The whole warp walks the loop (uniform control flow); lane 0 alone issues.  Descriptors of
+        // one operand differ only in the start-address field, so only their low words are computed.
+        // In a CTA pair the leading CTA's warp issues for both; the peer's has nothing to do.
+        if (leader) {
+            const uint32_t lead = lane == 0 ? 1u : 0u;
+            // warp r of `rings` issuing warps takes the CTA's tiles r, r + rings, ... and the stages
+            // [r * ring_stages, (r + 1) * ring_stages); accumulator stages advance by `rings` as well
+            // In pair mode both warps walk the whole ring, stage by stage together: warp r issues for the
+            // r-th tile of each pair, on the r-th activation tile of the stage and the shared weight tile.
+            constexpr int rings = MODE == 1 ? 2 : 1;
+            constexpr int tile_step = (MODE == 0 || MODE == 3) ? 1 : 2;
+            const int ring = warp == 1 ? 0 : 1;
+            const int ring_stages = g.stages / rings, stage0 = MODE == 1 ? ring * ring_stages : 0;
+            int stage = stage0;
+            uint32_t phase = 0;
+            int as = ring;
+            uint32_t aphase = 0;
+            bool ok = true;
+            const uint64_t adesc0 = make_smem_desc(base + L.a, g.bk);
+            const uint64_t bdesc0 = make_smem_desc(base + L.b, g.bk);
+            const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);        // the same for A and B
+            const uint32_t a_lo0 = (uint32_t)adesc0, b_lo0 = (uint32_t)bdesc0;
+            const uint32_t a_step = a_tile_bytes >> 4, b_step = b_tile_bytes >> 4;   // descriptor address units
+            const uint32_t a_grp = a_step * g.kgroup * (MODE == 2 ? 2 : 1), b_grp = b_step * g.kgroup;
+            const int ksteps_full = g.bk / 32;
+            const int groups = kblocks / g.kgroup;
+            const uint32_t idesc = g.idesc;
+            if (g.b_resident && tile0 < total_tiles && !mbar_wait(bres_bar, 0, abort_flag)) {
+                if (lead)
+                    atomicCAS(g.status, 0, kErrMmaFullWait);
+                *abort_flag = 1;
+                ok = false;
+            }
+            for (int tile = tile0 + ring * tstride; (MODE == 2 ? tile - ring * tstride : tile) < total_tiles && ok;
+                 tile += tile_step * tstride) {
+                // pair mode: the second warp of a pair without a second tile still takes part in the
+                // stage hand-over (its commits arrive at once), it just issues nothing
+                const bool have_tile = MODE != 2 || tile < total_tiles;
+                const uint32_t issue = have_tile ? lead : 0u;
+                if (have_tile && !mbar_wait(tempty_bar(as), aphase ^ 1, abort_flag)) {
+                    if (lead)
+                        atomicCAS(g.status, 0, kErrMmaTmemWait);
+                    *abort_flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(as * (g.bn + kOnes));
+                uint32_t accumulate = 0;
+                int chunk = 0;        // k-block of the tap
+                for (int grp = 0; grp < groups; ++grp) {
+                    if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
+                        if (lead)
+                            atomicCAS(g.status, 0, kErrMmaFullWait);
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    uint32_t a_lo = a_lo0 + stage * a_grp + (MODE == 2 ? ring * a_step : 0u);
+                    uint32_t b_lo = b_lo0 + (g.b_resident ? grp : stage) * b_grp;
+                    for (int j = 0; j < g.kgroup; ++j, a_lo += a_step, b_lo += b_step) {
+                        // a k-block is up to 4 MMAs of K = 32 bytes: +2 (16-byte units) inside the swizzle atom
+                        int ksteps = ksteps_full;
+                        if (++chunk == cchunks) {
+                            chunk = 0;
+                            ksteps = g.last_steps;
+                        }
+                        if (PAIR) {
+                            mma_i8_pair(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, issue);
+                            if (ksteps >= 2)
+                                mma_i8_pair(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, issue);
+                            if (ksteps >= 3)
+                                mma_i8_pair(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1, issue);
+                            if (ksteps == 4)
+                                mma_i8_pair(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1, issue);
+                            accumulate = 1;
+                            continue;
+                        }
+                        mma_i8(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, issue);
+                        accumulate = 1;
+                        if (ksteps >= 2)
+                            mma_i8(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, issue);
+                        if (ksteps >= 3)
+                            mma_i8(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1, issue);
+                        if (ksteps == 4)
+                            mma_i8(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1, issue);
+                    }
+                    if (PAIR) {
+                        // the stage is free again in both CTAs once these MMAs are done: one commit per CTA
+                        mma_commit_pair(cluster_addr(empty_bar(stage), 0), lead);
+                        mma_commit_pair(cluster_addr(empty_bar(stage), 1), lead);
+                    } else
+                    mma_commit(empty_bar(stage), lead);   // frees the smem stage when the group's MMAs are done
+                    if (++stage == stage0 + ring_stages) {
+                        stage = stage0;
+                        phase ^= 1;
+                    }
+                }
+                if (!ok)
+                    break;
+                if (PAIR) {
+                    mma_commit_pair(cluster_addr(tfull_bar(as), 0), issue);   // both CTAs' halves of the accumulator
+                    mma_commit_pair(cluster_addr(tfull_bar(as), 1), issue);
+                } else
+                mma_commit(tfull_bar(as), issue);         // accumulator complete
+                as += tile_step;
+                if (as >= g.acc_stages) {
+                    as -= g.acc_stages;
+                    aphase ^= 1;
+                }
+            }
+        }
+    } else if (warp < kMma2Warp) {
+        // ================= epilogue (warps 2..17) =================
+        // Two independent groups of 8 warps; group i owns accumulator stage i, i.e. every second
+        // tile of this CTA, with its own staging buffer, tables and named barriers, so that one
+        // group's waits and barriers overlap the other group's arithmetic.
+        const int group_warps = kEpiWarps / g.groups;      // 8 or 4: a multiple of four, one or two warps per lane quarter
+        const int group_threads = group_warps * 32;
+        const int group = (warp - 2) / group_warps;
+        const int gw = (warp - 2) % group_warps;     // warp inside the group
+        const int et = gw * 32 + lane;               // thread inside the group
+        const int quarter = warp & 3;                // TMEM lanes 32*quarter .. +31 belong to this warp
+        const int sub_warp = gw >> 2;                // which of the group's warps of that quarter
+        const int row = quarter * 32 + lane;         // accumulator row = pixel of the tile
+        int32_t *s_off = reinterpret_cast<int32_t *>(smem + L.tables + (size_t)group * g.bn * 12);
+        int32_t *s_mul = s_off + g.bn, *s_shift = s_mul + g.bn;
+        // one offset row for all pixels (1x1 and unpadded convs), in shared memory
+        constexpr bool one_class = EPI == kEpiFpOne || EPI == kEpiFpOneFull || EPI == kEpiIntOne || EPI == kEpiIntOneFull;
+        constexpr int form = EPI <= kEpiFpManyFull ? kEpiFp : EPI <= kEpiIntManyFull ? kEpiInt : kEpiGeneric;
+        constexpr bool full = EPI == kEpiAny || (EPI & 1) != 0;
+        const uint32_t out_bytes = (uint32_t)kTileM * g.bn;
+        // this thread's pixel inside a tile (tw, th are powers of two)
+        const int lw = row & (g.tw - 1), lh = (row >> g.tw_sh) & (g.th - 1), ln = row >> (g.tw_sh + g.th_sh);
+        int as = group;                              // accumulator stage of this group's current tile
+        uint32_t aphase = 0;
+        int cur_nt = -1;
+        bool store_pending = false;
+        uint8_t *s_out = smem + L.out + (size_t)group * out_bytes;
+
+        const EpiConsts ec = { g.ozp, g.qmax, g.relu_lo, g.ushift, g.rnd_hi, (float)g.ozp + 0.5f, g.out_flip,
+                               g.r_m[0], g.r_add[0], g.r_b[0], g.r_m[1], g.r_add[1], g.r_b[1], g.r_s0, g.r_ozp, g.r_lo };
+
+        // A tile's columns lie in the staging buffer as one or two segments, each a dense [pixel][width] box.  Each
+        // warp owns its 32 rows of the segments it computes (all of them where it is alone on its lane quarter,
+        // else the one of its number) and stores them with its own TMA store of the quarter box: no barrier between
+        // the warps of a group on the way of a tile.  Group barriers remain only where the shared tables are reloaded.
+        const int wpq = group_warps >> 2;                       // warps per lane quarter: 1 or 2
+        const int seg0 = wpq == 1 ? 0 : sub_warp, seg1 = wpq == 1 ? (g.seg_w[1] ? 2 : 1) : (g.seg_w[sub_warp & 1] ? seg0 + 1 : seg0);
+        // XOR mask of this row's 16-byte chunks in a segment of the given width (a power of two: TMA's swizzle; an odd
+        // number of chunks spreads over the banks by itself)
+        auto swizzle = [&](int w) { return w == 128 ? row & 7 : w == 64 ? (row >> 1) & 3 : w == 32 ? (row >> 2) & 1 : 0; };
+        const int p0 = quarter * 32;                            // first pixel of this warp's rows inside a tile
+        const int qlw = p0 & (g.tw - 1), qlh = (p0 >> g.tw_sh) & (g.th - 1), qln = p0 >> (g.tw_sh + g.th_sh);
+        pdl_wait();            // the output may be what the launch before this one still reads
+        bool failed = false;   // a wait ran out: skip the work of the remaining tiles, keep meeting the group barriers
+
+        TileWalker tw;
+        walker_init(tw);
+        for (int i = 0; i < group; ++i)
+            tw.advance(g);
+        // a CTA pair's accumulator stages are handed back on the leading CTA's barrier
+        auto tempty_arrive = [&](int stage_idx) {
+            if (PAIR && !leader)
+                mbar_arrive_cluster(cluster_addr(tempty_bar(stage_idx), 0));
+            else
+                mbar_arrive(tempty_bar(stage_idx));
+        };
+        for (int tile = tile0 + group * tstride; tile < total_tiles; tile += g.groups * tstride) {
+            const int nt = tw.nt;
+            const int ow0 = tw.wi(g) << g.tw_sh, oh0 = tw.hi(g) << g.th_sh, n0 = tw.ni(g) * g.tn;
+            const int k0 = nt * g.bn;
+            const int ow = ow0 + lw, oh = oh0 + lh, img = n0 + ln;
+            const bool pix_valid = ow < g.ow && oh < g.oh && img < g.n;
+            const uint8_t *res_row = g.res;
+            if ((HAS_RES && g.res != nullptr) && pix_valid)
+                res_row += (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
+            int wz_t = 0;       // wzp != 128: this pixel's correction, the same for every channel
+            int cls = 0;
+            if (!one_class)
+                cls = (int)g.row_cls[min(oh, g.oh - 1)] * g.n_col_cls + (int)g.col_cls[min(ow, g.ow - 1)];
+
+            // per-channel tables change with the channel tile: the group meets before (everyone is
+            // past the previous tile's reads) and after the reload
+            if (nt != cur_nt) {
+                epi_bar_sync(group, group_threads);
+                for (int j = et; j < g.bn; j += group_threads) {
+                    s_mul[j] = g.mul[k0 + j];
+                    if (EPI == kEpiAny)
+                        s_shift[j] = g.shift[k0 + j];
+                    if (one_class)
+                        s_off[j] = g.off32[k0 + j];
+                }
+                epi_bar_sync(group, group_threads);
+                cur_nt = nt;
+            }
+            if (!failed) {
+                // this warp's previous store must have finished reading its part of the staging buffer
+                if (store_pending) {
+                    if (lane == 0)
+                        tma_store_wait_read();
+                    __syncwarp();
+                }
+                if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(as), aphase, abort_flag))) {
+                    if (lane == 0) {
+                        atomicCAS(g.status, 0, kErrEpilogueWait);
+                        *abort_flag = 1;
+                    }
+                    failed = true;
+                }
+            }
+            if (!failed) {
+                tc_fence_after();
+                const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * (g.bn + kOnes));
+                if (HAS_WZP) {
+                    uint32_t xs;
+                    tmem_ld1(t_row + g.bn, xs);
+                    tmem_ld_wait();
+                    wz_t = -g.wzp_d * (int)xs;
+                }
+                const int32_t *off_row = g.off32 + (size_t)cls * g.kpad + k0;
+                const uint32_t tab = smem_u32(s_off), pitch = (uint32_t)g.bn * 4;
+                const uint32_t tempty = PAIR && !leader ? cluster_addr(tempty_bar(as), 0) : tempty_bar(as);
+                const bool has_res = HAS_RES && g.res != nullptr;
+                if (seg0 == seg1) {
+                    tc_fence_before();
+                    if (lane == 0)
+                        tempty_arrive(as);
+                }
+                for (int seg = seg0; seg < seg1; ++seg) {
+                    const int w = g.seg_w[seg], c0 = seg ? g.seg_w[0] : 0;
+                    const uint32_t row_out = smem_u32(s_out) + (uint32_t)(kTileM * c0 + row * w);
+                    epi_segment<form, one_class, full, HAS_WZP, HAS_RES>(
+                        t_row + c0, w >> 4, tab + c0 * 4, pitch, off_row + c0, ec, wz_t, has_res && pix_valid ? res_row + c0 : nullptr, row_out,
+                        (uint32_t)swizzle(w) << 4, seg + 1 == seg1 ? tempty : 0u, PAIR && !leader);
+                }
+
+                if (g.use_tma_store) {
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        for (int seg = seg0; seg < seg1; ++seg) {
+                            const int c0 = seg ? g.seg_w[0] : 0;
+                            if (k0 + c0 < g.cout)       // (the store clips what lies past Cout inside a segment)
+                                tma_store_4d(&maps.y[seg], smem_u32(s_out + (size_t)kTileM * c0 + p0 * g.seg_w[seg]),
+                                             k0 + c0, ow0 + qlw, oh0 + qlh, n0 + qln);
+                        }
+                        tma_store_commit();
+                    }
+                    store_pending = true;
+                } else {
+                    // plain stores for channel counts the TMA store cannot address (Cout % 16 != 0): pixel by pixel, the
+                    // lanes side by side along the channels the warp computed, by words where Cout allows
+                    __syncwarp();
+                    const int nvalid = min(g.bn, g.cout - k0), unit = (g.cout & 3) == 0 ? 4 : 1;
+                    for (int pr = 0; pr < 32; ++pr) {
+                        if (!__shfl_sync(0xffffffffu, (int)pix_valid, pr))
+                            continue;
+                        const int prow = p0 + pr;
+                        const int plw = prow & (g.tw - 1), plh = (prow >> g.tw_sh) & (g.th - 1), pln = prow >> (g.tw_sh + g.th_sh);
+                        uint8_t *dst = g.y + (((size_t)(n0 + pln) * g.oh + (oh0 + plh)) * g.ow + (ow0 + plw)) * g.cout + k0;
+                        for (int seg = seg0; seg < seg1; ++seg) {
+                            const int w = g.seg_w[seg], c0 = seg ? g.seg_w[0] : 0;
+                            const int psw = w == 128 ? prow & 7 : w == 64 ? (prow >> 1) & 3 : w == 32 ? (prow >> 2) & 1 : 0;
+                            const uint8_t *src = s_out + (size_t)kTileM * c0 + prow * w;
+                            for (int j = lane * unit; j < min(w, nvalid - c0); j += 32 * unit) {
+                                const uint8_t *from = src + (((j >> 4) ^ psw) << 4) + (j & 15);
+                                if (unit == 4)
+                                    *reinterpret_cast<uint32_t *>(dst + c0 + j) = *reinterpret_cast<const uint32_t *>(from);
+                                else
+                                    dst[c0 + j] = *from;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            as += g.groups;                          // the group's next tile: stage (as + groups) mod acc_stages
+            if (as >= g.acc_stages) {
+                as -= g.acc_stages;
+                aphase ^= 1;
+            }
+            for (int i = 0; i < g.groups; ++i)
+                tw.advance(g);
+        }
+        if (store_pending && lane == 0)
+            tma_store_wait_all();
+    }
+
+    // ---- common exit: every role gets here (all waits are bounded) ---------------------------------
+    tc_fence_before();
+    __syncthreads();
+    if (PAIR)
+        cluster_sync_all();     // neither CTA leaves (or gives tensor memory back) while its peer still works on the pair
+    if (warp == 1) {
+        tc_fence_after();
+        if (PAIR)
+            tmem_dealloc_pair(tmem_base, g.tmem_cols);
+        else
+            tmem_dealloc(tmem_base, g.tmem_cols);
+    }
+}
+
+
+// The kernels, by EpiVariant; nullptr where a combination is not built.  The instantiations are spread over
+// conv_igemm_inst_*.cu, which compile side by side.
+typedef void (*IgemmKernel)(const IgemmMaps, const IgemmArgs);
+IgemmKernel igemm_kernel_mode0(int epi);
+IgemmKernel igemm_kernel_mode1(int epi);
+IgemmKernel igemm_kernel_mode2(int epi);
+IgemmKernel igemm_kernel_mode3(int epi);                // none for variants that only short reductions have
+IgemmKernel igemm_kernel_wzp(int epi);                  // a weight zero point other than 128
+IgemmKernel igemm_kernel_residual(int epi);             // a residual add: none for the Full variants and kEpiAny
+
+}  // namespace b200

@@ -20,6 +20,7 @@ struct SmallArgs {
     int tw_sh, th_sh, tn;              // M-tile box (ow, oh, image) of 128 pixels: log2, log2, images
     int tiles_w, tiles_h, n_tiles_n;
     int bk, kblocks, cchunks;          // k-block bytes per pixel, k-blocks of a tile, k-blocks per tap
+    int cpad, last_steps;              // weights' pitch per tap; 32-byte steps of a tap's last k-block that hold channels
     int bn;                            // output channels per tile
     int split;                         // CTAs (one cluster) that share a tile's k-blocks: 1, 2, 4 or 8
     int slots;                         // k-blocks in flight

@@ -157,10 +157,11 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
         const uint32_t a_dst = base + lane * a_tile, b_dst = base + L.b + lane * L.b_tile;
         const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;
         auto load_b = [&](int kb) {
+            const int tap = kb / g.cchunks, kc = tap * g.cpad + (kb - tap * g.cchunks) * g.bk;
             mbar_expect_tx(full_bar(lane), tx);
-            tma_load_2d(b_dst, &maps.b, full_bar(lane), kb * g.bk, k0);
+            tma_load_2d(b_dst, &maps.b, full_bar(lane), kc, k0);
             if (g.wzp_d)
-                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(lane), kb * g.bk, 0);
+                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(lane), kc, 0);
         };
         int kb = kb0 + lane;
         bool active = lane < g.slots && kb < kb1;
@@ -205,8 +206,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
         const uint32_t lead = lane == 0 ? 1u : 0u;
         const uint64_t adesc0 = make_smem_desc(base, g.bk), bdesc0 = make_smem_desc(base + L.b, g.bk);
         const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);
-        const int ksteps = g.bk / 32;
-        int slot = 0;
+        int slot = 0, chunk = kb0 % g.cchunks;
         uint32_t phase = 0, accumulate = 0;
         bool ok = true;
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -219,6 +219,8 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
             }
             tc_fence_after();
             const uint32_t a_lo = (uint32_t)adesc0 + slot * (a_tile >> 4), b_lo = (uint32_t)bdesc0 + slot * (L.b_tile >> 4);
+            const int ksteps = chunk == g.cchunks - 1 ? g.last_steps : g.bk / 32;
+            chunk = chunk == g.cchunks - 1 ? 0 : chunk + 1;
             for (int j = 0; j < ksteps; ++j) {
                 mma_i8(tmem_base, a_lo + 2 * j, b_lo + 2 * j, desc_hi, g.idesc, accumulate, lead);
                 accumulate = 1;
