@@ -37,6 +37,8 @@ inline cudaStream_t as_stream(b200_stream_t s) { return reinterpret_cast<cudaStr
 
 // Per-device int the kernels with bounded waits write a code into when a wait runs out.
 int status_word_ptr(int **dev_ptr);
+// Queues a kernel that moves the current device's status word to *host (pinned) and clears it.
+int status_publish_launch(int *host, cudaStream_t st);
 
 // Device copy of a 256-byte lookup table, uploaded the first time this table is seen on the current device
 // and cached for the life of the process (runtime.cu).

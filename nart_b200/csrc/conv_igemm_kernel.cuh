@@ -264,18 +264,29 @@ __device__ __forceinline__ void sts4(uint32_t addr, uint4 v)
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// Sixteen accumulator columns of this thread's row, requantized and packed.  tab: shared address of the columns' offsets,
-// multipliers and shifts, `pitch` bytes apart; off: the border class's offsets in global memory where the layer has
-// several (ONE false); rv: the residual's bytes (RES).
-template <int FORM, bool ONE, bool FULL, bool WZP, bool RES>
-__device__ __forceinline__ uint4 epi_half(const uint32_t (&v)[16], const uint32_t tab, const uint32_t pitch, const int32_t *off,
-                                          const EpiConsts &ec, const int wz, const uint4 rv)
+// eltwise SUM of the four bytes of y (a conv's output) and x (the residual), as eltwise_sum_kernel forms it
+__device__ __forceinline__ uint32_t add_residual(const uint32_t y, const uint32_t x, const EpiConsts &ec)
 {
-    uint32_t packed[4];
+    int q[4];
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
-        const int4 o = ONE ? lds4(tab + q4 * 16) : __ldg(reinterpret_cast<const int4 *>(off + q4 * 4));
-        const int4 m = lds4(tab + pitch + q4 * 16);
+    for (int i = 0; i < 4; ++i) {
+        const int a = (int)__byte_perm(y, 0, 0x4440 | i), b = (int)__byte_perm(x, 0, 0x4440 | i);
+        const int t = ((a * ec.r_m0 + ec.r_add0) >> ec.r_b0) + ((b * ec.r_m1 + ec.r_add1) >> ec.r_b1);
+        q[i] = max((t >> ec.r_s0) + ec.r_ozp, ec.r_lo);
+    }
+    return pack_sat_u8x4(q[0], q[1], q[2], q[3]);
+}
+
+// N accumulator columns of this thread's row, requantized and packed.  mul, shift: shared addresses of the columns'
+// constants; the offsets are in shared memory (OFF_SHARED: off_s) or global memory (off_g).
+template <int FORM, bool OFF_SHARED, bool FULL, bool WZP, int N>
+__device__ __forceinline__ void epi_pack(const uint32_t (&v)[N], const uint32_t off_s, const int32_t *off_g, const uint32_t mul, const uint32_t shift,
+                                         const EpiConsts &ec, const int wz, uint32_t (&packed)[N / 4])
+{
+#pragma unroll
+    for (int q4 = 0; q4 < N / 4; ++q4) {
+        const int4 o = OFF_SHARED ? lds4(off_s + q4 * 16) : __ldg(reinterpret_cast<const int4 *>(off_g + q4 * 4));
+        const int4 m = lds4(mul + q4 * 16);
         int a[4] = { (int)v[q4 * 4] + o.x, (int)v[q4 * 4 + 1] + o.y, (int)v[q4 * 4 + 2] + o.z, (int)v[q4 * 4 + 3] + o.w };
         const int mm[4] = { m.x, m.y, m.z, m.w };
         if (WZP) {
@@ -299,7 +310,7 @@ __device__ __forceinline__ uint4 epi_half(const uint32_t (&v)[16], const uint32_
                     q[i] = max(q[i], ec.relu_lo);
             }
         } else {
-            const int4 sh = lds4(tab + 2 * pitch + q4 * 16);
+            const int4 sh = lds4(shift + q4 * 16);
             const int ss[4] = { sh.x, sh.y, sh.z, sh.w };
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -312,24 +323,29 @@ __device__ __forceinline__ uint4 epi_half(const uint32_t (&v)[16], const uint32_
             for (int i = 0; i < 4; ++i)
                 q[i] = max(min(q[i], ec.qmax), ec.relu_lo);
         }
-        if (RES) {
-            // fused eltwise SUM with the residual bytes rv: the conv's own value is first saturated as
-            // it would have been stored (floor, then 0..255), then both inputs go through
-            // (x * m + add) >> b, the sum through >> s0 plus the output zero point and floor
-            const uint32_t rw = q4 == 0 ? rv.x : q4 == 1 ? rv.y : q4 == 2 ? rv.z : rv.w;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int y = min(max(q[i], ec.relu_lo), 255), x = (int)__byte_perm(rw, 0, 0x4440 | i);
-                const int t = ((y * ec.r_m0 + ec.r_add0) >> ec.r_b0) + ((x * ec.r_m1 + ec.r_add1) >> ec.r_b1);
-                q[i] = max((t >> ec.r_s0) + ec.r_ozp, ec.r_lo);
-            }
-        }
         packed[q4] = pack_sat_u8x4(q[0], q[1], q[2], q[3]);
         if (FULL)
             packed[q4] ^= ec.out_flip;
     }
-    return make_uint4(packed[0], packed[1], packed[2], packed[3]);
 }
+
+// Sixteen columns of the persistent kernel's tables: offsets, multipliers and shifts `pitch` bytes apart; rv: the
+// residual's bytes (RES).
+template <int FORM, bool ONE, bool FULL, bool WZP, bool RES>
+__device__ __forceinline__ uint4 epi_half(const uint32_t (&v)[16], const uint32_t tab, const uint32_t pitch, const int32_t *off,
+                                          const EpiConsts &ec, const int wz, const uint4 rv)
+{
+    uint32_t p[4];
+    epi_pack<FORM, ONE, FULL, WZP>(v, tab, off, tab + pitch, tab + 2 * pitch, ec, wz, p);
+    if (RES) {
+        p[0] = add_residual(p[0], rv.x, ec);
+        p[1] = add_residual(p[1], rv.y, ec);
+        p[2] = add_residual(p[2], rv.z, ec);
+        p[3] = add_residual(p[3], rv.w, ec);
+    }
+    return make_uint4(p[0], p[1], p[2], p[3]);
+}
+
 
 // The n16 groups of sixteen columns of one segment for this thread's row: the tensor-memory read of the next group is in
 // flight while one is requantized (two register sets).  row_out: shared address of the row in the staging buffer, whose

@@ -181,7 +181,6 @@ struct ConvIgemmPlan {
     int32_t *off32_dev = nullptr;   // [n_cls][kpad] accumulator offsets
     int32_t *off_form_dev = nullptr;    // the same plus kFpMagic (kEpiFp)
     int32_t *mul_form_dev = nullptr;    // [kpad]
-    uint32_t *mult_dev = nullptr;   // [kpad]
     int32_t *shift_dev = nullptr;   // [kpad]
     uint8_t *row_cls_dev = nullptr, *col_cls_dev = nullptr;
     int rev = 0;                    // reversed tile traversal (conv_igemm_set_reverse)
@@ -192,6 +191,7 @@ struct ConvIgemmPlan {
     bool has_res = false;
     int r_m[2] = { 0, 0 }, r_add[2] = { 0, 0 }, r_b[2] = { 1, 1 };
     int r_s0 = 1, r_ozp = 0, r_lo = 0;
+    int small_bn = 0, small_split = 0;
     bool small_ok = true;           // one tile per CTA where a launch leaves SMs without a tile
     int8_t *ones_dev = nullptr;     // wzp != 128: [16][r][s][c], the first row ones where the window has a channel
     bool attr_set = false;
@@ -301,7 +301,17 @@ int conv_igemm_create(
     }
     ConvIgemmPlan *p = new ConvIgemmPlan();
     p->g = g;
-    p->small_ok = !(getenv("B200_IGEMM_SMALL") && atoi(getenv("B200_IGEMM_SMALL")) == 0);   // tuning aid
+    if (const char *e = getenv("B200_IGEMM_SMALL")) {           // tuning aid: 0, or <channels per tile>x<CTAs per tile>
+        int bn = 0, split = 0;
+        if (sscanf(e, "%dx%d", &bn, &split) == 2) {
+            if ((bn == 16 || bn == 32 || bn == 64 || bn == 128) && (split == 1 || split == 2 || split == 4 || split == 8) && bn / split >= 8) {
+                p->small_bn = bn;
+                p->small_split = split;
+            }
+        } else if (atoi(e) == 0) {
+            p->small_ok = false;
+        }
+    }
     p->saved.reserve(ConvIgemmPlan::kMaxSaved);   // launches never grow it: a later run touches no heap
     p->a_wide = a_row_swizzled ? 1 : 0;
     // K of an 8-bit MMA is 32 bytes: the channel count is rounded up to a multiple of 32 in the
@@ -512,10 +522,8 @@ int conv_igemm_create(
             mag += std::abs((int)w_s8[(size_t)k * g.c * taps + i]);
         reach[k] += 255 * mag + 255ll * (g.wzp_d < 0 ? -g.wzp_d : g.wzp_d) * g.c * taps;
     }
-    std::vector<uint32_t> multp(p->kpad, 0);
     std::vector<int32_t> shiftp(p->kpad, 33);
     for (int k = 0; k < g.k; ++k) {
-        multp[k] = mult[k];
         shiftp[k] = shift[k];
     }
     // The form of the epilogue's arithmetic (EpiForm).
@@ -573,7 +581,6 @@ int conv_igemm_create(
     if (rc == B200_OK) rc = up(mulp.data(), mulp.size() * 4, (void **)&p->mul_form_dev);
     if (rc == B200_OK && p->form == kEpiFp) rc = up(off_form.data(), off_form.size() * 4, (void **)&p->off_form_dev);
     if (rc == B200_OK) rc = up(off32_all.data(), off32_all.size() * 4, (void **)&p->off32_dev);
-    if (rc == B200_OK) rc = up(multp.data(), multp.size() * 4, (void **)&p->mult_dev);
     if (rc == B200_OK) rc = up(shiftp.data(), shiftp.size() * 4, (void **)&p->shift_dev);
     if (rc == B200_OK) rc = up(row_cls.data(), row_cls.size(), (void **)&p->row_cls_dev);
     if (rc == B200_OK) rc = up(col_cls.data(), col_cls.size(), (void **)&p->col_cls_dev);
@@ -594,7 +601,6 @@ void conv_igemm_destroy(ConvIgemmPlan *p)
     cudaFree(p->off_form_dev);
     cudaFree(p->mul_form_dev);
     cudaFree(p->off32_dev);
-    cudaFree(p->mult_dev);
     cudaFree(p->shift_dev);
     cudaFree(p->row_cls_dev);
     cudaFree(p->col_cls_dev);
@@ -727,7 +733,7 @@ static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int
     return encode(map, const_cast<int8_t *>(w), 2, dims, strides, box, swizzle_for(p->bk));
 }
 
-// Fills l.smaps / l.sargs if the launch leaves SMs without a tile; l.small says so.
+// Fills l.smaps / l.sargs if the launch is one for conv_small_kernel; l.small says so.
 static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status, int tw, int th, int tn, ConvIgemmPlan::Launch &l)
 {
     const ConvGeom &g = p->g;
@@ -741,8 +747,12 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.last_steps = (p->cpad - (a.cchunks - 1) * p->bk) / 32;
     a.kblocks = g.r * g.s * a.cchunks;
     a.bk = p->bk;
-    if (!conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, &a.bn, &a.split))
+    if (p->small_bn && p->small_split <= a.kblocks) {              // tuning aid
+        a.bn = p->small_bn;
+        a.split = p->small_split;
+    } else if (!conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, &a.bn, &a.split)) {
         return B200_OK;
+    }
     a.n = n; a.oh = g.oh; a.ow = g.ow; a.cout = g.k;
     a.r = g.r; a.s = g.s; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
     for (a.tw_sh = 0; (1 << a.tw_sh) < tw; ++a.tw_sh) {}
@@ -750,10 +760,12 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.tn = tn;
     a.n_tiles_n = (g.k + a.bn - 1) / a.bn;
     a.a_wide = p->a_wide;
-    a.off32 = p->off32_dev; a.mult = p->mult_dev; a.shift = p->shift_dev;
+    a.form = p->form;
+    a.off32 = p->off_form_dev ? p->off_form_dev : p->off32_dev; a.mul = p->mul_form_dev; a.shift = p->shift_dev;
+    a.ushift = p->ushift; a.rnd_hi = p->rnd_hi;
     a.row_cls = p->row_cls_dev; a.col_cls = p->col_cls_dev;
     a.n_col_cls = p->n_col_cls; a.n_cls = p->n_row_cls * p->n_col_cls; a.kpad = p->kpad;
-    a.ozp = g.ozp; a.qmax = g.qmax; a.relu_lo = g.relu_lo; a.out_flip = g.act_signed ? 0x80 : 0;
+    a.ozp = g.ozp; a.qmax = g.qmax; a.relu_lo = g.relu_lo; a.out_flip = g.act_signed ? 0x80808080u : 0u;
     a.wzp_d = g.wzp_d;
     a.y = y;
     a.status = status;

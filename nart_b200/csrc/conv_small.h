@@ -26,22 +26,28 @@ struct SmallArgs {
     int slots;                         // k-blocks in flight
     int a_wide;                        // see IgemmArgs::a_wide
     uint32_t idesc, tmem_cols;
-    const int32_t *off32;              // [n_cls][kpad] accumulator offsets
-    const uint32_t *mult;              // [kpad]
-    const int32_t *shift;              // [kpad]
+    int form;                          // EpiForm, and its constants (see IgemmArgs)
+    const int32_t *off32;              // [n_cls][kpad]
+    const int32_t *mul, *shift;        // [kpad]
+    int ushift, rnd_hi;
     const uint8_t *row_cls, *col_cls;  // [oh], [ow]
     int n_col_cls, n_cls, kpad;
-    int ozp, qmax, relu_lo, out_flip;  // out_flip: 0x80 for int8 outputs, else 0
+    int ozp, qmax, relu_lo;
+    uint32_t out_flip;                 // 0x80808080 for int8 outputs, else 0
     int wzp_d;                         // weight zero point - 128; not 0: the tile has the window-sum column
     uint8_t *y;
+    const uint8_t *res;                // not nullptr: sum = eltwise SUM of y and res (constants as in IgemmArgs)
+    uint8_t *sum;
+    int r_m[2], r_add[2], r_b[2];
+    int r_s0, r_ozp, r_lo;
     int *status;
     const uint8_t *next_ro;            // see IgemmArgs::next_ro
     uint32_t next_ro_bytes;
 };
 
-// How to cut m_tiles x (k output channels) x kblocks for this kernel: channels per tile and CTAs per tile.  False when
-// the launch has more tiles than SMs whatever the cut: the persistent kernel is the one for it.
-bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int *bn, int *split);
+// How to cut m_tiles x (k output channels) x kblocks for this kernel: channels per tile and CTAs per tile.  False where
+// the persistent kernel, with bn_p channels per tile, is the better one.
+bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int bn_p, int *bn, int *split);
 // Completes bn-dependent fields (slots, idesc, tmem_cols) and launches.
 size_t conv_small_smem(SmallArgs &a, bool act_signed);
 int conv_small_launch(const SmallMaps &maps, const SmallArgs &a, int m_tiles, size_t smem, size_t bytes, cudaStream_t st);

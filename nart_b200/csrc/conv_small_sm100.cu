@@ -10,11 +10,14 @@
 //     shared memory: CTA r of the cluster receives and finishes channels [r * bn / split, (r + 1) * bn / split);
 //   * every k-block of a CTA has a slot of its own where they fit, the weights' loads are issued before
 //     griddepcontrol.wait, and constants reach shared memory while the operands are on their way;
-//   * 192 threads and as little shared memory as that needs, so that the next launch's CTAs are resident beside these.
-// Roles: warp 0 TMA (one lane per slot), warp 1 tensor memory and MMAs, warps 2-5 epilogue.
+//   * 320 threads and as little shared memory as that needs, so that the next launch's CTAs are resident beside these.
+// Roles: warp 0 TMA (one lane per slot), warp 1 tensor memory and MMAs, warps 2-9 epilogue, two per lane quarter.  The
+// epilogue is the persistent kernel's arithmetic (EpiForm); requantizing channel by channel with a shift each, as this kernel
+// first did, took 0.9 us per 16 channels of a tile, most of a 64-channel launch's time.
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "conv_igemm_kernel.cuh"
 #include "conv_small.h"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
@@ -23,7 +26,8 @@ namespace b200 {
 
 namespace {
 
-constexpr int kSmallThreads = 192;
+constexpr int kSmallEpiThreads = 256;
+constexpr int kSmallThreads = 64 + kSmallEpiThreads;
 constexpr int kSmallM = 128;            // pixels per tile
 constexpr int kSmallSlots = 16;
 constexpr int kSmallClsCols = 4096;     // border classes x channels that are staged in shared memory; more are read in place
@@ -40,7 +44,7 @@ __host__ __device__ inline SmallLayout small_layout(const SmallArgs &g)
     L.b = o;
     L.b_tile = ((uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk + 1023u) & ~1023u;
     o += g.slots * L.b_tile;
-    L.red = o;                                              // [split][bn / split][128] partial accumulators
+    L.red = o;                                              // [split][channel quad][128][4] partial accumulators
     o += g.split > 1 ? (uint32_t)g.bn * kSmallM * 4 : 0;
     L.xred = o;                                             // [split][128] partial window sums
     o += g.split > 1 && g.wzp_d ? (uint32_t)g.split * kSmallM * 4 : 0;
@@ -61,42 +65,68 @@ __host__ __device__ inline SmallLayout small_layout(const SmallArgs &g)
     return L;
 }
 
+__device__ __forceinline__ void st_cluster4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v)
 {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-// N channels from accumulators `acc` (one pixel): requantized, packed, stored at `dst`; k: the first channel.
+// Where a CTA's tables lie (shared addresses), and this thread's border class's offsets.
+struct SmallTables {
+    uint32_t off_s, mul, shift;
+    const int32_t *off_g;               // nullptr: staged at off_s
+};
+
+// N channels from accumulators `acc` (one pixel), the first at channel j of the tile and k of the layer: requantized,
+// packed, stored at element `at` of the output, and with the residual added at the same element of its sum.
 template <int N>
-__device__ __forceinline__ void store_channels(const int (&acc)[N], const SmallArgs &g, const int *s_mult, const int *s_shift, const int32_t *off,
-                                               int xcorr, int j, int k, uint8_t *dst)
+__device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const SmallArgs &g, const EpiConsts &ec, const SmallTables &t, int xcorr,
+                                               int j, int k, size_t at)
 {
     uint32_t w[N / 4];
-#pragma unroll
-    for (int q = 0; q < N / 4; ++q) {
-        int v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int i = 4 * q + e;
-            v[e] = sat_relu(requant_raw(acc[i] + off[j + i] + xcorr, (uint32_t)s_mult[j + i], s_shift[j + i], g.ozp), g.qmax, g.relu_lo) ^ g.out_flip;
-        }
-        w[q] = pack4(v[0], v[1], v[2], v[3]);
-    }
-    if (k + N <= g.cout && (g.cout & (N - 1)) == 0) {
-        if constexpr (N == 16)
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (t.off_g == nullptr) {
+        if (g.form == kEpiFp)
+            epi_pack<kEpiFp, true, true, true>(acc, t.off_s + j * 4, nullptr, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
+        else if (g.form == kEpiInt)
+            epi_pack<kEpiInt, true, true, true>(acc, t.off_s + j * 4, nullptr, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
         else
-            *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
-    } else if ((g.cout & 3) == 0) {
+            epi_pack<kEpiGeneric, true, true, true>(acc, t.off_s + j * 4, nullptr, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
+    } else {
+        if (g.form == kEpiFp)
+            epi_pack<kEpiFp, false, true, true>(acc, 0, t.off_g + j, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
+        else if (g.form == kEpiInt)
+            epi_pack<kEpiInt, false, true, true>(acc, 0, t.off_g + j, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
+        else
+            epi_pack<kEpiGeneric, false, true, true>(acc, 0, t.off_g + j, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
+    }
+    auto store = [&](uint8_t *dst) {
+        if (k + N <= g.cout && (g.cout & (N - 1)) == 0) {
+            if constexpr (N == 16)
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+            else
+                *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
+        } else if ((g.cout & 3) == 0) {
+#pragma unroll
+            for (int q = 0; q < N / 4; ++q)
+                if (k + 4 * q < g.cout)
+                    reinterpret_cast<uint32_t *>(dst)[q] = w[q];
+        } else {
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (k + i < g.cout)
+                    dst[i] = (uint8_t)(w[i / 4] >> (8 * (i % 4)));
+        }
+    };
+    store(g.y + at);
+    if (g.res) {            // (Cout is a multiple of 32 then)
+        const uint32_t *x = reinterpret_cast<const uint32_t *>(g.res + at);
 #pragma unroll
         for (int q = 0; q < N / 4; ++q)
-            if (k + 4 * q < g.cout)
-                reinterpret_cast<uint32_t *>(dst)[q] = w[q];
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            if (k + i < g.cout)
-                dst[i] = (uint8_t)(w[i / 4] >> (8 * (i % 4)));
+            w[q] = add_residual(w[q], __ldg(x + q), ec);
+        store(g.sum + at);
     }
 }
 
@@ -236,40 +266,46 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
             mma_commit(acc_bar, lead);
     }
 
-    // ================= epilogue (warps 2..5) =================
+    // ================= epilogue (warps 2..9) =================
     const int quarter = warp & 3;                       // tensor-memory lanes of this warp
+    const int half = (warp - 2) >> 2;                   // which of the two warps of the quarter
     const int row = quarter * 32 + lane;
     const int bnl = g.bn / split;                       // channels this CTA finishes
-    int *s_mult = reinterpret_cast<int *>(smem + L.mult), *s_shift = reinterpret_cast<int *>(smem + L.shift);
-    int32_t *s_off = reinterpret_cast<int32_t *>(smem + L.off);
     const bool off_staged = g.n_cls * g.bn <= kSmallClsCols;
     const int lw = row & ((1 << g.tw_sh) - 1), lh = (row >> g.tw_sh) & ((1 << g.th_sh) - 1), ln = row >> (g.tw_sh + g.th_sh);
     const int ow = (twi << g.tw_sh) + lw, oh = (thi << g.th_sh) + lh, img = tni * g.tn + ln;
     const bool pix_valid = ow < g.ow && oh < g.oh && img < g.n;
-    uint8_t *dst = g.y + (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
-    const int32_t *off = nullptr;
+    const size_t at = (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
+    const EpiConsts ec = { g.ozp, g.qmax, g.relu_lo, g.ushift, g.rnd_hi, (float)g.ozp + 0.5f, g.out_flip,
+                           g.r_m[0], g.r_add[0], g.r_b[0], g.r_m[1], g.r_add[1], g.r_b[1], g.r_s0, g.r_ozp, g.r_lo };
+    SmallTables t = { base + L.off, base + L.mult, base + L.shift, nullptr };
     const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
     bool ok = true;
     if (warp >= 2) {
+        int *s_mult = reinterpret_cast<int *>(smem + L.mult), *s_shift = reinterpret_cast<int *>(smem + L.shift);
+        int32_t *s_off = reinterpret_cast<int32_t *>(smem + L.off);
         const int et = threadIdx.x - 64;
         if (et == 0 && g.next_ro_bytes != 0) {
             const uint32_t granules = g.next_ro_bytes >> 4, per = (granules + gridDim.x - 1) / gridDim.x, from = blockIdx.x * per;
             if (from < granules)
                 asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g.next_ro + ((size_t)from << 4)), "r"(min(per, granules - from) << 4) : "memory");
         }
-        for (int j = et; j < g.bn; j += 128) {
+        for (int j = et; j < g.bn; j += kSmallEpiThreads) {
             const bool in = k0 + j < g.kpad;
-            s_mult[j] = in ? (int)__ldg(g.mult + k0 + j) : 0;
+            s_mult[j] = in ? __ldg(g.mul + k0 + j) : 0;
             s_shift[j] = in ? __ldg(g.shift + k0 + j) : 33;
         }
         if (off_staged)
-            for (int i = et; i < g.n_cls * g.bn; i += 128) {
+            for (int i = et; i < g.n_cls * g.bn; i += kSmallEpiThreads) {
                 const int c = i / g.bn, j = i - c * g.bn;
                 s_off[i] = k0 + j < g.kpad ? __ldg(g.off32 + (size_t)c * g.kpad + k0 + j) : 0;
             }
         const int cls = (int)__ldg(g.row_cls + min(oh, g.oh - 1)) * g.n_col_cls + (int)__ldg(g.col_cls + min(ow, g.ow - 1));
-        off = off_staged ? s_off + cls * g.bn : g.off32 + (size_t)cls * g.kpad + k0;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (off_staged)
+            t.off_s += (uint32_t)(cls * g.bn) * 4;
+        else
+            t.off_g = g.off32 + (size_t)cls * g.kpad + k0;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         ok = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag));
         if (!ok && lane == 0) {
             atomicCAS(g.status, 0, kErrSmallEpilogue);
@@ -285,34 +321,29 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 tmem_ld_wait();
                 xcorr = -g.wzp_d * (int)xs;
             }
-            for (int c0 = 0; c0 < g.bn && k0 + c0 < g.cout; c0 += 16) {
+            for (int c0 = half * 16; c0 < g.bn && k0 + c0 < g.cout; c0 += 32) {
                 uint32_t v[16];
                 tmem_ld16(t_row + c0, v);
                 tmem_ld_wait();
-                int acc[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    acc[i] = (int)v[i];
                 if (pix_valid)
-                    store_channels<16>(acc, g, s_mult, s_shift, off, xcorr, c0, k0 + c0, dst + c0);
+                    store_channels<16>(v, g, ec, t, xcorr, c0, k0 + c0, at + c0);
                 __syncwarp();
             }
         } else if (ok) {
-            // this CTA's partial sums to the CTAs that finish them: [source rank][channel][pixel]
-            for (int c0 = 0; c0 < g.bn; c0 += 16) {
+            // this CTA's partial sums to the CTAs that finish them, four channels of 32 neighbouring pixels a store
+            for (int c0 = half * 16; c0 < g.bn; c0 += 32) {
                 uint32_t v[16];
                 tmem_ld16(t_row + c0, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int h = 0; h < 16; h += 8) {       // bn / split is a multiple of 8
-                    const int owner = (c0 + h) / bnl, j = (c0 + h) - owner * bnl;
-                    const uint32_t to = cluster_addr(base + L.red + (uint32_t)((rank * bnl + j) * kSmallM + row) * 4, (uint32_t)owner);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        st_cluster(to + i * (kSmallM * 4), v[h + i]);
+                    const int owner = (c0 + h) / bnl, ch = ((c0 + h) - owner * bnl) >> 2;
+                    const uint32_t to = cluster_addr(base + L.red + (uint32_t)(((rank * (bnl >> 2) + ch) * kSmallM + row) * 16), (uint32_t)owner);
+                    st_cluster4(to, v[h], v[h + 1], v[h + 2], v[h + 3]);
+                    st_cluster4(to + kSmallM * 16, v[h + 4], v[h + 5], v[h + 6], v[h + 7]);
                 }
             }
-            if (g.wzp_d) {
+            if (g.wzp_d && half == 0) {
                 uint32_t xs;
                 tmem_ld1(t_row + g.bn, xs);
                 tmem_ld_wait();
@@ -325,7 +356,6 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
         __syncthreads();
         cluster_sync_all();
         if (warp >= 2 && ok && pix_valid) {
-            const int *red = reinterpret_cast<const int *>(smem + L.red);
             int xcorr = 0;
             if (g.wzp_d) {
                 const int *xred = reinterpret_cast<const int *>(smem + L.xred);
@@ -334,16 +364,17 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 xcorr *= g.wzp_d;
             }
             const int c1 = rank * bnl;                  // first channel of this CTA's share
-            for (int j = 0; j < bnl && k0 + c1 + j < g.cout; j += 8) {
-                int acc[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    acc[i] = red[(j + i) * kSmallM + row];
-                for (int s = 1; s < split; ++s)
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        acc[i] += red[(s * bnl + j + i) * kSmallM + row];
-                store_channels<8>(acc, g, s_mult, s_shift, off, xcorr, c1 + j, k0 + c1 + j, dst + c1 + j);
+            for (int j = half * 8; j < bnl && k0 + c1 + j < g.cout; j += 16) {
+                uint32_t acc[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
+                const uint32_t from = base + L.red + (uint32_t)(((j >> 2) * kSmallM + row) * 16);
+#pragma unroll 4
+                for (int s = 0; s < split; ++s) {
+                    const int4 a = lds4(from + (uint32_t)(s * kSmallM * bnl) * 4);
+                    const int4 b = lds4(from + (uint32_t)(s * kSmallM * bnl) * 4 + kSmallM * 16);
+                    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+                    acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+                }
+                store_channels<8>(acc, g, ec, t, xcorr, c1 + j, k0 + c1 + j, at + c1 + j);
             }
         }
     }
@@ -357,32 +388,43 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
 
 }  // namespace
 
-bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int *bn_out, int *split_out)
+bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int bn_p, int *bn_out, int *split_out)
 {
-    const int sms = sm_count();
-    const int k16 = (k + 15) / 16 * 16;
-    double best = 1e30;
+    // Microseconds on this GPU, fitted to sweeps over both kernels' tilings of ResNet-50's and MobileNetV2's layers at
+    // batches 1 to 32.  What counts: a k-block's rows through the SM's TMA unit (0.25 us for 128 rows of 64 bytes, 0.37 of
+    // 128), the epilogue behind the last MMA, and the cluster's exchange of partial sums.
+    const int sms = sm_count(), extra = wzp ? 16 : 0, k16 = (k + 15) / 16 * 16;
+    const double row = 0.13 + 0.0019 * bk;
+    double best;
+    {   // the persistent kernel: a round's loads and the epilogue of the round before it overlap
+        const int rounds = (m_tiles * ((k + bn_p - 1) / bn_p) + sms - 1) / sms;
+        const double load = kblocks * row * (bn_p > 128 ? 1.4 : 1.1), epi = 0.008 * bn_p;
+        best = 3.4 + rounds * (load > epi ? load : epi) + (load > epi ? epi : load);
+    }
+    bool small = false;
     for (int bn = 16; bn <= 128; bn *= 2) {
-        if (bn > k16 && bn != 16 && bn / 2 >= k16)
+        if (bn > 16 && bn / 2 >= k16)
             break;
         const int tiles = m_tiles * ((k + bn - 1) / bn);
-        for (int split = 1; split <= 8 && split <= kblocks; split *= 2) {
-            if (tiles * split > sms || bn / split < 8)
+        for (int split = 1; split <= 8 && split <= kblocks && bn / split >= 8; split *= 2) {
+            const int ctas = tiles * split, kb = (kblocks + split - 1) / split;
+            // two CTAs share an SM where both fit its shared memory; clusters of four and eight leave SMs of a GPC over
+            const int slots = kb < 4 ? kb : 4;
+            const bool two = split == 1 && slots * (kSmallM + bn + extra) * bk <= 104 * 1024;
+            if (ctas > (split == 8 ? sms * 2 / 3 : split == 4 ? sms * 7 / 8 : two ? 2 * sms : sms))
                 continue;
-            // nanoseconds on this GPU: the operands of a CTA's k-blocks through its memory port, its MMAs one
-            // after the other, the reduction, the share of the epilogue that follows the last MMA
-            const int kb = (kblocks + split - 1) / split;
-            const double load = kb * (double)(kSmallM + bn + (wzp ? 16 : 0)) * bk / 110.0;
-            const double mma = kb * (bk / 32) * (bn + (wzp ? 16 : 0) > 128 ? 38.0 : 34.0);
-            const double cost = (load > mma ? load : mma) + (split > 1 ? 900.0 + bn * 4.0 : 0.0) + bn / split * 10.0;
+            const double load = kb * (row + 0.0003 * (bn + extra));
+            const double epi = split > 1 ? 0.6 + 0.012 * bn + 0.7 * ctas / sms + (split == 8 ? 0.5 : 0.0) : bn > 32 ? 0.0125 * (bn - 32) : 0.0;
+            const double cost = ctas > sms ? 3.2 + (load + epi) * ctas / sms : 2.3 + load + epi;
             if (cost < best) {
                 best = cost;
+                small = true;
                 *bn_out = bn;
                 *split_out = split;
             }
         }
     }
-    return best < 1e30;
+    return small;
 }
 
 size_t conv_small_smem(SmallArgs &a, bool act_signed)

@@ -275,7 +275,9 @@ static int pool_pair_pick(int method, int vec, const uint8_t *x, uint8_t *y, con
 // the padded window size (pool.c:217-221) and come from a small host-built table indexed by how
 // many rows / columns the window loses at the far edge.  The sums run on 16-bit lanes: pool_prepare
 // admits at most 257 taps, 65535 a lane.
-template <int VEC>
+// LANES > 1: that many neighbouring lanes share an output, taking every LANES-th round of taps, for launches with few
+// outputs and large windows, whose time is one thread's chain of loads (2048 channels of one 7x7 map: 10.8 us with one).
+template <int VEC, int LANES = 1>
 __global__ void __launch_bounds__(256) pool_avg_kernel(
     const uint8_t *__restrict__ x, uint8_t *__restrict__ y, PoolGeom g, PoolAvgTab tab)
 {
@@ -284,8 +286,10 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
     constexpr int W = (VEC + 3) / 4;
     const uint32_t cv = (uint32_t)(g.c / VEC);
     const size_t total = (size_t)g.n * g.oh * g.ow * cv;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (size_t)gridDim.x * blockDim.x) {
+    const int sub = threadIdx.x & (LANES - 1);
+    // (LANES > 1 is launched with whole warps of work only, so that all lanes reach the shuffles)
+    for (size_t idx = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES; idx < total;
+         idx += (size_t)gridDim.x * blockDim.x / LANES) {
         int ci = (int)(idx % cv);
         size_t pix = idx / cv;
         int ox = (int)(pix % g.ow);
@@ -309,7 +313,11 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
         constexpr int UNR = 8;
         const uint8_t *base = x + (((size_t)n * g.h + hs) * g.w + ws) * g.c + (size_t)ci * VEC;
         int ty = 0, tx = 0;
-        for (int t = 0; t < cnt; t += UNR) {
+        if (LANES > 1 && wd > 0) {
+            ty = sub * UNR / wd;
+            tx = sub * UNR - ty * wd;
+        }
+        for (int t = sub * UNR; t < cnt; t += UNR * LANES) {
             uint32_t v[UNR][W];
 #pragma unroll
             for (int u = 0; u < UNR; ++u) {
@@ -332,7 +340,19 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
                     sum[j].lo += b.lo;
                     sum[j].hi += b.hi;
                 }
+            if (LANES > 1 && t + UNR * LANES < cnt) {
+                const int at = t + UNR * LANES;
+                ty = at / wd;
+                tx = at - ty * wd;
+            }
         }
+#pragma unroll
+        for (int m = 1; m < LANES; m *= 2)
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                sum[j].lo += __shfl_xor_sync(0xffffffffu, sum[j].lo, m);
+                sum[j].hi += __shfl_xor_sync(0xffffffffu, sum[j].hi, m);
+            }
         uint32_t o[W];
 #pragma unroll
         for (int j = 0; j < W; ++j)
@@ -348,7 +368,8 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
             v = min(max(v, 0), g.qmax);
             o[j / 4] |= (uint32_t)v << (8 * (j % 4));
         }
-        store_words<VEC>(y + pix * g.c + (size_t)ci * VEC, o);
+        if (sub == 0)
+            store_words<VEC>(y + pix * g.c + (size_t)ci * VEC, o);
     }
 }
 
@@ -468,7 +489,9 @@ int pool_launch(
     // the loop over the window is a chain of loads (2048 channels of 7x7, batch 256)
     if (method == 1 && vec == 16 && (size_t)n * g.oh * g.ow * (c / 16) < (size_t)sm_count() * 1024)
         vec = 4;
-    const size_t blocks = ((size_t)n * g.oh * g.ow * (c / vec) + 255) / 256;
+    const size_t outs = (size_t)n * g.oh * g.ow * (c / vec), blocks = (outs + 255) / 256;
+    if (method == 1 && vec == 4 && outs % 4 == 0 && outs * 8 <= (size_t)sm_count() * 2048 && g.kernel_h * g.kernel_w >= 16)
+        return launch_kernel(pool_avg_kernel<4, 8>, dim3((unsigned)((outs * 8 + 255) / 256)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
     if (method == 0) {
         if (vec == 16) return launch_kernel(pool_max_kernel<16>, dim3(resident_grid<pool_max_kernel<16>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
         if (vec == 4) return launch_kernel(pool_max_kernel<4>, dim3(resident_grid<pool_max_kernel<4>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
