@@ -264,6 +264,34 @@ __device__ __forceinline__ void sts4(uint32_t addr, uint4 v)
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+__device__ __forceinline__ uint32_t lds1(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// n bytes of a staged row to global memory, whatever the alignment of dst, by `lanes` neighbouring lanes (`sub` is this one's
+// number): aligned words, funnel-shifted out of two staged ones, and the bytes before and behind them.
+// load(off): the staged word at byte off, a multiple of 4.
+__device__ __forceinline__ int copy_lanes(int n) { return n <= 16 ? 4 : n <= 32 ? 8 : n <= 64 ? 16 : 32; }
+template <typename Load>
+__device__ __forceinline__ void copy_row(uint8_t *dst, int n, int sub, int lanes, Load load)
+{
+    const int head = min((int)((0u - (uint32_t)(uintptr_t)dst) & 3u), n), words = (n - head) >> 2, tail = (n - head) & 3;
+    for (int w = sub; w < words; w += lanes) {
+        const uint32_t a = load(4 * w), b = head ? load(4 * w + 4) : 0u;
+        *reinterpret_cast<uint32_t *>(dst + head + 4 * w) = __funnelshift_r(a, b, 8 * head);
+    }
+    if (sub < head)
+        dst[sub] = (uint8_t)(load(0) >> (8 * sub));
+    const int back = lanes - 1 - sub;
+    if (back < tail) {
+        const int off = head + 4 * words + back;
+        dst[off] = (uint8_t)(load(off & ~3) >> (8 * (off & 3)));
+    }
+}
+
 // eltwise SUM of the four bytes of y (a conv's output) and x (the residual), as eltwise_sum_kernel forms it
 __device__ __forceinline__ uint32_t add_residual(const uint32_t y, const uint32_t x, const EpiConsts &ec)
 {
@@ -907,27 +935,24 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
                     }
                     store_pending = true;
                 } else {
-                    // plain stores for channel counts the TMA store cannot address (Cout % 16 != 0): pixel by pixel, the
-                    // lanes side by side along the channels the warp computed, by words where Cout allows
+                    // channel counts the TMA store cannot address (Cout % 16 != 0): pixel by pixel, the lanes side by side along
+                    // the channels the warp computed
                     __syncwarp();
-                    const int nvalid = min(g.bn, g.cout - k0), unit = (g.cout & 3) == 0 ? 4 : 1;
-                    for (int pr = 0; pr < 32; ++pr) {
-                        if (!__shfl_sync(0xffffffffu, (int)pix_valid, pr))
+                    const unsigned valid = __ballot_sync(0xffffffffu, pix_valid);
+                    for (int seg = seg0; seg < seg1; ++seg) {
+                        const int w = g.seg_w[seg], c0 = seg ? g.seg_w[0] : 0, n = min(w, g.cout - k0 - c0);
+                        if (n <= 0)
                             continue;
-                        const int prow = p0 + pr;
-                        const int plw = prow & (g.tw - 1), plh = (prow >> g.tw_sh) & (g.th - 1), pln = prow >> (g.tw_sh + g.th_sh);
-                        uint8_t *dst = g.y + (((size_t)(n0 + pln) * g.oh + (oh0 + plh)) * g.ow + (ow0 + plw)) * g.cout + k0;
-                        for (int seg = seg0; seg < seg1; ++seg) {
-                            const int w = g.seg_w[seg], c0 = seg ? g.seg_w[0] : 0;
-                            const int psw = w == 128 ? prow & 7 : w == 64 ? (prow >> 1) & 3 : w == 32 ? (prow >> 2) & 1 : 0;
-                            const uint8_t *src = s_out + (size_t)kTileM * c0 + prow * w;
-                            for (int j = lane * unit; j < min(w, nvalid - c0); j += 32 * unit) {
-                                const uint8_t *from = src + (((j >> 4) ^ psw) << 4) + (j & 15);
-                                if (unit == 4)
-                                    *reinterpret_cast<uint32_t *>(dst + c0 + j) = *reinterpret_cast<const uint32_t *>(from);
-                                else
-                                    dst[c0 + j] = *from;
-                            }
+                        const int lanes = copy_lanes(n);
+                        for (int pr = lane / lanes; pr < 32; pr += 32 / lanes) {
+                            if (!((valid >> pr) & 1))
+                                continue;
+                            const int prow = p0 + pr;
+                            const int plw = prow & (g.tw - 1), plh = (prow >> g.tw_sh) & (g.th - 1), pln = prow >> (g.tw_sh + g.th_sh);
+                            uint8_t *dst = g.y + (((size_t)(n0 + pln) * g.oh + (oh0 + plh)) * g.ow + (ow0 + plw)) * g.cout + k0 + c0;
+                            const uint32_t psw = w == 128 ? prow & 7 : w == 64 ? (prow >> 1) & 3 : w == 32 ? (prow >> 2) & 1 : 0;
+                            const uint32_t src = smem_u32(s_out) + (uint32_t)(kTileM * c0 + prow * w);
+                            copy_row(dst, n, lane & (lanes - 1), lanes, [&](int off) { return lds1(src + ((uint32_t)off ^ (psw << 4))); });
                         }
                     }
                     __syncwarp();

@@ -35,7 +35,7 @@ constexpr int kSmallClsCols = 4096;     // border classes x channels that are st
 constexpr int kErrSmallProducer = 0x201, kErrSmallFull = 0x202, kErrSmallEpilogue = 0x203;
 
 struct SmallLayout {
-    uint32_t b, b_tile, red, xred, mult, shift, off, bars, tmem_slot, abort_flag, total;
+    uint32_t b, b_tile, red, xred, mult, shift, off, stage, stage_pitch, bars, tmem_slot, abort_flag, total;
 };
 __host__ __device__ inline SmallLayout small_layout(const SmallArgs &g)
 {
@@ -55,6 +55,11 @@ __host__ __device__ inline SmallLayout small_layout(const SmallArgs &g)
     L.off = o;
     o += g.n_cls * g.bn <= kSmallClsCols ? (uint32_t)g.n_cls * g.bn * 4 : 0;
     o = (o + 15u) & ~15u;
+    // Cout % 16 != 0: the tile's bytes pass through shared memory, so that whole words reach global memory (a byte store
+    // per channel and pixel took 20 us for 218 channels of 6776 pixels)
+    L.stage = o;
+    L.stage_pitch = (uint32_t)(g.bn / g.split) + 16;
+    o += g.cout % 16 != 0 ? kSmallM * L.stage_pitch : 0;
     L.bars = o;                                             // full[slots], empty[slots], accumulator
     o += (2 * kSmallSlots + 1) * 8;
     L.tmem_slot = o;
@@ -80,11 +85,11 @@ struct SmallTables {
     const int32_t *off_g;               // nullptr: staged at off_s
 };
 
-// N channels from accumulators `acc` (one pixel), the first at channel j of the tile and k of the layer: requantized,
-// packed, stored at element `at` of the output, and with the residual added at the same element of its sum.
+// N channels from accumulators `acc` (one pixel), the first at channel j of the tile: requantized, packed, stored at element
+// `at` of the output, and with the residual added at the same element of its sum; or at the shared address `stage`.
 template <int N>
 __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const SmallArgs &g, const EpiConsts &ec, const SmallTables &t, int xcorr,
-                                               int j, int k, size_t at)
+                                               int j, size_t at, uint32_t stage)
 {
     uint32_t w[N / 4];
     if (t.off_g == nullptr) {
@@ -102,23 +107,18 @@ __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const S
         else
             epi_pack<kEpiGeneric, false, true, true>(acc, 0, t.off_g + j, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
     }
+    if (stage != 0) {
+        if constexpr (N == 16)
+            sts4(stage, make_uint4(w[0], w[1], w[2], w[3]));
+        else
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(stage), "r"(w[0]), "r"(w[1]) : "memory");
+        return;
+    }
     auto store = [&](uint8_t *dst) {
-        if (k + N <= g.cout && (g.cout & (N - 1)) == 0) {
-            if constexpr (N == 16)
-                *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-            else
-                *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
-        } else if ((g.cout & 3) == 0) {
-#pragma unroll
-            for (int q = 0; q < N / 4; ++q)
-                if (k + 4 * q < g.cout)
-                    reinterpret_cast<uint32_t *>(dst)[q] = w[q];
-        } else {
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-                if (k + i < g.cout)
-                    dst[i] = (uint8_t)(w[i / 4] >> (8 * (i % 4)));
-        }
+        if constexpr (N == 16)
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        else
+            *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
     };
     store(g.y + at);
     if (g.res) {            // (Cout is a multiple of 32 then)
@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                            g.r_m[0], g.r_add[0], g.r_b[0], g.r_m[1], g.r_add[1], g.r_b[1], g.r_s0, g.r_ozp, g.r_lo };
     SmallTables t = { base + L.off, base + L.mult, base + L.shift, nullptr };
     const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const uint32_t stage = g.cout % 16 != 0 ? base + L.stage + (uint32_t)row * L.stage_pitch : 0u;
     bool ok = true;
     if (warp >= 2) {
         int *s_mult = reinterpret_cast<int *>(smem + L.mult), *s_shift = reinterpret_cast<int *>(smem + L.shift);
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 tmem_ld16(t_row + c0, v);
                 tmem_ld_wait();
                 if (pix_valid)
-                    store_channels<16>(v, g, ec, t, xcorr, c0, k0 + c0, at + c0);
+                    store_channels<16>(v, g, ec, t, xcorr, c0, at + c0, stage ? stage + c0 : 0u);
                 __syncwarp();
             }
         } else if (ok) {
@@ -374,7 +375,24 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                     acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
                     acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
                 }
-                store_channels<8>(acc, g, ec, t, xcorr, c1 + j, k0 + c1 + j, at + c1 + j);
+                store_channels<8>(acc, g, ec, t, xcorr, c1 + j, at + c1 + j, stage ? stage + j : 0u);
+            }
+        }
+    }
+    if (stage != 0 && warp >= 2) {
+        asm volatile("bar.sync 1, 256;" ::: "memory");      // both warps of a quarter have staged their channels
+        const int c1 = rank * bnl, n = min(bnl, g.cout - k0 - c1);
+        const unsigned valid = __ballot_sync(0xffffffffu, pix_valid && ok);
+        if (n > 0) {
+            const int lanes = copy_lanes(n), step = 32 / lanes;
+            for (int pr = half * step + lane / lanes; pr < 32; pr += 2 * step) {
+                if (!((valid >> pr) & 1))
+                    continue;
+                const int prow = quarter * 32 + pr;
+                const int plw = prow & ((1 << g.tw_sh) - 1), plh = (prow >> g.tw_sh) & ((1 << g.th_sh) - 1), pln = prow >> (g.tw_sh + g.th_sh);
+                uint8_t *dst = g.y + (((size_t)(tni * g.tn + pln) * g.oh + (thi << g.th_sh) + plh) * g.ow + (twi << g.tw_sh) + plw) * g.cout + k0 + c1;
+                const uint32_t src = base + L.stage + (uint32_t)prow * L.stage_pitch;
+                copy_row(dst, n, lane & (lanes - 1), lanes, [&](int off) { return lds1(src + off); });
             }
         }
     }

@@ -359,7 +359,8 @@ TILING_SHAPES = [(1, 512, 512, 7, 7, 3, 1, 128, False), (1, 256, 64, 14, 13, 3, 
                  (1, 1024, 256, 5, 6, 1, 1, 140, False), (3, 64, 40, 30, 31, 3, 1, 128, True), (40, 64, 272, 30, 31, 1, 1, 101, False),
                  (50, 128, 256, 28, 29, 1, 1, 101, False), (40, 32, 64, 33, 30, 3, 1, 128, True), (40, 24, 100, 30, 31, 1, 1, 128, False),
                  (2, 24, 100, 9, 8, 3, 1, 77, False), (40, 20, 18, 30, 31, 3, 1, 131, False), (2, 7, 33, 12, 11, 3, 2, 128, True),
-                 (2, 3, 32, 33, 35, 7, 2, 60, False), (30, 3, 24, 40, 41, 3, 2, 128, False), (1, 1, 16, 9, 9, 3, 1, 128, False)]
+                 (2, 3, 32, 33, 35, 7, 2, 60, False), (30, 3, 24, 40, 41, 3, 2, 128, False), (1, 1, 16, 9, 9, 3, 1, 128, False),
+                 (1, 512, 219, 9, 7, 3, 1, 128, False), (2, 64, 37, 9, 8, 1, 1, 90, True), (40, 8, 218, 30, 31, 1, 1, 128, False)]
 
 
 @pytest.mark.parametrize("n,c,k,h,w,ks,st,wzp,signed", TILING_SHAPES)
