@@ -18,12 +18,11 @@
 // border class.  The host builds off[class][k] = bias[k] - izp * sum_{taps valid in class} w[k].
 //
 // Warp roles (576 threads, one CTA per SM, persistent over tiles):
-//   warp 0      TMA producer (one lane per pipeline slot)
+//   warp 0      TMA producer (one elected lane)
 //   warp 1      tensor-memory allocation, MMA issue (one elected lane)
 //   warps 2..17 epilogue, two groups of 8 warps (two per tensor-memory lane quarter) or, for narrow
 //               channel tiles with a short mainloop, four groups of 4 warps; group i
 //               owns accumulator stage i: tcgen05.ld -> requantize -> pack -> swizzled smem -> TMA store
-//   warp 18     a second MMA-issuing warp in the instantiations for narrow tiles (MODE 1, 2)
 // One accumulator stage per group in tensor memory lets the epilogue of tile i overlap the mainloop
 // of the next tiles and their epilogues (the other groups).  MODE 3 runs on clusters of two CTAs that
 // share every MMA (tcgen05 cta_group::2, M = 256), each CTA loading its own operands with plain TMA
@@ -45,13 +44,11 @@ constexpr int kMaxAccStages = 4;              // accumulator stages in tensor me
 #define B200_EPI_WARPS 16
 #endif
 constexpr int kEpiWarps = B200_EPI_WARPS;     // split into 2 groups of 8 warps or 4 groups of 4
-constexpr int kMma2Warp = 2 + kEpiWarps;        // the second MMA-issuing warp, behind the epilogue warps
 constexpr int kThreads = 64 + kEpiWarps * 32;
-constexpr int kThreads2 = kThreads + 32;         // with the second MMA-issuing warp
 constexpr int kTileM = 128;
 constexpr int kMaxStages = 8;
 constexpr int kGroupBytes = 32 * 1024;        // target size of one pipeline stage (a group of k-blocks)
-constexpr int kMaxGroup = 10;                 // three stages of a group must fit the producer's 32 lanes
+constexpr int kMaxGroup = 10;
 
 // device status codes (which wait gave up)
 constexpr int kErrProducerWait = 0x101;
@@ -84,7 +81,6 @@ struct IgemmArgs {
     int groups;          // epilogue groups (2 or 4); group i takes every groups-th tile of the CTA
     int acc_stages;      // accumulator stages in tensor memory (a multiple of groups, at most 4)
     int kgroup;          // k-blocks per pipeline stage (divides the k-blocks of a tile): one barrier round trip per group
-    uint32_t rcp_cchunks, rcp_s;   // ceil(2^30 / (c / bk)), ceil(2^30 / s): k-block index -> tap, tap -> row
     int b_resident;      // 1: all k-blocks of B stay in shared memory (one channel tile, weights fit)
     int a_wide;          // 1: 32-channel rows stored pre-swizzled; A is fetched as whole rows of pixels
     int seg_w[2];        // column segments of a tile: widths in bytes (the second may be 0), see epilogue_segments
@@ -457,12 +453,10 @@ __host__ __device__ inline SmemLayout smem_layout(int a_slots, int b_slots, int 
 
 // HAS_RES: the instantiation whose epilogue can add a residual tensor; plans without a fused add run the
 // other one, which carries none of that code.
-// MODE 0: one MMA-issuing warp.  MODE 1 and 2 add a second one (one more warp in the block):
-//   1: the CTA's tiles alternate between the two warps, each on its own half of the stage ring;
-//   2: the CTA's tiles go in pairs that share every weight k-block: a stage holds the activation
-//      tiles of both and ONE weight tile, each warp issues the MMAs of its own tile of the pair.
+// MODE 0: tile by tile.  MODE 2: the CTA's tiles go in pairs that share every weight k-block: a stage holds the activation
+// tiles of both and ONE weight tile.  MODE 3: CTA pairs.
 template <int EPI, bool HAS_RES, bool HAS_WZP, int MODE>
-__global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ IgemmArgs g)
+__global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ IgemmArgs g)
 {
     extern __shared__ uint8_t smem_raw[];
     // the swizzle patterns are functions of the absolute shared address: align the base to 1024
@@ -480,7 +474,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
     const int bnl = PAIR ? g.bn >> 1 : g.bn + kOnes;     // rows of B this CTA holds
     const SmemLayout L = smem_layout(MODE == 2 ? 2 * slots : slots, g.b_resident ? kblocks_all : slots, g.bk, g.bn, g.groups, bnl);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform, and known to be
     const int lane = threadIdx.x & 31;
     const uint32_t a_tile_bytes = (uint32_t)kTileM * g.bk;
     const uint32_t b_tile_bytes = ((uint32_t)bnl * g.bk + 1023u) & ~1023u;
@@ -496,7 +490,7 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
     if (threadIdx.x == 0) {
         for (int s = 0; s < g.stages; ++s) {
             mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), MODE == 2 ? 2 : 1);   // pair mode: both issuing warps release a stage
+            mbar_init(empty_bar(s), 1);
         }
         mbar_init(bres_bar, 1);
         for (int s = 0; s < g.acc_stages; ++s) {
@@ -554,249 +548,251 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
 
     if (warp == 0) {
         // ================= TMA producer =================
-        // The pipeline's k-blocks form one sequence over this CTA's tiles; slot l = q mod slots
-        // (slots = stages * kgroup <= 32) holds k-block q.  Lane l owns slot l for the whole kernel and
-        // issues the loads of k-blocks l, l + slots, ...: the lanes work side by side, so the latency
-        // of one lane's bookkeeping (decode the k-block, wait for the stage, issue) is shared by
-        // `slots` k-blocks.  The first lane of a group posts the group's byte count; a load of another
-        // lane may complete before that (the transaction count is signed), the phase cannot, because
-        // the arrival is still pending.
+        // One thread walks the k-blocks of this CTA's tiles in order: wait for the stage of the next group of k-blocks, post
+        // the group's byte count, issue its loads.  The chain of instructions of one k-block bounds the mainloop (its MMAs take
+        // 64 .. 512 cycles), so addresses and coordinates advance by counters: chunk -> tap -> tile, with what depends on the
+        // tap or the tile worked out when that changes.
         //
-        // With two MMA-issuing warps the ring is split in two halves, one per warp: the lanes of half
-        // r load the k-blocks of the CTA's tiles r, r + 2, ... only, so that every stage barrier has
-        // one consumer that meets its phases in order.
-        const int slots = g.stages * g.kgroup;
-        //
-        // Pair mode: one ring; slot l holds, for k-block q of the PAIR sequence, the activation tiles of
-        // the pair's two tiles and the one weight tile both use (the host has checked that the two
-        // tiles share their channel tile).
-        constexpr int rings = MODE == 1 ? 2 : 1;
-        constexpr int tiles_per_step = (MODE == 0 || MODE == 3) ? 1 : 2;   // tiles a lane moves on by when its k-block wraps
-        const int ring_slots = slots / rings;
-        if (lane < slots && tile0 < total_tiles) {
-            const int stage = lane / g.kgroup;
-            const int ring = lane / ring_slots, rl = lane - ring * ring_slots;
-            const bool first = lane == stage * g.kgroup;
-            const uint32_t fb = full_bar(stage), eb = empty_bar(stage);
-            const uint32_t a_dst = base + L.a + lane * a_tile_bytes * (MODE == 2 ? 2 : 1), b_dst = base + L.b + lane * b_tile_bytes;
+        // Two tiles per stage (MODE 2): a k-block is the activation tiles of both and the one weight tile they share (the host
+        // has checked that).
+        if (tile0 < total_tiles) {
+            const uint32_t bk = g.bk, kgroup = g.kgroup;
             // a CTA pair: the leading CTA's barrier counts the bytes of both CTAs
-            const uint32_t tx_bytes = (a_tile_bytes + (g.b_resident ? 0u : (uint32_t)bnl * g.bk)) * (uint32_t)g.kgroup * (PAIR ? 2u : 1u);
-            const uint32_t fb_lead = PAIR ? cluster_addr(fb, 0) : fb;
+            const uint32_t tx_bytes = (a_tile_bytes + (g.b_resident ? 0u : (uint32_t)bnl * bk)) * kgroup * (PAIR ? 2u : 1u);
+            const uint32_t a_slot = a_tile_bytes * (MODE == 2 ? 2 : 1), b_slot = b_tile_bytes;
             // weights are written once, at preparation: they need not wait for the launch before this one
-            if (g.b_resident && lane == 0) {
+            if (g.b_resident) {
                 // one channel tile and weights that fit: every k-block of B is loaded once and stays
-                mbar_expect_tx(bres_bar, (uint32_t)kblocks * bnl * g.bk);
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    const int tap = kb / cchunks, kc = tap * g.c + (kb - tap * cchunks) * g.bk;
-                    tma_load_2d(base + L.b + kb * b_tile_bytes, &maps.b, bres_bar, kc, 0);
-                    if (HAS_WZP)
-                        tma_load_2d(base + L.b + kb * b_tile_bytes + g.bn * g.bk, &maps.ones, bres_bar, kc, 0);
-                }
-            }
-            const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;   // strides are 1 or 2
-            // this lane's first k-block
-            int kb = rl % kblocks;
-            int tile = tile0;
-            TileWalker tw;
-            walker_init(tw);
-            for (int i = (rl / kblocks) * tiles_per_step + ring; i > 0; --i) {
-                tile += tstride;
-                tw.advance(g);
-            }
-            uint32_t phase = 0;
-            pdl_wait();
-            // Every pass of the loop each lane polls its own stage once (without suspending: a blocked
-            // lane would hold back the ready ones); a lane whose stage is free issues its loads and
-            // moves on to its next k-block, the others poll again in the next pass.  No lane ever waits
-            // for another lane's stage.
-            const unsigned lanes_mask = slots >= 32 ? 0xffffffffu : ((1u << slots) - 1u);
-            bool active = tile < total_tiles;
-            long long t0 = clock64();
-            int spins = 0;
-            while (__any_sync(lanes_mask, active)) {
-                if (active) {
-                    if (mbar_test_wait(eb, phase ^ 1)) {
-                        // k-block -> (tap row, tap column, channel chunk); the divisions are multiplications
-                        // by reciprocals the host rounded up (exact for operands below 2^15)
-                        const int tap = (int)(((uint64_t)(uint32_t)kb * g.rcp_cchunks) >> 30);
-                        const int cc = (kb - tap * cchunks) * g.bk;
-                        const int rr = (int)(((uint64_t)(uint32_t)tap * g.rcp_s) >> 30);
-                        const int ss = tap - rr * g.s;
-                        // input row of output row oh for this tap: ih = oh*stride + d, d = rr - pad
-                        //   = stride * (oh + (d - p) / stride) + p with p = d mod stride (0 <= p < stride)
-                        const int dh = rr - g.pad_h, ph = dh & sh_h;
-                        const int dw = ss - g.pad_w, pw = dw & sh_w;
-                        const int yh = (tw.hi(g) << g.th_sh) + ((dh - ph) >> sh_h);
-                        const int xw = (tw.wi(g) << g.tw_sh) + ((dw - pw) >> sh_w);
-                        const int n0 = tw.ni(g) * g.tn;
-                        const CUtensorMap *amap = &maps.a[ph * 2 + pw];
-                        if (PAIR) {
-                            if (first && leader)
-                                mbar_expect_tx(fb, tx_bytes);
-                            tma_load_4d_pair(a_dst, amap, fb_lead, cc, xw, yh, n0);
-                            tma_load_2d_pair(b_dst, &maps.b, fb_lead, tap * g.c + cc, tw.nt * g.bn + (int)cta_rank * bnl);
-                        } else if (MODE == 2) {
-                            // the pair's second tile (absent behind an odd number of tiles): same tap, its own pixels
-                            const bool second = tile + (int)gridDim.x < total_tiles;
-                            mbar_expect_tx(fb, tx_bytes + (second ? a_tile_bytes : 0u));
-                            tma_load_4d(a_dst, amap, fb, cc, xw, yh, n0);
-                            if (second) {
-                                TileWalker t2 = tw;
-                                t2.advance(g);
-                                tma_load_4d(a_dst + a_tile_bytes, amap, fb, cc, (t2.wi(g) << g.tw_sh) + ((dw - pw) >> sh_w),
-                                            (t2.hi(g) << g.th_sh) + ((dh - ph) >> sh_h), t2.ni(g) * g.tn);
-                            }
-                        } else {
-                        if (first)
-                            mbar_expect_tx(fb, tx_bytes);
-                        if (g.a_wide)   // rows of tw pixels x 32 bytes, in 8-byte elements
-                            tma_load_3d(a_dst, amap, fb, xw << 2, yh, n0);
-                        else
-                            tma_load_4d(a_dst, amap, fb, cc, xw, yh, n0);
-                        }
-                        if (!g.b_resident && !PAIR) {
-                            tma_load_2d(b_dst, &maps.b, fb, tap * g.c + cc, tw.nt * g.bn);
+                if (elect_one())
+                    mbar_expect_tx(bres_bar, (uint32_t)kblocks * bnl * bk);
+                __syncwarp();
+                uint32_t dst = base + L.b;
+                for (int tap = 0; tap < g.r * g.s; ++tap)
+                    for (int c = 0; c < cchunks; ++c, dst += b_slot) {
+                        const int kc = tap * g.c + c * (int)bk;
+                        if (elect_one()) {
+                            tma_load_2d(dst, &maps.b, bres_bar, kc, 0);
                             if (HAS_WZP)
-                                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, fb, tap * g.c + cc, 0);
+                                tma_load_2d(dst + g.bn * bk, &maps.ones, bres_bar, kc, 0);
                         }
-                        phase ^= 1;
-                        kb += ring_slots;
-                        while (kb >= kblocks) {
-                            kb -= kblocks;
-                            for (int i = 0; i < tiles_per_step; ++i) {
-                                tile += tstride;
-                                tw.advance(g);
-                            }
-                        }
-                        active = tile < total_tiles;
-                        t0 = clock64();
-                        spins = 0;
-                    } else if ((++spins & 255) == 0 && (*abort_flag != 0 || clock64() - t0 > kWaitCycles)) {
-                        atomicCAS(g.status, 0, kErrProducerWait);
-                        *abort_flag = 1;
-                        active = false;
                     }
-                }
             }
-        }
-        // every load is on its way: the next launch's blocks may come (a block per SM that waits for longer
-        // would keep the SM from the launches of other streams)
-        pdl_trigger();
-    } else if (warp == 1 || ((MODE == 1 || MODE == 2) && warp == kMma2Warp)) {
-        // ================= MMA issuer =================
-        // The whole warp walks the loop (uniform control flow); lane 0 alone issues.  Descriptors of
-        // one operand differ only in the start-address field, so only their low words are computed.
-        // In a CTA pair the leading CTA's warp issues for both; the peer's has nothing to do.
-        if (leader) {
-            const uint32_t lead = lane == 0 ? 1u : 0u;
-            // warp r of `rings` issuing warps takes the CTA's tiles r, r + rings, ... and the stages
-            // [r * ring_stages, (r + 1) * ring_stages); accumulator stages advance by `rings` as well
-            // In pair mode both warps walk the whole ring, stage by stage together: warp r issues for the
-            // r-th tile of each pair, on the r-th activation tile of the stage and the shared weight tile.
-            constexpr int rings = MODE == 1 ? 2 : 1;
-            constexpr int tile_step = (MODE == 0 || MODE == 3) ? 1 : 2;
-            const int ring = warp == 1 ? 0 : 1;
-            const int ring_stages = g.stages / rings, stage0 = MODE == 1 ? ring * ring_stages : 0;
-            int stage = stage0;
-            uint32_t phase = 0;
-            int as = ring;
-            uint32_t aphase = 0;
-            bool ok = true;
-            const uint64_t adesc0 = make_smem_desc(base + L.a, g.bk);
-            const uint64_t bdesc0 = make_smem_desc(base + L.b, g.bk);
-            const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);        // the same for A and B
-            const uint32_t a_lo0 = (uint32_t)adesc0, b_lo0 = (uint32_t)bdesc0;
-            const uint32_t a_step = a_tile_bytes >> 4, b_step = b_tile_bytes >> 4;   // descriptor address units
-            const uint32_t a_grp = a_step * g.kgroup * (MODE == 2 ? 2 : 1), b_grp = b_step * g.kgroup;
-            const int ksteps_full = g.bk / 32;
-            const int groups = kblocks / g.kgroup;
-            const uint32_t idesc = g.idesc;
-            if (g.b_resident && tile0 < total_tiles && !mbar_wait(bres_bar, 0, abort_flag)) {
-                if (lead)
-                    atomicCAS(g.status, 0, kErrMmaFullWait);
-                *abort_flag = 1;
-                ok = false;
-            }
-            for (int tile = tile0 + ring * tstride; (MODE == 2 ? tile - ring * tstride : tile) < total_tiles && ok;
-                 tile += tile_step * tstride) {
-                // pair mode: the second warp of a pair without a second tile still takes part in the
-                // stage hand-over (its commits arrive at once), it just issues nothing
-                const bool have_tile = MODE != 2 || tile < total_tiles;
-                const uint32_t issue = have_tile ? lead : 0u;
-                if (have_tile && !mbar_wait(tempty_bar(as), aphase ^ 1, abort_flag)) {
-                    if (lead)
-                        atomicCAS(g.status, 0, kErrMmaTmemWait);
-                    *abort_flag = 1;
-                    break;
+            const int groups = kblocks / (int)kgroup;
+            const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;         // strides are 1 or 2
+            const int c_end = cchunks * (int)bk, c_pitch = g.c, taps_w = g.s, pad_w = g.pad_w, pad_h = g.pad_h;
+            const uint32_t bars_end = full_bar(g.stages);
+            uint32_t fb = full_bar(0), a_dst = base + L.a, b_dst = base + L.b, phase = 1;
+            uint32_t fb_lead = PAIR ? cluster_addr(fb, 0) : 0u;
+            const uint32_t fb_lead0 = fb_lead;
+            constexpr uint32_t to_empty = 8u * kMaxStages;
+            int tile = tile0;
+            TileWalker tw, tw2;
+            walker_init(tw);
+            if (MODE == 2)
+                tw2 = tw;
+            pdl_wait();
+            const bool load_b = !g.b_resident, a_wide = MODE != 2 && MODE != 3 && g.a_wide;
+            for (bool ok = true; ok && tile < total_tiles;) {
+                const int x0 = tw.wi(g) << g.tw_sh, y0 = tw.hi(g) << g.th_sh, n0 = tw.ni(g) * g.tn;
+                const int b_row = tw.nt * g.bn + (PAIR ? (int)cta_rank * bnl : 0);
+                bool second = false;
+                int dx2 = 0, dy2 = 0, n2 = 0;
+                if (MODE == 2) {
+                    tw2.advance(g);
+                    second = tile + tstride < total_tiles;
+                    dx2 = (tw2.wi(g) << g.tw_sh) - x0;
+                    dy2 = (tw2.hi(g) << g.th_sh) - y0;
+                    n2 = tw2.ni(g) * g.tn;
                 }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(as * (g.bn + kOnes));
-                uint32_t accumulate = 0;
-                int chunk = 0;        // k-block of the tap
+                const uint32_t tx = tx_bytes + (MODE == 2 && second ? a_tile_bytes : 0u);       // (MODE 2: kgroup is 1)
+                // k-blocks left of the group, of the tap; position of the tap
+                int cc = 0, kc = 0, kc0 = 0, rr = 0, ss = 0;
+                // input row of output row oh for this tap: ih = oh*stride + d, d = rr - pad
+                //   = stride * (oh + (d - p) / stride) + p with p = d mod stride (0 <= p < stride)
+                int dh = -pad_h, ph = dh & sh_h, yh = y0 + ((dh - ph) >> sh_h);
+                int dw = -pad_w, pw = dw & sh_w, xw = x0 + ((dw - pw) >> sh_w);
+                const CUtensorMap *amap = &maps.a[ph * 2 + pw];
                 for (int grp = 0; grp < groups; ++grp) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
-                        if (lead)
-                            atomicCAS(g.status, 0, kErrMmaFullWait);
+                    if (!mbar_wait_warp(fb + to_empty, phase, abort_flag)) {
+                        if (lane == 0)
+                            atomicCAS(g.status, 0, kErrProducerWait);
                         *abort_flag = 1;
                         ok = false;
                         break;
                     }
+                    if ((!PAIR || leader) && elect_one())
+                        mbar_expect_tx(fb, tx);
+                    for (int j = 0; j < (int)kgroup; ++j) {
+                        if (elect_one()) {
+                            if (PAIR) {
+                                tma_load_4d_pair(a_dst, amap, fb_lead, cc, xw, yh, n0);
+                                tma_load_2d_pair(b_dst, &maps.b, fb_lead, kc, b_row);
+                            } else {
+                                if (a_wide)                     // rows of tw pixels x 32 bytes, in 8-byte elements
+                                    tma_load_3d(a_dst, amap, fb, xw << 2, yh, n0);
+                                else
+                                    tma_load_4d(a_dst, amap, fb, cc, xw, yh, n0);
+                                if (MODE == 2 && second)        // the pair's second tile: same tap, its own pixels
+                                    tma_load_4d(a_dst + a_tile_bytes, amap, fb, cc, xw + dx2, yh + dy2, n2);
+                                if (load_b) {
+                                    tma_load_2d(b_dst, &maps.b, fb, kc, b_row);
+                                    if (HAS_WZP)
+                                        tma_load_2d(b_dst + g.bn * bk, &maps.ones, fb, kc, 0);
+                                }
+                            }
+                        }
+                        a_dst += a_slot;
+                        b_dst += b_slot;
+                        cc += bk;
+                        kc += bk;
+                        if (cc >= c_end) {
+                            cc = 0;
+                            kc = kc0 += c_pitch;
+                            ++ss;
+                            if (ss == taps_w) {
+                                ss = 0;
+                                ++rr;
+                                dh = rr - pad_h, ph = dh & sh_h, yh = y0 + ((dh - ph) >> sh_h);
+                            }
+                            dw = ss - pad_w, pw = dw & sh_w, xw = x0 + ((dw - pw) >> sh_w);
+                            amap = &maps.a[ph * 2 + pw];
+                        }
+                    }
+                    fb += 8;
+                    fb_lead += 8;
+                    if (fb == bars_end) {
+                        fb = bar0;
+                        fb_lead = fb_lead0;
+                        a_dst = base + L.a;
+                        b_dst = base + L.b;
+                        phase ^= 1;
+                    }
+                }
+                tile += MODE == 2 ? 2 * tstride : tstride;
+                tw.advance(g);
+                if (MODE == 2) {
+                    tw.advance(g);
+                    tw2.advance(g);
+                }
+            }
+        }
+        __syncwarp();
+        // every load is on its way: the next launch's blocks may come (a block per SM that waits for longer
+        // would keep the SM from the launches of other streams)
+        pdl_trigger();
+    } else if (warp == 1) {
+        // ================= MMA issuer =================
+        // One thread.  Descriptors of one operand differ only in the start-address field, so only their low words are
+        // computed.  In a CTA pair the leading CTA's thread issues for both; the peer's has nothing to do.
+        if (leader) {
+            const int ring = g.stages, kgroup = g.kgroup, ksteps_full = g.bk / 32, last_steps = g.last_steps;
+            int stage = 0;
+            uint32_t phase = 0;
+            int as = 0;
+            uint32_t aphase = 0;
+            bool ok = true;
+            const uint64_t adesc0 = make_smem_desc(base + L.a, g.bk);
+            const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);        // the same for A and B
+            const uint32_t a_lo0 = (uint32_t)adesc0, b_lo0 = (uint32_t)make_smem_desc(base + L.b, g.bk);
+            const uint32_t a_step = (a_tile_bytes >> 4) * (MODE == 2 ? 2 : 1), b_step = b_tile_bytes >> 4;   // descriptor address units
+            uint32_t a_lo = a_lo0, b_lo = b_lo0;
+            const int groups = kblocks / kgroup;
+            const uint32_t idesc = g.idesc, acc_cols = (uint32_t)(g.bn + kOnes);
+            const bool resident = g.b_resident;
+            auto give_up = [&](int code) {
+                if (lane == 0)
+                    atomicCAS(g.status, 0, code);
+                *abort_flag = 1;
+                ok = false;
+            };
+            if (resident && tile0 < total_tiles && !mbar_wait_warp(bres_bar, 0, abort_flag))
+                give_up(kErrMmaFullWait);
+            for (int tile = tile0; tile < total_tiles && ok; tile += MODE == 2 ? 2 * tstride : tstride) {
+                // (MODE 2: the last step may lack the second tile)
+                const bool second = MODE == 2 && tile + tstride < total_tiles;
+                if (!mbar_wait_warp(tempty_bar(as), aphase ^ 1, abort_flag) || (second && !mbar_wait_warp(tempty_bar(as + 1), aphase ^ 1, abort_flag))) {
+                    give_up(kErrMmaTmemWait);
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)as * acc_cols;
+                uint32_t accumulate = 0;
+                int chunk = 0;        // k-block of the tap
+                if (resident)
+                    b_lo = b_lo0;
+                for (int grp = 0; grp < groups; ++grp) {
+                    if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
+                        give_up(kErrMmaFullWait);
+                        break;
+                    }
                     tc_fence_after();
-                    uint32_t a_lo = a_lo0 + stage * a_grp + (MODE == 2 ? ring * a_step : 0u);
-                    uint32_t b_lo = b_lo0 + (g.b_resident ? grp : stage) * b_grp;
-                    for (int j = 0; j < g.kgroup; ++j, a_lo += a_step, b_lo += b_step) {
+                    for (int j = 0; j < kgroup; ++j, a_lo += a_step, b_lo += b_step) {
                         // a k-block is up to 4 MMAs of K = 32 bytes: +2 (16-byte units) inside the swizzle atom
                         int ksteps = ksteps_full;
                         if (++chunk == cchunks) {
                             chunk = 0;
-                            ksteps = g.last_steps;
+                            ksteps = last_steps;
                         }
-                        if (PAIR) {
-                            mma_i8_pair(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, issue);
+                        auto block = [&](uint32_t d, uint32_t a) {
+                            auto mma = [&](int k, uint32_t acc) {
+                                if (PAIR)
+                                    mma_i8_pair(d, a + 2 * k, b_lo + 2 * k, desc_hi, idesc, acc);
+                                else
+                                    mma_i8(d, a + 2 * k, b_lo + 2 * k, desc_hi, idesc, acc);
+                            };
+                            mma(0, accumulate);
                             if (ksteps >= 2)
-                                mma_i8_pair(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, issue);
+                                mma(1, 1);
                             if (ksteps >= 3)
-                                mma_i8_pair(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1, issue);
+                                mma(2, 1);
                             if (ksteps == 4)
-                                mma_i8_pair(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1, issue);
-                            accumulate = 1;
-                            continue;
+                                mma(3, 1);
+                        };
+                        if (elect_one()) {
+                            block(d_tmem, a_lo);
+                            if (MODE == 2 && second)
+                                block(d_tmem + acc_cols, a_lo + (a_tile_bytes >> 4));
                         }
-                        mma_i8(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate, issue);
+                        __syncwarp();
                         accumulate = 1;
-                        if (ksteps >= 2)
-                            mma_i8(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1, issue);
-                        if (ksteps >= 3)
-                            mma_i8(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1, issue);
-                        if (ksteps == 4)
-                            mma_i8(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1, issue);
                     }
-                    if (PAIR) {
-                        // the stage is free again in both CTAs once these MMAs are done: one commit per CTA
-                        mma_commit_pair(cluster_addr(empty_bar(stage), 0), lead);
-                        mma_commit_pair(cluster_addr(empty_bar(stage), 1), lead);
-                    } else
-                    mma_commit(empty_bar(stage), lead);   // frees the smem stage when the group's MMAs are done
-                    if (++stage == stage0 + ring_stages) {
-                        stage = stage0;
+                    if (elect_one()) {
+                        if (PAIR) {
+                            // the stage is free again in both CTAs once these MMAs are done: one commit per CTA
+                            mma_commit_pair(cluster_addr(empty_bar(stage), 0));
+                            mma_commit_pair(cluster_addr(empty_bar(stage), 1));
+                        } else
+                            mma_commit(empty_bar(stage));   // frees the smem stage when the group's MMAs are done
+                        if (grp + 1 == groups) {            // accumulator complete
+                            if (PAIR) {                     // both CTAs' halves of it
+                                mma_commit_pair(cluster_addr(tfull_bar(as), 0));
+                                mma_commit_pair(cluster_addr(tfull_bar(as), 1));
+                            } else
+                                mma_commit(tfull_bar(as));
+                            if (MODE == 2 && second)
+                                mma_commit(tfull_bar(as + 1));
+                        }
+                    }
+                    __syncwarp();
+                    if (++stage == ring) {
+                        stage = 0;
                         phase ^= 1;
+                        a_lo = a_lo0;
+                        if (!resident)
+                            b_lo = b_lo0;
                     }
                 }
                 if (!ok)
                     break;
-                if (PAIR) {
-                    mma_commit_pair(cluster_addr(tfull_bar(as), 0), issue);   // both CTAs' halves of the accumulator
-                    mma_commit_pair(cluster_addr(tfull_bar(as), 1), issue);
-                } else
-                mma_commit(tfull_bar(as), issue);         // accumulator complete
-                as += tile_step;
+                as += MODE == 2 ? 2 : 1;
                 if (as >= g.acc_stages) {
                     as -= g.acc_stages;
                     aphase ^= 1;
                 }
             }
         }
-    } else if (warp < kMma2Warp) {
+        __syncwarp();
+    } else {
         // ================= epilogue (warps 2..17) =================
         // Two independent groups of 8 warps; group i owns accumulator stage i, i.e. every second
         // tile of this CTA, with its own staging buffer, tables and named barriers, so that one
@@ -989,7 +985,6 @@ __global__ void __launch_bounds__((MODE == 1 || MODE == 2) ? kThreads2 : kThread
 // conv_igemm_inst_*.cu, which compile side by side.
 typedef void (*IgemmKernel)(const IgemmMaps, const IgemmArgs);
 IgemmKernel igemm_kernel_mode0(int epi);
-IgemmKernel igemm_kernel_mode1(int epi);
 IgemmKernel igemm_kernel_mode2(int epi);
 IgemmKernel igemm_kernel_mode3(int epi);                // none for variants that only short reductions have
 IgemmKernel igemm_kernel_wzp(int epi);                  // a weight zero point other than 128

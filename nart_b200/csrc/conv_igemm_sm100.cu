@@ -95,10 +95,12 @@ __global__ void __launch_bounds__(128, 1) mma_i8_peak_kernel(int mmas, int *stat
                 phase[b] ^= 1;
             }
             const uint32_t d = tmem_base + (uint32_t)b * 256u;
+            if (elect_one()) {
 #pragma unroll 4
-            for (int j = 0; j < kPeakGroup; ++j)
-                mma_i8(d, a_lo + 2 * (j & 3), b_lo + 2 * (j & 3), desc_hi, idesc, j ? 1u : 0u, lead);
-            mma_commit(smem_u32(&bars[b]), lead);
+                for (int j = 0; j < kPeakGroup; ++j)
+                    mma_i8(d, a_lo + 2 * (j & 3), b_lo + 2 * (j & 3), desc_hi, idesc, j ? 1u : 0u);
+                mma_commit(smem_u32(&bars[b]));
+            }
         }
         // the last groups must have finished before tensor memory goes back
         for (int t = groups < 2 ? 0 : groups - 2; t < groups && ok; ++t) {
@@ -168,7 +170,7 @@ struct ConvIgemmPlan {
     ConvGeom g;
     int groups = 2, acc_stages = 2;
     int cpad = 0;                   // input channels rounded up to a multiple of 32
-    int bk = 0, bn = 0, stages = 0, kgroup = 1, kpad = 0, b_resident = 0, a_wide = 0, mma_warps = 1, pair = 0;
+    int bk = 0, bn = 0, stages = 0, kgroup = 1, kpad = 0, b_resident = 0, a_wide = 0, pair = 0;
     // Two CTAs of a cluster per MMA (kernel MODE 3).  Whether a launch uses it depends on the batch: the pair
     // wins 3-6 % once every cluster walks many tiles and loses a little on short launches (cluster launch,
     // two cluster-wide syncs), so the plan carries both configurations and build_launch picks.
@@ -409,18 +411,6 @@ int conv_igemm_create(
         while (stages > 2 && (!fits(stages, kgroup) || stages * kgroup > 32))
             --stages;
         // a deep ring lets the producer run several tiles ahead when a tile has few k-blocks
-        // Narrow channel tiles make short MMAs, and one thread issues those no faster than one per
-        // ~100 cycles whatever their size: two issuing warps, each on its own half of the ring and on
-        // every second tile, keep the tensor pipe fed (3x3 64-channel layer: 0.082 -> 0.061 ms; 256-wide
-        // tiles gain nothing).
-        p->mma_warps = (p->bn <= 128 && stages >= 4 && !ones) ? 2 : 1;
-        if (const char *e = getenv("B200_IGEMM_MMA_WARPS")) {   // tuning aid: 1, or 2 when the ring has four stages or more
-            int v = atoi(e);
-            if (v == 1 || (v == 2 && stages >= 4 && !ones))
-                p->mma_warps = v;
-        }
-        if (p->mma_warps == 2)
-            stages &= ~1;
         // Pair mode (see the kernel's MODE 2): wide k-blocks of a layer with one channel tile, where the
         // operand loads from L2 set the pace: two tiles per stage share one weight tile.
         // (3x3 128-channel layer 0.047 -> 0.043 ms.  256-wide tiles lose: their two accumulators fill the
@@ -433,7 +423,6 @@ int conv_igemm_create(
                 --st;
             if (fits2(st)) {
                 p->pair = 1;
-                p->mma_warps = 2;
                 stages = st;
             }
         }
@@ -454,7 +443,7 @@ int conv_igemm_create(
                 int st = kMaxStages;
                 while (st > 2 && (!fits_p(st, kgroup) || st * kgroup > 32))
                     --st;
-                if (fits_p(st, kgroup) && p->mma_warps == 1) {
+                if (fits_p(st, kgroup)) {
                     p->pair_ok = 1;
                     p->stages_pair = st;
                 }
@@ -635,8 +624,8 @@ void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
     }
     const bool cta_pair = l && l->cta_pair;
     const char *mode = cta_pair ? "cta-pair (cta_group::2, M=256)" : p->pair ? "tile pairs on one weight tile"
-        : p->pair_ok ? "one issuing warp (cta pairs on long launches)"
-        : p->mma_warps == 2 ? "two issuing warps" : "one issuing warp";
+        : p->pair_ok ? "tile by tile (cta pairs on long launches)"
+        : "tile by tile";
     snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d stages=%d kgroup=%d groups=%d acc_stages=%d %s%s%s%s", p->bn, p->bk,
              cta_pair ? p->stages_pair : p->stages, p->kgroup, p->groups, p->acc_stages, mode, p->b_resident ? ", weights resident" : "",
              p->form == kEpiFp ? ", fp32 epilogue" : p->form == kEpiInt ? ", uniform-shift epilogue" : ", generic requantize",
@@ -844,8 +833,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     a.bk = p->bk; a.bn = p->bn; a.stages = l.cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
     a.cchunks = (p->cpad + p->bk - 1) / p->bk;
     a.last_steps = (p->cpad - (a.cchunks - 1) * p->bk) / 32;
-    a.rcp_cchunks = (uint32_t)(((1ull << 30) + (uint64_t)a.cchunks - 1) / (uint64_t)a.cchunks);
-    a.rcp_s = (uint32_t)(((1ull << 30) + (uint64_t)g.s - 1) / (uint64_t)g.s); a.b_resident = p->b_resident; a.a_wide = p->a_wide;
+    a.b_resident = p->b_resident; a.a_wide = p->a_wide;
     for (a.tw_sh = 0; (1 << a.tw_sh) < a.tw; ++a.tw_sh) {}
     for (a.th_sh = 0; (1 << a.th_sh) < a.th; ++a.th_sh) {}
     // instruction descriptor: D = S32 (2 at bit 4), A = unsigned 8-bit (0 at bit 7), B = signed 8-bit
@@ -899,8 +887,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     l.kernel = res ? igemm_kernel_residual(p->variant)
         : g.wzp_d ? igemm_kernel_wzp(p->variant)
         : l.cta_pair ? igemm_kernel_mode3(p->variant)
-        : p->pair ? igemm_kernel_mode2(p->variant)
-        : p->mma_warps == 2 ? igemm_kernel_mode1(p->variant) : igemm_kernel_mode0(p->variant);
+        : p->pair ? igemm_kernel_mode2(p->variant) : igemm_kernel_mode0(p->variant);
     if (!l.kernel)
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no kernel of epilogue variant %d for this launch", p->variant);
     const int total_tiles = a.tiles_w * a.tiles_h * a.tiles_n * a.n_tiles_n;
@@ -962,8 +949,7 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
     const size_t bytes = (size_t)n * ((size_t)p->g.h * p->g.w * p->g.c + (size_t)p->g.oh * p->g.ow * p->g.k) + p->w_bytes;
     if (l.small)
         return conv_small_launch(l.smaps, l.sargs, l.m_tiles, l.smem, bytes, st);
-    const bool two_warps = l.cta_pair == 0 && res == nullptr && p->g.wzp_d == 0 && (p->pair || p->mma_warps == 2);
-    return launch_kernel(l.kernel, l.grid, dim3(two_warps ? kThreads2 : kThreads), l.smem, st, bytes, l.cta_pair ? 2 : 1, l.maps, l.args);
+    return launch_kernel(l.kernel, l.grid, dim3(kThreads), l.smem, st, bytes, l.cta_pair ? 2 : 1, l.maps, l.args);
 }
 
 // Everything the first launch of any plan would otherwise do once per process or device: the driver
@@ -975,7 +961,7 @@ int conv_igemm_warm()
         return fail(B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     B200_TRY(conv_small_warm());
     for (int epi = 0; epi < kEpiVariants; ++epi)
-        for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode1(epi), igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
+        for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
                                igemm_kernel_wzp(epi), igemm_kernel_residual(epi) })
             if (k)
                 B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));

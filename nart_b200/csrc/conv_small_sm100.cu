@@ -183,57 +183,68 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
 
     if (warp == 0) {
         // ================= TMA =================
-        const uint32_t tx = a_tile + (uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk;
-        const uint32_t a_dst = base + lane * a_tile, b_dst = base + L.b + lane * L.b_tile;
-        const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;
-        auto load_b = [&](int kb) {
-            const int tap = kb / g.cchunks, kc = tap * g.cpad + (kb - tap * g.cchunks) * g.bk;
-            mbar_expect_tx(full_bar(lane), tx);
-            tma_load_2d(b_dst, &maps.b, full_bar(lane), kc, k0);
-            if (g.wzp_d)
-                tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(lane), kc, 0);
-        };
-        int kb = kb0 + lane;
-        bool active = lane < g.slots && kb < kb1;
-        if (active)
-            load_b(kb);             // weights are constant: the launch before this one does not matter to them
-        pdl_wait();
-        bool first = true;
-        uint32_t phase = 0;
-        long long t0 = clock64();
-        int spins = 0;
-        while (__any_sync(0xffffffffu, active)) {
-            if (active) {
-                if (first || mbar_test_wait(empty_bar(lane), phase ^ 1)) {
-                    if (!first)
-                        load_b(kb);
-                    const int tap = kb / g.cchunks, cc = (kb - tap * g.cchunks) * g.bk;
-                    const int rr = tap / g.s, ss = tap - rr * g.s;
-                    // see the producer of conv_igemm_i8_kernel
-                    const int dh = rr - g.pad_h, ph = dh & sh_h, dw = ss - g.pad_w, pw = dw & sh_w;
-                    const int yh = (thi << g.th_sh) + ((dh - ph) >> sh_h), xw = (twi << g.tw_sh) + ((dw - pw) >> sh_w), n0 = tni * g.tn;
-                    const CUtensorMap *amap = &maps.a[ph * 2 + pw];
-                    if (g.a_wide)
-                        tma_load_3d(a_dst, amap, full_bar(lane), xw << 2, yh, n0);
-                    else
-                        tma_load_4d(a_dst, amap, full_bar(lane), cc, xw, yh, n0);
-                    first = false;
+        // one thread, in order: the weights of the first `slots` k-blocks (constant, the launch before this one does not matter
+        // to them), and behind its wait the k-blocks one by one
+        if (elect_one()) {
+            const uint32_t tx = a_tile + (uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk;
+            const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;
+            auto load_b = [&](int slot, int kc) {
+                const uint32_t b_dst = base + L.b + slot * L.b_tile;
+                mbar_expect_tx(full_bar(slot), tx);
+                tma_load_2d(b_dst, &maps.b, full_bar(slot), kc, k0);
+                if (g.wzp_d)
+                    tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(slot), kc, 0);
+            };
+            const int tap0 = kb0 / g.cchunks, chunk0 = kb0 - tap0 * g.cchunks;
+            int chunk = chunk0, tap_c = tap0 * g.cpad;
+            auto advance = [&] {
+                if (++chunk == g.cchunks) {
+                    chunk = 0;
+                    tap_c += g.cpad;
+                    return true;
+                }
+                return false;
+            };
+            for (int kb = kb0, slot = 0; slot < g.slots && kb < kb1; ++kb, ++slot) {
+                load_b(slot, tap_c + chunk * g.bk);
+                advance();
+            }
+            pdl_wait();
+            chunk = chunk0;
+            tap_c = tap0 * g.cpad;
+            int rr = tap0 / g.s, ss = tap0 - rr * g.s, slot = 0;
+            uint32_t phase = 1;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (kb >= kb0 + g.slots) {
+                    if (!mbar_wait(empty_bar(slot), phase, abort_flag)) {
+                        atomicCAS(g.status, 0, kErrSmallProducer);
+                        *abort_flag = 1;
+                        break;
+                    }
+                    load_b(slot, tap_c + chunk * g.bk);
+                }
+                // see the producer of conv_igemm_i8_kernel
+                const int dh = rr - g.pad_h, ph = dh & sh_h, dw = ss - g.pad_w, pw = dw & sh_w;
+                const int yh = (thi << g.th_sh) + ((dh - ph) >> sh_h), xw = (twi << g.tw_sh) + ((dw - pw) >> sh_w), n0 = tni * g.tn;
+                const CUtensorMap *amap = &maps.a[ph * 2 + pw];
+                if (g.a_wide)
+                    tma_load_3d(base + slot * a_tile, amap, full_bar(slot), xw << 2, yh, n0);
+                else
+                    tma_load_4d(base + slot * a_tile, amap, full_bar(slot), chunk * g.bk, xw, yh, n0);
+                if (advance() && ++ss == g.s) {
+                    ss = 0;
+                    ++rr;
+                }
+                if (++slot == g.slots) {
+                    slot = 0;
                     phase ^= 1;
-                    kb += g.slots;
-                    active = kb < kb1;
-                    t0 = clock64();
-                    spins = 0;
-                } else if ((++spins & 255) == 0 && (*abort_flag != 0 || clock64() - t0 > kWaitCycles)) {
-                    atomicCAS(g.status, 0, kErrSmallProducer);
-                    *abort_flag = 1;
-                    active = false;
                 }
             }
         }
+        __syncwarp();
         pdl_trigger();
     } else if (warp == 1) {
         // ================= MMA =================
-        const uint32_t lead = lane == 0 ? 1u : 0u;
         const uint64_t adesc0 = make_smem_desc(base, g.bk), bdesc0 = make_smem_desc(base + L.b, g.bk);
         const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);
         int slot = 0, chunk = kb0 % g.cchunks;
@@ -241,7 +252,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
         bool ok = true;
         for (int kb = kb0; kb < kb1; ++kb) {
             if (!mbar_wait(full_bar(slot), phase, abort_flag)) {
-                if (lead)
+                if (lane == 0)
                     atomicCAS(g.status, 0, kErrSmallFull);
                 *abort_flag = 1;
                 ok = false;
@@ -251,19 +262,22 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
             const uint32_t a_lo = (uint32_t)adesc0 + slot * (a_tile >> 4), b_lo = (uint32_t)bdesc0 + slot * (L.b_tile >> 4);
             const int ksteps = chunk == g.cchunks - 1 ? g.last_steps : g.bk / 32;
             chunk = chunk == g.cchunks - 1 ? 0 : chunk + 1;
-            for (int j = 0; j < ksteps; ++j) {
-                mma_i8(tmem_base, a_lo + 2 * j, b_lo + 2 * j, desc_hi, g.idesc, accumulate, lead);
-                accumulate = 1;
+            if (elect_one()) {
+                for (int j = 0; j < ksteps; ++j) {
+                    mma_i8(tmem_base, a_lo + 2 * j, b_lo + 2 * j, desc_hi, g.idesc, accumulate);
+                    accumulate = 1;
+                }
+                if (kb + g.slots < kb1)
+                    mma_commit(empty_bar(slot));
             }
-            if (kb + g.slots < kb1)
-                mma_commit(empty_bar(slot), lead);
+            accumulate = 1;
             if (++slot == g.slots) {
                 slot = 0;
                 phase ^= 1;
             }
         }
-        if (ok)
-            mma_commit(acc_bar, lead);
+        if (ok && elect_one())
+            mma_commit(acc_bar);
     }
 
     // ================= epilogue (warps 2..9) =================

@@ -67,6 +67,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return true;
 }
 
+// The same for a converged warp: one answer for all lanes, which the compiler knows to be uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3)
 {
     asm volatile(
@@ -168,53 +174,51 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols)
 // One MMA over both CTAs of a pair (M = 256): rows 0..127 of A and D live in the leading CTA, rows 128..255 in
 // its peer, each CTA holds half of B's rows; the descriptors are this (the leading) CTA's shared addresses.
 __device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
-                                            uint32_t accumulate, uint32_t issue)
+                                            uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
         "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
         "mov.b64 da, {%1, %3};\n\t"
         "mov.b64 db, {%2, %3};\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(issue)
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // Arrival on `bar` (a shared::cluster address, this CTA's or the peer's) when every MMA of the pair issued so
 // far has completed.  One such commit per CTA that has to hear of it: no multicast form is used.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint32_t issue)
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar)
 {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(bar), "r"(issue)
-        : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// True in one lane of the (converged) warp, always the same one.  Single-thread instructions -- MMAs, commits, TMA
+// copies -- stand directly under this, in loops that the whole warp walks with uniform counters: their operands then live
+// in uniform registers.  Under a comparison of the lane number, or in a loop that one lane walks alone, the compiler cannot
+// tell that one lane is active and wraps each of them in a walk over the active lanes (four MMAs and a commit cost the
+// issuing warp ~450 cycles that way).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
 }
 // D[tmem] (+)= A[smem] * B[smem]^T, 8-bit integer operands, int32 accumulate.  The descriptors
-// come as low words plus the high word both share; `issue` predicates the instruction.
-__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
-                                       uint32_t accumulate, uint32_t issue)
+// come as low words plus the high word both share.
+__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
         "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
         "mov.b64 da, {%1, %3};\n\t"
         "mov.b64 db, {%2, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(issue)
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // The barrier gets one arrival when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint32_t bar, uint32_t issue)
+__device__ __forceinline__ void mma_commit(uint32_t bar)
 {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(bar), "r"(issue)
-        : "memory");
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
 {
