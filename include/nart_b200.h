@@ -121,6 +121,7 @@ B200_API void b200_get_quant_scale(float x, int bits, uint32_t *mult, int8_t *sh
  *   B200_IGEMM_GROUPS=<2|4>                  epilogue groups (4 needs four accumulators in tensor memory)
  *   B200_IGEMM_ACC=<2|4>                     accumulator stages in tensor memory
  *   B200_IGEMM_KGROUP=<1..10>                k-blocks per pipeline stage (must divide a tile's k-blocks)
+ *   B200_IGEMM_RINGS=<1|2>                   pipelines per block
  *   B200_IGEMM_PAIR=0                        never pair tiles on one weight tile
  *   B200_IGEMM_CTA_PAIR=<0|1>                never / wherever possible run on CTA pairs (tcgen05 cta_group::2)
  *   B200_IGEMM_SMALL=<0|BNxS>                never one tile per CTA or cluster (launches that leave SMs without a tile), or

@@ -23,6 +23,7 @@
 //   warps 2..17 epilogue, two groups of 8 warps (two per tensor-memory lane quarter) or, for narrow
 //               channel tiles with a short mainloop, four groups of 4 warps; group i
 //               owns accumulator stage i: tcgen05.ld -> requantize -> pack -> swizzled smem -> TMA store
+//   warps 18, 19  the producer and the MMA issuer of a second pipeline (MODE 1)
 // One accumulator stage per group in tensor memory lets the epilogue of tile i overlap the mainloop
 // of the next tiles and their epilogues (the other groups).  MODE 3 runs on clusters of two CTAs that
 // share every MMA (tcgen05 cta_group::2, M = 256), each CTA loading its own operands with plain TMA
@@ -45,6 +46,8 @@ constexpr int kMaxAccStages = 4;              // accumulator stages in tensor me
 #endif
 constexpr int kEpiWarps = B200_EPI_WARPS;     // split into 2 groups of 8 warps or 4 groups of 4
 constexpr int kThreads = 64 + kEpiWarps * 32;
+constexpr int kRing1Warp = 2 + kEpiWarps;       // MODE 1: the second pipeline's producer, and behind it its MMA issuer
+constexpr int kThreads2 = kThreads + 64;
 constexpr int kTileM = 128;
 constexpr int kMaxStages = 8;
 constexpr int kGroupBytes = 32 * 1024;        // target size of one pipeline stage (a group of k-blocks)
@@ -453,10 +456,11 @@ __host__ __device__ inline SmemLayout smem_layout(int a_slots, int b_slots, int 
 
 // HAS_RES: the instantiation whose epilogue can add a residual tensor; plans without a fused add run the
 // other one, which carries none of that code.
-// MODE 0: tile by tile.  MODE 2: the CTA's tiles go in pairs that share every weight k-block: a stage holds the activation
+// MODE 0: tile by tile.  MODE 1: two pipelines, each with its own producer, MMA issuer and half of the stages, take the CTA's
+// tiles in turn: the producer's and the issuer's chains of instructions set the pace of short k-blocks.  MODE 2: the CTA's tiles go in pairs that share every weight k-block: a stage holds the activation
 // tiles of both and ONE weight tile.  MODE 3: CTA pairs.
 template <int EPI, bool HAS_RES, bool HAS_WZP, int MODE>
-__global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ IgemmArgs g)
+__global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ IgemmArgs g)
 {
     extern __shared__ uint8_t smem_raw[];
     // the swizzle patterns are functions of the absolute shared address: align the base to 1024
@@ -546,7 +550,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
     const int cchunks = g.cchunks;
     const int kblocks = g.r * g.s * cchunks;
 
-    if (warp == 0) {
+    // this warp's pipeline (MODE 1), its stages and its first tile
+    constexpr int tile_step = MODE == 1 || MODE == 2 ? 2 : 1;
+    const int ring = MODE == 1 && warp >= kRing1Warp ? 1 : 0, ring_stages = MODE == 1 ? g.stages >> 1 : g.stages;
+    const int ring_tile0 = tile0 + ring * tstride, stage0 = ring * ring_stages;
+    if (warp == 0 || (MODE == 1 && warp == kRing1Warp)) {
         // ================= TMA producer =================
         // One thread walks the k-blocks of this CTA's tiles in order: wait for the stage of the next group of k-blocks, post
         // the group's byte count, issue its loads.  The chain of instructions of one k-block bounds the mainloop (its MMAs take
@@ -555,13 +563,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
         //
         // Two tiles per stage (MODE 2): a k-block is the activation tiles of both and the one weight tile they share (the host
         // has checked that).
-        if (tile0 < total_tiles) {
+        if (ring_tile0 < total_tiles) {
             const uint32_t bk = g.bk, kgroup = g.kgroup;
             // a CTA pair: the leading CTA's barrier counts the bytes of both CTAs
             const uint32_t tx_bytes = (a_tile_bytes + (g.b_resident ? 0u : (uint32_t)bnl * bk)) * kgroup * (PAIR ? 2u : 1u);
             const uint32_t a_slot = a_tile_bytes * (MODE == 2 ? 2 : 1), b_slot = b_tile_bytes;
             // weights are written once, at preparation: they need not wait for the launch before this one
-            if (g.b_resident) {
+            if (g.b_resident && ring == 0) {
                 // one channel tile and weights that fit: every k-block of B is loaded once and stays
                 if (elect_one())
                     mbar_expect_tx(bres_bar, (uint32_t)kblocks * bnl * bk);
@@ -580,14 +588,17 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
             const int groups = kblocks / (int)kgroup;
             const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;         // strides are 1 or 2
             const int c_end = cchunks * (int)bk, c_pitch = g.c, taps_w = g.s, pad_w = g.pad_w, pad_h = g.pad_h;
-            const uint32_t bars_end = full_bar(g.stages);
-            uint32_t fb = full_bar(0), a_dst = base + L.a, b_dst = base + L.b, phase = 1;
+            const uint32_t bars0 = full_bar(stage0), bars_end = full_bar(stage0 + ring_stages);
+            const uint32_t a_dst0 = base + L.a + (uint32_t)(stage0 * g.kgroup) * a_slot, b_dst0 = base + L.b + (uint32_t)(stage0 * g.kgroup) * b_slot;
+            uint32_t fb = bars0, a_dst = a_dst0, b_dst = b_dst0, phase = 1;
             uint32_t fb_lead = PAIR ? cluster_addr(fb, 0) : 0u;
             const uint32_t fb_lead0 = fb_lead;
             constexpr uint32_t to_empty = 8u * kMaxStages;
-            int tile = tile0;
+            int tile = ring_tile0;
             TileWalker tw, tw2;
             walker_init(tw);
+            if (MODE == 1 && ring == 1)
+                tw.advance(g);
             if (MODE == 2)
                 tw2 = tw;
             pdl_wait();
@@ -661,40 +672,42 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
                     fb += 8;
                     fb_lead += 8;
                     if (fb == bars_end) {
-                        fb = bar0;
+                        fb = bars0;
                         fb_lead = fb_lead0;
-                        a_dst = base + L.a;
-                        b_dst = base + L.b;
+                        a_dst = a_dst0;
+                        b_dst = b_dst0;
                         phase ^= 1;
                     }
                 }
-                tile += MODE == 2 ? 2 * tstride : tstride;
+                tile += tile_step * tstride;
                 tw.advance(g);
-                if (MODE == 2) {
+                if (tile_step == 2)
                     tw.advance(g);
+                if (MODE == 2)
                     tw2.advance(g);
-                }
             }
         }
         __syncwarp();
         // every load is on its way: the next launch's blocks may come (a block per SM that waits for longer
         // would keep the SM from the launches of other streams)
-        pdl_trigger();
-    } else if (warp == 1) {
+        if (ring == 0)
+            pdl_trigger();
+    } else if (warp == 1 || (MODE == 1 && warp == kRing1Warp + 1)) {
         // ================= MMA issuer =================
         // One thread.  Descriptors of one operand differ only in the start-address field, so only their low words are
         // computed.  In a CTA pair the leading CTA's thread issues for both; the peer's has nothing to do.
         if (leader) {
-            const int ring = g.stages, kgroup = g.kgroup, ksteps_full = g.bk / 32, last_steps = g.last_steps;
-            int stage = 0;
+            const int kgroup = g.kgroup, ksteps_full = g.bk / 32, last_steps = g.last_steps;
+            int stage = stage0;
             uint32_t phase = 0;
-            int as = 0;
+            int as = ring;
             uint32_t aphase = 0;
             bool ok = true;
             const uint64_t adesc0 = make_smem_desc(base + L.a, g.bk);
             const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);        // the same for A and B
-            const uint32_t a_lo0 = (uint32_t)adesc0, b_lo0 = (uint32_t)make_smem_desc(base + L.b, g.bk);
             const uint32_t a_step = (a_tile_bytes >> 4) * (MODE == 2 ? 2 : 1), b_step = b_tile_bytes >> 4;   // descriptor address units
+            const uint32_t a_lo0 = (uint32_t)adesc0 + (uint32_t)(stage0 * kgroup) * a_step;
+            const uint32_t b_lo0 = (uint32_t)make_smem_desc(base + L.b, g.bk) + (g.b_resident ? 0u : (uint32_t)(stage0 * kgroup) * b_step);
             uint32_t a_lo = a_lo0, b_lo = b_lo0;
             const int groups = kblocks / kgroup;
             const uint32_t idesc = g.idesc, acc_cols = (uint32_t)(g.bn + kOnes);
@@ -705,9 +718,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
                 *abort_flag = 1;
                 ok = false;
             };
-            if (resident && tile0 < total_tiles && !mbar_wait_warp(bres_bar, 0, abort_flag))
+            if (resident && ring_tile0 < total_tiles && !mbar_wait_warp(bres_bar, 0, abort_flag))
                 give_up(kErrMmaFullWait);
-            for (int tile = tile0; tile < total_tiles && ok; tile += MODE == 2 ? 2 * tstride : tstride) {
+            for (int tile = ring_tile0; tile < total_tiles && ok; tile += tile_step * tstride) {
                 // (MODE 2: the last step may lack the second tile)
                 const bool second = MODE == 2 && tile + tstride < total_tiles;
                 if (!mbar_wait_warp(tempty_bar(as), aphase ^ 1, abort_flag) || (second && !mbar_wait_warp(tempty_bar(as + 1), aphase ^ 1, abort_flag))) {
@@ -774,8 +787,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
                         }
                     }
                     __syncwarp();
-                    if (++stage == ring) {
-                        stage = 0;
+                    if (++stage == stage0 + ring_stages) {
+                        stage = stage0;
                         phase ^= 1;
                         a_lo = a_lo0;
                         if (!resident)
@@ -784,7 +797,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
                 }
                 if (!ok)
                     break;
-                as += MODE == 2 ? 2 : 1;
+                as += tile_step;
                 if (as >= g.acc_stages) {
                     as -= g.acc_stages;
                     aphase ^= 1;
@@ -985,6 +998,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_igemm_i8_kernel(const __grid
 // conv_igemm_inst_*.cu, which compile side by side.
 typedef void (*IgemmKernel)(const IgemmMaps, const IgemmArgs);
 IgemmKernel igemm_kernel_mode0(int epi);
+IgemmKernel igemm_kernel_mode1(int epi);
 IgemmKernel igemm_kernel_mode2(int epi);
 IgemmKernel igemm_kernel_mode3(int epi);                // none for variants that only short reductions have
 IgemmKernel igemm_kernel_wzp(int epi);                  // a weight zero point other than 128

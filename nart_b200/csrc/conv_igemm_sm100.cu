@@ -170,7 +170,7 @@ struct ConvIgemmPlan {
     ConvGeom g;
     int groups = 2, acc_stages = 2;
     int cpad = 0;                   // input channels rounded up to a multiple of 32
-    int bk = 0, bn = 0, stages = 0, kgroup = 1, kpad = 0, b_resident = 0, a_wide = 0, pair = 0;
+    int bk = 0, bn = 0, stages = 0, kgroup = 1, kpad = 0, b_resident = 0, a_wide = 0, rings = 1, pair = 0;
     // Two CTAs of a cluster per MMA (kernel MODE 3).  Whether a launch uses it depends on the batch: the pair
     // wins 3-6 % once every cluster walks many tiles and loses a little on short launches (cluster launch,
     // two cluster-wide syncs), so the plan carries both configurations and build_launch picks.
@@ -411,6 +411,16 @@ int conv_igemm_create(
         while (stages > 2 && (!fits(stages, kgroup) || stages * kgroup > 32))
             --stages;
         // a deep ring lets the producer run several tiles ahead when a tile has few k-blocks
+        // Two pipelines (the kernel's MODE 1) where the k-blocks are short: an MMA of a tile this narrow takes 64 cycles or
+        // less, and one producer thread needs ~300 cycles for a k-block (3x3 64-channel layer, 56x56, batch 256: 84 -> 51 us).
+        p->rings = (p->bn <= 128 && stages >= 4 && !ones) ? 2 : 1;
+        if (const char *e = getenv("B200_IGEMM_RINGS")) {   // tuning aid: 1, or 2 when the ring has four stages or more
+            int v = atoi(e);
+            if (v == 1 || (v == 2 && stages >= 4 && !ones))
+                p->rings = v;
+        }
+        if (p->rings == 2)
+            stages &= ~1;
         // Pair mode (see the kernel's MODE 2): wide k-blocks of a layer with one channel tile, where the
         // operand loads from L2 set the pace: two tiles per stage share one weight tile.
         // (3x3 128-channel layer 0.047 -> 0.043 ms.  256-wide tiles lose: their two accumulators fill the
@@ -423,6 +433,7 @@ int conv_igemm_create(
                 --st;
             if (fits2(st)) {
                 p->pair = 1;
+                p->rings = 1;
                 stages = st;
             }
         }
@@ -443,7 +454,7 @@ int conv_igemm_create(
                 int st = kMaxStages;
                 while (st > 2 && (!fits_p(st, kgroup) || st * kgroup > 32))
                     --st;
-                if (fits_p(st, kgroup)) {
+                if (fits_p(st, kgroup) && p->rings == 1) {
                     p->pair_ok = 1;
                     p->stages_pair = st;
                 }
@@ -625,7 +636,7 @@ void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
     const bool cta_pair = l && l->cta_pair;
     const char *mode = cta_pair ? "cta-pair (cta_group::2, M=256)" : p->pair ? "tile pairs on one weight tile"
         : p->pair_ok ? "tile by tile (cta pairs on long launches)"
-        : "tile by tile";
+        : p->rings == 2 ? "two pipelines" : "tile by tile";
     snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d stages=%d kgroup=%d groups=%d acc_stages=%d %s%s%s%s", p->bn, p->bk,
              cta_pair ? p->stages_pair : p->stages, p->kgroup, p->groups, p->acc_stages, mode, p->b_resident ? ", weights resident" : "",
              p->form == kEpiFp ? ", fp32 epilogue" : p->form == kEpiInt ? ", uniform-shift epilogue" : ", generic requantize",
@@ -887,7 +898,8 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     l.kernel = res ? igemm_kernel_residual(p->variant)
         : g.wzp_d ? igemm_kernel_wzp(p->variant)
         : l.cta_pair ? igemm_kernel_mode3(p->variant)
-        : p->pair ? igemm_kernel_mode2(p->variant) : igemm_kernel_mode0(p->variant);
+        : p->pair ? igemm_kernel_mode2(p->variant)
+        : p->rings == 2 ? igemm_kernel_mode1(p->variant) : igemm_kernel_mode0(p->variant);
     if (!l.kernel)
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no kernel of epilogue variant %d for this launch", p->variant);
     const int total_tiles = a.tiles_w * a.tiles_h * a.tiles_n * a.n_tiles_n;
@@ -949,7 +961,8 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
     const size_t bytes = (size_t)n * ((size_t)p->g.h * p->g.w * p->g.c + (size_t)p->g.oh * p->g.ow * p->g.k) + p->w_bytes;
     if (l.small)
         return conv_small_launch(l.smaps, l.sargs, l.m_tiles, l.smem, bytes, st);
-    return launch_kernel(l.kernel, l.grid, dim3(kThreads), l.smem, st, bytes, l.cta_pair ? 2 : 1, l.maps, l.args);
+    const bool two_rings = !l.cta_pair && !res && p->g.wzp_d == 0 && !p->pair && p->rings == 2;
+    return launch_kernel(l.kernel, l.grid, dim3(two_rings ? kThreads2 : kThreads), l.smem, st, bytes, l.cta_pair ? 2 : 1, l.maps, l.args);
 }
 
 // Everything the first launch of any plan would otherwise do once per process or device: the driver
@@ -961,7 +974,7 @@ int conv_igemm_warm()
         return fail(B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     B200_TRY(conv_small_warm());
     for (int epi = 0; epi < kEpiVariants; ++epi)
-        for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
+        for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode1(epi), igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
                                igemm_kernel_wzp(epi), igemm_kernel_residual(epi) })
             if (k)
                 B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
