@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
     const uint32_t base = (raw_addr + 1023u) & ~1023u;
     uint8_t *smem = smem_raw + (base - raw_addr);
     const SmallLayout L = small_layout(g);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // (the warp: known to be uniform)
     const uint32_t bars = base + L.bars;
     auto full_bar = [&](int s) { return bars + 8u * s; };
     auto empty_bar = [&](int s) { return bars + 8u * (kSmallSlots + s); };
@@ -183,17 +183,19 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
 
     if (warp == 0) {
         // ================= TMA =================
-        // one thread, in order: the weights of the first `slots` k-blocks (constant, the launch before this one does not matter
-        // to them), and behind its wait the k-blocks one by one
-        if (elect_one()) {
+        // in order: the weights of the first `slots` k-blocks (constant, the launch before this one does not matter to them),
+        // and behind its wait the k-blocks one by one; uniform loops around elect_one(), see there
+        {
             const uint32_t tx = a_tile + (uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk;
             const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;
             auto load_b = [&](int slot, int kc) {
                 const uint32_t b_dst = base + L.b + slot * L.b_tile;
-                mbar_expect_tx(full_bar(slot), tx);
-                tma_load_2d(b_dst, &maps.b, full_bar(slot), kc, k0);
-                if (g.wzp_d)
-                    tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(slot), kc, 0);
+                if (elect_one()) {
+                    mbar_expect_tx(full_bar(slot), tx);
+                    tma_load_2d(b_dst, &maps.b, full_bar(slot), kc, k0);
+                    if (g.wzp_d)
+                        tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(slot), kc, 0);
+                }
             };
             const int tap0 = kb0 / g.cchunks, chunk0 = kb0 - tap0 * g.cchunks;
             int chunk = chunk0, tap_c = tap0 * g.cpad;
@@ -216,8 +218,9 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
             uint32_t phase = 1;
             for (int kb = kb0; kb < kb1; ++kb) {
                 if (kb >= kb0 + g.slots) {
-                    if (!mbar_wait(empty_bar(slot), phase, abort_flag)) {
-                        atomicCAS(g.status, 0, kErrSmallProducer);
+                    if (!mbar_wait_warp(empty_bar(slot), phase, abort_flag)) {
+                        if (lane == 0)
+                            atomicCAS(g.status, 0, kErrSmallProducer);
                         *abort_flag = 1;
                         break;
                     }
@@ -227,10 +230,12 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 const int dh = rr - g.pad_h, ph = dh & sh_h, dw = ss - g.pad_w, pw = dw & sh_w;
                 const int yh = (thi << g.th_sh) + ((dh - ph) >> sh_h), xw = (twi << g.tw_sh) + ((dw - pw) >> sh_w), n0 = tni * g.tn;
                 const CUtensorMap *amap = &maps.a[ph * 2 + pw];
-                if (g.a_wide)
-                    tma_load_3d(base + slot * a_tile, amap, full_bar(slot), xw << 2, yh, n0);
-                else
-                    tma_load_4d(base + slot * a_tile, amap, full_bar(slot), chunk * g.bk, xw, yh, n0);
+                if (elect_one()) {
+                    if (g.a_wide)
+                        tma_load_3d(base + slot * a_tile, amap, full_bar(slot), xw << 2, yh, n0);
+                    else
+                        tma_load_4d(base + slot * a_tile, amap, full_bar(slot), chunk * g.bk, xw, yh, n0);
+                }
                 if (advance() && ++ss == g.s) {
                     ss = 0;
                     ++rr;
@@ -251,7 +256,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
         uint32_t phase = 0, accumulate = 0;
         bool ok = true;
         for (int kb = kb0; kb < kb1; ++kb) {
-            if (!mbar_wait(full_bar(slot), phase, abort_flag)) {
+            if (!mbar_wait_warp(full_bar(slot), phase, abort_flag)) {
                 if (lane == 0)
                     atomicCAS(g.status, 0, kErrSmallFull);
                 *abort_flag = 1;
@@ -263,13 +268,17 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
             const int ksteps = chunk == g.cchunks - 1 ? g.last_steps : g.bk / 32;
             chunk = chunk == g.cchunks - 1 ? 0 : chunk + 1;
             if (elect_one()) {
-                for (int j = 0; j < ksteps; ++j) {
-                    mma_i8(tmem_base, a_lo + 2 * j, b_lo + 2 * j, desc_hi, g.idesc, accumulate);
-                    accumulate = 1;
-                }
+                mma_i8(tmem_base, a_lo, b_lo, desc_hi, g.idesc, accumulate);
+                if (ksteps >= 2)
+                    mma_i8(tmem_base, a_lo + 2, b_lo + 2, desc_hi, g.idesc, 1);
+                if (ksteps >= 3)
+                    mma_i8(tmem_base, a_lo + 4, b_lo + 4, desc_hi, g.idesc, 1);
+                if (ksteps == 4)
+                    mma_i8(tmem_base, a_lo + 6, b_lo + 6, desc_hi, g.idesc, 1);
                 if (kb + g.slots < kb1)
                     mma_commit(empty_bar(slot));
             }
+            __syncwarp();
             accumulate = 1;
             if (++slot == g.slots) {
                 slot = 0;
