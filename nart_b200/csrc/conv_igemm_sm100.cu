@@ -1,5 +1,6 @@
 // Host side of the implicit-GEMM convolution (kernels: conv_igemm_kernel.cuh, conv_small_sm100.cu): plans -- weights
 // repacked, tiling, epilogue form and constants -- and launches, with their tensor maps.
+#include <atomic>
 #include <cuda.h>
 #include <math.h>
 #include <stdlib.h>
@@ -179,6 +180,7 @@ struct ConvIgemmPlan {
     int n_row_cls = 0, n_col_cls = 0;
     int seg_w[2] = { 0, 0 };        // see epilogue_segments
     int form = kEpiGeneric, variant = kEpiAny, ushift = 0, rnd_hi = 0;      // see EpiForm, EpiVariant
+    uint8_t *block_dev = nullptr;   // the device memory behind all of these
     int8_t *w_dev = nullptr;        // [kpad][r][s][c]
     int32_t *off32_dev = nullptr;   // [n_cls][kpad] accumulator offsets
     int32_t *off_form_dev = nullptr;    // the same plus kFpMagic (kEpiFp)
@@ -234,6 +236,26 @@ static void epilogue_segments(int bn, int warps_per_quarter, int (&w)[2])
         for (a = (t + 1) / 2; !good(a) || !good(t - a); ++a) {}
     w[0] = a * 16;
     w[1] = (t - a) * 16;
+}
+
+// One filter's weights [c][taps] to [taps][pitch], with the sum of each tap.
+void weights_tap_major(const int8_t *w, int c, int taps, int8_t *dst, int pitch, int32_t *sums)
+{
+    for (int t = 0; t < taps; ++t) {
+        int8_t *row = dst + (size_t)t * pitch;
+        int32_t sum = 0;
+        if (taps == 1) {
+            memcpy(row, w, c);
+            for (int i = 0; i < c; ++i)
+                sum += w[i];
+        } else {
+            for (int i = 0; i < c; ++i) {
+                row[i] = w[(size_t)i * taps + t];
+                sum += row[i];
+            }
+        }
+        sums[t] = sum;
+    }
 }
 
 int conv_igemm_supported(const ConvGeom &g, char *why, size_t why_len)
@@ -471,10 +493,9 @@ int conv_igemm_create(
     const int taps = g.r * g.s;
     // ---- weights [kpad][r][s][c] ---------------------------------------------------------------
     std::vector<int8_t> wp((size_t)p->kpad * taps * p->cpad, 0);
+    std::vector<int32_t> wtap((size_t)g.k * taps);       // sum over channels per (k, tap)
     for (int k = 0; k < g.k; ++k)
-        for (int c = 0; c < g.c; ++c)
-            for (int t = 0; t < taps; ++t)
-                wp[((size_t)k * taps + t) * p->cpad + c] = w_s8[((size_t)k * g.c + c) * taps + t];
+        weights_tap_major(&w_s8[(size_t)k * g.c * taps], g.c, taps, &wp[(size_t)k * taps * p->cpad], p->cpad, &wtap[(size_t)k * taps]);
     // ---- border classes and offsets ---------------------------------------------------------------
     std::vector<uint8_t> row_cls, col_cls;
     std::vector<std::vector<char>> row_valid, col_valid;
@@ -486,11 +507,6 @@ int conv_igemm_create(
         delete p;
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): too many border classes");
     }
-    std::vector<long long> wtap((size_t)g.k * taps, 0);   // sum over channels per (k, tap)
-    for (int k = 0; k < g.k; ++k)
-        for (int c = 0; c < g.c; ++c)
-            for (int t = 0; t < taps; ++t)
-                wtap[(size_t)k * taps + t] += w_s8[((size_t)k * g.c + c) * taps + t];
     std::vector<int32_t> off32_all((size_t)p->n_row_cls * p->n_col_cls * p->kpad, 0);
     std::vector<long long> reach(g.k, 0);            // a bound of |accumulator + offset| per channel, whatever the input
     for (int rc = 0; rc < p->n_row_cls; ++rc)
@@ -517,10 +533,11 @@ int conv_igemm_create(
                 reach[k] = std::max(reach[k], off32 < 0 ? -off32 : off32);
             }
     for (int k = 0; k < g.k; ++k) {
-        long long mag = 0;
+        const int8_t *row = &w_s8[(size_t)k * g.c * taps];
+        int mag = 0;                            // (fits: at most 128 x 32767 k-blocks x 128 channels)
         for (int i = 0; i < g.c * taps; ++i)
-            mag += std::abs((int)w_s8[(size_t)k * g.c * taps + i]);
-        reach[k] += 255 * mag + 255ll * (g.wzp_d < 0 ? -g.wzp_d : g.wzp_d) * g.c * taps;
+            mag += row[i] < 0 ? -row[i] : row[i];
+        reach[k] += 255ll * mag + 255ll * (g.wzp_d < 0 ? -g.wzp_d : g.wzp_d) * g.c * taps;
     }
     std::vector<int32_t> shiftp(p->kpad, 33);
     for (int k = 0; k < g.k; ++k) {
@@ -563,11 +580,6 @@ int conv_igemm_create(
     }
     if (p->pair_ok && !igemm_kernel_mode3(p->variant))      // built for long reductions only
         p->pair_ok = 0;
-    auto up = [](const void *src, size_t bytes, void **dst) -> int {
-        B200_CUDA_TRY(cudaMalloc(dst, bytes));
-        B200_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
-        return B200_OK;
-    };
     std::vector<int8_t> one_row;
     if (ones) {
         one_row.assign((size_t)16 * taps * p->cpad, 0);
@@ -576,14 +588,41 @@ int conv_igemm_create(
                 one_row[(size_t)t * p->cpad + c] = 1;
     }
     p->w_bytes = wp.size();
-    int rc = up(wp.data(), wp.size(), (void **)&p->w_dev);
-    if (rc == B200_OK && ones) rc = up(one_row.data(), one_row.size(), (void **)&p->ones_dev);
-    if (rc == B200_OK) rc = up(mulp.data(), mulp.size() * 4, (void **)&p->mul_form_dev);
-    if (rc == B200_OK && p->form == kEpiFp) rc = up(off_form.data(), off_form.size() * 4, (void **)&p->off_form_dev);
-    if (rc == B200_OK) rc = up(off32_all.data(), off32_all.size() * 4, (void **)&p->off32_dev);
-    if (rc == B200_OK) rc = up(shiftp.data(), shiftp.size() * 4, (void **)&p->shift_dev);
-    if (rc == B200_OK) rc = up(row_cls.data(), row_cls.size(), (void **)&p->row_cls_dev);
-    if (rc == B200_OK) rc = up(col_cls.data(), col_cls.size(), (void **)&p->col_cls_dev);
+    // one device block for the weights and all tables: an allocation and a copy each cost more than the small tables hold
+    struct { const void *src; size_t bytes; void **dst; } parts[] = {
+        { wp.data(), wp.size(), (void **)&p->w_dev },
+        { one_row.data(), one_row.size(), (void **)&p->ones_dev },
+        { mulp.data(), mulp.size() * 4, (void **)&p->mul_form_dev },
+        { off_form.data(), p->form == kEpiFp ? off_form.size() * 4 : 0, (void **)&p->off_form_dev },
+        { off32_all.data(), off32_all.size() * 4, (void **)&p->off32_dev },
+        { shiftp.data(), shiftp.size() * 4, (void **)&p->shift_dev },
+        { row_cls.data(), row_cls.size(), (void **)&p->row_cls_dev },
+        { col_cls.data(), col_cls.size(), (void **)&p->col_cls_dev },
+    };
+    size_t small = 0;       // what goes behind the weights, copied together
+    for (auto &q : parts)
+        small += q.src == wp.data() ? 0 : (q.bytes + 255) / 256 * 256;
+    const size_t behind = (wp.size() + 255) / 256 * 256;
+    std::vector<uint8_t> tables(small);
+    auto upload_all = [&]() -> int {
+        B200_CUDA_TRY(cudaMalloc((void **)&p->block_dev, behind + small));
+        size_t at = 0;
+        for (auto &q : parts) {
+            if (q.src == wp.data()) {
+                *q.dst = p->block_dev;
+                continue;
+            }
+            if (q.bytes == 0)
+                continue;
+            memcpy(&tables[at], q.src, q.bytes);
+            *q.dst = p->block_dev + behind + at;
+            at += (q.bytes + 255) / 256 * 256;
+        }
+        B200_CUDA_TRY(cudaMemcpy(p->block_dev, wp.data(), wp.size(), cudaMemcpyHostToDevice));
+        B200_CUDA_TRY(cudaMemcpy(p->block_dev + behind, tables.data(), at, cudaMemcpyHostToDevice));
+        return B200_OK;
+    };
+    const int rc = upload_all();
     if (rc != B200_OK) {
         conv_igemm_destroy(p);
         return rc;
@@ -596,14 +635,7 @@ void conv_igemm_destroy(ConvIgemmPlan *p)
 {
     if (!p)
         return;
-    cudaFree(p->w_dev);
-    cudaFree(p->ones_dev);
-    cudaFree(p->off_form_dev);
-    cudaFree(p->mul_form_dev);
-    cudaFree(p->off32_dev);
-    cudaFree(p->shift_dev);
-    cudaFree(p->row_cls_dev);
-    cudaFree(p->col_cls_dev);
+    cudaFree(p->block_dev);
     delete p;
 }
 
@@ -972,12 +1004,20 @@ int conv_igemm_warm()
 {
     if (!encode_fn())
         return fail(B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    // once per device: the attributes belong to the loaded module (256 devices and more are set up on every call)
+    static std::atomic<bool> done[256];
+    int device = 0;
+    B200_CUDA_TRY(cudaGetDevice(&device));
+    if (device < 256 && done[device].load(std::memory_order_acquire))
+        return B200_OK;
     B200_TRY(conv_small_warm());
     for (int epi = 0; epi < kEpiVariants; ++epi)
         for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode1(epi), igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
                                igemm_kernel_wzp(epi), igemm_kernel_residual(epi) })
             if (k)
                 B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    if (device < 256)
+        done[device].store(true, std::memory_order_release);
     return B200_OK;
 }
 

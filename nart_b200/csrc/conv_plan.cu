@@ -141,15 +141,12 @@ int b200_conv2d_create(
     // ---- direct-kernel tables (always built: the accumulator-dumping entry uses them) --------
     const int cg4 = (cg + 3) / 4 * 4;
     std::vector<int8_t> w_pack((size_t)g.k * taps * cg4, 0);
-    std::vector<int32_t> bias_fold(g.k);
+    std::vector<int32_t> bias_fold(g.k), tap_sum(taps);
     for (int k = 0; k < g.k; ++k) {
+        weights_tap_major(&w_s8[(size_t)k * cg * taps], cg, taps, &w_pack[(size_t)k * taps * cg4], cg4, tap_sum.data());
         long long wsum = 0;
-        for (int c = 0; c < cg; ++c)
-            for (int t = 0; t < taps; ++t) {
-                int8_t v = w_s8[((size_t)k * cg + c) * taps + t];
-                w_pack[((size_t)k * taps + t) * cg4 + c] = v;
-                wsum += v;
-            }
+        for (int t = 0; t < taps; ++t)
+            wsum += tap_sum[t];
         long long bf = (long long)(bias ? bias[k] : 0) - (long long)g.izp * wsum;
         bias_fold[k] = (int32_t)(uint32_t)(unsigned long long)bf;   // modulo 2^32
     }

@@ -120,6 +120,7 @@ int conv_pad_channels_launch(const uint8_t *x, uint8_t *y, size_t pixels, int c,
 
 // Implicit-GEMM (tcgen05) convolution plan; defined in conv_igemm_sm100.cu.
 struct ConvIgemmPlan;
+void weights_tap_major(const int8_t *w, int c, int taps, int8_t *dst, int pitch, int32_t *sums);
 int conv_igemm_supported(const ConvGeom &g, char *why, size_t why_len);
 int conv_igemm_create(
     const ConvGeom &g, const std::vector<int8_t> &w_s8 /* [k][c][r][s] */, const int32_t *bias,
