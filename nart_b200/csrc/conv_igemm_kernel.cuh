@@ -419,6 +419,106 @@ __device__ __forceinline__ void epi_segment(uint32_t t_col, const int n16, uint3
     }
 }
 
+// ---- one offset row for all pixels: fragment layout ----------------------------------------------------------------
+// A thread that holds a whole row of the tile reads the constants of every column, and 32 lanes that read the same 16 bytes
+// still fill 512 bytes of registers: 2300 cycles of shared-memory traffic for a tile of 256 columns, which bound the layers
+// with a short reduction.  Here a thread holds two columns of every eight, of four rows: a quarter of the constants.  They
+// lie in pairs of columns, { offset, offset, multiplier, multiplier }.
+// 1x1 64 -> 256, 56x56, batch 256: 63.2 -> FRAG us.
+__device__ __forceinline__ void sts_u16(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"((uint16_t)v) : "memory");
+}
+template <int FORM, bool FULL>
+__device__ __forceinline__ uint32_t requant2(uint32_t v0, uint32_t v1, const int4 &k, const EpiConsts &ec)
+{
+    const int a0 = (int)v0 + k.x, a1 = (int)v1 + k.y;
+    int q0, q1;
+    if constexpr (FORM == kEpiFp) {
+        fp_requant_pair(a0, a1, k.z, k.w, ec.add, q0, q1);
+        q0 = FULL ? q0 - kFpOne : __viaddmax_s32(q0, -kFpOne, ec.relu_lo);
+        q1 = FULL ? q1 - kFpOne : __viaddmax_s32(q1, -kFpOne, ec.relu_lo);
+    } else {
+        const long long rnd = (long long)((unsigned long long)(uint32_t)ec.rnd_hi << 32);
+        q0 = (int)(((long long)a0 * k.z + rnd) >> 32) >> ec.ushift;
+        q1 = (int)(((long long)a1 * k.w + rnd) >> 32) >> ec.ushift;
+        if (!FULL) {
+            q0 = max(q0, ec.relu_lo);
+            q1 = max(q1, ec.relu_lo);
+        }
+    }
+    if (FULL) {
+        q0 = max(min(q0, ec.qmax), ec.relu_lo);
+        q1 = max(min(q1, ec.qmax), ec.relu_lo);
+    }
+    uint32_t out;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(out) : "r"(q1), "r"(q0), "r"(0));
+    return FULL ? out ^ ec.out_flip : out;
+}
+// 8 X columns: two halves of sixteen rows.  row_out: shared address of this thread's first row (lane / 4), col its chunk of
+// sixteen columns there; pitch8: bytes of eight rows.
+template <int FORM, bool FULL, int X>
+__device__ __forceinline__ void frag_half(const uint32_t (&v)[4 * X], const int4 (&k)[X], const EpiConsts &ec, uint32_t row_out, uint32_t pitch8,
+                                          uint32_t chunk, uint32_t sw16, uint32_t in_chunk)
+{
+#pragma unroll
+    for (int j = 0; j < X; ++j) {
+        const uint32_t at = row_out + (((chunk + (j >> 1)) << 4) ^ sw16) + (j & 1) * 8 + in_chunk;
+        sts_u16(at, requant2<FORM, FULL>(v[4 * j], v[4 * j + 1], k[j], ec));
+        sts_u16(at + pitch8, requant2<FORM, FULL>(v[4 * j + 2], v[4 * j + 3], k[j], ec));
+    }
+}
+template <int FORM, bool FULL>
+__device__ __forceinline__ void frag_segment(uint32_t t_col, const int n16, uint32_t tab, const EpiConsts &ec, uint32_t row_out, const uint32_t pitch8,
+                                             const uint32_t sw16, const uint32_t tempty, const bool remote)
+{
+    constexpr uint32_t kHalf = 16u << 16;           // sixteen lanes of tensor memory
+    const uint32_t q = threadIdx.x & 3, in_chunk = 2 * q;
+    tab += q * 16;
+    auto drained = [&]() {
+        if (tempty != 0) {
+            tc_fence_before();
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) {
+                if (remote)
+                    mbar_arrive_cluster(tempty);
+                else
+                    mbar_arrive(tempty);
+            }
+        }
+    };
+    uint32_t va[16], vb[16];
+    const int n32 = n16 >> 1;
+    if (n32 > 0)
+        tmem_ld_frag<4>(t_col, va);
+#pragma unroll 1
+    for (int h = 0; h < n32; ++h, tab += 256) {
+        int4 k[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            k[j] = lds4(tab + 64 * j);
+        tmem_ld_wait();
+        tmem_ld_frag<4>(t_col + h * 32 + kHalf, vb);
+        frag_half<FORM, FULL, 4>(va, k, ec, row_out, pitch8, 2 * h, sw16, in_chunk);
+        tmem_ld_wait();
+        if (h + 1 < n32)
+            tmem_ld_frag<4>(t_col + h * 32 + 32, va);
+        else if (!(n16 & 1))
+            drained();
+        frag_half<FORM, FULL, 4>(vb, k, ec, row_out + 2 * pitch8, pitch8, 2 * h, sw16, in_chunk);
+    }
+    if (n16 & 1) {
+        uint32_t v0[8], v1[8];
+        tmem_ld_frag<2>(t_col + n32 * 32, v0);
+        tmem_ld_frag<2>(t_col + n32 * 32 + kHalf, v1);
+        const int4 k[2] = { lds4(tab), lds4(tab + 64) };
+        tmem_ld_wait();
+        drained();
+        frag_half<FORM, FULL, 2>(v0, k, ec, row_out, pitch8, 2 * n32, sw16, in_chunk);
+        frag_half<FORM, FULL, 2>(v1, k, ec, row_out + 2 * pitch8, pitch8, 2 * n32, sw16, in_chunk);
+    }
+}
+
 // ---- shared memory layout (dynamic, base aligned to 1024) ---------------------------------------
 //   [stages x A tile (128 x bk)] [stages x B tile (bn x bk)] [2 x output staging 128 x bn]
 //   [per epilogue group: offsets, multipliers, shifts, bn x 4 each] [barriers][tmem address][abort flag]
@@ -824,6 +924,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
         constexpr bool one_class = EPI == kEpiFpOne || EPI == kEpiFpOneFull || EPI == kEpiIntOne || EPI == kEpiIntOneFull;
         constexpr int form = EPI <= kEpiFpManyFull ? kEpiFp : EPI <= kEpiIntManyFull ? kEpiInt : kEpiGeneric;
         constexpr bool full = EPI == kEpiAny || (EPI & 1) != 0;
+        constexpr bool frag = one_class && !HAS_RES && !HAS_WZP;
         const uint32_t out_bytes = (uint32_t)kTileM * g.bn;
         // this thread's pixel inside a tile (tw, th are powers of two)
         const int lw = row & (g.tw - 1), lh = (row >> g.tw_sh) & (g.th - 1), ln = row >> (g.tw_sh + g.th_sh);
@@ -880,6 +981,12 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
             if (nt != cur_nt) {
                 epi_bar_sync(group, group_threads);
                 for (int j = et; j < g.bn; j += group_threads) {
+                    if (frag) {         // pairs of columns: { offset, offset, multiplier, multiplier }
+                        const int at = (j >> 1) * 4 + (j & 1);
+                        s_off[at] = g.off32[k0 + j];
+                        s_off[at + 2] = g.mul[k0 + j];
+                        continue;
+                    }
                     s_mul[j] = g.mul[k0 + j];
                     if (EPI == kEpiAny)
                         s_shift[j] = g.shift[k0 + j];
@@ -924,10 +1031,17 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                 }
                 for (int seg = seg0; seg < seg1; ++seg) {
                     const int w = g.seg_w[seg], c0 = seg ? g.seg_w[0] : 0;
-                    const uint32_t row_out = smem_u32(s_out) + (uint32_t)(kTileM * c0 + row * w);
-                    epi_segment<form, one_class, full, HAS_WZP, HAS_RES>(
-                        t_row + c0, w >> 4, tab + c0 * 4, pitch, off_row + c0, ec, wz_t, has_res && pix_valid ? res_row + c0 : nullptr, row_out,
-                        (uint32_t)swizzle(w) << 4, seg + 1 == seg1 ? tempty : 0u, PAIR && !leader);
+                    if constexpr (frag) {
+                        const int frow = p0 + (lane >> 2);
+                        const uint32_t fsw = w == 128 ? frow & 7 : w == 64 ? (frow >> 1) & 3 : w == 32 ? (frow >> 2) & 1 : 0;
+                        frag_segment<form, full>(t_row + c0, w >> 4, tab + c0 * 8, ec, smem_u32(s_out) + (uint32_t)(kTileM * c0 + frow * w), 8 * w, fsw << 4,
+                                                 seg + 1 == seg1 ? tempty : 0u, PAIR && !leader);
+                    } else {
+                        const uint32_t row_out = smem_u32(s_out) + (uint32_t)(kTileM * c0 + row * w);
+                        epi_segment<form, one_class, full, HAS_WZP, HAS_RES>(
+                            t_row + c0, w >> 4, tab + c0 * 4, pitch, off_row + c0, ec, wz_t, has_res && pix_valid ? res_row + c0 : nullptr, row_out,
+                            (uint32_t)swizzle(w) << 4, seg + 1 == seg1 ? tempty : 0u, PAIR && !leader);
+                    }
                 }
 
                 if (g.use_tma_store) {

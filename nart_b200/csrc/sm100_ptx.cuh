@@ -253,6 +253,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
         : "r"(taddr)
         : "memory");
 }
+// X blocks of eight columns of 16 lanes: thread t holds, of block j, the columns 2 (t % 4) and the next of lane t / 4 in
+// v[4 j], v[4 j + 1] and of lane t / 4 + 8 in v[4 j + 2], v[4 j + 3].
+template <int X>
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&v)[4 * X])
+{
+    static_assert(X == 2 || X == 4, "columns: 16 or 32");
+    if constexpr (X == 4)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(taddr)
+            : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "r"(taddr)
+                     : "memory");
+}
 __device__ __forceinline__ void tmem_ld1(uint32_t taddr, uint32_t &v)
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(taddr) : "memory");
