@@ -6,15 +6,15 @@ namespace b200 {
 IgemmKernel igemm_kernel_mode1(int epi)
 {
     switch (epi) {
-    case kEpiFpOne: return conv_igemm_i8_kernel<kEpiFpOne, false, false, 1>;
-    case kEpiFpOneFull: return conv_igemm_i8_kernel<kEpiFpOneFull, false, false, 1>;
-    case kEpiFpMany: return conv_igemm_i8_kernel<kEpiFpMany, false, false, 1>;
-    case kEpiFpManyFull: return conv_igemm_i8_kernel<kEpiFpManyFull, false, false, 1>;
-    case kEpiIntOne: return conv_igemm_i8_kernel<kEpiIntOne, false, false, 1>;
-    case kEpiIntOneFull: return conv_igemm_i8_kernel<kEpiIntOneFull, false, false, 1>;
-    case kEpiIntMany: return conv_igemm_i8_kernel<kEpiIntMany, false, false, 1>;
-    case kEpiIntManyFull: return conv_igemm_i8_kernel<kEpiIntManyFull, false, false, 1>;
-    case kEpiAny: return conv_igemm_i8_kernel<kEpiAny, false, false, 1>;
+    case kEpiFpOne: return conv_igemm_i8_kernel<kEpiFpOne, false, false, 1, false>;
+    case kEpiFpOneFull: return conv_igemm_i8_kernel<kEpiFpOneFull, false, false, 1, false>;
+    case kEpiFpMany: return conv_igemm_i8_kernel<kEpiFpMany, false, false, 1, false>;
+    case kEpiFpManyFull: return conv_igemm_i8_kernel<kEpiFpManyFull, false, false, 1, false>;
+    case kEpiIntOne: return conv_igemm_i8_kernel<kEpiIntOne, false, false, 1, false>;
+    case kEpiIntOneFull: return conv_igemm_i8_kernel<kEpiIntOneFull, false, false, 1, false>;
+    case kEpiIntMany: return conv_igemm_i8_kernel<kEpiIntMany, false, false, 1, false>;
+    case kEpiIntManyFull: return conv_igemm_i8_kernel<kEpiIntManyFull, false, false, 1, false>;
+    case kEpiAny: return conv_igemm_i8_kernel<kEpiAny, false, false, 1, false>;
     default: return nullptr;
     }
 }

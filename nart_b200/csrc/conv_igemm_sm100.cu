@@ -931,6 +931,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         : g.wzp_d ? igemm_kernel_wzp(p->variant)
         : l.cta_pair ? igemm_kernel_mode3(p->variant)
         : p->pair ? igemm_kernel_mode2(p->variant)
+        : !a.use_tma_store ? igemm_kernel_ragged(p->variant, p->rings == 2)
         : p->rings == 2 ? igemm_kernel_mode1(p->variant) : igemm_kernel_mode0(p->variant);
     if (!l.kernel)
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no kernel of epilogue variant %d for this launch", p->variant);
@@ -1012,7 +1013,8 @@ int conv_igemm_warm()
         return B200_OK;
     B200_TRY(conv_small_warm());
     for (int epi = 0; epi < kEpiVariants; ++epi)
-        for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode1(epi), igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
+        for (IgemmKernel k : { igemm_kernel_mode0(epi), igemm_kernel_mode1(epi), igemm_kernel_ragged(epi, false), igemm_kernel_ragged(epi, true),
+                               igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
                                igemm_kernel_wzp(epi), igemm_kernel_residual(epi) })
             if (k)
                 B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
