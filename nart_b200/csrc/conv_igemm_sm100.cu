@@ -435,7 +435,8 @@ int conv_igemm_create(
         // a deep ring lets the producer run several tiles ahead when a tile has few k-blocks
         // Two pipelines (the kernel's MODE 1) where the k-blocks are short: an MMA of a tile this narrow takes 64 cycles or
         // less, and one producer thread needs ~300 cycles for a k-block (3x3 64-channel layer, 56x56, batch 256: 84 -> 51 us).
-        p->rings = (p->bn <= 128 && stages >= 4 && !ones) ? 2 : 1;
+        // Tiles of 80 channels and more with a short reduction wait for their epilogue (16 -> 96, 112x112: 110 us, with two 119).
+        p->rings = (p->bn <= 128 && (p->bn <= 64 || kblocks * p->bk > 256) && stages >= 4 && !ones) ? 2 : 1;
         if (const char *e = getenv("B200_IGEMM_RINGS")) {   // tuning aid: 1, or 2 when the ring has four stages or more
             int v = atoi(e);
             if (v == 1 || (v == 2 && stages >= 4 && !ones))
@@ -870,8 +871,8 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
             p->max_clusters = nc < sms / 2 ? nc : sms / 2;
         }
         const int pair_tiles = (a.tiles_w * a.tiles_h * a.tiles_n + 1) / 2 * (p->kpad / p->bn);
-        // long launches only: at least six pair tiles for every cluster
-        l.cta_pair = (p->pair_want == 1 || pair_tiles >= 6 * p->max_clusters) ? 1 : 0;
+        // a pair tile for every cluster at least (3x3 256 -> 256, 14x14, batch 256: 26.5 -> 25.8 us; 3x3 s2 512 -> 512: 34.1 -> 31.1)
+        l.cta_pair = (p->pair_want == 1 || pair_tiles >= p->max_clusters) ? 1 : 0;
     }
     a.bk = p->bk; a.bn = p->bn; a.stages = l.cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
     a.cchunks = (p->cpad + p->bk - 1) / p->bk;
