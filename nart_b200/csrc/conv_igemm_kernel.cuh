@@ -424,7 +424,7 @@ __device__ __forceinline__ void epi_segment(uint32_t t_col, const int n16, uint3
 // still fill 512 bytes of registers: 2300 cycles of shared-memory traffic for a tile of 256 columns, which bound the layers
 // with a short reduction.  Here a thread holds two columns of every eight, of four rows: a quarter of the constants.  They
 // lie in pairs of columns, { offset, offset, multiplier, multiplier }.
-// 1x1 64 -> 256, 56x56, batch 256: 63.2 -> FRAG us.
+// 1x1 64 -> 256, 56x56, batch 256: 63.2 -> 64.3 us, bound by instruction issue either way; 256 -> 1024, 14x14: 26.1 -> 22.4.
 __device__ __forceinline__ void sts_u16(uint32_t addr, uint32_t v)
 {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"((uint16_t)v) : "memory");
@@ -758,7 +758,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
             const bool load_b = !g.b_resident, a_wide = MODE != 2 && MODE != 3 && g.a_wide;
             // Groups of several k-blocks, up to 32 a tile: lane i knows where k-block i lies (offsets from the tile's first pixel,
             // map, channel, weight column), and the warp takes four entries at a time by shuffles.  The counters below are one
-            // chain of instructions, ~190 cycles a k-block.  (3x3 64 -> 64, 56x56, batch 256: 51 -> TAB us)
+            // chain of instructions, ~190 cycles a k-block.  (3x3 64 -> 64, 56x56, batch 256: 51.2 -> 49.4 us)
             const bool table = (MODE == 0 || MODE == 1) && kgroup > 1 && kblocks <= 32;
             uint32_t tab = 0;
             int tab_kc = 0;
