@@ -423,17 +423,15 @@ __device__ __forceinline__ void epi_segment(uint32_t t_col, const int n16, uint3
 // A thread that holds a whole row of the tile reads the constants of every column, and 32 lanes that read the same 16 bytes
 // still fill 512 bytes of registers: 2300 cycles of shared-memory traffic for a tile of 256 columns, which bound the layers
 // with a short reduction.  Here a thread holds two columns of every eight, of four rows: a quarter of the constants.  They
-// lie in pairs of columns, { offset, offset, multiplier, multiplier }.
-// 1x1 64 -> 256, 56x56, batch 256: 63.2 -> 64.3 us, bound by instruction issue either way; 256 -> 1024, 14x14: 26.1 -> 22.4.
-__device__ __forceinline__ void sts_u16(uint32_t addr, uint32_t v)
-{
-    asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"((uint16_t)v) : "memory");
-}
+// lie in pairs of columns, { offset, offset, multiplier, multiplier }.  The weight tile's rows are in an order that gives a
+// thread four neighbouring channels of every sixteen, one word of the staging buffer: accumulator column 8 j + 2 q + e is
+// channel 4 q + 2 j + e (the tensor map of the weights does that, see encode_weights).
+// 1x1 256 -> 1024, 14x14, batch 256: 26.1 -> 23.0 us; 64 -> 256, 56x56, bound by instruction issue: 63.2 -> 63.7..
+__device__ __forceinline__ void sts1(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 template <int FORM, bool FULL>
-__device__ __forceinline__ uint32_t requant2(uint32_t v0, uint32_t v1, const int4 &k, const EpiConsts &ec)
+__device__ __forceinline__ void requant2(uint32_t v0, uint32_t v1, const int4 &k, const EpiConsts &ec, int &q0, int &q1)
 {
     const int a0 = (int)v0 + k.x, a1 = (int)v1 + k.y;
-    int q0, q1;
     if constexpr (FORM == kEpiFp) {
         fp_requant_pair(a0, a1, k.z, k.w, ec.add, q0, q1);
         q0 = FULL ? q0 - kFpOne : __viaddmax_s32(q0, -kFpOne, ec.relu_lo);
@@ -451,8 +449,14 @@ __device__ __forceinline__ uint32_t requant2(uint32_t v0, uint32_t v1, const int
         q0 = max(min(q0, ec.qmax), ec.relu_lo);
         q1 = max(min(q1, ec.qmax), ec.relu_lo);
     }
-    uint32_t out;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(out) : "r"(q1), "r"(q0), "r"(0));
+}
+template <int FORM, bool FULL>
+__device__ __forceinline__ uint32_t requant4(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, const int4 &k0, const int4 &k1, const EpiConsts &ec)
+{
+    int q[4];
+    requant2<FORM, FULL>(v0, v1, k0, ec, q[0], q[1]);
+    requant2<FORM, FULL>(v2, v3, k1, ec, q[2], q[3]);
+    const uint32_t out = pack_sat_u8x4(q[0], q[1], q[2], q[3]);
     return FULL ? out ^ ec.out_flip : out;
 }
 // 8 X columns: two halves of sixteen rows.  row_out: shared address of this thread's first row (lane / 4), col its chunk of
@@ -462,10 +466,10 @@ __device__ __forceinline__ void frag_half(const uint32_t (&v)[4 * X], const int4
                                           uint32_t chunk, uint32_t sw16, uint32_t in_chunk)
 {
 #pragma unroll
-    for (int j = 0; j < X; ++j) {
-        const uint32_t at = row_out + (((chunk + (j >> 1)) << 4) ^ sw16) + (j & 1) * 8 + in_chunk;
-        sts_u16(at, requant2<FORM, FULL>(v[4 * j], v[4 * j + 1], k[j], ec));
-        sts_u16(at + pitch8, requant2<FORM, FULL>(v[4 * j + 2], v[4 * j + 3], k[j], ec));
+    for (int j = 0; j < X; j += 2) {
+        const uint32_t at = row_out + (((chunk + (j >> 1)) << 4) ^ sw16) + in_chunk;
+        sts1(at, requant4<FORM, FULL>(v[4 * j], v[4 * j + 1], v[4 * j + 4], v[4 * j + 5], k[j], k[j + 1], ec));
+        sts1(at + pitch8, requant4<FORM, FULL>(v[4 * j + 2], v[4 * j + 3], v[4 * j + 6], v[4 * j + 7], k[j], k[j + 1], ec));
     }
 }
 template <int FORM, bool FULL>
@@ -473,8 +477,8 @@ __device__ __forceinline__ void frag_segment(uint32_t t_col, const int n16, uint
                                              const uint32_t sw16, const uint32_t tempty, const bool remote)
 {
     constexpr uint32_t kHalf = 16u << 16;           // sixteen lanes of tensor memory
-    const uint32_t q = threadIdx.x & 3, in_chunk = 2 * q;
-    tab += q * 16;
+    const uint32_t q = threadIdx.x & 3, in_chunk = 4 * q;
+    tab += q * 32;
     auto drained = [&]() {
         if (tempty != 0) {
             tc_fence_before();
@@ -496,7 +500,7 @@ __device__ __forceinline__ void frag_segment(uint32_t t_col, const int n16, uint
         int4 k[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            k[j] = lds4(tab + 64 * j);
+            k[j] = lds4(tab + (j >> 1) * 128 + (j & 1) * 16);
         tmem_ld_wait();
         tmem_ld_frag<4>(t_col + h * 32 + kHalf, vb);
         frag_half<FORM, FULL, 4>(va, k, ec, row_out, pitch8, 2 * h, sw16, in_chunk);
@@ -511,7 +515,7 @@ __device__ __forceinline__ void frag_segment(uint32_t t_col, const int n16, uint
         uint32_t v0[8], v1[8];
         tmem_ld_frag<2>(t_col + n32 * 32, v0);
         tmem_ld_frag<2>(t_col + n32 * 32 + kHalf, v1);
-        const int4 k[2] = { lds4(tab), lds4(tab + 64) };
+        const int4 k[2] = { lds4(tab), lds4(tab + 16) };
         tmem_ld_wait();
         drained();
         frag_half<FORM, FULL, 2>(v0, k, ec, row_out, pitch8, 2 * n32, sw16, in_chunk);
@@ -703,6 +707,18 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
     };
     const int cchunks = g.cchunks;
     const int kblocks = g.r * g.s * cchunks;
+    constexpr bool one_class = EPI == kEpiFpOne || EPI == kEpiFpOneFull || EPI == kEpiIntOne || EPI == kEpiIntOneFull;
+    constexpr bool frag = one_class && !HAS_RES && !HAS_WZP;     // (the host permutes the weight rows by the same rule)
+    auto load_weights = [&](uint32_t dst, uint32_t bar, int kc, int row) {
+        if constexpr (frag && PAIR)
+            tma_load_5d_pair(dst, &maps.b, bar, kc, 0, 0, 0, row >> 4);
+        else if constexpr (frag)
+            tma_load_5d(dst, &maps.b, bar, kc, 0, 0, 0, row >> 4);
+        else if constexpr (PAIR)
+            tma_load_2d_pair(dst, &maps.b, bar, kc, row);
+        else
+            tma_load_2d(dst, &maps.b, bar, kc, row);
+    };
 
     // this warp's pipeline (MODE 1), its stages and its first tile
     constexpr int tile_step = MODE == 1 || MODE == 2 ? 2 : 1;
@@ -733,7 +749,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                     for (int c = 0; c < cchunks; ++c, dst += b_slot) {
                         const int kc = tap * g.c + c * (int)bk;
                         if (elect_one()) {
-                            tma_load_2d(dst, &maps.b, bres_bar, kc, 0);
+                            load_weights(dst, bres_bar, kc, 0);
                             if (HAS_WZP)
                                 tma_load_2d(dst + g.bn * bk, &maps.ones, bres_bar, kc, 0);
                         }
@@ -823,7 +839,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                                         else
                                             tma_load_4d(a_at, m, fb, (int)(e[u] >> 16) << 5, x, y, n0);
                                         if (load_b) {
-                                            tma_load_2d(b_at, &maps.b, fb, ekc[u], b_row);
+                                            load_weights(b_at, fb, ekc[u], b_row);
                                             if (HAS_WZP)
                                                 tma_load_2d(b_at + g.bn * bk, &maps.ones, fb, ekc[u], 0);
                                         }
@@ -838,7 +854,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                         if (elect_one()) {
                             if (PAIR) {
                                 tma_load_4d_pair(a_dst, amap, fb_lead, cc, xw, yh, n0);
-                                tma_load_2d_pair(b_dst, &maps.b, fb_lead, kc, b_row);
+                                load_weights(b_dst, fb_lead, kc, b_row);
                             } else {
                                 if (a_wide)                     // rows of tw pixels x 32 bytes, in 8-byte elements
                                     tma_load_3d(a_dst, amap, fb, xw << 2, yh, n0);
@@ -847,7 +863,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                                 if (MODE == 2 && second)        // the pair's second tile: same tap, its own pixels
                                     tma_load_4d(a_dst + a_tile_bytes, amap, fb, cc, xw + dx2, yh + dy2, n2);
                                 if (load_b) {
-                                    tma_load_2d(b_dst, &maps.b, fb, kc, b_row);
+                                    load_weights(b_dst, fb, kc, b_row);
                                     if (HAS_WZP)
                                         tma_load_2d(b_dst + g.bn * bk, &maps.ones, fb, kc, 0);
                                 }
@@ -1022,10 +1038,8 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
         int32_t *s_off = reinterpret_cast<int32_t *>(smem + L.tables + (size_t)group * g.bn * 12);
         int32_t *s_mul = s_off + g.bn, *s_shift = s_mul + g.bn;
         // one offset row for all pixels (1x1 and unpadded convs), in shared memory
-        constexpr bool one_class = EPI == kEpiFpOne || EPI == kEpiFpOneFull || EPI == kEpiIntOne || EPI == kEpiIntOneFull;
         constexpr int form = EPI <= kEpiFpManyFull ? kEpiFp : EPI <= kEpiIntManyFull ? kEpiInt : kEpiGeneric;
         constexpr bool full = EPI == kEpiAny || (EPI & 1) != 0;
-        constexpr bool frag = one_class && !HAS_RES && !HAS_WZP;
         const uint32_t out_bytes = (uint32_t)kTileM * g.bn;
         // this thread's pixel inside a tile (tw, th are powers of two)
         const int lw = row & (g.tw - 1), lh = (row >> g.tw_sh) & (g.th - 1), ln = row >> (g.tw_sh + g.th_sh);

@@ -757,9 +757,16 @@ static int encode_activations(const ConvIgemmPlan *p, const uint8_t *x, int n, i
 }
 
 // Tensor map of [rows][r*s*c] weights in boxes of `box_rows` rows and one k-block.
-static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int box_rows, CUtensorMap *map)
+// frag: the row order of the fragment epilogue (frag_segment): row 8 j + 2 q + e of every sixteen is channel 4 q + 2 j + e.
+static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int box_rows, CUtensorMap *map, bool frag = false)
 {
     const int ktot = p->g.r * p->g.s * p->cpad;
+    if (frag) {
+        cuuint64_t dims[5] = { (cuuint64_t)ktot, 2, 4, 2, (cuuint64_t)(rows / 16) };
+        cuuint64_t strides[4] = { (cuuint64_t)ktot, 4 * (cuuint64_t)ktot, 2 * (cuuint64_t)ktot, 16 * (cuuint64_t)ktot };
+        cuuint32_t box[5] = { (cuuint32_t)p->bk, 2, 4, 2, (cuuint32_t)(box_rows / 16) };
+        return encode(map, const_cast<int8_t *>(w), 5, dims, strides, box, swizzle_for(p->bk));
+    }
     cuuint64_t dims[2] = { (cuuint64_t)ktot, (cuuint64_t)rows };
     cuuint64_t strides[1] = { (cuuint64_t)ktot };
     cuuint32_t box[2] = { (cuuint32_t)p->bk, (cuuint32_t)box_rows };
@@ -909,7 +916,8 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
 
     // ---- tensor maps -------------------------------------------------------------------------------
     B200_TRY(encode_activations(p, x, n, a.tw, a.th, a.tn, l.maps.a));
-    B200_TRY(encode_weights(p, p->w_dev, p->kpad, l.cta_pair ? p->bn / 2 : p->bn, &l.maps.b));   // a CTA of a pair loads half the rows
+    const bool frag = !res && !g.wzp_d && p->n_row_cls * p->n_col_cls == 1 && p->variant != kEpiAny;   // as the kernel's `frag`
+    B200_TRY(encode_weights(p, p->w_dev, p->kpad, l.cta_pair ? p->bn / 2 : p->bn, &l.maps.b, frag));   // a CTA of a pair loads half the rows
     l.maps.ones = l.maps.b;
     if (p->ones_dev)
         B200_TRY(encode_weights(p, p->ones_dev, 16, 16, &l.maps.ones));
