@@ -388,7 +388,7 @@ B200_API int b200_case_run_host(
 B200_API int b200_case_submit_host(
     b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs);
 B200_API int b200_case_wait(b200_case_t *cs);
-/* Number of kernels one b200_case_run_device launches. */
+/* Number of kernels one b200_case_run_device launches.  (A residual add that a small conv launch forms itself still counts.) */
 B200_API int b200_case_launch_count(const b200_case_t *cs, int32_t *launches);
 /* Folds residual adds into the convs that feed them (default: off; call before b200_case_prepare).
  * Off by default because on B200 the conv epilogue is bound by instruction issue, not by memory:

@@ -426,7 +426,7 @@ __device__ __forceinline__ void epi_segment(uint32_t t_col, const int n16, uint3
 // lie in pairs of columns, { offset, offset, multiplier, multiplier }.  The weight tile's rows are in an order that gives a
 // thread four neighbouring channels of every sixteen, one word of the staging buffer: accumulator column 8 j + 2 q + e is
 // channel 4 q + 2 j + e (the tensor map of the weights does that, see encode_weights).
-// 1x1 256 -> 1024, 14x14, batch 256: 26.1 -> 23.0 us; 64 -> 256, 56x56, bound by instruction issue: 63.2 -> 63.7..
+// 1x1 256 -> 1024, 14x14, batch 256: 26.1 -> 23.0 us; 64 -> 256, 56x56, bound by instruction issue: 63.2 -> 63.7.
 __device__ __forceinline__ void sts1(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 template <int FORM, bool FULL>
 __device__ __forceinline__ void requant2(uint32_t v0, uint32_t v1, const int4 &k, const EpiConsts &ec, int &q0, int &q1)

@@ -204,6 +204,9 @@ struct ConvIgemmPlan {
     struct Launch {
         const uint8_t *x;
         const uint8_t *res;
+        const uint8_t *sum_res;     // ConvSum
+        uint8_t *sum;
+        bool summed;
         uint8_t *y;
         int n;
         int *status;
@@ -774,7 +777,7 @@ static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int
 }
 
 // Fills l.smaps / l.sargs if the launch is one for conv_small_kernel; l.small says so.
-static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status, int tw, int th, int tn, ConvIgemmPlan::Launch &l)
+static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status, int tw, int th, int tn, const ConvSum *ws, ConvIgemmPlan::Launch &l)
 {
     const ConvGeom &g = p->g;
     SmallArgs &a = l.sargs;
@@ -810,6 +813,16 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.y = y;
     a.status = status;
     a.next_ro = p->next_ro; a.next_ro_bytes = p->next_ro_bytes;
+    if (ws && g.k % 16 == 0 && !g.act_signed) {         // (other channel counts leave through staged rows)
+        const int ci = ws->conv_input, other = 1 - ci;
+        const EltwiseArgs &e = *ws->elt;
+        a.res = ws->res;
+        a.sum = ws->sum;
+        a.r_m[0] = e.m[ci]; a.r_add[0] = e.add[ci]; a.r_b[0] = e.b[ci];
+        a.r_m[1] = e.m[other]; a.r_add[1] = e.add[other]; a.r_b[1] = e.b[other];
+        a.r_s0 = e.s0; a.r_ozp = e.ozp; a.r_lo = e.relu_lo;
+        l.summed = true;
+    }
     const size_t smem = conv_small_smem(a, g.act_signed != 0);
     if (smem > 227 * 1024)
         return B200_OK;
@@ -824,12 +837,13 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     return B200_OK;
 }
 
-static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status_word, const uint8_t *res, ConvIgemmPlan::Launch &l)
+static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status_word, const uint8_t *res, const ConvSum *ws, ConvIgemmPlan::Launch &l)
 {
     const ConvGeom &g = p->g;
     if ((((uintptr_t)x | (uintptr_t)y) & 15) != 0)
         return fail(B200_ERR_INVALID, "conv(igemm): x and y must be 16-byte aligned");
     l.x = x; l.res = res; l.y = y; l.n = n; l.status = status_word;
+    l.sum_res = ws ? ws->res : nullptr; l.sum = ws ? ws->sum : nullptr; l.summed = false;
     l.small = false;
     l.cta_pair = 0;
     IgemmArgs &a = l.args;
@@ -855,7 +869,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         p->attr_set = true;
     }
     if (!res && p->small_ok && !(p->pair_ok && p->pair_want == 1)) {
-        B200_TRY(build_small(p, x, n, y, a.status, a.tw, a.th, a.tn, l));
+        B200_TRY(build_small(p, x, n, y, a.status, a.tw, a.th, a.tn, ws, l));
         if (l.small)
             return B200_OK;
     }
@@ -969,8 +983,11 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     return B200_OK;
 }
 
-int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st, int *status_word, const uint8_t *res)
+int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st, int *status_word, const uint8_t *res,
+                      const ConvSum *with_sum, bool *summed)
 {
+    if (summed)
+        *summed = false;
     if (n == 0)
         return B200_OK;
     if (p->g.wzp_d != 0 && res != nullptr)
@@ -981,14 +998,15 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
         return fail(B200_ERR_INVALID, "conv(igemm): this conv was fused with a residual add and needs the residual tensor");
     if (res != nullptr && (((uintptr_t)res) & 15) != 0)
         return fail(B200_ERR_INVALID, "conv(igemm): the residual tensor must be 16-byte aligned");
-    auto matches = [&](const ConvIgemmPlan::Launch &l) { return l.x == x && l.y == y && l.n == n && l.status == status_word && l.res == res; };
+    auto matches = [&](const ConvIgemmPlan::Launch &l) { return l.x == x && l.y == y && l.n == n && l.status == status_word && l.res == res
+               && l.sum_res == (with_sum ? with_sum->res : nullptr) && l.sum == (with_sum ? with_sum->sum : nullptr); };
     if (p->last >= p->saved.size() || !matches(p->saved[p->last])) {
         size_t i = 0;
         while (i < p->saved.size() && !matches(p->saved[i]))
             ++i;
         if (i == p->saved.size()) {
             ConvIgemmPlan::Launch l;
-            B200_TRY(build_launch(p, x, n, y, status_word, res, l));
+            B200_TRY(build_launch(p, x, n, y, status_word, res, with_sum, l));
             if (p->saved.size() < ConvIgemmPlan::kMaxSaved) {
                 p->saved.push_back(l);
             } else {
@@ -1001,6 +1019,8 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
     }
     const ConvIgemmPlan::Launch &l = p->saved[p->last];
     const size_t bytes = (size_t)n * ((size_t)p->g.h * p->g.w * p->g.c + (size_t)p->g.oh * p->g.ow * p->g.k) + p->w_bytes;
+    if (summed)
+        *summed = l.small && l.summed;
     if (l.small)
         return conv_small_launch(l.smaps, l.sargs, l.m_tiles, l.smem, bytes, st);
     const bool two_rings = !l.cta_pair && !res && p->g.wzp_d == 0 && !p->pair && p->rings == 2;

@@ -91,7 +91,16 @@ template <int N>
 __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const SmallArgs &g, const EpiConsts &ec, const SmallTables &t, int xcorr,
                                                int j, size_t at, uint32_t stage)
 {
-    uint32_t w[N / 4];
+    uint32_t w[N / 4], x[N / 4];
+    if (g.res) {            // on its way while the accumulators are requantized (Cout is a multiple of 16 then)
+        if constexpr (N == 16) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(g.res + at));
+            x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+        } else {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(g.res + at));
+            x[0] = v.x, x[1] = v.y;
+        }
+    }
     if (t.off_g == nullptr) {
         if (g.form == kEpiFp)
             epi_pack<kEpiFp, true, true, true>(acc, t.off_s + j * 4, nullptr, t.mul + j * 4, t.shift + j * 4, ec, xcorr, w);
@@ -121,11 +130,10 @@ __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const S
             *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
     };
     store(g.y + at);
-    if (g.res) {            // (Cout is a multiple of 32 then)
-        const uint32_t *x = reinterpret_cast<const uint32_t *>(g.res + at);
+    if (g.res) {
 #pragma unroll
         for (int q = 0; q < N / 4; ++q)
-            w[q] = add_residual(w[q], __ldg(x + q), ec);
+            w[q] = add_residual(w[q], x[q], ec);
         store(g.sum + at);
     }
 }

@@ -132,8 +132,16 @@ int conv_igemm_create(
 // status_word: device int that a bounded wait writes its code into; nullptr = the per-device word
 // that b200_device_status reads.
 // res: the second input of a fused residual add (conv_igemm_set_residual), else nullptr.
+// An eltwise SUM of the conv's output and `res` that the conv's launch may form as well (the small kernel does): both tensors
+// are written.  conv_input: which of the SUM's inputs the conv's output is.
+struct ConvSum {
+    const uint8_t *res;
+    uint8_t *sum;
+    const EltwiseArgs *elt;
+    int conv_input;
+};
 int conv_igemm_launch(ConvIgemmPlan *plan, const uint8_t *x, int n, uint8_t *y, cudaStream_t st,
-                      int *status_word = nullptr, const uint8_t *res = nullptr);
+                      int *status_word = nullptr, const uint8_t *res = nullptr, const ConvSum *with_sum = nullptr, bool *summed = nullptr);
 // Fuses y = eltwise_sum(conv(x), res) into the epilogue: `e` holds the eltwise constants and
 // conv_input says which of its two inputs is this conv's output.  B200_ERR_UNSUPPORTED when the
 // plan's epilogue form cannot take it (the caller then keeps the separate eltwise kernel).
