@@ -100,3 +100,33 @@ def test_case_fusion_on_and_off_agree(port):
     assert_same(outs[0].view(np.uint32), want_logits.view(np.uint32), "fused case vs restatement")
     assert_same(outs[1].view(np.uint32), want_logits.view(np.uint32), "unfused case vs restatement")
     assert launches[0] == launches[1] - 16      # the 16 residual adds of ResNet-50 ride in conv epilogues
+
+
+# (n, c, h, w, k, kernel): one tile and several, split reductions
+SUM_SHAPES = [(1, 512, 5, 6, 64, 3), (2, 64, 14, 13, 48, 1), (1, 64, 9, 8, 16, 1), (1, 32, 56, 56, 256, 1)]
+
+
+@pytest.mark.parametrize("conv_input", [0, 1])
+@pytest.mark.parametrize("n,c,h,w,k,ks", SUM_SHAPES)
+def test_case_sums_behind_small_convs(port, n, c, h, w, k, ks, conv_input):
+    """A conv and the residual add behind it, both read by the host."""
+    from nart_b200.case import Case
+    x, wt, bias, walpha = conv_inputs(5 + k, n, c, h, w, k, ks, ks, 1)
+    res = np.random.default_rng(k).integers(0, 256, (n, k, h, w), dtype=np.uint8)
+    q = dict(ialpha=0.031, izp=121, walpha=walpha, wzp=128, oalpha=0.05 * np.sqrt(c * ks * ks) / 4, ozp=113)
+    y = port.conv2d_u8(x, wt, bias, (1, 1), (ks // 2, ks // 2), 1, q["ialpha"], q["izp"], walpha, 128, q["oalpha"], q["ozp"])
+    both = lambda a, b: [a, b] if conv_input == 0 else [b, a]
+    ia, iz = both(np.float32(q["oalpha"]), 0.043), both(q["ozp"], 97)
+    want = port.eltwise_sum_u8(both(y, res), ia, iz, 0.06, 9, relu=True)
+    cs = Case()
+    tx, tr = cs.input_u8(c, h, w), cs.input_u8(k, h, w)
+    ty = cs.conv2d(tx, wt, bias, pad=(ks // 2, ks // 2), **q)
+    ts = cs.eltwise_sum(both(ty, tr), ia, iz, 0.06, 9, relu=True)
+    cs.output_u8(ty)
+    cs.output_u8(ts)
+    cs.prepare(n)
+    for _ in range(2):
+        got_y, got_s = cs.run_host([x, res], [(np.uint8, (k, h, w))] * 2)
+        assert_same(got_y.reshape(y.shape), y, "conv")
+        assert_same(got_s.reshape(want.shape), want, "sum")
+    cs.close()
