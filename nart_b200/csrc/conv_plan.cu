@@ -5,6 +5,7 @@
 // bias.  b200_conv2d_run then only launches.
 #include <cmath>
 #include <cstdlib>
+#include <mutex>
 #include <string.h>
 
 #include <vector>
@@ -27,6 +28,51 @@ int upload(const std::vector<T> &v, T **dev)
     return B200_OK;
 }
 
+// A plan's scratch tensors (they grow with the batch, so the first run allocates them).  Small ones come from a pool per device
+// that keeps up to 64 MB of what destroyed plans gave back: mapping fresh device memory costs 0.3 .. 2.6 ms, taking it from
+// the pool some 10 us.  Larger ones are allocated and released on their own.
+constexpr size_t kScratchKeep = (size_t)64 << 20;
+int scratch_alloc(uint8_t **p, size_t bytes)
+{
+    struct Pool {
+        cudaMemPool_t pool = nullptr;
+        cudaStream_t stream = nullptr;
+    };
+    static std::mutex mu;
+    static Pool pools[64];
+    int device = 0;
+    B200_CUDA_TRY(cudaGetDevice(&device));
+    if (bytes > kScratchKeep || device >= 64)
+        return b200_malloc((void **)p, bytes);
+    std::lock_guard<std::mutex> lock(mu);
+    Pool &q = pools[device];
+    if (!q.stream)
+        B200_CUDA_TRY(cudaStreamCreateWithFlags(&q.stream, cudaStreamNonBlocking));
+    if (!q.pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        B200_CUDA_TRY(cudaMemPoolCreate(&pool, &props));
+        uint64_t keep = kScratchKeep;
+        B200_CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        q.pool = pool;
+    }
+    B200_CUDA_TRY(cudaMallocFromPoolAsync((void **)p, bytes, q.pool, q.stream));
+    B200_CUDA_TRY(cudaStreamSynchronize(q.stream));
+    return B200_OK;
+}
+// (cudaFree does not wait for the users of pool memory)
+cudaError_t scratch_free(uint8_t *p)
+{
+    if (!p)
+        return cudaSuccess;
+    const cudaError_t e = cudaDeviceSynchronize();
+    const cudaError_t f = cudaFree(p);
+    return e != cudaSuccess ? e : f;
+}
+
 void destroy_conv(b200_conv *cv)
 {
     if (!cv)
@@ -42,8 +88,8 @@ void destroy_conv(b200_conv *cv)
     cudaFree(cv->direct.shift_dev);
     if (cv->igemm)
         conv_igemm_destroy(cv->igemm);
-    cudaFree(cv->scratch);
-    cudaFree(cv->padded);
+    scratch_free(cv->scratch);
+    scratch_free(cv->padded);
     delete cv;
 }
 
@@ -395,10 +441,10 @@ int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
     auto grow = [](uint8_t *&buf, size_t &have, size_t need) -> int {
         if (need <= have)
             return B200_OK;
-        B200_CUDA_TRY(cudaFree(buf));
+        B200_CUDA_TRY(scratch_free(buf));
         buf = nullptr;
         have = 0;
-        B200_TRY(b200_malloc((void **)&buf, need));
+        B200_TRY(scratch_alloc(&buf, need));
         have = need;
         return B200_OK;
     };

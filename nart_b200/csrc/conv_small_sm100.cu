@@ -87,12 +87,12 @@ struct SmallTables {
 
 // N channels from accumulators `acc` (one pixel), the first at channel j of the tile: requantized, packed, stored at element
 // `at` of the output, and with the residual added at the same element of its sum; or at the shared address `stage`.
-template <int N>
+template <int N, bool SUM>
 __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const SmallArgs &g, const EpiConsts &ec, const SmallTables &t, int xcorr,
                                                int j, size_t at, uint32_t stage)
 {
     uint32_t w[N / 4], x[N / 4];
-    if (g.res) {            // on its way while the accumulators are requantized (Cout is a multiple of 16 then)
+    if (SUM) {            // on its way while the accumulators are requantized (Cout is a multiple of 16 then)
         if constexpr (N == 16) {
             const uint4 v = __ldg(reinterpret_cast<const uint4 *>(g.res + at));
             x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
@@ -130,7 +130,7 @@ __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const S
             *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
     };
     store(g.y + at);
-    if (g.res) {
+    if (SUM) {
 #pragma unroll
         for (int q = 0; q < N / 4; ++q)
             w[q] = add_residual(w[q], x[q], ec);
@@ -138,6 +138,8 @@ __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const S
     }
 }
 
+// SUM: the instantiation that also forms a residual add (ConvSum); the other one carries none of that code.
+template <bool SUM>
 __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_constant__ SmallMaps maps, const __grid_constant__ SmallArgs g)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -358,7 +360,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 tmem_ld16(t_row + c0, v);
                 tmem_ld_wait();
                 if (pix_valid)
-                    store_channels<16>(v, g, ec, t, xcorr, c0, at + c0, stage ? stage + c0 : 0u);
+                    store_channels<16, SUM>(v, g, ec, t, xcorr, c0, at + c0, stage ? stage + c0 : 0u);
                 __syncwarp();
             }
         } else if (ok) {
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                     acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
                     acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
                 }
-                store_channels<8>(acc, g, ec, t, xcorr, c1 + j, at + c1 + j, stage ? stage + j : 0u);
+                store_channels<8, SUM>(acc, g, ec, t, xcorr, c1 + j, at + c1 + j, stage ? stage + j : 0u);
             }
         }
     }
@@ -493,12 +495,13 @@ size_t conv_small_smem(SmallArgs &a, bool act_signed)
 
 int conv_small_launch(const SmallMaps &maps, const SmallArgs &a, int m_tiles, size_t smem, size_t bytes, cudaStream_t st)
 {
-    return launch_kernel(conv_small_kernel, dim3((unsigned)(m_tiles * a.n_tiles_n * a.split)), dim3(kSmallThreads), smem, st, bytes, a.split, maps, a);
+    return launch_kernel(a.res ? conv_small_kernel<true> : conv_small_kernel<false>, dim3((unsigned)(m_tiles * a.n_tiles_n * a.split)), dim3(kSmallThreads), smem, st, bytes, a.split, maps, a);
 }
 
 int conv_small_warm()
 {
-    B200_CUDA_TRY(cudaFuncSetAttribute(conv_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    for (auto k : { conv_small_kernel<false>, conv_small_kernel<true> })
+        B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     return B200_OK;
 }
 
