@@ -848,17 +848,23 @@ int b200_case_profile(b200_case_t *cs, float *ms_per_launch, int32_t *kinds, int
     return B200_OK;
 }
 
-// The device address of a small pinned host buffer, or nullptr.
+// The device address of a small pinned host buffer that the layout kernels can use in place of a staging buffer, or nullptr.
+// Their widest access is 16 bytes (float tensors of one pixel or one channel), so the address has to be a multiple of
+// that; a staging buffer's is, a row of a caller's array need not be.  Pinned memory may end inside the buffer.
 static void *direct_view(const void *host, size_t bytes)
 {
-    if (bytes > kDirectBytes)
+    if (bytes == 0 || bytes > kDirectBytes)
         return nullptr;
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaPointerAttributes first, last;
+    if (cudaPointerGetAttributes(&first, host) != cudaSuccess
+        || cudaPointerGetAttributes(&last, static_cast<const uint8_t *>(host) + bytes - 1) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || ((uintptr_t)first.devicePointer & 15) != 0
+        || static_cast<uint8_t *>(first.devicePointer) + bytes - 1 != last.devicePointer)
+        return nullptr;
+    return first.devicePointer;
 }
 
 int b200_case_run_host(
