@@ -867,6 +867,45 @@ static void *direct_view(const void *host, size_t bytes)
     return first.devicePointer;
 }
 
+// The buffers of one b200_case_run_host: whatever happens, no later run sees them, and a run that failed half-way is through
+// with them when the caller gets them back.
+struct DirectBuffers {
+    b200_case_t *cs;
+    cudaStream_t st;
+    bool done = false;
+    ~DirectBuffers()
+    {
+        if (!done)
+            cudaStreamSynchronize(st);
+        for (auto *ios : { &cs->inputs, &cs->outputs })
+            for (auto &io : *ios)
+                io.direct = nullptr;
+    }
+};
+
+static int run_on_host_buffers(b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs, b200_stream_t stream)
+{
+    DirectBuffers buffers{ cs, as_stream(stream) };
+    for (size_t i = 0; i < cs->inputs.size(); ++i) {
+        CaseIO &io = cs->inputs[i];
+        if (batch > 0 && !inputs[i])
+            return fail(B200_ERR_INVALID, "case_run_host: input %zu is NULL", i);
+        io.direct = direct_view(inputs[i], io.bytes_per_image * batch);
+        if (!io.direct)
+            B200_TRY(b200_memcpy_h2d(io.staging, inputs[i], io.bytes_per_image * batch, stream));
+    }
+    for (size_t i = 0; i < cs->outputs.size(); ++i)
+        cs->outputs[i].direct = direct_view(outputs[i], cs->outputs[i].bytes_per_image * batch);
+    B200_TRY(b200_case_run_device(cs, batch, stream));
+    for (size_t i = 0; i < cs->outputs.size(); ++i)
+        if (!cs->outputs[i].direct)
+            B200_TRY(b200_memcpy_d2h(outputs[i], cs->outputs[i].staging, cs->outputs[i].bytes_per_image * batch, stream));
+    B200_TRY(status_publish_launch(cs->status_host, as_stream(stream)));
+    B200_TRY(b200_stream_synchronize(stream));
+    buffers.done = true;
+    return B200_OK;
+}
+
 int b200_case_run_host(
     b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs,
     b200_stream_t stream)
@@ -879,25 +918,7 @@ int b200_case_run_host(
         return fail(B200_ERR_INVALID, "case_run_host: batch %d outside 0..%d", batch, cs->max_batch);
     if (!cs->status_host)
         B200_CUDA_TRY(cudaMallocHost((void **)&cs->status_host, sizeof(int)));
-    for (size_t i = 0; i < cs->inputs.size(); ++i) {
-        CaseIO &io = cs->inputs[i];
-        io.direct = direct_view(inputs[i], io.bytes_per_image * batch);
-        if (!io.direct)
-            B200_TRY(b200_memcpy_h2d(io.staging, inputs[i], io.bytes_per_image * batch, stream));
-    }
-    for (size_t i = 0; i < cs->outputs.size(); ++i)
-        cs->outputs[i].direct = direct_view(outputs[i], cs->outputs[i].bytes_per_image * batch);
-    int rc = b200_case_run_device(cs, batch, stream);
-    for (size_t i = 0; i < cs->outputs.size() && rc == B200_OK; ++i)
-        if (!cs->outputs[i].direct)
-            rc = b200_memcpy_d2h(outputs[i], cs->outputs[i].staging, cs->outputs[i].bytes_per_image * batch, stream);
-    if (rc == B200_OK)
-        rc = status_publish_launch(cs->status_host, as_stream(stream));
-    for (auto *ios : { &cs->inputs, &cs->outputs })
-        for (auto &io : *ios)
-            io.direct = nullptr;
-    B200_TRY(rc);
-    B200_TRY(b200_stream_synchronize(stream));
+    B200_TRY(run_on_host_buffers(cs, batch, inputs, outputs, stream));
     const int word = *cs->status_host;
     if (word != 0)
         return fail(B200_ERR_DEVICE_WAIT, "case_run_host: a device-side wait ran out (code 0x%x)", word);

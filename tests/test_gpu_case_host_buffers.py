@@ -39,3 +39,27 @@ def test_rows_of_pinned_arrays(k, f32_in):
     assert np.array_equal(got[1:1 + n * k].reshape(n, k), np.concatenate(want))
     assert got[0] == 7.0 and got[-1] == 7.0
     cs.close()
+
+
+def test_a_failed_host_run_leaves_no_buffer_behind():
+    """A run that fails on a later input must not leave run_device reading the pinned buffer of an earlier one."""
+    from nart_b200.case import Case
+    c, h, w = 4, 6, 6
+    cs = Case()
+    a, b = cs.input_u8(c, h, w), cs.input_u8(c, h, w)
+    cs.output_u8(cs.eltwise_sum([a, b], [0.02, 0.02], [0, 0], 0.04, 0))
+    cs.prepare(1)
+    rng = np.random.default_rng(11)
+    x = [torch.from_numpy(rng.integers(0, 256, (1, c, h, w), dtype=np.uint8)).pin_memory() for _ in range(2)]
+    (want,) = cs.run_host([t.numpy().copy() for t in x], [(np.uint8, (c, h, w))])       # fills the staging buffers
+    with pytest.raises(Exception, match="input 1 is NULL"):
+        cs.run_host_ptrs(1, [x[0].data_ptr(), None], [x[1].data_ptr()])
+    x[0].zero_()
+    cs.run_device(1)
+    torch.cuda.synchronize()
+    from nart_b200._lib import check, lib
+    got = np.empty_like(want)
+    check(lib.b200_memcpy_d2h(got.ctypes.data, cs.io_device_ptr(True, 0), got.nbytes, None))
+    torch.cuda.synchronize()
+    assert np.array_equal(got, want)
+    cs.close()
