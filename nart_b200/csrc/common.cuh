@@ -62,6 +62,23 @@ struct FastDiv {
 #endif
 };
 
+// Another device as the current one for the time of a scope.
+struct DeviceGuard {
+    int before = -1;
+    explicit DeviceGuard(int device)
+    {
+        int now = device;
+        if (cudaGetDevice(&now) == cudaSuccess && now != device && cudaSetDevice(device) == cudaSuccess)
+            before = now;
+    }
+    ~DeviceGuard()
+    {
+        if (before >= 0)
+            cudaSetDevice(before);
+    }
+    DeviceGuard(const DeviceGuard &) = delete;
+};
+
 // Number of SMs of the current device (cached).
 int sm_count();
 

@@ -63,11 +63,12 @@ int scratch_alloc(uint8_t **p, size_t bytes)
     B200_CUDA_TRY(cudaStreamSynchronize(q.stream));
     return B200_OK;
 }
-// (cudaFree does not wait for the users of pool memory)
-cudaError_t scratch_free(uint8_t *p)
+// (cudaFree does not wait for the users of pool memory: `device`, the plan's own, need not be the current one)
+cudaError_t scratch_free(uint8_t *p, int device)
 {
     if (!p)
         return cudaSuccess;
+    const DeviceGuard on(device);
     const cudaError_t e = cudaDeviceSynchronize();
     const cudaError_t f = cudaFree(p);
     return e != cudaSuccess ? e : f;
@@ -88,8 +89,8 @@ void destroy_conv(b200_conv *cv)
     cudaFree(cv->direct.shift_dev);
     if (cv->igemm)
         conv_igemm_destroy(cv->igemm);
-    scratch_free(cv->scratch);
-    scratch_free(cv->padded);
+    scratch_free(cv->scratch, cv->device);
+    scratch_free(cv->padded, cv->device);
     delete cv;
 }
 
@@ -438,10 +439,11 @@ int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
     if (!conv || n < 0)
         return fail(B200_ERR_INVALID, "conv(reserve): bad argument");
     const ConvGeom &g = conv->g;
-    auto grow = [](uint8_t *&buf, size_t &have, size_t need) -> int {
+    auto grow = [conv](uint8_t *&buf, size_t &have, size_t need) -> int {
         if (need <= have)
             return B200_OK;
-        B200_CUDA_TRY(scratch_free(buf));
+        const DeviceGuard on(conv->device);
+        B200_CUDA_TRY(scratch_free(buf, conv->device));
         buf = nullptr;
         have = 0;
         B200_TRY(scratch_alloc(&buf, need));
