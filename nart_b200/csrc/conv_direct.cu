@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) conv_direct_kernel(
         }
     }
     uint8_t *py = y + pix * g.k + k0 + kq * 4;
-    if (nk == 4 && (((size_t)g.k | (size_t)k0) & 3) == 0) {
+    if (nk == 4 && (((uintptr_t)y | (size_t)g.k | (size_t)k0) & 3) == 0) {
         *reinterpret_cast<uint32_t *>(py) = pack4(q[0], q[1], q[2], q[3]);
     } else {
         for (int j = 0; j < nk; ++j)

@@ -419,6 +419,10 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
         return B200_OK;
     if (conv->fused_residual)
         return fail(B200_ERR_INVALID, "conv: this plan has a residual add, run it with b200_conv2d_run_residual");
+    // Channel counts that AUTO pads would otherwise run on the CUDA cores, which take outputs at any address; the tensor-core
+    // path stores 16 bytes at a time.
+    if (conv->pad_c && ((uintptr_t)y & 15) != 0)
+        return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, as_stream(stream));
     B200_TRY(b200_conv2d_reserve(conv, n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
     const ConvGeom &g = conv->pad_c ? conv->g_pad : conv->g;
     if (conv->pad_c) {

@@ -35,3 +35,23 @@ def test_plan_destroyed_while_another_device_is_current():
         _plan(24, 144, hw)(other)
         torch.cuda.synchronize()
         assert all(torch.equal(g, want) for g in got)
+
+
+@pytest.mark.parametrize("c,k,hw", [(24, 18, 5), (20, 20, 3), (3, 17, 7), (40, 64, 3)])
+def test_output_at_any_address(c, k, hw):
+    """Images one by one into the rows of a larger output tensor: rows of k * hw * hw bytes, in a buffer at an odd address."""
+    from nart_b200 import ops
+    from nart_b200._lib import check, lib
+    n = 4
+    x = torch.randint(0, 256, (n, hw, hw, c), device="cuda", dtype=torch.uint8)
+    plan = _plan(c, k, hw)
+    want = _plan(c, k, hw, algo=ops.ALGO_DIRECT)(x)
+    row = k * hw * hw
+    for shift in (0, 1, 4):
+        y = torch.full((n * row + shift + 1,), 7, device="cuda", dtype=torch.uint8)
+        torch.cuda.synchronize()
+        for i in range(n):
+            check(lib.b200_conv2d_run(plan._h, x[i:i + 1].data_ptr(), 1, y.data_ptr() + shift + i * row, None))
+        torch.cuda.synchronize()
+        assert torch.equal(y[shift:shift + n * row].view(n, hw, hw, k), want)
+        assert int(y[-1]) == 7 and (shift == 0 or int(y[0]) == 7)
