@@ -181,14 +181,19 @@ B200_API int b200_conv2d_out_dims(const b200_conv_t *conv, int32_t *oh, int32_t 
 B200_API int b200_conv2d_algo(const b200_conv_t *conv);
 /* One line of text naming the kernel variant and tiling the plan resolved to (for logs and tuning). */
 B200_API int b200_conv2d_describe(const b200_conv_t *conv, char *buf, size_t len);
-/* x: device NHWC [n][h][w][c]; y: device NHWC [n][oh][ow][k].  Plans with a scratch tensor (the
- * row-lowered 4-channel stem; channel counts that are no multiple of 16, copied into padded tensors) grow it, with a device synchronization,
- * the first time a larger batch arrives; the old tensor is freed then. */
+/* x: device NHWC [n][h][w][c]; y: device NHWC [n][oh][ow][k].
+ * Row-lowered plans of 4-channel images have one scratch tensor: it grows, with a device synchronization, the first time
+ * a larger batch arrives (the old tensor is freed then), and runs that overlap on the GPU (different streams, no
+ * dependency between them) race on it.
+ * Channel counts that are no multiple of 16 are copied into padded tensors on the way to the tensor cores.  Such a plan
+ * may be run by several streams and threads at once, and under capture: the stream that ran it first keeps a buffer in the
+ * plan, a run on another stream takes one from a memory pool in stream order, a captured run leaves the graph one of its
+ * own.  Without memory for it, and for outputs that are not 16-byte aligned, the CUDA-core kernel runs instead. */
 B200_API int b200_conv2d_run(
     b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, b200_stream_t stream);
-/* Sizes the plan's scratch tensors for batches of up to n images now, so that no later run
- * allocates or frees (a CUDA graph captured from a run keeps the scratch address it saw).
- * No counterpart in the reference; a no-op for plans without scratch. */
+/* Sizes the plan's scratch for batches of up to n images now.  Row-lowered plans of 4-channel images: no later run allocates
+ * or frees (a CUDA graph captured from a run keeps the scratch address it saw).  Padded channel counts: nor does one
+ * on the stream that runs the plan first.  No counterpart in the reference; a no-op for plans without scratch. */
 B200_API int b200_conv2d_reserve(b200_conv_t *conv, int32_t n);
 /* As b200_conv2d_run, also writing the int32 accumulators (bias included) as NHWC int32.
  * Debug/verification entry; always takes the CUDA-core path. */

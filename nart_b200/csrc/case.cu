@@ -340,6 +340,7 @@ int b200_case_conv2d(
             p.group = c_in;
     }
     B200_TRY(b200_conv2d_create(&p, wsrc, bsrc, &op.conv));
+    op.conv->one_owner = true;
     int32_t oh, ow;
     b200_conv2d_out_dims(op.conv, &oh, &ow);
     op.out = new_tensor(cs, params->k, oh, ow, k_phys);
@@ -365,6 +366,7 @@ int b200_case_ip(
     op.ins = { in };
     B200_TRY(b200_ip_create(
         ti.c, ti.h, ti.w, k, ialpha, izp, walpha, n_walpha, wzp, oalpha, ozp, obits, weights, bias, &op.conv));
+    op.conv->one_owner = true;
     op.out = new_tensor(cs, k, 1, 1, k);
     *out = op.out;
     cs->ops.push_back(op);

@@ -554,11 +554,14 @@ __global__ void __launch_bounds__(256) conv_pad_channels_kernel(
         y[idx] = o[0];
 }
 
+static int pad_vectors(int c_pad) { return c_pad == 4 ? 1 : c_pad / 16; }
+bool conv_pad_channels_fits(size_t pixels, int c_pad) { return pixels * pad_vectors(c_pad) < 0x7fffff00ull; }
+
 int conv_pad_channels_launch(const uint8_t *x, uint8_t *y, size_t pixels, int c, int c_pad, uint8_t fill, cudaStream_t st)
 {
-    const int vecs = c_pad == 4 ? 1 : c_pad / 16;
+    const int vecs = pad_vectors(c_pad);
     const size_t total = pixels * vecs;
-    if (total >= 0x7fffff00ull)
+    if (!conv_pad_channels_fits(pixels, c_pad))
         return fail(B200_ERR_UNSUPPORTED, "conv(pad): tensor too large");
     const dim3 grid((unsigned)((total + 255) / 256));
     const uint32_t fill4 = (uint32_t)fill * 0x01010101u;

@@ -29,23 +29,24 @@ int upload(const std::vector<T> &v, T **dev)
 }
 
 // A plan's scratch tensors (they grow with the batch, so the first run allocates them).  Small ones come from a pool per device
-// that keeps up to 64 MB of what destroyed plans gave back: mapping fresh device memory costs 0.3 .. 2.6 ms, taking it from
-// the pool some 10 us.  Larger ones are allocated and released on their own.
+// that keeps up to 64 MB of what was given back: mapping fresh device memory costs 0.3 .. 2.6 ms, taking it from the pool
+// some 10 us.
 constexpr size_t kScratchKeep = (size_t)64 << 20;
-int scratch_alloc(uint8_t **p, size_t bytes)
+struct ScratchPool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;      // for allocations that belong to no stream of a caller
+};
+// The current device's
+int scratch_pool(ScratchPool *out)
 {
-    struct Pool {
-        cudaMemPool_t pool = nullptr;
-        cudaStream_t stream = nullptr;
-    };
     static std::mutex mu;
-    static Pool pools[64];
+    static ScratchPool pools[64];
     int device = 0;
     B200_CUDA_TRY(cudaGetDevice(&device));
-    if (bytes > kScratchKeep || device >= 64)
-        return b200_malloc((void **)p, bytes);
+    if (device >= 64)
+        return fail(B200_ERR_UNSUPPORTED, "conv: no scratch pool for device %d", device);
     std::lock_guard<std::mutex> lock(mu);
-    Pool &q = pools[device];
+    ScratchPool &q = pools[device];
     if (!q.stream)
         B200_CUDA_TRY(cudaStreamCreateWithFlags(&q.stream, cudaStreamNonBlocking));
     if (!q.pool) {
@@ -59,7 +60,27 @@ int scratch_alloc(uint8_t **p, size_t bytes)
         B200_CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
         q.pool = pool;
     }
-    B200_CUDA_TRY(cudaMallocFromPoolAsync((void **)p, bytes, q.pool, q.stream));
+    *out = q;
+    return B200_OK;
+}
+int pool_alloc(uint8_t **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st)
+{
+    *p = nullptr;
+    const cudaError_t e = cudaMallocFromPoolAsync((void **)p, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        *p = nullptr;
+        return fail(B200_ERR_NOMEM, "conv: scratch of %zu bytes", bytes);
+    }
+    B200_CUDA_TRY(e);
+    return B200_OK;
+}
+int scratch_alloc(uint8_t **p, size_t bytes)
+{
+    ScratchPool q;
+    if (bytes > kScratchKeep || scratch_pool(&q) != B200_OK)
+        return b200_malloc((void **)p, bytes);
+    B200_TRY(pool_alloc(p, bytes, q.pool, q.stream));
     B200_CUDA_TRY(cudaStreamSynchronize(q.stream));
     return B200_OK;
 }
@@ -91,7 +112,91 @@ void destroy_conv(b200_conv *cv)
         conv_igemm_destroy(cv->igemm);
     scratch_free(cv->scratch, cv->device);
     scratch_free(cv->padded, cv->device);
+    scratch_free(cv->home, cv->device);
     delete cv;
+}
+
+// The channel-padded copy of the activations, and the rows it is lowered to, for n images
+struct PaddedBytes {
+    size_t padded, lowered;
+    PaddedBytes(const b200_conv *cv, int32_t n)
+        : padded((size_t)n * cv->g.h * cv->g.w * cv->pad_c), lowered(cv->lowered ? (size_t)n * cv->g.h * cv->g.ow * (kLowerWindow * 4) : 0) {}
+    size_t lowered_at() const { return (padded + 255) & ~(size_t)255; }
+    size_t total() const { return lowered_at() + lowered; }
+};
+
+// The launches of a plan on the tensor cores
+int conv_run_igemm(b200_conv *cv, const uint8_t *x, int32_t n, uint8_t *y, uint8_t *padded, uint8_t *lowered, cudaStream_t st)
+{
+    const ConvGeom &g = cv->pad_c ? cv->g_pad : cv->g;
+    if (cv->pad_c) {
+        B200_TRY(conv_pad_channels_launch(x, padded, (size_t)n * g.h * g.w, cv->g.c, cv->pad_c, (uint8_t)g.izp, st));
+        x = padded;
+    }
+    if (cv->lowered) {
+        B200_TRY(conv_lower_rows_launch(g, x, n, lowered, st));
+        x = lowered;
+    }
+    return conv_igemm_launch(cv->igemm, x, n, y, st);
+}
+
+// A padded plan without an owner who orders its runs.  The stream that runs it first keeps a scratch buffer in the plan; a
+// run on another stream takes one from the pool for its own launches, and a run under capture leaves the graph a buffer of the
+// graph's own (an allocation node), as a captured address must outlive the plan's growth.  All of it is ordered by the
+// stream: no run waits for the device.  B200_ERR_NOMEM: nothing has been launched.
+int conv_run_padded(b200_conv *cv, const uint8_t *x, int32_t n, uint8_t *y, cudaStream_t st)
+{
+    const PaddedBytes need(cv, n);
+    ScratchPool q;
+    B200_TRY(scratch_pool(&q));
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;      // unique among all streams the process ever has, unlike the handle
+    B200_CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    if (capture == cudaStreamCaptureStatusNone)         // (not permitted under capture)
+        B200_CUDA_TRY(cudaStreamGetId(st, &id));
+    if (capture != cudaStreamCaptureStatusNone || (cv->home_taken && cv->home_stream != id)) {
+        uint8_t *block = nullptr;
+        B200_TRY(pool_alloc(&block, need.total(), q.pool, st));
+        const int rc = conv_run_igemm(cv, x, n, y, block, block + need.lowered_at(), st);
+        const cudaError_t e = cudaFreeAsync(block, st);
+        B200_TRY(rc);
+        B200_CUDA_TRY(e);
+        return B200_OK;
+    }
+    if (cv->home_bytes < need.total()) {
+        uint8_t *old = cv->home;
+        cv->home = nullptr;
+        cv->home_bytes = 0;
+        if (old)
+            B200_CUDA_TRY(cudaFreeAsync(old, st));
+        B200_TRY(pool_alloc(&cv->home, need.total(), q.pool, st));
+        cv->home_bytes = need.total();
+    }
+    cv->home_taken = true;
+    cv->home_stream = id;
+    return conv_run_igemm(cv, x, n, y, cv->home, cv->home + need.lowered_at(), st);
+}
+
+// Scratch tensors that serve every run of the plan, for n images
+int reserve_owned(b200_conv *conv, int32_t n)
+{
+    const PaddedBytes need(conv, n);
+    auto grow = [conv](uint8_t *&buf, size_t &have, size_t need) -> int {
+        if (need <= have)
+            return B200_OK;
+        const DeviceGuard on(conv->device);
+        B200_CUDA_TRY(scratch_free(buf, conv->device));
+        buf = nullptr;
+        have = 0;
+        B200_TRY(scratch_alloc(&buf, need));
+        have = need;
+        return B200_OK;
+    };
+    if (conv->lowered)
+        B200_TRY(grow(conv->scratch, conv->scratch_bytes, need.lowered));
+    if (conv->pad_c)
+        B200_TRY(grow(conv->padded, conv->padded_bytes, need.padded));
+    return B200_OK;
 }
 
 }  // namespace
@@ -338,6 +443,11 @@ int b200_conv2d_create(
     }
     if (rc == B200_OK) {
         cv->algo = B200_CONV_ALGO_IGEMM;
+        // what a first run under capture could not set up; a failure only matters to a run, which reports it itself
+        ScratchPool q;
+        int *status = nullptr;
+        if (cv->pad_c && (scratch_pool(&q) != B200_OK || conv_igemm_warm() != B200_OK || status_word_ptr(&status) != B200_OK))
+            cudaGetLastError();
     } else {
         cv->pad_c = 0;
         if (rc != B200_ERR_UNSUPPORTED || p->algo == B200_CONV_ALGO_IGEMM) {
@@ -419,45 +529,48 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
         return B200_OK;
     if (conv->fused_residual)
         return fail(B200_ERR_INVALID, "conv: this plan has a residual add, run it with b200_conv2d_run_residual");
-    // Channel counts that AUTO pads would otherwise run on the CUDA cores, which take outputs at any address; the tensor-core
-    // path stores 16 bytes at a time.
-    if (conv->pad_c && ((uintptr_t)y & 15) != 0)
-        return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, as_stream(stream));
-    B200_TRY(b200_conv2d_reserve(conv, n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
-    const ConvGeom &g = conv->pad_c ? conv->g_pad : conv->g;
-    if (conv->pad_c) {
-        B200_TRY(conv_pad_channels_launch(x, conv->padded, (size_t)n * g.h * g.w, conv->g.c, conv->pad_c, (uint8_t)g.izp, as_stream(stream)));
-        x = conv->padded;
+    cudaStream_t st = as_stream(stream);
+    if (conv->algo != B200_CONV_ALGO_IGEMM)
+        return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st);
+    // Channel counts that AUTO pads would otherwise run on the CUDA cores, which take outputs at any address, any size and need
+    // no memory; the tensor-core path stores 16 bytes at a time.
+    if (conv->pad_c && (((uintptr_t)y & 15) != 0 || !conv_pad_channels_fits((size_t)n * conv->g.h * conv->g.w, conv->pad_c)))
+        return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st);
+    std::lock_guard<std::mutex> lock(conv->mu);
+    if (conv->pad_c && !conv->one_owner) {
+        const int rc = conv_run_padded(conv, x, n, y, st);
+        return rc == B200_ERR_NOMEM ? conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st) : rc;
     }
-    if (conv->lowered) {
-        B200_TRY(conv_lower_rows_launch(g, x, n, conv->scratch, as_stream(stream)));
-        return conv_igemm_launch(conv->igemm, conv->scratch, n, y, as_stream(stream));
-    }
-    if (conv->algo == B200_CONV_ALGO_IGEMM)
-        return conv_igemm_launch(conv->igemm, x, n, y, as_stream(stream));
-    return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, as_stream(stream));
+    B200_TRY(reserve_owned(conv, n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
+    return conv_run_igemm(conv, x, n, y, conv->padded, conv->scratch, st);
 }
 
 int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
 {
     if (!conv || n < 0)
         return fail(B200_ERR_INVALID, "conv(reserve): bad argument");
-    const ConvGeom &g = conv->g;
-    auto grow = [conv](uint8_t *&buf, size_t &have, size_t need) -> int {
-        if (need <= have)
-            return B200_OK;
-        const DeviceGuard on(conv->device);
-        B200_CUDA_TRY(scratch_free(buf, conv->device));
-        buf = nullptr;
-        have = 0;
-        B200_TRY(scratch_alloc(&buf, need));
-        have = need;
+    std::lock_guard<std::mutex> lock(conv->mu);
+    if (!conv->pad_c || conv->one_owner) {
+        const int rc = reserve_owned(conv, n);
+        if (rc != B200_ERR_NOMEM || !conv->pad_c)
+            return rc;
+        conv->algo = B200_CONV_ALGO_DIRECT;         // needs no scratch
+        conv->pad_c = 0;
+        conv->lowered = false;
         return B200_OK;
-    };
-    if (conv->lowered)
-        B200_TRY(grow(conv->scratch, conv->scratch_bytes, (size_t)n * g.h * g.ow * (kLowerWindow * 4)));
-    if (conv->pad_c)
-        B200_TRY(grow(conv->padded, conv->padded_bytes, (size_t)n * g.h * g.w * conv->pad_c));
+    }
+    const size_t need = PaddedBytes(conv, n).total();
+    if (need <= conv->home_bytes)
+        return B200_OK;
+    const DeviceGuard on(conv->device);
+    ScratchPool q;
+    B200_TRY(scratch_pool(&q));
+    B200_CUDA_TRY(scratch_free(conv->home, conv->device));
+    conv->home = nullptr;
+    conv->home_bytes = 0;
+    B200_TRY(pool_alloc(&conv->home, need, q.pool, q.stream));
+    B200_CUDA_TRY(cudaStreamSynchronize(q.stream));
+    conv->home_bytes = need;
     return B200_OK;
 }
 

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <vector>
 
 #include "nart_b200.h"
@@ -116,6 +117,7 @@ constexpr int kLowerWindow = 8;
 int conv_lower_rows_launch(const ConvGeom &g, const uint8_t *x, int n, uint8_t *out, cudaStream_t st);
 
 // NHWC tensor of `pixels` x c bytes into one of c_pad channels (4 or a multiple of 16), the rest `fill`.
+bool conv_pad_channels_fits(size_t pixels, int c_pad);       // 31-bit indices
 int conv_pad_channels_launch(const uint8_t *x, uint8_t *y, size_t pixels, int c, int c_pad, uint8_t fill, cudaStream_t st);
 
 // Implicit-GEMM (tcgen05) convolution plan; defined in conv_igemm_sm100.cu.
@@ -188,6 +190,15 @@ struct b200_conv {
     b200::ConvGeom g_pad;
     uint8_t *padded = nullptr;      // [n][h][w][pad_c]
     size_t padded_bytes = 0;
+    // One owner orders all runs of the plan, on whatever streams, and keeps it longer than the graphs it captures (the case
+    // runner): `scratch` and `padded` serve every run.  Else a padded plan may be run by several streams and threads at
+    // once, as the CUDA-core kernel it replaces: see conv_run_padded.
+    bool one_owner = false;
+    uint8_t *home = nullptr;        // the scratch of the stream that ran the plan first
+    size_t home_bytes = 0;
+    bool home_taken = false;
+    unsigned long long home_stream = 0;
+    std::mutex mu;                  // one run's launches, and the launch cache of `igemm`, at a time
     float oalpha = 0.f;             // output scale, kept for b200_conv2d_fuse_residual_add
     bool fused_residual = false;    // the plan computes eltwise_sum(conv(x), res)
 };

@@ -37,6 +37,106 @@ def test_plan_destroyed_while_another_device_is_current():
         assert all(torch.equal(g, want) for g in got)
 
 
+def _direct(c, k, hw):
+    from nart_b200 import ops
+    return _plan(c, k, hw, algo=ops.ALGO_DIRECT)
+
+
+# (channels, output channels, map, batch): 24 -> 32 channels; an image of 3 channels, which is lowered as well
+SHARED = [(24, 144, 56, 16), (3, 32, 56, 16)]
+
+
+@pytest.mark.parametrize("c,k,hw,n", SHARED)
+def test_one_plan_on_several_streams(c, k, hw, n):
+    plan = _plan(c, k, hw)
+    xs = [torch.randint(0, 256, (n + i, hw, hw, c), device="cuda", dtype=torch.uint8) for i in range(4)]
+    want = [_direct(c, k, hw)(x) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    plan(xs[-1])
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)       # all is queued before any of it runs
+    for st in streams:
+        st.wait_stream(torch.cuda.current_stream())
+    got = []
+    for _ in range(25):
+        for x, st in zip(xs, streams):
+            with torch.cuda.stream(st):
+                got.append(plan(x))
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % len(xs)]), i
+
+
+@pytest.mark.parametrize("c,k,hw,n", SHARED)
+def test_one_plan_in_several_threads(c, k, hw, n):
+    import threading
+    plan = _plan(c, k, hw)
+    xs = [torch.randint(0, 256, (n, hw, hw, c), device="cuda", dtype=torch.uint8) for _ in range(4)]
+    want = [_direct(c, k, hw)(x) for x in xs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i, stream):
+        with torch.cuda.stream(stream):
+            got = [plan(xs[i]) for _ in range(40)]
+            torch.cuda.current_stream().synchronize()
+        bad.extend(i for y in got if not torch.equal(y, want[i]))
+
+    shared = torch.cuda.Stream()        # two threads on one stream, two on their own
+    threads = [threading.Thread(target=work, args=(i, shared if i < 2 else torch.cuda.Stream())) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+@pytest.mark.parametrize("c,k,hw,n", SHARED)
+def test_first_run_under_capture_and_replays_beside_growth(c, k, hw, n):
+    plan, direct = _plan(c, k, hw), _direct(c, k, hw)
+    x = torch.randint(0, 256, (2, hw, hw, c), device="cuda", dtype=torch.uint8)
+    big = torch.randint(0, 256, (3 * n, hw, hw, c), device="cuda", dtype=torch.uint8)
+    want_big = direct(big)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = plan(x)
+        z = plan(x[1:])
+    for seed in range(3):
+        x.random_(0, 256)
+        want = direct(x)
+        torch.cuda.synchronize()
+        eager = [plan(big[:n * (seed + 1)]) for _ in range(3)]      # grows the plan's own buffer
+        g.replay()
+        eager += [plan(big[:n * (seed + 1)]) for _ in range(3)]
+        torch.cuda.synchronize()
+        assert torch.equal(y, want) and torch.equal(z, want[1:])
+        assert all(torch.equal(e, want_big[:n * (seed + 1)]) for e in eager)
+
+
+def test_first_run_of_a_process_under_capture():
+    """Nothing that a capture forbids is left to the first run."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from tests.test_gpu_conv_scratch import _direct, _plan
+plan = _plan(24, 144, 14)
+x = torch.randint(0, 256, (2, 14, 14, 24), device="cuda", dtype=torch.uint8)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    y = plan(x)
+g.replay()
+torch.cuda.synchronize()
+assert torch.equal(y, _direct(24, 144, 14)(x))
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+
+
 @pytest.mark.parametrize("c,k,hw", [(24, 18, 5), (20, 20, 3), (3, 17, 7), (40, 64, 3)])
 def test_output_at_any_address(c, k, hw):
     """Images one by one into the rows of a larger output tensor: rows of k * hw * hw bytes, in a buffer at an odd address."""
