@@ -988,6 +988,8 @@ int b200_case_launch_count(const b200_case_t *cs, int32_t *launches)
     for (const auto &op : cs->ops) {
         if (op.conv && op.conv->lowered)
             ++n;   // the row-lowering kernel runs ahead of the convolution kernel
+        if (op.conv && op.conv->pad_c)
+            ++n;   // and the copy into a padded tensor ahead of both
         if (op.skipped)
             --n;   // an eltwise op that runs inside a conv's epilogue
     }

@@ -155,3 +155,18 @@ def test_output_at_any_address(c, k, hw):
         torch.cuda.synchronize()
         assert torch.equal(y[shift:shift + n * row].view(n, hw, hw, k), want)
         assert int(y[-1]) == 7 and (shift == 0 or int(y[0]) == 7)
+
+
+def test_case_counts_the_copy_into_the_padded_tensor(port):
+    from nart_b200.case import Case
+    rng = np.random.default_rng(5)
+    x = rng.integers(0, 256, (2, 20, 9, 9), dtype=np.uint8)
+    wt = rng.integers(0, 256, (32, 20, 3, 3), dtype=np.uint8)
+    q = dict(ialpha=0.02, izp=120, walpha=np.float32([0.005]), oalpha=0.5, ozp=99)
+    cs = Case()
+    cs.output_u8(cs.conv2d(cs.input_u8(20, 9, 9), wt, None, pad=(1, 1), **q))
+    cs.prepare(2)
+    assert cs.launch_count() == 4       # input layout, padding, convolution, output layout
+    (got,) = cs.run_host([x], [(np.uint8, (32, 9, 9))])
+    cs.close()
+    assert np.array_equal(got, port.conv2d_u8(x, wt, np.zeros(32, np.int32), (1, 1), (1, 1), 1, 0.02, 120, q["walpha"], 128, 0.5, 99))
