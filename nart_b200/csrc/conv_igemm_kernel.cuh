@@ -775,7 +775,8 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
             // Groups of several k-blocks, up to 32 a tile: lane i knows where k-block i lies (offsets from the tile's first pixel,
             // map, channel, weight column), and the warp takes four entries at a time by shuffles.  The counters below are one
             // chain of instructions, ~190 cycles a k-block.  (3x3 64 -> 64, 56x56, batch 256: 51.2 -> 49.4 us)
-            const bool table = (MODE == 0 || MODE == 1) && kgroup > 1 && kblocks <= 32;
+            // An offset has seven bits: -64 from the padding up to 31 from at most 32 taps.
+            const bool table = (MODE == 0 || MODE == 1) && kgroup > 1 && kblocks <= 32 && pad_h <= 64 && pad_w <= 64;
             uint32_t tab = 0;
             int tab_kc = 0;
             if (table) {

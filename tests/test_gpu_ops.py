@@ -515,3 +515,17 @@ def test_conv_picks_cta_pairs_on_long_launches(ops, port):
     want = port.conv2d_u8(x[pick], wt, bias, (1, 1), (1, 1), 1, walpha=walpha, relu=True, **q)
     assert_same(to_host_nchw(y[pick]), want, "long launch on cta pairs")
     assert_same(to_host_nchw(y_small[[0, 7]]), want[:2], "short launch on single CTAs")
+
+
+@pytest.mark.parametrize("pad,ks,st,c", [(64, 3, 1, 64), (65, 3, 1, 64), (70, 3, 2, 64), (130, 1, 1, 256), (70, (3, 2), 1, 32)])
+def test_conv_wide_padding(ops, pad, ks, st, c):
+    """Padding far beyond the kernel, on launches that fill the GPU: against the CUDA-core kernel."""
+    import torch
+    r, s = ks if isinstance(ks, tuple) else (ks, ks)
+    n, k, h, w = 3, 64, 13, 17
+    x, wt, bias, walpha = conv_inputs(pad, n, c, h, w, k, r, s)
+    q = dict(in_hw=(h, w), stride=(st, st), pad=(pad, pad), ialpha=0.02, izp=117, walpha=walpha, oalpha=0.01 * np.sqrt(c * r * s), ozp=99)
+    want = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **q)(to_dev_nhwc(x))
+    got = ops.Conv2d(wt, bias, algo=ops.ALGO_IGEMM, **q)(to_dev_nhwc(x))
+    assert ops.device_status() == 0
+    assert len(torch.unique(want)) > 100 and torch.equal(got, want)
