@@ -219,6 +219,11 @@ PyObject *eltwise_sum(PyObject *, PyObject *const *args, Py_ssize_t nargs)
             return nullptr;
         if (!first)
             first = t;
+        // the kernel reads as many bytes of every input as the first one has
+        if (t->numel() < first->numel() || t->device() != first->device()) {
+            PyErr_SetString(PyExc_ValueError, "eltwise: an input is smaller than the first one, or on another device");
+            return nullptr;
+        }
         xs[i] = u8(*t);
         ia[i] = (float)PyFloat_AsDouble(PyList_GET_ITEM(lists[1], i));
         iz[i] = (uint8_t)PyLong_AsLongLong(PyList_GET_ITEM(lists[2], i));

@@ -529,3 +529,16 @@ def test_conv_wide_padding(ops, pad, ks, st, c):
     got = ops.Conv2d(wt, bias, algo=ops.ALGO_IGEMM, **q)(to_dev_nhwc(x))
     assert ops.device_status() == 0
     assert len(torch.unique(want)) > 100 and torch.equal(got, want)
+
+
+def test_eltwise_refuses_an_input_that_is_smaller_than_the_first(ops):
+    import torch
+    big = torch.zeros((2, 5, 5, 16), device="cuda", dtype=torch.uint8)
+    q = dict(oalpha=0.04, ozp=3)
+    for shape in [(2, 5, 4, 16), (1, 5, 5, 16), (0, 5, 5, 16)]:
+        with pytest.raises(ValueError, match="smaller than the first"):
+            ops.add(big, torch.zeros(shape, device="cuda", dtype=torch.uint8), (0.02, 0.02), (0, 0), **q)
+        with pytest.raises(ValueError, match="smaller than the first"):
+            ops.eltwise_sum([big, big, torch.zeros(shape, device="cuda", dtype=torch.uint8)], (0.02,) * 3, (0,) * 3, **q)
+    # another shape of the same size is the same bytes
+    assert torch.equal(ops.add(big, big.view(2, 25, 16), (0.02, 0.02), (0, 0), **q), ops.add(big, big, (0.02, 0.02), (0, 0), **q))
