@@ -189,7 +189,24 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t nargs)
     B200_PY_CATCH
 }
 
-// eltwise_sum(xs, ialpha, izp, coeff or None, oalpha, ozp, obits, relu); the first four are lists of one length
+// float(o) and int(o), which take more than the plain conversions above: an integral float, a text
+float as_float(PyObject *o)
+{
+    PyObject *f = PyNumber_Float(o);
+    const double v = f ? PyFloat_AsDouble(f) : 0.0;
+    Py_XDECREF(f);
+    return (float)v;
+}
+uint8_t as_byte(PyObject *o)
+{
+    PyObject *i = PyNumber_Long(o);
+    const unsigned long long v = i ? PyLong_AsUnsignedLongLongMask(i) : 0;
+    Py_XDECREF(i);
+    return (uint8_t)v;
+}
+
+// eltwise_sum(xs, ialpha, izp, coeff or None, oalpha, ozp, obits, relu); the first four are lists of one length (zero points
+// that are not given are 0)
 PyObject *eltwise_sum(PyObject *, PyObject *const *args, Py_ssize_t nargs)
 {
     B200_PY_TRY
@@ -199,9 +216,9 @@ PyObject *eltwise_sum(PyObject *, PyObject *const *args, Py_ssize_t nargs)
     constexpr Py_ssize_t kMost = 64;      // the library declines more than four with a message of its own
     PyObject *lists[4] = { args[0], args[1], args[2], args[3] };
     const bool has_coeff = lists[3] != Py_None;
-    Py_ssize_t n = PyList_Check(lists[0]) ? PyList_GET_SIZE(lists[0]) : 0;
+    Py_ssize_t n = PyList_Check(lists[0]) ? PyList_GET_SIZE(lists[0]) : 0, n_zp = PyList_Check(lists[2]) ? PyList_GET_SIZE(lists[2]) : -1;
     for (int l = 0; l < (has_coeff ? 4 : 3); ++l)
-        if (!PyList_Check(lists[l]) || PyList_GET_SIZE(lists[l]) != n || n < 1 || n > kMost) {
+        if (!PyList_Check(lists[l]) || (l != 2 && PyList_GET_SIZE(lists[l]) != n) || n_zp > n || n < 1 || n > kMost) {
             PyErr_SetString(PyExc_ValueError, "eltwise: inputs, scales, zero points and coefficients must have one length");
             return nullptr;
         }
@@ -225,9 +242,9 @@ PyObject *eltwise_sum(PyObject *, PyObject *const *args, Py_ssize_t nargs)
             return nullptr;
         }
         xs[i] = u8(*t);
-        ia[i] = (float)PyFloat_AsDouble(PyList_GET_ITEM(lists[1], i));
-        iz[i] = (uint8_t)PyLong_AsLongLong(PyList_GET_ITEM(lists[2], i));
-        cf[i] = has_coeff ? (float)PyFloat_AsDouble(PyList_GET_ITEM(lists[3], i)) : 1.0f;
+        ia[i] = as_float(PyList_GET_ITEM(lists[1], i));
+        iz[i] = i < n_zp ? as_byte(PyList_GET_ITEM(lists[2], i)) : 0;
+        cf[i] = has_coeff ? as_float(PyList_GET_ITEM(lists[3], i)) : 1.0f;
         if (PyErr_Occurred())
             return nullptr;
     }

@@ -542,3 +542,17 @@ def test_eltwise_refuses_an_input_that_is_smaller_than_the_first(ops):
             ops.eltwise_sum([big, big, torch.zeros(shape, device="cuda", dtype=torch.uint8)], (0.02,) * 3, (0,) * 3, **q)
     # another shape of the same size is the same bytes
     assert torch.equal(ops.add(big, big.view(2, 25, 16), (0.02, 0.02), (0, 0), **q), ops.add(big, big, (0.02, 0.02), (0, 0), **q))
+
+
+def test_eltwise_takes_numbers_of_any_kind(ops):
+    """Zero points and scales as int() and float() take them; zero points that are left out are 0."""
+    import torch
+    x, y = (torch.randint(0, 256, (2, 3, 5, 16), device="cuda", dtype=torch.uint8) for _ in range(2))
+    want = ops.eltwise_sum([x, y], [0.02, 0.03], [7, 0], 0.05, 9, coeff=[1.0, 2.0])
+    for izp in ([7.0, 0.0], np.float32([7, 0]), np.uint8([7, 0]), torch.tensor([7, 0]), [7], (7 + 256, 0)):
+        assert torch.equal(ops.eltwise_sum([x, y], [0.02, 0.03], izp, 0.05, 9, coeff=[1, 2]), want)
+    assert torch.equal(ops.eltwise_sum((x, y), np.float64([0.02, 0.03]), [7, 0], 0.05, 9, coeff=np.int32([1, 2])), want)
+    with pytest.raises(Exception):
+        ops.eltwise_sum([x, y], [0.02, 0.03], [7, 0, 0], 0.05, 9)
+    with pytest.raises(Exception):
+        ops.eltwise_sum([x, y], [0.02], [7, 0], 0.05, 9)
