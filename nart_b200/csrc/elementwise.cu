@@ -226,38 +226,55 @@ __global__ void __launch_bounds__(kLayoutThreads) nhwc_to_nchw_kernel(
     }
 }
 
-template <typename TIn, typename Fn>
-static int nchw_to_nhwc_launch(const TIn *x, uint8_t *y, int n, int c, int P, int c_pad, int fill, Fn fn, cudaStream_t st)
+// The kernels number pixels with 32 bits: larger batches go in several launches.  run(first image, images) does one.
+template <typename Run>
+static int in_image_slices(int n, int P, int channels, Run run)
 {
-    const size_t pixels = (size_t)n * P;
-    const size_t groups = ((size_t)c_pad + TC - 1) / TC, blocks = (pixels + kLayoutThreads - 1) / kLayoutThreads * groups;
-    if (pixels > 0xffffff00ull || blocks > 0x7fffffffull)
-        return fail(B200_ERR_UNSUPPORTED, "layout: more than 2^32 pixels or 2^31 blocks");
-    const dim3 grid((unsigned)blocks);
-    const size_t bytes = pixels * (c * sizeof(TIn) + c_pad);
-    const bool a16 = c_pad % 16 == 0 && ((uintptr_t)y & 15) == 0, a4 = c_pad % 4 == 0 && ((uintptr_t)y & 3) == 0;
-    if (a16)
-        return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 16>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
-    if (a4)
-        return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 4>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
-    return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 1>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+    const size_t groups = ((size_t)channels + TC - 1) / TC;
+    const size_t blocks = 0x7fffffffull / groups;                       // of kLayoutThreads pixels
+    const size_t most = blocks * kLayoutThreads < 0xffffff00ull ? blocks * kLayoutThreads : 0xffffff00ull;
+    const size_t images = (size_t)P > most ? 0 : most / P;
+    if (images == 0)
+        return fail(B200_ERR_UNSUPPORTED, "layout: more than 2^31 blocks an image");
+    for (size_t i = 0; i < (size_t)n; i += images)
+        B200_TRY(run(i, (size_t)n - i < images ? (size_t)n - i : images));
+    return B200_OK;
+}
+
+template <typename TIn, typename Fn>
+static int nchw_to_nhwc_launch(const TIn *x0, uint8_t *y0, int n, int c, int P, int c_pad, int fill, Fn fn, cudaStream_t st)
+{
+    return in_image_slices(n, P, c_pad, [=](size_t first, size_t images) {
+        const TIn *x = x0 + first * c * P;
+        uint8_t *y = y0 + first * c_pad * P;
+        const size_t pixels = images * P, groups = ((size_t)c_pad + TC - 1) / TC;
+        const dim3 grid((unsigned)((pixels + kLayoutThreads - 1) / kLayoutThreads * groups));
+        const size_t bytes = pixels * (c * sizeof(TIn) + c_pad);
+        const bool a16 = c_pad % 16 == 0 && ((uintptr_t)y & 15) == 0, a4 = c_pad % 4 == 0 && ((uintptr_t)y & 3) == 0;
+        if (a16)
+            return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 16>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+        if (a4)
+            return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 4>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+        return launch_kernel(nchw_to_nhwc_kernel<TIn, Fn, 1>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, fill, pixels, groups, fn);
+    });
 }
 
 template <typename TOut, typename Fn>
-static int nhwc_to_nchw_launch(const uint8_t *x, TOut *y, int n, int c, int P, int c_pad, Fn fn, cudaStream_t st)
+static int nhwc_to_nchw_launch(const uint8_t *x0, TOut *y0, int n, int c, int P, int c_pad, Fn fn, cudaStream_t st)
 {
-    const size_t pixels = (size_t)n * P;
-    const size_t groups = ((size_t)c + TC - 1) / TC, blocks = (pixels + kLayoutThreads - 1) / kLayoutThreads * groups;
-    if (pixels > 0xffffff00ull || blocks > 0x7fffffffull)
-        return fail(B200_ERR_UNSUPPORTED, "layout: more than 2^32 pixels or 2^31 blocks");
-    const dim3 grid((unsigned)blocks);
-    const size_t bytes = pixels * (c * sizeof(TOut) + c_pad);
-    const bool a16 = c_pad % 16 == 0 && ((uintptr_t)x & 15) == 0, a4 = c_pad % 4 == 0 && ((uintptr_t)x & 3) == 0;
-    if (a16)
-        return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 16>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
-    if (a4)
-        return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 4>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
-    return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 1>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
+    return in_image_slices(n, P, c, [=](size_t first, size_t images) {
+        const uint8_t *x = x0 + first * c_pad * P;
+        TOut *y = y0 + first * c * P;
+        const size_t pixels = images * P, groups = ((size_t)c + TC - 1) / TC;
+        const dim3 grid((unsigned)((pixels + kLayoutThreads - 1) / kLayoutThreads * groups));
+        const size_t bytes = pixels * (c * sizeof(TOut) + c_pad);
+        const bool a16 = c_pad % 16 == 0 && ((uintptr_t)x & 15) == 0, a4 = c_pad % 4 == 0 && ((uintptr_t)x & 3) == 0;
+        if (a16)
+            return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 16>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
+        if (a4)
+            return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 4>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
+        return launch_kernel(nhwc_to_nchw_kernel<TOut, Fn, 1>, grid, dim3(kLayoutThreads), 0, st, bytes, 1, x, y, c, P, c_pad, pixels, groups, fn);
+    });
 }
 
 // Flat variants (no layout change): 4 elements per thread.

@@ -556,3 +556,11 @@ def test_eltwise_takes_numbers_of_any_kind(ops):
         ops.eltwise_sum([x, y], [0.02, 0.03], [7, 0, 0], 0.05, 9)
     with pytest.raises(Exception):
         ops.eltwise_sum([x, y], [0.02], [7, 0], 0.05, 9)
+
+
+def test_layout_of_more_pixels_than_32_bits_number(ops):
+    import torch
+    n, h, w = 3, 40000, 40000
+    x = torch.randint(0, 256, (n, 1, h, w), device="cuda", dtype=torch.uint8)
+    assert torch.equal(ops.nchw_to_nhwc(x).view(-1), x.view(-1))
+    assert torch.equal(ops.nhwc_to_nchw(x.view(n, h, w, 1)), x)
