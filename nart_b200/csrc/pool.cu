@@ -476,8 +476,9 @@ int pool_launch(
                                                                            : 1;
     const size_t bytes = (size_t)n * c * (g.h * g.w + g.oh * g.ow);
     // two outputs per thread, unrolled window, 32-bit indices: the common window shapes
-    if (vec >= 4 && (size_t)n * g.h * g.w * (c / 4) < 0xffffffffull && (size_t)n * g.oh * ((g.ow + 1) / 2) * (c / vec) < 0xffffffffull - 256ull * 65536ull
-        && (method == 0 || g.avg32)) {
+    // (words of the input and, where the padding makes it the larger one, of the output; threads, with room for a grid past the end)
+    if (vec >= 4 && (size_t)n * g.h * g.w * (c / 4) < 0xffffffffull && (size_t)n * g.oh * g.ow * (c / 4) < 0xffffffffull
+        && (size_t)n * g.oh * ((g.ow + 1) / 2) * (c / vec) < 0xffffffffull - 256ull * 65536ull && (method == 0 || g.avg32)) {
         if (g.kernel_h == 3 && g.kernel_w == 3 && g.stride_w == 2)
             return pool_pair_pick<3, 3, 2>(method, vec, x, y, g, lut_dev, tab, bytes, st);
         if (g.kernel_h == 3 && g.kernel_w == 3 && g.stride_w == 1)

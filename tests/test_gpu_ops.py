@@ -564,3 +564,17 @@ def test_layout_of_more_pixels_than_32_bits_number(ops):
     x = torch.randint(0, 256, (n, 1, h, w), device="cuda", dtype=torch.uint8)
     assert torch.equal(ops.nchw_to_nhwc(x).view(-1), x.view(-1))
     assert torch.equal(ops.nhwc_to_nchw(x.view(n, h, w, 1)), x)
+
+
+@pytest.mark.parametrize("method", [0, 1])
+def test_pool_with_more_output_than_32_bit_offsets_reach(ops, method):
+    """One pixel with two of padding all round: nine times as many outputs, 17 GB of them."""
+    import torch
+    c = 16
+    n = (1 << 34) // (9 * c) + 1000
+    x = torch.randint(0, 256, (n, 1, 1, c), device="cuda", dtype=torch.uint8)
+    args = (method, (3, 3), (2, 2), (1, 1), False, 0.05, 3, 0.05, 3)
+    y = ops.pool(x, *args)
+    assert y.numel() > 1 << 34
+    for part in (slice(0, 500), slice(n // 2, n // 2 + 500), slice(n - 2000, n)):
+        assert torch.equal(y[part], ops.pool(x[part], *args))
