@@ -68,6 +68,7 @@ struct CaseIO {
     // the layout kernels themselves (b200_case_run_host); nullptr: the staging buffer.
     void *direct = nullptr;
     void *buffer() const { return direct ? direct : staging; }
+    int behind = 0;            // images that such runs have left out of the staging buffer (refresh_staging)
 };
 
 // b200_case_run_host keeps tensors of at most this size out of the copy engines: a copy of 150 KB and the hand-over to
@@ -109,6 +110,8 @@ struct b200_case {
     // next step wait for d2h_done before they overwrite the device staging buffers
     cudaEvent_t comp_done = nullptr, d2h_done = nullptr;
     bool submitted = false;
+    bool staging_known = false;        // the caller has a staging buffer's address: every run goes through them
+    cudaStream_t refresh_stream = nullptr;
     int *status_host = nullptr;        // pinned: the device status word as the end of a run found it
 };
 
@@ -235,6 +238,7 @@ int b200_case_destroy(b200_case_t *cs)
         if (gr.exec)
             cudaGraphExecDestroy(gr.exec);
     cudaFreeHost(cs->status_host);
+    if (cs->refresh_stream) cudaStreamDestroy(cs->refresh_stream);
     if (cs->h2d_done) cudaEventDestroy(cs->h2d_done);
     if (cs->after_inputs) cudaEventDestroy(cs->after_inputs);
     if (cs->comp_done) cudaEventDestroy(cs->comp_done);
@@ -596,17 +600,6 @@ int b200_case_io_bytes(const b200_case_t *cs, int32_t is_output, int32_t index, 
     return B200_OK;
 }
 
-int b200_case_io_device_ptr(const b200_case_t *cs, int32_t is_output, int32_t index, void **dev_ptr)
-{
-    if (!cs || !dev_ptr)
-        return fail(B200_ERR_INVALID, "case_io_device_ptr: NULL argument");
-    const CaseIO *io = get_io(cs, is_output, index);
-    if (!io || !cs->prepared)
-        return fail(B200_ERR_INVALID, "case_io_device_ptr: no such buffer (is the case prepared?)");
-    *dev_ptr = io->staging;
-    return B200_OK;
-}
-
 int b200_case_tensor_device_ptr(const b200_case_t *cs, int32_t tensor, void **dev_ptr)
 {
     if (!cs || !dev_ptr)
@@ -628,12 +621,66 @@ static int run_outputs(b200_case_t *cs, int32_t batch, b200_stream_t stream)
     return run_eager(cs, batch, stream, 3);
 }
 
+// Brings the staging buffers to what a host run that used the caller's buffers in their place would have left there: uint8
+// inputs and all outputs come back from their device tensors.  Nobody has waited for any of it until now, so it is done
+// before this returns.
+static int refresh_staging(b200_case_t *cs)
+{
+    bool any = false;
+    for (auto *ios : { &cs->inputs, &cs->outputs })
+        for (auto &io : *ios)
+            any = any || io.behind > 0;
+    if (!any)
+        return B200_OK;
+    if (!cs->refresh_stream)
+        B200_CUDA_TRY(cudaStreamCreateWithFlags(&cs->refresh_stream, cudaStreamNonBlocking));
+    const b200_stream_t st = reinterpret_cast<b200_stream_t>(cs->refresh_stream);
+    if (cs->submitted && cs->d2h_done)
+        B200_CUDA_TRY(cudaStreamWaitEvent(cs->refresh_stream, cs->d2h_done, 0));
+    for (auto *ios : { &cs->inputs, &cs->outputs })
+        for (auto &io : *ios) {
+            const CaseTensor &t = cs->tensors[io.tensor];
+            if (io.behind > 0 && io.is_f32)         // (an output: float inputs always pass through staging)
+                B200_TRY(b200_dequantize_u8(t.dev, (float *)io.staging, io.behind, t.c, t.h, t.w, io.alpha, io.zp, 1, st));
+            else if (io.behind > 0)
+                B200_TRY(b200_nhwc_to_nchw_u8(t.dev, (uint8_t *)io.staging, io.behind, t.c, t.h, t.w, t.c_phys, st));
+        }
+    B200_CUDA_TRY(cudaStreamSynchronize(cs->refresh_stream));
+    for (auto *ios : { &cs->inputs, &cs->outputs })
+        for (auto &io : *ios)
+            io.behind = 0;
+    return B200_OK;
+}
+
+int b200_case_io_device_ptr(const b200_case_t *cs, int32_t is_output, int32_t index, void **dev_ptr)
+{
+    if (!cs || !dev_ptr)
+        return fail(B200_ERR_INVALID, "case_io_device_ptr: NULL argument");
+    const CaseIO *io = get_io(cs, is_output, index);
+    if (!io || !cs->prepared)
+        return fail(B200_ERR_INVALID, "case_io_device_ptr: no such buffer (is the case prepared?)");
+    B200_TRY(refresh_staging(const_cast<b200_case_t *>(cs)));
+    const_cast<b200_case_t *>(cs)->staging_known = true;
+    *dev_ptr = io->staging;
+    return B200_OK;
+}
+
+static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream);
+
 int b200_case_run_device(b200_case_t *cs, int32_t batch, b200_stream_t stream)
 {
     if (!cs || !cs->prepared)
         return fail(B200_ERR_INVALID, "case_run: the case is not prepared");
     if (batch < 0 || batch > cs->max_batch)
         return fail(B200_ERR_INVALID, "case_run: batch %d outside 0..%d", batch, cs->max_batch);
+    if (batch == 0)
+        return B200_OK;
+    B200_TRY(refresh_staging(cs));
+    return run_batch(cs, batch, stream);
+}
+
+static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream)
+{
     if (batch == 0)
         return B200_OK;
     // the legacy default stream cannot be captured: graph mode needs a stream of its own
@@ -892,19 +939,27 @@ static int run_on_host_buffers(b200_case_t *cs, int32_t batch, const void *const
         CaseIO &io = cs->inputs[i];
         if (batch > 0 && !inputs[i])
             return fail(B200_ERR_INVALID, "case_run_host: input %zu is NULL", i);
-        io.direct = direct_view(inputs[i], io.bytes_per_image * batch);
+        if (!cs->staging_known && !io.is_f32)
+            io.direct = direct_view(inputs[i], io.bytes_per_image * batch);
+        if (!io.direct && io.behind > 0)
+            B200_TRY(refresh_staging(cs));
         if (!io.direct)
             B200_TRY(b200_memcpy_h2d(io.staging, inputs[i], io.bytes_per_image * batch, stream));
     }
-    for (size_t i = 0; i < cs->outputs.size(); ++i)
-        cs->outputs[i].direct = direct_view(outputs[i], cs->outputs[i].bytes_per_image * batch);
-    B200_TRY(b200_case_run_device(cs, batch, stream));
+    if (!cs->staging_known)
+        for (size_t i = 0; i < cs->outputs.size(); ++i)
+            cs->outputs[i].direct = direct_view(outputs[i], cs->outputs[i].bytes_per_image * batch);
+    B200_TRY(run_batch(cs, batch, stream));
     for (size_t i = 0; i < cs->outputs.size(); ++i)
         if (!cs->outputs[i].direct)
             B200_TRY(b200_memcpy_d2h(outputs[i], cs->outputs[i].staging, cs->outputs[i].bytes_per_image * batch, stream));
     B200_TRY(status_publish_launch(cs->status_host, as_stream(stream)));
     B200_TRY(b200_stream_synchronize(stream));
     buffers.done = true;
+    for (auto *ios : { &cs->inputs, &cs->outputs })
+        for (auto &io : *ios)
+            if (io.direct && io.behind < batch)
+                io.behind = batch;
     return B200_OK;
 }
 
@@ -944,6 +999,7 @@ int b200_case_submit_host(b200_case_t *cs, int32_t batch, const void *const *inp
         B200_CUDA_TRY(cudaEventCreateWithFlags(&cs->comp_done, cudaEventDisableTiming));
         B200_CUDA_TRY(cudaEventCreateWithFlags(&cs->d2h_done, cudaEventDisableTiming));
     }
+    B200_TRY(refresh_staging(cs));
     // the input staging buffer is free again once the previous run's layout kernels have read it
     if (cs->submitted)
         B200_CUDA_TRY(cudaStreamWaitEvent(cs->copy_stream, cs->after_inputs, 0));
@@ -952,7 +1008,7 @@ int b200_case_submit_host(b200_case_t *cs, int32_t batch, const void *const *inp
             cs->inputs[i].staging, inputs[i], cs->inputs[i].bytes_per_image * batch, cudaMemcpyHostToDevice, cs->copy_stream));
     B200_CUDA_TRY(cudaEventRecord(cs->h2d_done, cs->copy_stream));
     B200_CUDA_TRY(cudaStreamWaitEvent(cs->comp_stream, cs->h2d_done, 0));
-    B200_TRY(b200_case_run_device(cs, batch, reinterpret_cast<b200_stream_t>(cs->comp_stream)));
+    B200_TRY(run_batch(cs, batch, reinterpret_cast<b200_stream_t>(cs->comp_stream)));
     // the results leave on a stream of their own, so that the next step's kernels do not queue behind the copy
     B200_CUDA_TRY(cudaEventRecord(cs->comp_done, cs->comp_stream));
     B200_CUDA_TRY(cudaStreamWaitEvent(cs->out_stream, cs->comp_done, 0));

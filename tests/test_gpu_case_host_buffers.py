@@ -63,3 +63,88 @@ def test_a_failed_host_run_leaves_no_buffer_behind():
     torch.cuda.synchronize()
     assert np.array_equal(got, want)
     cs.close()
+
+
+def _staged_output(cs, want):
+    from nart_b200._lib import check, lib
+    got = np.empty_like(want)
+    check(lib.b200_memcpy_d2h(got.ctypes.data, cs.io_device_ptr(True, 0), got.nbytes, None))
+    torch.cuda.synchronize()
+    return got
+
+
+@pytest.mark.parametrize("ask_first", [False, True])
+def test_resident_run_after_host_runs(ask_first):
+    """run_device works on what the host runs before it brought to the device, image by image, and the staging buffers hold
+    what they copied in and out -- whether or not the host runs used the caller's pinned buffers in their place."""
+    from nart_b200.case import Case
+    c, h, w, n = 3, 6, 5, 4
+    rng = np.random.default_rng(12)
+    cs = Case()
+    t = cs.input_u8(c, h, w)
+    t = cs.conv2d(t, rng.integers(0, 256, (32, c, 3, 3), dtype=np.uint8), None, pad=(1, 1), ialpha=0.02, izp=120, walpha=0.005,
+                  oalpha=0.1, ozp=111)
+    cs.output_f32(t, 0.1, 111)
+    cs.prepare(n)
+    a, b = (rng.integers(0, 256, (n, c, h, w), dtype=np.uint8) for _ in range(2))
+    (want_a,), (want_b,) = (cs.run_host([v], [(np.float32, (32, h, w))]) for v in (a, b))
+    if ask_first:
+        cs.io_device_ptr(False, 0)
+    pin_a, pin_b = (torch.from_numpy(v).pin_memory() for v in (a, b))
+    y = torch.zeros((n, 32, h, w)).pin_memory()
+    cs.run_host_ptrs(n, [pin_a.data_ptr()], [y.data_ptr()])
+    assert np.array_equal(y.numpy(), want_a)
+    cs.run_host_ptrs(2, [pin_b.data_ptr()], [y.data_ptr()])
+    mixed = np.concatenate([want_b[:2], want_a[2:]])
+    assert np.array_equal(y.numpy(), mixed)
+    pin_a.zero_(), pin_b.zero_()
+    cs.run_device(n)
+    torch.cuda.synchronize()
+    assert np.array_equal(_staged_output(cs, mixed), mixed)
+    # and a caller who has the staging buffer's address finds a host run's results and inputs there
+    pin_b.copy_(torch.from_numpy(b))
+    cs.run_host_ptrs(n, [pin_b.data_ptr()], [y.data_ptr()])
+    assert np.array_equal(_staged_output(cs, want_b), want_b)
+    cs.run_device(n)
+    torch.cuda.synchronize()
+    assert np.array_equal(_staged_output(cs, want_b), want_b)
+    cs.close()
+
+
+def test_staging_address_asked_for_after_a_host_run():
+    """The first look at the staging buffers comes behind a host run on pinned buffers: both hold its data."""
+    from nart_b200._lib import check, lib
+    cs, c = _logits_case(10, False)
+    rng = np.random.default_rng(4)
+    x = rng.integers(0, 256, (2, c, 1, 1), dtype=np.uint8)
+    (want,) = cs.run_host([x], [(np.float32, (10,))])
+    cs.run_host([np.zeros_like(x)], [(np.float32, (10,))])
+    pin_x, pin_y = torch.from_numpy(x).pin_memory(), torch.zeros((2, 10)).pin_memory()
+    cs.run_host_ptrs(2, [pin_x.data_ptr()], [pin_y.data_ptr()])
+    assert np.array_equal(_staged_output(cs, want), want)
+    got = np.empty_like(x)
+    check(lib.b200_memcpy_d2h(got.ctypes.data, cs.io_device_ptr(False, 0), got.nbytes, None))
+    torch.cuda.synchronize()
+    assert np.array_equal(got, x)
+    cs.close()
+
+
+def test_parade_forward_after_run(tmp_path):
+    """Parade.forward runs on the data that Parade.run brought to the device."""
+    import os
+
+    from nart_b200 import art, engine, nets
+    spec = nets.resnet(18, seed=23, hw=64, width_div=4, spread=True, num_classes=10)
+    path = os.path.join(tmp_path, "engine.bin")
+    engine.write_engine(spec, path, batch=2)
+    parade = art.load_parade(path, art.create_context_for_target("b200"))
+    inputs, outputs = art.get_empty_io(parade)
+    (iname,), (oname,) = parade.get_input_names(), parade.get_output_names()
+    for seed in (5, 6):
+        inputs[iname][:] = np.random.default_rng(seed).integers(0, 256, inputs[iname].shape, dtype=np.uint8)
+        parade.run(inputs, outputs)
+        want = outputs[oname].copy()
+        outputs[oname].fill(0)
+        parade.forward()
+    assert np.array_equal(_staged_output(parade._case, want), want)
+    parade.close()
