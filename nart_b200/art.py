@@ -166,8 +166,8 @@ class Parade:
                 raise ValueError("output dtype not match")
         x = np.ascontiguousarray(x)
         given = [outputs[oname] for oname in self.get_output_names()]
-        direct = [isinstance(y, np.ndarray) and y.flags.c_contiguous and y.flags.writeable for y in given]
-        results = [y if ok else np.empty(y.shape, dtype=y.dtype) for y, ok in zip(given, direct)]
+        direct = [isinstance(y, np.ndarray) and y.flags.c_contiguous and y.flags.writeable and y.dtype.isnative for y in given]
+        results = [y if ok else np.empty(y.shape, dtype=y.dtype.newbyteorder("=")) for y, ok in zip(given, direct)]
         self._case.run_host_ptrs(self._batch, [x.ctypes.data], [y.ctypes.data for y in results], self._stream.cuda_stream)
         for y, got, ok in zip(given, results, direct):
             if not ok:

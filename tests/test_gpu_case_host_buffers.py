@@ -148,3 +148,26 @@ def test_parade_forward_after_run(tmp_path):
         parade.forward()
     assert np.array_equal(_staged_output(parade._case, want), want)
     parade.close()
+
+
+def test_parade_run_into_arrays_of_any_kind(tmp_path):
+    """Byte order, strides and alignment of the output arrays are the caller's: values are assigned, not bytes."""
+    import os
+
+    from nart_b200 import art, engine, nets
+    spec = nets.resnet(18, seed=23, hw=64, width_div=4, spread=True, num_classes=10)
+    path = os.path.join(tmp_path, "engine.bin")
+    engine.write_engine(spec, path, batch=2)
+    parade = art.load_parade(path, art.create_context_for_target("b200"))
+    inputs, outputs = art.get_empty_io(parade)
+    (iname,), (oname,) = parade.get_input_names(), parade.get_output_names()
+    inputs[iname][:] = np.random.default_rng(5).integers(0, 256, inputs[iname].shape, dtype=np.uint8)
+    parade.run(inputs, outputs)
+    want, shape = outputs[oname].copy(), outputs[oname].shape
+    assert len(np.unique(want)) > 3
+    kinds = [np.zeros(shape, ">f4"), np.zeros((2 * shape[0],) + shape[1:], np.float32)[::2], np.zeros(shape[:1] + (12, 1, 1), ">f4")[:, 1:11],
+             np.zeros(4 * want.size + 1, np.uint8)[1:].view(np.float32).reshape(shape)]
+    for y in kinds:
+        parade.run(inputs, {oname: y})
+        assert np.array_equal(y, want)
+    parade.close()
