@@ -200,7 +200,11 @@ class _PinnedMemory:
 
 
 def _pinned_zeros(shape, dtype) -> np.ndarray:
-    arr = np.asarray(_PinnedMemory(shape, np.dtype(dtype)))
+    from ._lib import B200Error
+    try:
+        arr = np.asarray(_PinnedMemory(shape, np.dtype(dtype)))
+    except B200Error:              # page-locked memory is a limited resource, and only the faster one
+        return np.zeros(shape, dtype=np.dtype(dtype))
     arr.fill(0)
     return arr
 
