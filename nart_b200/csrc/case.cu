@@ -924,8 +924,8 @@ struct DirectBuffers {
     bool done = false;
     ~DirectBuffers()
     {
-        if (!done)
-            cudaStreamSynchronize(st);
+        if (!done && cudaStreamSynchronize(st) != cudaSuccess)
+            cudaGetLastError();     // (the run's own error is the one that is reported)
         for (auto *ios : { &cs->inputs, &cs->outputs })
             for (auto &io : *ios)
                 io.direct = nullptr;

@@ -140,13 +140,14 @@ __global__ void __launch_bounds__(kLayoutThreads) nchw_to_nhwc_kernel(
             // 32 bytes of one pixel and not 32 lanes a word each of 32 pixels (16 M elements of 236 channels: 27.5 us so)
             __shared__ uint32_t tile[kLayoutThreads / 32][32][TC / 4 + 1];
             uint32_t (*t)[TC / 4 + 1] = tile[threadIdx.x / 32];
-            const unsigned lane = threadIdx.x & 31, active = __activemask();
+            const unsigned lane = threadIdx.x & 31;
+            const unsigned live = min(32u, pixels - (gp - lane));         // the lanes that are here: a prefix of the warp
+            const unsigned active = 0xffffffffu >> (32 - live);
 #pragma unroll
             for (int j = 0; j < TC / 4; ++j)
                 t[lane][j] = wv[j];
             __syncwarp(active);
             uint8_t *first = out + (size_t)(gp - lane) * c_pad + c0;      // the warp's first pixel
-            const unsigned live = __popc(active);                         // lanes below `pixels`: a prefix of the warp
             for (unsigned i = lane; i < live * (TC / 4); i += live)
                 *reinterpret_cast<uint32_t *>(first + (size_t)(i / (TC / 4)) * c_pad + (i % (TC / 4)) * 4) = t[i / (TC / 4)][i % (TC / 4)];
         }
