@@ -277,7 +277,7 @@ static int pool_pair_pick(int method, int vec, const uint8_t *x, uint8_t *y, con
 // admits at most 257 taps, 65535 a lane.
 // LANES > 1: that many neighbouring lanes share an output, taking every LANES-th round of taps, for launches with few
 // outputs and large windows, whose time is one thread's chain of loads (2048 channels of one 7x7 map: 10.8 us with one).
-template <int VEC, int LANES = 1>
+template <int VEC, int LANES = 1, bool ROWS = false>
 __global__ void __launch_bounds__(256) pool_avg_kernel(
     const uint8_t *__restrict__ x, uint8_t *__restrict__ y, PoolGeom g, PoolAvgTab tab)
 {
@@ -308,30 +308,10 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
         for (int j = 0; j < W; ++j)
             sum[j] = { 0u, 0u };
         const int wd = max(we - ws, 0), cnt = max(he - hs, 0) * wd;
-        // the window's taps as one sequence, eight per round, loaded before any is used: a large window (the
-        // global average of a 7x7 map is 49 taps) keeps several loads in flight
+        // eight taps per round, loaded before any is used: a large window (the global average of a 7x7 map is 49 taps)
+        // keeps several loads in flight
         constexpr int UNR = 8;
-        const uint8_t *base = x + (((size_t)n * g.h + hs) * g.w + ws) * g.c + (size_t)ci * VEC;
-        int ty = 0, tx = 0;
-        if (LANES > 1 && wd > 0) {
-            ty = sub * UNR / wd;
-            tx = sub * UNR - ty * wd;
-        }
-        for (int t = sub * UNR; t < cnt; t += UNR * LANES) {
-            uint32_t v[UNR][W];
-#pragma unroll
-            for (int u = 0; u < UNR; ++u) {
-#pragma unroll
-                for (int j = 0; j < W; ++j)
-                    v[u][j] = 0;
-                if (t + u < cnt) {
-                    load_words<VEC>(base + (size_t)(ty * g.w + tx) * g.c, v[u]);
-                    if (++tx == wd) {
-                        tx = 0;
-                        ++ty;
-                    }
-                }
-            }
+        auto add = [&](const uint32_t (&v)[UNR][W]) {
 #pragma unroll
             for (int u = 0; u < UNR; ++u)
 #pragma unroll
@@ -340,10 +320,51 @@ __global__ void __launch_bounds__(256) pool_avg_kernel(
                     sum[j].lo += b.lo;
                     sum[j].hi += b.hi;
                 }
-            if (LANES > 1 && t + UNR * LANES < cnt) {
-                const int at = t + UNR * LANES;
-                ty = at / wd;
-                tx = at - ty * wd;
+        };
+        if constexpr (ROWS) {
+            for (int iy = hs; iy < he; ++iy) {
+                const uint8_t *row = x + (((size_t)n * g.h + iy) * g.w) * g.c + (size_t)ci * VEC;
+                for (int ix = ws; ix < we; ix += UNR) {
+                    uint32_t v[UNR][W];
+#pragma unroll
+                    for (int u = 0; u < UNR; ++u) {
+#pragma unroll
+                        for (int j = 0; j < W; ++j)
+                            v[u][j] = 0;
+                        if (ix + u < we)
+                            load_words<VEC>(row + (size_t)(ix + u) * g.c, v[u]);
+                    }
+                    add(v);
+                }
+            }
+        } else {
+            const uint8_t *base = x + (((size_t)n * g.h + hs) * g.w + ws) * g.c + (size_t)ci * VEC;
+            int ty = 0, tx = 0;
+            if (LANES > 1 && wd > 0) {
+                ty = sub * UNR / wd;
+                tx = sub * UNR - ty * wd;
+            }
+            for (int t = sub * UNR; t < cnt; t += UNR * LANES) {
+                uint32_t v[UNR][W];
+#pragma unroll
+                for (int u = 0; u < UNR; ++u) {
+#pragma unroll
+                    for (int j = 0; j < W; ++j)
+                        v[u][j] = 0;
+                    if (t + u < cnt) {
+                        load_words<VEC>(base + (size_t)(ty * g.w + tx) * g.c, v[u]);
+                        if (++tx == wd) {
+                            tx = 0;
+                            ++ty;
+                        }
+                    }
+                }
+                add(v);
+                if (LANES > 1 && t + UNR * LANES < cnt) {
+                    const int at = t + UNR * LANES;
+                    ty = at / wd;
+                    tx = at - ty * wd;
+                }
             }
         }
 #pragma unroll
@@ -486,9 +507,10 @@ int pool_launch(
         if (g.kernel_h == 2 && g.kernel_w == 2 && g.stride_w == 2)
             return pool_pair_pick<2, 2, 2>(method, vec, x, y, g, lut_dev, tab, bytes, st);
     }
-    // an average whose 16-byte vectors would not give every SM a few warps goes by words: four times the threads, and
-    // the loop over the window is a chain of loads (2048 channels of 7x7, batch 256)
-    if (method == 1 && vec == 16 && (size_t)n * g.oh * g.ow * (c / 16) < (size_t)sm_count() * 1024)
+    // an average whose 16-byte vectors would leave the SMs a few warps each goes by words: four times the threads for a chain of
+    // loads (2048 channels of one 7x7 window, batch 256: 221 vectors an SM).  Beyond that the vectors win: 7x7 stride 7 on 256
+    // channels of 56 x 56, batch 64, 443 an SM: 23.1 us by words, 15.5; 7x7 on 64 of 71 x 71, batch 8, 913: 36.4 and 19.6.
+    if (method == 1 && vec == 16 && (size_t)n * g.oh * g.ow * (c / 16) < (size_t)sm_count() * 256)
         vec = 4;
     const size_t outs = (size_t)n * g.oh * g.ow * (c / vec), blocks = (outs + 255) / 256;
     if (method == 1 && vec == 4 && outs % 4 == 0 && outs * 8 <= (size_t)sm_count() * 2048 && g.kernel_h * g.kernel_w >= 16)
@@ -498,9 +520,18 @@ int pool_launch(
         if (vec == 4) return launch_kernel(pool_max_kernel<4>, dim3(resident_grid<pool_max_kernel<4>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
         return launch_kernel(pool_max_kernel<1>, dim3(resident_grid<pool_max_kernel<1>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, lut_dev);
     } else {
-        if (vec == 16) return launch_kernel(pool_avg_kernel<16>, dim3(resident_grid<pool_avg_kernel<16>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
-        if (vec == 4) return launch_kernel(pool_avg_kernel<4>, dim3(resident_grid<pool_avg_kernel<4>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
-        return launch_kernel(pool_avg_kernel<1>, dim3(resident_grid<pool_avg_kernel<1>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab);
+#define B200_AVG(...) return launch_kernel(pool_avg_kernel<__VA_ARGS__>, dim3(resident_grid<pool_avg_kernel<__VA_ARGS__>, 256>(blocks)), dim3(256), 0, st, bytes, 1, x, y, g, tab)
+        // A window's taps as one sequence take the fewest rounds of loads, which counts while a launch is one thread's chain of
+        // them; row by row they take fewer instructions, which counts once the GPU is full and where rows fill their rounds of
+        // eight (7x7 stride 1, 7 channels of 56 x 56, batch 64: 65.3 and 52.9 us; 40 channels of 14 x 14: 6.8 and 8.8).
+        // Sixteen channels a thread are bound by neither: 29.2 and 31.2 us (256 channels of 28 x 28, batch 32).
+        const bool rows = (g.kernel_w + 7) / 8 * 7 <= g.kernel_w && outs >= (size_t)sm_count() * (vec == 1 ? 1024 : 4096);
+        if (vec == 16) B200_AVG(16);
+        if (vec == 4 && rows) B200_AVG(4, 1, true);
+        if (vec == 4) B200_AVG(4);
+        if (rows) B200_AVG(1, 1, true);
+        B200_AVG(1);
+#undef B200_AVG
     }
 }
 

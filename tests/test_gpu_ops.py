@@ -578,3 +578,19 @@ def test_pool_with_more_output_than_32_bit_offsets_reach(ops, method):
     assert y.numel() > 1 << 34
     for part in (slice(0, 500), slice(n // 2, n // 2 + 500), slice(n - 2000, n)):
         assert torch.equal(y[part], ops.pool(x[part], *args))
+
+
+@pytest.mark.parametrize("c,h,w,n,ks,st,pad", [
+    (7, 40, 41, 70, 7, 1, 3),      # a byte a thread, row by row
+    (5, 9, 9, 3, 7, 1, 0),         # the same as one sequence
+    (20, 40, 41, 80, 8, 1, 0),     # a word a thread, row by row
+    (20, 9, 9, 3, 7, 2, 3),
+    (64, 19, 17, 4, 7, 1, 3),      # few vectors: by words
+    (64, 33, 35, 32, 5, 1, 2),     # vectors of sixteen channels
+    (16, 15, 15, 9, 15, 1, 7),
+])
+def test_average_pool_forms(ops, port, c, h, w, n, ks, st, pad):
+    x = np.random.default_rng(c + ks).integers(0, 256, (n, c, h, w), dtype=np.uint8)
+    for ceil in (0, 1):
+        q = ((ks, ks), (pad, pad), (st, st), ceil, 0.05, 33, 0.03, 12)
+        assert_same(to_host_nchw(ops.pool(to_dev_nhwc(x), 1, *q)), port.pool_u8(x, 1, *q), "average pool")
