@@ -322,8 +322,8 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_kernel(
 // is built); mult * 2^-shift is a float m (24 significant bits); acc * m + (zero point + 1/2) is formed by one
 // multiply-add rounded toward zero, which never crosses an integer, and 2^23 is added, again toward zero: the low
 // bits are then floor(acc * m + 1/2) + zero point for every result of 0 or more, and for every negative one the
-// low 16 bits are a negative 16-bit number (results stay below 2^13 in magnitude, checked as well).  Floor and
-// ceiling run on pairs of those.
+// low 16 bits are a negative 16-bit number (below 2^23 a float's last bit is a half: results stay within -2^14 .. 2^15,
+// checked as well).  Floor and ceiling run on pairs of those.
 // (A thread that walks whole columns, every input row loaded and transposed once, is no faster: its accumulators in
 // flight and weights leave 16 to 20 warps per SM, and its row loop's bookkeeping costs what the shared rows save.)
 // Weight table: [c/4][3 kernel rows][2 + (S == 2)][4 channels] words.  Requantize table: [c/4] 4 start values, 4 floats.

@@ -337,11 +337,20 @@ int b200_conv2d_create(
             }
             rc = upload(w3, &cv->direct.w_dw3_dev);
             if (rc == B200_OK) rc = upload(q3, &cv->direct.q_dw3_dev);
-            // its fp32 requantize: every accumulator (9 products of at most 255 * 128) below 2^22, every result below 2^13
+            // its fp32 requantize: every accumulator below 2^22, every result within the 16 bits it is clamped in (see
+            // conv_depthwise3x3_strip_kernel: half steps below zero).  Taps are 0 .. 255, so a channel's negative and positive
+            // weights bound its accumulators; 22 of 272 layers of MobileNetV2 with random weights miss a bound by their number.
             bool strip = g.stride_w == g.stride_h && (g.stride_w == 1 || g.stride_w == 2);
-            for (int k = 0; k < g.k; ++k)
-                strip = strip && std::abs((long long)bias_fold[k]) < (1 << 22) - 9 * 255 * 128
-                    && ldexp((std::abs((double)bias_fold[k]) + 9 * 255 * 128) * mult[k], -shift[k]) < 8000.0;
+            for (int k = 0; k < g.k; ++k) {
+                int neg = 0, pos = 0;
+                for (int t = 0; t < 9; ++t) {
+                    const int w = w_s8[(size_t)k * 9 + t];
+                    (w < 0 ? neg : pos) += w;
+                }
+                const long long lo = bias_fold[k] + 255ll * neg, hi = bias_fold[k] + 255ll * pos;
+                strip = strip && lo > -(1 << 22) && hi < (1 << 22) && ldexp((double)lo * mult[k], -shift[k]) > -16380.0
+                    && ldexp((double)hi * mult[k], -shift[k]) + g.ozp < 32760.0;
+            }
             if (rc == B200_OK && strip) {
                 // one kernel row against 3 + stride_w neighbouring input pixels (conv_depthwise3x3_strip_kernel)
                 const int nv = g.stride_w == 2 ? 3 : 2;

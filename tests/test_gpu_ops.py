@@ -594,3 +594,23 @@ def test_average_pool_forms(ops, port, c, h, w, n, ks, st, pad):
     for ceil in (0, 1):
         q = ((ks, ks), (pad, pad), (st, st), ceil, 0.05, 33, 0.03, 12)
         assert_same(to_host_nchw(ops.pool(to_dev_nhwc(x), 1, *q)), port.pool_u8(x, 1, *q), "average pool")
+
+
+@pytest.mark.parametrize("st", [(1, 1), (2, 2), (1, 2), (2, 1)])
+@pytest.mark.parametrize("reach", [200, 8000, 16000, 16800, 32000, 33500, 70000])
+def test_depthwise3x3_results_far_beyond_a_byte(ops, port, reach, st):
+    """Scales at which results reach to and beyond the 16 bits the fp32 requantize clamps in (2^15 above, 2^14 below): taps of
+    0 and 255 by the weights' signs, the whole range of accumulators among them."""
+    c, h, w = 16, 12, 15
+    rng = np.random.default_rng(reach + 10 * st[0] + st[1])
+    wt = rng.integers(-127, 128, (c, 1, 3, 3))
+    bias = rng.integers(-4096, 4097, c).astype(np.int32)
+    x = rng.integers(0, 256, (4, c, h, w), dtype=np.uint8)
+    for img, sign in ((1, 1), (2, -1)):
+        x[img] = np.tile(np.where(sign * wt[:, 0] > 0, 255, 0), (1, h // 3, w // 3)).astype(np.uint8)
+    most = float(np.maximum(255 * np.where(wt > 0, wt, 0).sum((1, 2, 3)), -255 * np.where(wt < 0, wt, 0).sum((1, 2, 3))).max())
+    for relu in (False, True):
+        q = dict(ialpha=0.02, izp=3, walpha=np.float32([0.01]), wzp=128, oalpha=float(np.float32(0.0002 * most / reach)), ozp=60)
+        want = port.conv2d_u8(x, (wt + 128).astype(np.uint8), bias, st, (1, 1), c, relu=relu, **q)
+        conv = ops.Conv2d((wt + 128).astype(np.uint8), bias, in_hw=(h, w), stride=st, pad=(1, 1), group=c, relu=relu, **q)
+        assert_same(to_host_nchw(conv(to_dev_nhwc(x))), want, "reach %d" % reach)
