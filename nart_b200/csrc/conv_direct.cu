@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------
-// Depthwise 3x3 with stride S (1 or 2) both ways: a thread computes two output pixels side by
-// side, in ROWS output rows, for four channels.  The two windows of a row cover 3 + S neighbouring input
+// Depthwise 3x3 with horizontal stride S (1 or 2): a thread computes two output pixels side by
+// side, in ROWS output rows (one unless the vertical stride is S too), for four channels.  The two windows of a row cover 3 + S neighbouring input
 // pixels per kernel row.  One transpose of the first four of those words gives, per channel, a
 // word (x0, x1, x2, x3) that serves both pixels: dp4a against (w0, w1, w2, 0) is the left pixel's
 // kernel row; the right pixel's is (0, w0, w1, w2) for S == 1, and for S == 2 (0, 0, w0, w1) plus
@@ -327,9 +327,12 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_kernel(
 // (A thread that walks whole columns, every input row loaded and transposed once, is no faster: its accumulators in
 // flight and weights leave 16 to 20 warps per SM, and its row loop's bookkeeping costs what the shared rows save.)
 // Weight table: [c/4][3 kernel rows][2 + (S == 2)][4 channels] words.  Requantize table: [c/4] 4 start values, 4 floats.
+// FP false, for scales whose results leave those bounds: the integers of conv_depthwise3x3_kernel, four constants a channel.
+// (144 channels of 56 x 56, batch 64: 37.1 us with 2 rows, 75.4 pixel by pixel.)
 // ---------------------------------------------------------------------------------------------
 struct DwArgs {
     int c4, h, w, oh, ow, pad_h, pad_w;
+    int stride_h, relu_lo;
     FastDiv by_c4, by_pairs, by_strips;         // channel words, pixel pairs of a row, strips of ROWS rows
     uint32_t total, izp4;
     float add;                                  // zero point + 1/2
@@ -362,10 +365,10 @@ __device__ __forceinline__ uint32_t clamp_s16x2(uint32_t v, uint32_t lo2)
     return d;
 }
 
-template <int ROWS, int S>
+template <int ROWS, int S, bool FP>
 __global__ void __launch_bounds__(128) conv_depthwise3x3_strip_kernel(
     const __grid_constant__ DwArgs g, const uint32_t *__restrict__ x, const uint4 *__restrict__ w3p, const uint4 *__restrict__ qf,
-    uint32_t *__restrict__ y)
+    const int4 *__restrict__ q3, uint32_t *__restrict__ y)
 {
     constexpr int IN_ROWS = 3 + (ROWS - 1) * S, IN_COLS = 3 + S, NV = S == 2 ? 3 : 2;
     const uint32_t idx = blockIdx.x * 128 + threadIdx.x;
@@ -383,10 +386,19 @@ __global__ void __launch_bounds__(128) conv_depthwise3x3_strip_kernel(
 #pragma unroll
         for (int v = 0; v < NV; ++v)
             wv[rr][v] = __ldg(w3p + ((size_t)ci * 3 + rr) * NV + v);
-    const uint4 start = __ldg(qf + ci * 2), mb = __ldg(qf + ci * 2 + 1);
+    uint4 start = make_uint4(0, 0, 0, 0), mb = start;
+    int4 q[4];
+    if (FP) {
+        start = __ldg(qf + ci * 2);
+        mb = __ldg(qf + ci * 2 + 1);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            q[j] = __ldg(q3 + ci * 4 + j);
+    }
     pdl_wait();
     pdl_trigger();
-    const int iy0 = oy * S - g.pad_h, ix0 = ox * S - g.pad_w;
+    const int iy0 = oy * (ROWS == 1 ? g.stride_h : S) - g.pad_h, ix0 = ox * S - g.pad_w;
     // byte offsets of 32 bits from the tensor's start (the launcher checks that it ends below 4 GB)
     auto at = [&](uint32_t off) { return __ldg(reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(x) + off)); };
     const uint32_t col_pitch = (uint32_t)g.c4 * 4, row_pitch = (uint32_t)g.w * col_pitch;
@@ -441,22 +453,35 @@ __global__ void __launch_bounds__(128) conv_depthwise3x3_strip_kernel(
             if (kr == 2 && (o == 0 || oy + o < g.oh)) {
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
-                    const uint32_t lo = clamp_s16x2(requant_pair(acc[o][p][0], acc[o][p][1], m0, m1, g.add), g.lo2);
-                    const uint32_t hi = clamp_s16x2(requant_pair(acc[o][p][2], acc[o][p][3], m2, m3, g.add), g.lo2);
+                    uint32_t out4;
+                    if (FP) {
+                        const uint32_t lo = clamp_s16x2(requant_pair(acc[o][p][0], acc[o][p][1], m0, m1, g.add), g.lo2);
+                        const uint32_t hi = clamp_s16x2(requant_pair(acc[o][p][2], acc[o][p][3], m2, m3, g.add), g.lo2);
+                        out4 = __byte_perm(lo, hi, 0x6420);
+                    } else {
+                        int r[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const long long off = (long long)(((unsigned long long)(uint32_t)q[j].y << 32) | (uint32_t)q[j].x);
+                            r[j] = max((int)(((long long)acc[o][p][j] * q[j].z + off) >> 32) >> q[j].w, g.relu_lo);
+                        }
+                        out4 = pack_sat_u8x4(r[0], r[1], r[2], r[3]);
+                    }
                     if (p == 0 || second)
-                        *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(y) + out + o * out_row + p * col_pitch) = __byte_perm(lo, hi, 0x6420);
+                        *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(y) + out + o * out_row + p * col_pitch) = out4;
                 }
             }
         }
     }
 }
 
-template <int ROWS, int S>
+template <int ROWS, int S, bool FP = true>
 static int depthwise3x3_strip_launch(const ConvGeom &g, const ConvDirectPlan &p, const uint8_t *x, int n, uint8_t *y, cudaStream_t st)
 {
     DwArgs a;
     a.c4 = g.c / 4; a.h = g.h; a.w = g.w; a.oh = g.oh; a.ow = g.ow; a.pad_h = g.pad_h; a.pad_w = g.pad_w;
     const uint32_t pairs = (uint32_t)(g.ow + 1) / 2, strips = (uint32_t)(g.oh + ROWS - 1) / ROWS;
+    a.stride_h = g.stride_h; a.relu_lo = g.relu_lo;
     a.by_c4 = FastDiv((uint32_t)a.c4);
     a.by_pairs = FastDiv(pairs);
     a.by_strips = FastDiv(strips);
@@ -465,9 +490,9 @@ static int depthwise3x3_strip_launch(const ConvGeom &g, const ConvDirectPlan &p,
     a.add = (float)g.ozp + 0.5f;
     a.lo2 = (uint32_t)(g.relu_lo > 0 ? g.relu_lo : 0) * 0x00010001u;
     return launch_kernel(
-        conv_depthwise3x3_strip_kernel<ROWS, S>, dim3((a.total + 127) / 128), dim3(128), 0, st, (size_t)n * g.c * (g.h * g.w + g.oh * g.ow), 1,
+        conv_depthwise3x3_strip_kernel<ROWS, S, FP>, dim3((a.total + 127) / 128), dim3(128), 0, st, (size_t)n * g.c * (g.h * g.w + g.oh * g.ow), 1,
         a, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint4 *>(p.w_dw3p_dev), reinterpret_cast<const uint4 *>(p.q_dw3p_dev),
-        reinterpret_cast<uint32_t *>(y));
+        p.q_dw3_dev, reinterpret_cast<uint32_t *>(y));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -587,6 +612,14 @@ int conv_direct_launch(
         // Rows per thread: as many as leave every SM about a thousand threads, of the heights that fit the map
         // (144 channels of 56 x 56, batch 256: 80.6 us with 4 rows, 71.2 with 7, 60.3 with 14; 960 of 7 x 7: 10.3 with 7,
         // 13.1 with 14; stride 2 to 28 x 28: 41.4 with 2, 34.4 with 4, 35.0 with 7).
+        const bool fp = p.q_dw3p_dev != nullptr;
+        if (g.stride_w != g.stride_h) {
+            if (g.stride_w == 1)
+                return fp ? depthwise3x3_strip_launch<1, 1>(g, p, x, n, y, st) : depthwise3x3_strip_launch<1, 1, false>(g, p, x, n, y, st);
+            return fp ? depthwise3x3_strip_launch<1, 2>(g, p, x, n, y, st) : depthwise3x3_strip_launch<1, 2, false>(g, p, x, n, y, st);
+        }
+        if (!fp)
+            return g.stride_w == 1 ? depthwise3x3_strip_launch<2, 1, false>(g, p, x, n, y, st) : depthwise3x3_strip_launch<2, 2, false>(g, p, x, n, y, st);
         const size_t per_row = (size_t)n * ((g.ow + 1) / 2) * (g.c / 4), few = (size_t)sm_count() * 1024;
         auto strips = [&](int rows) { return (size_t)((g.oh + rows - 1) / rows); };
         if (g.stride_w == 1) {

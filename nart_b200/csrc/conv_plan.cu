@@ -340,7 +340,8 @@ int b200_conv2d_create(
             // its fp32 requantize: every accumulator below 2^22, every result within the 16 bits it is clamped in (see
             // conv_depthwise3x3_strip_kernel: half steps below zero).  Taps are 0 .. 255, so a channel's negative and positive
             // weights bound its accumulators; 22 of 272 layers of MobileNetV2 with random weights miss a bound by their number.
-            bool strip = g.stride_w == g.stride_h && (g.stride_w == 1 || g.stride_w == 2);
+            const bool strip = g.stride_w == 1 || g.stride_w == 2;
+            bool fp = strip;
             for (int k = 0; k < g.k; ++k) {
                 int neg = 0, pos = 0;
                 for (int t = 0; t < 9; ++t) {
@@ -348,7 +349,7 @@ int b200_conv2d_create(
                     (w < 0 ? neg : pos) += w;
                 }
                 const long long lo = bias_fold[k] + 255ll * neg, hi = bias_fold[k] + 255ll * pos;
-                strip = strip && lo > -(1 << 22) && hi < (1 << 22) && ldexp((double)lo * mult[k], -shift[k]) > -16380.0
+                fp = fp && lo > -(1 << 22) && hi < (1 << 22) && ldexp((double)lo * mult[k], -shift[k]) > -16380.0
                     && ldexp((double)hi * mult[k], -shift[k]) + g.ozp < 32760.0;
             }
             if (rc == B200_OK && strip) {
@@ -370,8 +371,8 @@ int b200_conv2d_create(
                         }
                     }
                 rc = upload(w3p, &cv->direct.w_dw3p_dev);
-                std::vector<uint32_t> qf((size_t)g.c * 2);
-                for (int c = 0; c < g.c; ++c) {
+                std::vector<uint32_t> qf(fp ? (size_t)g.c * 2 : 0);
+                for (int c = 0; c < g.c && fp; ++c) {
                     const float m = ldexpf((float)mult[c], -shift[c]);      // exact: mult has 24 significant bits
                     qf[(size_t)(c / 4) * 8 + c % 4] = 0x4B400000u + (uint32_t)bias_fold[c];
                     memcpy(&qf[(size_t)(c / 4) * 8 + 4 + c % 4], &m, 4);

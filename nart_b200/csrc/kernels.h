@@ -94,9 +94,9 @@ struct ConvDirectPlan {
     // {folded 64-bit addend, mult, shift - 32}
     uint32_t *w_dw3_dev = nullptr;
     int4 *q_dw3_dev = nullptr;
-    // the same for two output pixels side by side (stride 1 or 2 both ways), see conv_depthwise3x3_strip_kernel:
+    // the same for two output pixels side by side (stride_w 1 or 2), see conv_depthwise3x3_strip_kernel:
     // [c/4][3 kernel rows][2 or 3][4 channels] words of one kernel row against 3 + stride_w input pixels, and
-    // [c/4] of four accumulator start values and four fp32 multipliers
+    // [c/4] of four accumulator start values and four fp32 multipliers (nullptr: results too large for its fp32 requantize)
     uint32_t *w_dw3p_dev = nullptr;
     uint32_t *q_dw3p_dev = nullptr;
     int32_t *bias_fold_dev = nullptr;
