@@ -490,7 +490,12 @@ size_t conv_small_smem(SmallArgs &a, bool act_signed)
         --a.slots;
     while (a.slots > 1 && small_layout(a).total > 227 * 1024)
         --a.slots;
-    return small_layout(a).total;
+    // A CTA waits for tensor memory (512 columns an SM) while its cluster waits for it, so CTAs of clusters must never fill an
+    // SM's columns against each other: two clusters could each hold what the other's peer waits for.  Three CTAs fit an
+    // SM's registers, and 128 columns each fit.  Those of 256 (a window-sum column beside 128 channels) ask for more than half
+    // of the shared memory, so that an SM holds one of them at most.  (CTAs without a cluster give theirs back by themselves.)
+    const size_t total = small_layout(a).total, half_sm = 116 * 1024;
+    return a.split > 1 && a.tmem_cols > 128 && total < half_sm ? half_sm : total;
 }
 
 int conv_small_launch(const SmallMaps &maps, const SmallArgs &a, int m_tiles, size_t smem, size_t bytes, cudaStream_t st)

@@ -614,3 +614,28 @@ def test_depthwise3x3_results_far_beyond_a_byte(ops, port, reach, st):
         want = port.conv2d_u8(x, (wt + 128).astype(np.uint8), bias, st, (1, 1), c, relu=relu, **q)
         conv = ops.Conv2d((wt + 128).astype(np.uint8), bias, in_hw=(h, w), stride=st, pad=(1, 1), group=c, relu=relu, **q)
         assert_same(to_host_nchw(conv(to_dev_nhwc(x))), want, "reach %d" % reach)
+
+
+def test_small_convs_with_wide_window_sum_tiles_on_many_streams(ops, monkeypatch):
+    """Clusters whose CTAs ask for 256 columns of tensor memory, and narrow ones, of several launches at once."""
+    import torch
+    plans = []
+    for tiling, c, k, ks, hw, wzp in (("128x2", 32, 256, 3, 24, 90), ("128x4", 32, 256, 3, 14, 140), ("128x8", 32, 128, 3, 20, 77),
+                                      ("16x2", 32, 64, 3, 12, 128), ("128x2", 16, 128, 3, 30, 101), ("64x4", 32, 128, 3, 14, 90)):
+        monkeypatch.setenv("B200_IGEMM_SMALL", tiling)
+        x, wt, bias, walpha = conv_inputs(hw, 2, c, hw, hw, k, ks, ks)
+        q = dict(in_hw=(hw, hw), pad=(ks // 2, ks // 2), ialpha=0.02, izp=117, wzp=wzp, walpha=walpha, oalpha=0.01 * np.sqrt(c) * ks, ozp=99)
+        xd = to_dev_nhwc(x)
+        plans.append((ops.Conv2d(wt, bias, algo=ops.ALGO_IGEMM, **q), xd, ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **q)(xd)))
+    streams = [torch.cuda.Stream() for _ in range(6)]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(40):
+        for s, st in enumerate(streams):
+            plan, xd, want = plans[(i + s) % len(plans)]
+            with torch.cuda.stream(st):
+                got.append((plan(xd), want))
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert all("one tile per cluster" in p.describe() for p, _, _ in plans)
+    assert all(torch.equal(a, b) for a, b in got)
