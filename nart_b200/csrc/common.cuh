@@ -44,8 +44,9 @@ int status_publish_launch(int *host, cudaStream_t st);
 // and cached for the life of the process (runtime.cu).
 int lut_cache_get(const uint8_t lut[256], const uint8_t **dev_ptr);
 
-// Division of 32-bit numbers below 2^31 by a launch constant: one high multiplication, one shift (the multiplier is
-// rounded up, 2^(31 + l) / d with 2^(l-1) < d <= 2^l, whose error stays below one part in 2^31).
+// Division of 32-bit numbers below 2^31 by a launch constant, after Granlund and Montgomery, "Division by invariant integers
+// using multiplication" (PLDI 1994): one high multiplication, one shift (the multiplier is rounded up, 2^(31 + l) / d
+// with 2^(l-1) < d <= 2^l, whose error stays below one part in 2^31).
 struct FastDiv {
     uint32_t d = 1, mul = 0x80000000u, shift = 0;
     FastDiv() = default;
@@ -192,12 +193,27 @@ __device__ __forceinline__ uint32_t pack_sat_u8x4(int a, int b, int c, int d)
     return out;
 }
 
-// 32-bit rounded shift for operands known to satisfy |x| + 2^(b-1) < 2^31, 1 <= b <= 30.
-__device__ __forceinline__ int rshift_rn32(int x, int b) { return (x + (1 << (b - 1))) >> b; }
 // 64-bit rounded shift, 1 <= b <= 62.
 __device__ __forceinline__ long long rshift_rn64(long long x, int b)
 {
     return (x + (1ll << (b - 1))) >> b;
+}
+
+// The bits of 2^23 + floor(((a0, a1) - 1.5 * 2^23) * (m0, m1) + add)
+__device__ __forceinline__ void fp_requant_pair(int a0, int a1, int m0, int m1, float add, int &q0, int &q1)
+{
+    asm("{\n\t.reg .b64 a, m, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 c, {%6, %6};\n\t"
+        "add.rn.f32x2 a, a, c;\n\t"
+        "mov.b64 m, {%4, %5};\n\t"
+        "mov.b64 d, {%7, %7};\n\t"
+        "fma.rz.f32x2 a, a, m, d;\n\t"
+        "mov.b64 c, {%8, %8};\n\t"
+        "add.rz.f32x2 a, a, c;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "=r"(q0), "=r"(q1)
+        : "r"(a0), "r"(a1), "r"(m0), "r"(m1), "f"(-12582912.f), "f"(add), "f"(8388608.f));
 }
 
 }  // namespace b200

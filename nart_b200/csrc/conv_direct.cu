@@ -339,22 +339,11 @@ struct DwArgs {
     uint32_t lo2;                               // floor, twice
 };
 
-// The bits of 2^23 + floor(((a0, a1) - 1.5 * 2^23) * (m0, m1) + add): their low halves in one word
-__device__ __forceinline__ uint32_t requant_pair(int a0, int a1, float m0, float m1, float add)
+// The low halves of two of fp_requant_pair's results in one word
+__device__ __forceinline__ uint32_t requant_pair(int a0, int a1, int m0, int m1, float add)
 {
-    uint32_t q0, q1;
-    asm("{\n\t.reg .b64 a, m, c, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\t"
-        "mov.b64 c, {%6, %6};\n\t"
-        "add.rn.f32x2 a, a, c;\n\t"
-        "mov.b64 m, {%4, %5};\n\t"
-        "mov.b64 d, {%7, %7};\n\t"
-        "fma.rz.f32x2 a, a, m, d;\n\t"
-        "mov.b64 c, {%8, %8};\n\t"
-        "add.rz.f32x2 a, a, c;\n\t"
-        "mov.b64 {%0, %1}, a;\n\t}"
-        : "=r"(q0), "=r"(q1)
-        : "r"(a0), "r"(a1), "f"(m0), "f"(m1), "f"(-12582912.f), "f"(add), "f"(8388608.f));
+    int q0, q1;
+    fp_requant_pair(a0, a1, m0, m1, add, q0, q1);
     return __byte_perm(q0, q1, 0x5410);
 }
 __device__ __forceinline__ uint32_t clamp_s16x2(uint32_t v, uint32_t lo2)
@@ -426,7 +415,7 @@ __global__ void __launch_bounds__(128) conv_depthwise3x3_strip_kernel(
         for (int p = 0; p < 2; ++p) {
             acc[o][p][0] = (int)start.x; acc[o][p][1] = (int)start.y; acc[o][p][2] = (int)start.z; acc[o][p][3] = (int)start.w;
         }
-    const float m0 = __uint_as_float(mb.x), m1 = __uint_as_float(mb.y), m2 = __uint_as_float(mb.z), m3 = __uint_as_float(mb.w);
+    const int m0 = (int)mb.x, m1 = (int)mb.y, m2 = (int)mb.z, m3 = (int)mb.w;       // bits of floats
     const uint32_t out_row = (uint32_t)g.ow * col_pitch;
     const uint32_t out = ((img * (uint32_t)g.oh + (uint32_t)oy) * (uint32_t)g.ow + (uint32_t)ox) * col_pitch + ci * 4;
     const bool second = ox + 1 < g.ow;

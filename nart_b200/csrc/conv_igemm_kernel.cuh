@@ -202,25 +202,10 @@ struct TileWalker {
     __device__ __forceinline__ int ni(const IgemmArgs &g) const { return (g.rev && tni < g.tiles_n) ? g.tiles_n - 1 - tni : tni; }
 };
 
-// Named barriers of one epilogue group (ids 1 + 2g and 2 + 2g for group g).
+// The named barrier of one epilogue group.
 __device__ __forceinline__ void epi_bar_sync(int group, int group_threads)
 {
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + 2 * group), "r"(group_threads) : "memory");
-}
-// AND-reduction of a predicate over the threads of one epilogue group: every thread gets
-// the same answer, so all of them leave the tile loop together.
-__device__ __forceinline__ bool epi_bar_all(int group, int group_threads, bool pred)
-{
-    uint32_t out;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %1, 0;\n\t"
-        "barrier.cta.red.and.pred q, %3, %2, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(out)
-        : "r"((uint32_t)pred), "r"(group_threads), "r"(2 + 2 * group)
-        : "memory");
-    return out != 0;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(group_threads) : "memory");
 }
 
 // ---- epilogue arithmetic ------------------------------------------------------------------------
@@ -233,23 +218,6 @@ struct EpiConsts {
 
 constexpr int kFpMagic = 0x4B400000;    // bits of 1.5 * 2^23
 constexpr int kFpOne = 0x4B000000;      // bits of 2^23
-
-// The bits of 2^23 + floor(((a0, a1) - 1.5 * 2^23) * (m0, m1) + add)
-__device__ __forceinline__ void fp_requant_pair(int a0, int a1, int m0, int m1, float add, int &q0, int &q1)
-{
-    asm("{\n\t.reg .b64 a, m, c, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\t"
-        "mov.b64 c, {%6, %6};\n\t"
-        "add.rn.f32x2 a, a, c;\n\t"
-        "mov.b64 m, {%4, %5};\n\t"
-        "mov.b64 d, {%7, %7};\n\t"
-        "fma.rz.f32x2 a, a, m, d;\n\t"
-        "mov.b64 c, {%8, %8};\n\t"
-        "add.rz.f32x2 a, a, c;\n\t"
-        "mov.b64 {%0, %1}, a;\n\t}"
-        : "=r"(q0), "=r"(q1)
-        : "r"(a0), "r"(a1), "r"(m0), "r"(m1), "f"(-12582912.f), "f"(add), "f"(8388608.f));
-}
 
 // (volatile: the constants of later columns are not loaded ahead, there are no registers for them)
 __device__ __forceinline__ int4 lds4(uint32_t addr)
@@ -726,7 +694,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
     const int ring_tile0 = tile0 + ring * tstride, stage0 = ring * ring_stages;
     if (warp == 0 || (MODE == 1 && warp == kRing1Warp)) {
         // ================= TMA producer =================
-        // One thread walks the k-blocks of this CTA's tiles in order: wait for the stage of the next group of k-blocks, post
+        // The warp walks the k-blocks of this CTA's tiles in order, one elected lane issues: wait for the stage of the next group of k-blocks, post
         // the group's byte count, issue its loads.  The chain of instructions of one k-block bounds the mainloop (its MMAs take
         // 64 .. 512 cycles), so addresses and coordinates advance by counters: chunk -> tap -> tile, with what depends on the
         // tap or the tile worked out when that changes.
@@ -912,8 +880,8 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
             pdl_trigger();
     } else if (warp == 1 || (MODE == 1 && warp == kRing1Warp + 1)) {
         // ================= MMA issuer =================
-        // One thread.  Descriptors of one operand differ only in the start-address field, so only their low words are
-        // computed.  In a CTA pair the leading CTA's thread issues for both; the peer's has nothing to do.
+        // The warp walks, one elected lane issues.  Descriptors of one operand differ only in the start-address field, so only their low words are
+        // computed.  In a CTA pair the leading CTA's warp issues for both; the peer's has nothing to do.
         if (leader) {
             const int kgroup = g.kgroup, ksteps_full = g.bk / 32, last_steps = g.last_steps;
             int stage = stage0;

@@ -11,7 +11,7 @@
 //   * every k-block of a CTA has a slot of its own where they fit, the weights' loads are issued before
 //     griddepcontrol.wait, and constants reach shared memory while the operands are on their way;
 //   * 320 threads and as little shared memory as that needs, so that the next launch's CTAs are resident beside these.
-// Roles: warp 0 TMA (one lane per slot), warp 1 tensor memory and MMAs, warps 2-9 epilogue, two per lane quarter.  The
+// Roles: warp 0 TMA (one elected lane), warp 1 tensor memory and MMAs, warps 2-9 epilogue, two per lane quarter.  The
 // epilogue is the persistent kernel's arithmetic (EpiForm); requantizing channel by channel with a shift each, as this kernel
 // first did, took 0.9 us per 16 channels of a tile, most of a 64-channel launch's time.
 #include <stdlib.h>
