@@ -153,7 +153,11 @@ def run_reference_arm(a):
     procs = max(1, min(os.cpu_count() or 1, 64))
     import multiprocessing as mp
     import oracle
-    kind = "reference" if oracle.have_ref() else "port"
+    if not oracle.have_ref():
+        print(json.dumps(dict(impl="reference", unavailable="the compiled reference (oracle/_ref/libnart_ref.so) is not on this "
+                                                            "machine and its sources are not either")))
+        return 0
+    kind = "reference"
     ctx = mp.get_context("spawn")
     times = []
     with ctx.Pool(procs, initializer=_cpu_init, initargs=(kind,)) as pool:
