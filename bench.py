@@ -9,8 +9,8 @@ collective is on the data path.  A step is one pass of the whole network over on
 
   value     whole-job images/s with the input batch already resident in HBM (CUDA events, max
             over ranks).
-  e2e       the same through the host-buffer entry point b200_case_run_host: pinned host input
-            copied host->device and the logits copied device->host inside every step.
+  e2e       the same through the host-buffer entry points b200_case_submit_host and b200_case_wait: pinned host
+            input copied host->device and the logits copied device->host inside every step.
   roofline  the tensor-core convolution kernel (all of its launches in a step): algorithmic bytes
             and ops over the kernel's own time, measured with CUDA events around every launch.
   cpu_baseline / --impl reference
@@ -33,9 +33,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 BATCH = 256
-# DRAM bytes per launch of the conv kernel, averaged over the 54 launches of one batch-256 step:
-# dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this script (3.850 GB per step)
-IGEMM_DRAM_BYTES_PER_LAUNCH = 3.850e9 / 54
+# DRAM bytes per launch of the conv kernels, averaged over the 54 launches of one batch-256 step:
+# dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this script (3.828 GB per step)
+IGEMM_DRAM_BYTES_PER_LAUNCH = 3.828e9 / 54
 WORKLOAD = "ResNet-50 v1.5 int8, batch 256 per GPU, 3x224x224 uint8 input, synthetic per-layer quantization"
 SEED = 3
 
@@ -569,8 +569,8 @@ def run_gpu_arm(a):
                         host_numa="rank 0: " + numa),
             roofline=dict(bound="hbm", achieved=hbm_ach, peak=peaks["hbm_gbs"], unit="GB/s", frac=hbm_ach / peaks["hbm_gbs"],
                           traffic=IGEMM_DRAM_BYTES_PER_LAUNCH if batch == BATCH else None,
-                          traffic_source="ncu dram__bytes_read.sum + dram__bytes_write.sum over the 54 launches of one "
-                                         "step at batch 256, average per launch (profiles/resnet50_b256_igemm_dram_traffic.md)",
+                          traffic_source="not measured in this run: ncu dram__bytes_read.sum + dram__bytes_write.sum over the 54 "
+                                         "conv launches of one step at batch 256, average per launch, captured with these kernels",
                           algorithmic_bytes_per_launch=igemm_bytes / max(1, igemm_launches),
                           kernel="conv_igemm_i8_kernel", launches_per_step=igemm_launches // a.steps,
                           peak_source=peaks["src"]),
