@@ -372,7 +372,7 @@ B200_API int b200_case_tensor_dims(
 B200_API int b200_case_io_bytes(
     const b200_case_t *cs, int32_t is_output, int32_t index, size_t *bytes_per_image);
 /* Device staging buffer of the i-th input / output (host layout, NCHW), for callers that keep
- * data resident. */
+ * data resident.  From the first call on, host runs of the case copy everything through these buffers. */
 B200_API int b200_case_io_device_ptr(
     const b200_case_t *cs, int32_t is_output, int32_t index, void **dev_ptr);
 /* Device NHWC buffer of any tensor after a run (verification). */
@@ -380,7 +380,8 @@ B200_API int b200_case_tensor_device_ptr(const b200_case_t *cs, int32_t tensor, 
 /* parade_run on data already resident in the input staging buffers; asynchronous on `stream`. */
 B200_API int b200_case_run_device(b200_case_t *cs, int32_t batch, b200_stream_t stream);
 /* parade_run with host buffers: copies every input host->device, runs, copies every output
- * device->host and synchronizes.  inputs[i] / outputs[i]: batch x bytes_per_image. */
+ * device->host and synchronizes.  inputs[i] / outputs[i]: batch x bytes_per_image.  Small pinned buffers are read and
+ * written in place by the layout kernels; a b200_case_run_device behind such a run works on its data all the same. */
 B200_API int b200_case_run_host(
     b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs,
     b200_stream_t stream);
@@ -396,9 +397,8 @@ B200_API int b200_case_wait(b200_case_t *cs);
 /* Number of kernels one b200_case_run_device launches.  (A residual add that a small conv launch forms itself still counts.) */
 B200_API int b200_case_launch_count(const b200_case_t *cs, int32_t *launches);
 /* Folds residual adds into the convs that feed them (default: off; call before b200_case_prepare).
- * Off by default because on B200 the conv epilogue is bound by instruction issue, not by memory:
- * ResNet-50 at batch 256 runs 3.43 ms per step fused against 3.23 ms with the adds as kernels of
- * their own, although the fused form moves 2.7 GB less.
+ * Off by default: ResNet-50 at batch 256 runs 2.80 ms per step fused against 2.67 ms with the adds as kernels of
+ * their own, although the fused form moves 2.7 GB less (its epilogue is the slower one).
  * A two-input eltwise SUM whose later-produced input is the output of a tensor-core conv that
  * nothing else reads then runs in that conv's epilogue (b200_conv2d_fuse_residual_add) and its own
  * kernel is skipped; results are unchanged.  No counterpart in the reference's CPU module, whose

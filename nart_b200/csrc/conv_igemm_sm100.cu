@@ -892,7 +892,8 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
             p->max_clusters = nc < sms / 2 ? nc : sms / 2;
         }
         const int pair_tiles = (a.tiles_w * a.tiles_h * a.tiles_n + 1) / 2 * (p->kpad / p->bn);
-        // a pair tile for every cluster at least (3x3 256 -> 256, 14x14, batch 256: 26.5 -> 25.8 us; 3x3 s2 512 -> 512: 34.1 -> 31.1)
+        // a pair tile for every cluster at least (one buffer, queued: 3x3 256 -> 256, 14x14, batch 256: 26.5 -> 25.8 us; 3x3 s2
+        // 512 -> 512: 34.1 -> 31.1)
         l.cta_pair = (p->pair_want == 1 || pair_tiles >= p->max_clusters) ? 1 : 0;
     }
     a.bk = p->bk; a.bn = p->bn; a.stages = l.cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
