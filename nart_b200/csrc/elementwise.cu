@@ -278,36 +278,55 @@ static int nhwc_to_nchw_launch(const uint8_t *x0, TOut *y0, int n, int c, int P,
     });
 }
 
-// Flat variants (no layout change): 4 elements per thread.
-template <typename Fn>
+// Flat variants (no layout change): 4 elements per thread, as vectors where both addresses allow it (VEC).
+template <typename Fn, bool VEC>
 __global__ void quantize_flat_kernel(const float *__restrict__ in, uint8_t *__restrict__ out, size_t count, Fn fn)
 {
     pdl_wait();
     pdl_trigger();
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i + 4 <= count) {
+    if (VEC && i + 4 <= count) {
         float4 v = *reinterpret_cast<const float4 *>(in + i);
         *reinterpret_cast<uint32_t *>(out + i) = fn.word(v.x, v.y, v.z, v.w);
     } else {
-        for (; i < count; ++i)
+        const size_t end = i + 4 < count ? i + 4 : count;
+        for (; i < end; ++i)
             out[i] = fn(in[i]);
     }
 }
 
-template <typename Fn>
+template <typename Fn, bool VEC>
 __global__ void dequantize_flat_kernel(const uint8_t *__restrict__ in, float *__restrict__ out, size_t count, Fn fn)
 {
     pdl_wait();
     pdl_trigger();
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i + 4 <= count) {
+    if (VEC && i + 4 <= count) {
         uint32_t q = *reinterpret_cast<const uint32_t *>(in + i);
         *reinterpret_cast<float4 *>(out + i) = make_float4(
             fn((uint8_t)q), fn((uint8_t)(q >> 8)), fn((uint8_t)(q >> 16)), fn((uint8_t)(q >> 24)));
     } else {
-        for (; i < count; ++i)
+        const size_t end = i + 4 < count ? i + 4 : count;
+        for (; i < end; ++i)
             out[i] = fn(in[i]);
     }
+}
+
+template <typename Fn>
+static int quantize_flat_launch(const float *x, uint8_t *y, size_t count, Fn fn, cudaStream_t st)
+{
+    const dim3 grid((unsigned)(((count + 3) / 4 + 255) / 256));
+    if ((((uintptr_t)x & 15) | ((uintptr_t)y & 3)) == 0)
+        return launch_kernel(quantize_flat_kernel<Fn, true>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
+    return launch_kernel(quantize_flat_kernel<Fn, false>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
+}
+template <typename Fn>
+static int dequantize_flat_launch(const uint8_t *x, float *y, size_t count, Fn fn, cudaStream_t st)
+{
+    const dim3 grid((unsigned)(((count + 3) / 4 + 255) / 256));
+    if ((((uintptr_t)x & 3) | ((uintptr_t)y & 15)) == 0)
+        return launch_kernel(dequantize_flat_kernel<Fn, true>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
+    return launch_kernel(dequantize_flat_kernel<Fn, false>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -601,11 +620,8 @@ int b200_quantize_u8(
     if (nhwc && !(c == 1 || P == 1)) {
         return nchw_to_nhwc_launch(x, y, n, c, P, c, 0, fn, as_stream(stream));
     } else {
-        size_t count = (size_t)n * c * P;
-        size_t threads = (count + 3) / 4;
-        B200_TRY((launch_kernel(quantize_flat_kernel<QuantizeFn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
+        return quantize_flat_launch(x, y, (size_t)n * c * P, fn, as_stream(stream));
     }
-    return B200_OK;
 }
 
 int b200_dequantize_u8(
@@ -623,11 +639,8 @@ int b200_dequantize_u8(
     if (nhwc && !(c == 1 || P == 1)) {
         return nhwc_to_nchw_launch(x, y, n, c, P, c, fn, as_stream(stream));
     } else {
-        size_t count = (size_t)n * c * P;
-        size_t threads = (count + 3) / 4;
-        B200_TRY((launch_kernel(dequantize_flat_kernel<DequantizeFn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
+        return dequantize_flat_launch(x, y, (size_t)n * c * P, fn, as_stream(stream));
     }
-    return B200_OK;
 }
 
 int b200_quantize_s8(
@@ -648,11 +661,8 @@ int b200_quantize_s8(
     if (nhwc && !(c == 1 || P == 1)) {
         return nchw_to_nhwc_launch(x, y, n, c, P, c, 0, fn, as_stream(stream));
     } else {
-        size_t count = (size_t)n * c * P;
-        size_t threads = (count + 3) / 4;
-        B200_TRY((launch_kernel(quantize_flat_kernel<QuantizeS8Fn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
+        return quantize_flat_launch(x, y, (size_t)n * c * P, fn, as_stream(stream));
     }
-    return B200_OK;
 }
 
 int b200_dequantize_s8(
@@ -670,11 +680,8 @@ int b200_dequantize_s8(
     if (nhwc && !(c == 1 || P == 1)) {
         return nhwc_to_nchw_launch(x, y, n, c, P, c, fn, as_stream(stream));
     } else {
-        size_t count = (size_t)n * c * P;
-        size_t threads = (count + 3) / 4;
-        B200_TRY((launch_kernel(dequantize_flat_kernel<DequantizeS8Fn>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), count * 5, 1, x, y, count, fn)));
+        return dequantize_flat_launch(x, y, (size_t)n * c * P, fn, as_stream(stream));
     }
-    return B200_OK;
 }
 
 int b200_nchw_to_nhwc_u8(

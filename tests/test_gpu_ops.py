@@ -639,3 +639,19 @@ def test_small_convs_with_wide_window_sum_tiles_on_many_streams(ops, monkeypatch
     assert ops.device_status() == 0
     assert all("one tile per cluster" in p.describe() for p, _, _ in plans)
     assert all(torch.equal(a, b) for a, b in got)
+
+
+@pytest.mark.parametrize("shape", [(5, 7, 1, 1), (5, 1, 3, 3), (4, 10, 1, 1), (3, 6, 3, 5)])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_quantize_and_dequantize_at_any_address(ops, shape, shift):
+    """Views that start anywhere in a larger tensor, with and without a layout change."""
+    import torch
+    n = int(np.prod(shape))
+    xf = torch.randn(n + 4, device="cuda")[shift:shift + n].view(shape)
+    xb = torch.randint(0, 256, (n + 4,), device="cuda", dtype=torch.uint8)[shift:shift + n].view(shape[0], shape[2], shape[3], shape[1])
+    for nhwc in (True, False):
+        b = xb if nhwc else xb.view(shape)
+        assert torch.equal(ops.quantize(xf, 0.02, 100, 8, nhwc), ops.quantize(xf.clone(), 0.02, 100, 8, nhwc))
+        assert torch.equal(ops.quantize_s8(xf, 0.02, 8, nhwc), ops.quantize_s8(xf.clone(), 0.02, 8, nhwc))
+        assert torch.equal(ops.dequantize(b, 0.02, 100, nhwc), ops.dequantize(b.clone(), 0.02, 100, nhwc))
+        assert torch.equal(ops.dequantize_s8(b.view(torch.int8), 0.02, nhwc), ops.dequantize_s8(b.clone().view(torch.int8), 0.02, nhwc))
