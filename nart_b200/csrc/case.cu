@@ -96,7 +96,7 @@ struct b200_case {
     // CUDA graph of one run, per (batch, stream); off by default
     bool use_graph = false;
     struct Graph {
-        int batch;
+        int batch, part;         // part: see run_ops
         cudaStream_t stream;
         int runs_seen;           // eager runs at this batch before capturing (the first one allocates)
         cudaGraphExec_t exec;
@@ -112,6 +112,9 @@ struct b200_case {
     bool submitted = false;
     bool staging_known = false;        // the caller has a staging buffer's address: every run goes through them
     cudaStream_t refresh_stream = nullptr;
+    // host runs in two parts (split_host_run): the copies, behind what `stream` has before them
+    cudaStream_t part_stream = nullptr;
+    cudaEvent_t part_event = nullptr;
     int *status_host = nullptr;        // pinned: the device status word as the end of a run found it
 };
 
@@ -239,6 +242,8 @@ int b200_case_destroy(b200_case_t *cs)
             cudaGraphExecDestroy(gr.exec);
     cudaFreeHost(cs->status_host);
     if (cs->refresh_stream) cudaStreamDestroy(cs->refresh_stream);
+    if (cs->part_event) cudaEventDestroy(cs->part_event);
+    if (cs->part_stream) cudaStreamDestroy(cs->part_stream);
     if (cs->h2d_done) cudaEventDestroy(cs->h2d_done);
     if (cs->after_inputs) cudaEventDestroy(cs->after_inputs);
     if (cs->comp_done) cudaEventDestroy(cs->comp_done);
@@ -610,7 +615,8 @@ int b200_case_tensor_device_ptr(const b200_case_t *cs, int32_t tensor, void **de
 }
 
 // phase: 0 = whole run, 1 = input layout kernels only, 2 = ops and outputs only
-static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int phase = 0);
+// first: the images [first, first + batch); op0, op1: of the ops, those (all of them by default)
+static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int phase = 0, int32_t first = 0, size_t op0 = 0, size_t op1 = SIZE_MAX);
 
 // The ops (phase 2) and then the output kernels (phase 3), which stay outside a captured graph: they write the
 // device staging buffers that the previous submitted step's device-to-host copy may still be reading.
@@ -666,6 +672,7 @@ int b200_case_io_device_ptr(const b200_case_t *cs, int32_t is_output, int32_t in
 }
 
 static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream);
+static int run_ops(b200_case_t *cs, int32_t batch, int part, b200_stream_t stream);
 
 int b200_case_run_device(b200_case_t *cs, int32_t batch, b200_stream_t stream)
 {
@@ -698,39 +705,89 @@ static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream)
         B200_TRY(run_eager(cs, batch, stream, 2));
         return run_outputs(cs, batch, stream);
     }
-    // Graph mode: the first run at a batch size is eager (plans build their tensor maps and scratch
-    // then), the second is captured, later ones replay the captured launches back to back.
-    cudaStream_t cst = as_stream(stream);
-    b200_case::Graph *gr = nullptr;
-    for (auto &g0 : cs->graphs)
-        if (g0.batch == batch && g0.stream == cst)
-            gr = &g0;
-    if (!gr) {
-        cs->graphs.push_back({ batch, cst, 0, nullptr });
-        gr = &cs->graphs.back();
-    }
     // the input layout kernels stay outside the graph: a pipelined caller refills the input staging
     // buffer as soon as they are done (b200_case_submit_host)
-    if (gr->exec) {
-        B200_TRY(run_eager(cs, batch, stream, 1));
-        if (cs->after_inputs)
-            B200_CUDA_TRY(cudaEventRecord(cs->after_inputs, cst));
-        B200_CUDA_TRY(cudaGraphLaunch(gr->exec, cst));
-        return run_outputs(cs, batch, stream);
-    }
-    if (gr->runs_seen++ == 0) {
-        B200_TRY(run_eager(cs, batch, stream, 1));
-        if (cs->after_inputs)
-            B200_CUDA_TRY(cudaEventRecord(cs->after_inputs, cst));
-        B200_TRY(run_eager(cs, batch, stream, 2));
-        return run_outputs(cs, batch, stream);
-    }
     B200_TRY(run_eager(cs, batch, stream, 1));
     if (cs->after_inputs)
-        B200_CUDA_TRY(cudaEventRecord(cs->after_inputs, cst));
+        B200_CUDA_TRY(cudaEventRecord(cs->after_inputs, as_stream(stream)));
+    B200_TRY(run_ops(cs, batch, 0, stream));
+    return run_outputs(cs, batch, stream);
+}
+
+// A host run whose images take long to copy: the first part of them goes through the first ops of the case while the others are
+// on their way (ResNet-18, 64 images: 185 us of copy).  Parts of a multiple of 16 images, so that every tensor of the second one is
+// aligned; the ops whose time on the first part the copy of the second covers.
+static int32_t first_part(int32_t batch) { return batch / 32 * 16; }
+static size_t head_ops(const b200_case_t *cs, int32_t batch)
+{
+    const int32_t n1 = first_part(batch);
+    double copy = 0.0;                                      // us, of the second part
+    for (const auto &io : cs->inputs)
+        copy += (double)io.bytes_per_image * (batch - n1) / 52e3;
+    if (n1 == 0 || copy < 20.0)
+        return 0;
+    size_t n = 0, whole = 0;
+    for (double t = 0.0; n < cs->ops.size(); ) {
+        const CaseOp &op = cs->ops[n];
+        if (!op.skipped) {
+            double bytes = (double)cs->tensors[op.out].bytes_per_image(), macs = 0.0;
+            for (int in : op.ins)
+                bytes += (double)cs->tensors[in].bytes_per_image();
+            if (op.kind == OpKind::Conv) {
+                const ConvGeom &g = op.conv->g;
+                macs = (double)g.oh * g.ow * g.k * (g.c / g.group) * g.r * g.s;
+            }
+            t += 2.5 + n1 * (bytes / 4e6 + macs / 0.6e9);
+        }
+        if (t > copy)
+            break;
+        ++n;
+        // (a conv and the SUM that its launch may form stay together)
+        bool pair = false;
+        for (size_t i = 0; i < n; ++i)
+            pair = pair || cs->ops[i].sum_op >= (int)n;
+        if (!pair)
+            whole = n;
+    }
+    return whole;
+}
+
+// The ops in graph mode: the first run at a batch size is eager (plans build their tensor maps and scratch
+// then), the second is captured, later ones replay the captured launches back to back.
+// part: 0 all of it; 1 the first ops (head_ops) on the images of the first part; 2 these ops on the other images, and all
+// others on all images.
+static int run_ops(b200_case_t *cs, int32_t batch, int part, b200_stream_t stream)
+{
+    cudaStream_t cst = as_stream(stream);
+    auto launch = [&]() -> int {
+        if (part == 0)
+            return run_eager(cs, batch, stream, 2);
+        const int32_t n1 = first_part(batch);
+        const size_t head = head_ops(cs, batch);
+        if (part == 1)
+            return run_eager(cs, n1, stream, 2, 0, 0, head);
+        B200_TRY(run_eager(cs, batch - n1, stream, 2, n1, 0, head));
+        return run_eager(cs, batch, stream, 2, 0, head);
+    };
+    if (!cs->use_graph)
+        return launch();
+    b200_case::Graph *gr = nullptr;
+    for (auto &g0 : cs->graphs)
+        if (g0.batch == batch && g0.part == part && g0.stream == cst)
+            gr = &g0;
+    if (!gr) {
+        cs->graphs.push_back({ batch, part, cst, 0, nullptr });
+        gr = &cs->graphs.back();
+    }
+    if (gr->exec) {
+        B200_CUDA_TRY(cudaGraphLaunch(gr->exec, cst));
+        return B200_OK;
+    }
+    if (gr->runs_seen++ == 0)
+        return launch();
     cudaGraph_t graph = nullptr;
     B200_CUDA_TRY(cudaStreamBeginCapture(cst, cudaStreamCaptureModeThreadLocal));
-    int rc = run_eager(cs, batch, stream, 2);
+    int rc = launch();
     cudaError_t ce = cudaStreamEndCapture(cst, &graph);
     if (rc != B200_OK || ce != cudaSuccess || !graph) {
         if (graph)
@@ -739,8 +796,7 @@ static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream)
         cs->use_graph = false;   // something on the path cannot be captured: stay eager
         if (rc != B200_OK)
             return rc;
-        B200_TRY(run_eager(cs, batch, stream, 2));
-        return run_outputs(cs, batch, stream);
+        return launch();
     }
     ce = cudaGraphInstantiate(&gr->exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -748,14 +804,13 @@ static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream)
         gr->exec = nullptr;
         cudaGetLastError();
         cs->use_graph = false;
-        B200_TRY(run_eager(cs, batch, stream, 2));
-        return run_outputs(cs, batch, stream);
+        return launch();
     }
     B200_CUDA_TRY(cudaGraphLaunch(gr->exec, cst));
-    return run_outputs(cs, batch, stream);
+    return B200_OK;
 }
 
-static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int phase)
+static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int phase, int32_t first, size_t op0, size_t op1)
 {
     // Launch overlap for cases whose launches are short on average (ResNet-50 at batch 32: 14 MB and 0.97 -> 0.90 ms);
     // at batch 256 (116 MB) it gains 1 % on one stream and costs 2 % with batches in flight on three.
@@ -775,38 +830,43 @@ static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int p
         return B200_OK;
     };
     // phase 0: everything; 1: the input layout kernels; 2: the ops; 3: the output kernels
+    auto at = [cs, first](int t) { return cs->tensors[t].dev + cs->tensors[t].bytes_per_image() * first; };
     for (auto &io : cs->inputs) {
         if (phase >= 2)
             break;
         CaseTensor &t = cs->tensors[io.tensor];
+        const void *from = static_cast<const uint8_t *>(io.buffer()) + io.bytes_per_image * first;
         if (io.is_f32)
             B200_TRY(b200_quantize_u8(
-                (const float *)io.buffer(), t.dev, batch, t.c, t.h, t.w, io.alpha, io.zp, io.bits, 1, stream));
+                (const float *)from, at(io.tensor), batch, t.c, t.h, t.w, io.alpha, io.zp, io.bits, 1, stream));
         else
             B200_TRY(b200_nchw_to_nhwc_u8(
-                (const uint8_t *)io.buffer(), t.dev, batch, t.c, t.h, t.w, t.c_phys, 0, stream));
+                (const uint8_t *)from, at(io.tensor), batch, t.c, t.h, t.w, t.c_phys, 0, stream));
         B200_TRY(mark(0));
     }
     if (phase == 1)
         return B200_OK;
-    for (auto &op : cs->ops) {
+    for (size_t oi = op0; oi < cs->ops.size() && oi < op1; ++oi) {
+        CaseOp &op = cs->ops[oi];
         int kind = 0;
         if (phase == 3)
             break;
         if (op.skipped)
             continue;
+        const uint8_t *x = at(op.ins[0]);
+        uint8_t *y = at(op.out);
         CaseTensor &to = cs->tensors[op.out];
         const CaseTensor &ti = cs->tensors[op.ins[0]];
         switch (op.kind) {
         case OpKind::Conv:
             if (op.residual >= 0)
-                B200_TRY(b200_conv2d_run_residual(op.conv, ti.dev, batch, cs->tensors[op.residual].dev, to.dev, stream));
+                B200_TRY(b200_conv2d_run_residual(op.conv, x, batch, at(op.residual), y, stream));
             else if (op.sum_op >= 0 && !prof) {
                 CaseOp &add = cs->ops[op.sum_op];
-                const ConvSum ws = { cs->tensors[add.ins[1 - op.sum_input]].dev, cs->tensors[add.out].dev, &add.elt, op.sum_input };
-                B200_TRY(conv_igemm_launch(op.conv->igemm, ti.dev, batch, to.dev, as_stream(stream), nullptr, nullptr, &ws, &add.summed));
+                const ConvSum ws = { at(add.ins[1 - op.sum_input]), at(add.out), &add.elt, op.sum_input };
+                B200_TRY(conv_igemm_launch(op.conv->igemm, x, batch, y, as_stream(stream), nullptr, nullptr, &ws, &add.summed));
             } else
-                B200_TRY(b200_conv2d_run(op.conv, ti.dev, batch, to.dev, stream));
+                B200_TRY(b200_conv2d_run(op.conv, x, batch, y, stream));
             kind = b200_conv2d_algo(op.conv) == B200_CONV_ALGO_IGEMM ? 1 : 2;
             break;
         case OpKind::Eltwise: {
@@ -814,17 +874,17 @@ static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int p
                 continue;
             const uint8_t *xs[4];
             for (size_t i = 0; i < op.ins.size(); ++i)
-                xs[i] = cs->tensors[op.ins[i]].dev;
-            B200_TRY(eltwise_launch(op.elt, op.elt_fast, xs, to.dev, to.bytes_per_image() * batch, op.reverse, as_stream(stream)));
+                xs[i] = at(op.ins[i]);
+            B200_TRY(eltwise_launch(op.elt, op.elt_fast, xs, y, to.bytes_per_image() * batch, op.reverse, as_stream(stream)));
             kind = 3;
             break;
         }
         case OpKind::Relu:
-            B200_TRY(lut_u8_launch(ti.dev, to.dev, to.bytes_per_image() * batch, op.lut_dev, as_stream(stream)));
+            B200_TRY(lut_u8_launch(x, y, to.bytes_per_image() * batch, op.lut_dev, as_stream(stream)));
             kind = 4;
             break;
         case OpKind::Pool:
-            B200_TRY(pool_launch(ti.dev, to.dev, batch, ti.c_phys, op.method, op.pg, op.lut_dev, op.ptab, as_stream(stream)));
+            B200_TRY(pool_launch(x, y, batch, ti.c_phys, op.method, op.pg, op.lut_dev, op.ptab, as_stream(stream)));
             kind = 5;
             break;
         }
@@ -926,15 +986,46 @@ struct DirectBuffers {
     {
         if (!done && cudaStreamSynchronize(st) != cudaSuccess)
             cudaGetLastError();     // (the run's own error is the one that is reported)
+        if (!done && cs->part_stream && cudaStreamSynchronize(cs->part_stream) != cudaSuccess)
+            cudaGetLastError();
         for (auto *ios : { &cs->inputs, &cs->outputs })
             for (auto &io : *ios)
                 io.direct = nullptr;
     }
 };
 
+// The copies in two parts, and the ops with them; the outputs as well.
+static int split_host_run(b200_case_t *cs, int32_t batch, const void *const *inputs, b200_stream_t stream)
+{
+    cudaStream_t cst = as_stream(stream);
+    if (!cs->part_stream)
+        B200_CUDA_TRY(cudaStreamCreateWithFlags(&cs->part_stream, cudaStreamNonBlocking));
+    if (!cs->part_event)
+        B200_CUDA_TRY(cudaEventCreateWithFlags(&cs->part_event, cudaEventDisableTiming));
+    B200_CUDA_TRY(cudaEventRecord(cs->part_event, cst));
+    B200_CUDA_TRY(cudaStreamWaitEvent(cs->part_stream, cs->part_event, 0));
+    const int32_t n1 = first_part(batch);
+    for (int part = 1; part <= 2; ++part) {
+        const int32_t first = part == 1 ? 0 : n1, count = part == 1 ? n1 : batch - n1;
+        for (size_t i = 0; i < cs->inputs.size(); ++i) {
+            const size_t each = cs->inputs[i].bytes_per_image;
+            B200_CUDA_TRY(cudaMemcpyAsync(static_cast<uint8_t *>(cs->inputs[i].staging) + each * first, static_cast<const uint8_t *>(inputs[i]) + each * first,
+                                          each * count, cudaMemcpyHostToDevice, cs->part_stream));
+        }
+        B200_CUDA_TRY(cudaEventRecord(cs->part_event, cs->part_stream));
+        B200_CUDA_TRY(cudaStreamWaitEvent(cst, cs->part_event, 0));
+        B200_TRY(run_eager(cs, count, stream, 1, first));
+        if (part == 2 && cs->after_inputs)
+            B200_CUDA_TRY(cudaEventRecord(cs->after_inputs, cst));
+        B200_TRY(run_ops(cs, batch, part, stream));
+    }
+    return run_outputs(cs, batch, stream);
+}
+
 static int run_on_host_buffers(b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs, b200_stream_t stream)
 {
     DirectBuffers buffers{ cs, as_stream(stream) };
+    bool split = cs->use_graph && !cs->profiling && stream != nullptr && head_ops(cs, batch) > 1;
     for (size_t i = 0; i < cs->inputs.size(); ++i) {
         CaseIO &io = cs->inputs[i];
         if (batch > 0 && !inputs[i])
@@ -943,13 +1034,18 @@ static int run_on_host_buffers(b200_case_t *cs, int32_t batch, const void *const
             io.direct = direct_view(inputs[i], io.bytes_per_image * batch);
         if (!io.direct && io.behind > 0)
             B200_TRY(refresh_staging(cs));
-        if (!io.direct)
-            B200_TRY(b200_memcpy_h2d(io.staging, inputs[i], io.bytes_per_image * batch, stream));
+        split = split && !io.direct;
     }
+    for (size_t i = 0; i < cs->inputs.size() && !split; ++i)
+        if (!cs->inputs[i].direct)
+            B200_TRY(b200_memcpy_h2d(cs->inputs[i].staging, inputs[i], cs->inputs[i].bytes_per_image * batch, stream));
     if (!cs->staging_known)
         for (size_t i = 0; i < cs->outputs.size(); ++i)
             cs->outputs[i].direct = direct_view(outputs[i], cs->outputs[i].bytes_per_image * batch);
-    B200_TRY(run_batch(cs, batch, stream));
+    if (split)
+        B200_TRY(split_host_run(cs, batch, inputs, stream));
+    else
+        B200_TRY(run_batch(cs, batch, stream));
     for (size_t i = 0; i < cs->outputs.size(); ++i)
         if (!cs->outputs[i].direct)
             B200_TRY(b200_memcpy_d2h(outputs[i], cs->outputs[i].staging, cs->outputs[i].bytes_per_image * batch, stream));

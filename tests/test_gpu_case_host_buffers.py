@@ -171,3 +171,39 @@ def test_parade_run_into_arrays_of_any_kind(tmp_path):
         parade.run(inputs, {oname: y})
         assert np.array_equal(y, want)
     parade.close()
+
+
+class _Buffer:
+    """Device memory as a torch tensor."""
+
+    def __init__(self, ptr, shape, typestr):
+        self.__cuda_array_interface__ = dict(data=(ptr, False), shape=shape, typestr=typestr, version=3)
+
+
+@pytest.mark.parametrize("net,hw,batch", [("resnet18", 128, 48), ("mobilenet_v2", 160, 33), ("resnet50", 112, 70)])
+@pytest.mark.parametrize("pinned", [True, False])
+def test_images_that_are_copied_in_two_parts(net, hw, batch, pinned):
+    """Graph mode, images of some megabytes: eager, captured and replayed runs with other images each time, against runs on
+    images that are on the device already; smaller batches of the same case, and a run without a graph, in between."""
+    from nart_b200 import nets
+    spec = nets.mobilenet_v2(seed=3, hw=hw, spread=True) if net == "mobilenet_v2" else nets.resnet(int(net[6:]), seed=3, hw=hw, spread=True, width_div=2)
+    cs, _ = nets.to_case(spec, batch)
+    ref, _ = nets.to_case(spec, batch)
+    cs.use_graph(True)
+    stream = torch.cuda.Stream()
+    x_dev = torch.as_tensor(_Buffer(ref.io_device_ptr(False, 0), (batch, 3, hw, hw), "|u1"), device="cuda")
+    y_dev = torch.as_tensor(_Buffer(ref.io_device_ptr(True, 0), (batch, 1000), "<f4"), device="cuda")
+    x, y = torch.empty((batch, 3, hw, hw), dtype=torch.uint8), torch.empty((batch, 1000), dtype=torch.float32)
+    if pinned:
+        x, y = x.pin_memory(), y.pin_memory()
+    for i, n in enumerate([batch, batch, batch, 7, batch, 32, 32, batch, batch]):
+        x.random_(0, 256)
+        cs.use_graph(i != 4)
+        cs.run_host_ptrs(n, [x.data_ptr()], [y.data_ptr()], stream.cuda_stream)
+        x_dev.copy_(x)
+        torch.cuda.synchronize()
+        ref.run_device(n, 0)
+        torch.cuda.synchronize()
+        assert torch.equal(y[:n], y_dev[:n].cpu()), i
+    cs.close()
+    ref.close()
