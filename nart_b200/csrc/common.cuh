@@ -39,6 +39,13 @@ inline cudaStream_t as_stream(b200_stream_t s) { return reinterpret_cast<cudaStr
 int status_word_ptr(int **dev_ptr);
 // Queues a kernel that moves the current device's status word to *host (pinned) and clears it.
 int status_publish_launch(int *host, cudaStream_t st);
+__device__ __forceinline__ void status_publish(int *word, int *host)
+{
+    const int v = *word;
+    *host = v;
+    if (v != 0)
+        *word = 0;
+}
 
 // Device copy of a 256-byte lookup table, uploaded the first time this table is seen on the current device
 // and cached for the life of the process (runtime.cu).

@@ -295,11 +295,14 @@ __global__ void quantize_flat_kernel(const float *__restrict__ in, uint8_t *__re
     }
 }
 
+// word: a status word that leaves for the host with this launch (see status_publish_launch), or nullptr
 template <typename Fn, bool VEC>
-__global__ void dequantize_flat_kernel(const uint8_t *__restrict__ in, float *__restrict__ out, size_t count, Fn fn)
+__global__ void dequantize_flat_kernel(const uint8_t *__restrict__ in, float *__restrict__ out, size_t count, Fn fn, int *word, int *host)
 {
     pdl_wait();
     pdl_trigger();
+    if (word != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
+        status_publish(word, host);
     size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (VEC && i + 4 <= count) {
         uint32_t q = *reinterpret_cast<const uint32_t *>(in + i);
@@ -321,12 +324,12 @@ static int quantize_flat_launch(const float *x, uint8_t *y, size_t count, Fn fn,
     return launch_kernel(quantize_flat_kernel<Fn, false>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
 }
 template <typename Fn>
-static int dequantize_flat_launch(const uint8_t *x, float *y, size_t count, Fn fn, cudaStream_t st)
+static int dequantize_flat_launch(const uint8_t *x, float *y, size_t count, Fn fn, cudaStream_t st, int *word = nullptr, int *host = nullptr)
 {
     const dim3 grid((unsigned)(((count + 3) / 4 + 255) / 256));
     if ((((uintptr_t)x & 3) | ((uintptr_t)y & 15)) == 0)
-        return launch_kernel(dequantize_flat_kernel<Fn, true>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
-    return launch_kernel(dequantize_flat_kernel<Fn, false>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn);
+        return launch_kernel(dequantize_flat_kernel<Fn, true>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn, word, host);
+    return launch_kernel(dequantize_flat_kernel<Fn, false>, grid, dim3(256), 0, st, count * 5, 1, x, y, count, fn, word, host);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -642,6 +645,21 @@ int b200_dequantize_u8(
         return dequantize_flat_launch(x, y, (size_t)n * c * P, fn, as_stream(stream));
     }
 }
+
+}  // extern "C"
+
+// b200_dequantize_u8 of one pixel an image, which also moves the current device's status word to *host
+int b200::dequantize_and_publish(const uint8_t *x, float *y, size_t count, float ialpha, uint8_t izp, int *host, cudaStream_t st)
+{
+    int *word = nullptr;
+    B200_TRY(status_word_ptr(&word));
+    DequantizeFn fn;
+    fn.alpha = ialpha;
+    fn.zp = izp;
+    return dequantize_flat_launch(x, y, count, fn, st, word, host);
+}
+
+extern "C" {
 
 int b200_quantize_s8(
     const float *x, int8_t *y8, int32_t n, int32_t c, int32_t h, int32_t w, float oalpha, uint8_t obits,

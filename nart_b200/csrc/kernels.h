@@ -34,6 +34,8 @@ int pool_launch(
     const uint8_t *x, uint8_t *y, int n, int c, int method, const PoolGeom &g, const uint8_t *lut_dev,
     const PoolAvgTab &tab, cudaStream_t st);
 
+int dequantize_and_publish(const uint8_t *x, float *y, size_t count, float ialpha, uint8_t izp, int *host, cudaStream_t st);
+
 // ---- relu -----------------------------------------------------------------------------------
 int relu_build_lut(
     float ialpha, uint8_t izp, float oalpha, uint8_t ozp, uint8_t obits, uint8_t lut[256]);

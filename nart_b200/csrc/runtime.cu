@@ -55,10 +55,7 @@ int status_word_ptr(int **dev_ptr)
 static __global__ void status_publish_kernel(int *word, int *host)
 {
     pdl_wait();
-    const int v = *word;
-    *host = v;
-    if (v != 0)
-        *word = 0;
+    status_publish(word, host);
 }
 
 int status_publish_launch(int *host, cudaStream_t st)
