@@ -34,7 +34,10 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
+#include "conv_small.h"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 
@@ -124,6 +127,15 @@ struct IgemmArgs {
     // number of clusters.
     int pm_tiles;            // pair tiles along M: ceil(m_tiles / 2)
     int step_pm;
+};
+// MODES 4 and 5: one box of activations for all taps of a channel chunk (and parity plane), box_bytes of shared memory each; the
+// groups of eight accumulator rows lie box_group pixels apart in it
+struct IgemmBoxArgs : IgemmArgs {
+    HaloTiles halo;
+    uint32_t box_bytes;
+    int box_group;
+    int a_pitch;             // shared memory a pixel takes: bk bytes; 16 with
+    int quads;               // 1: pixels of 16 channels, several neighbours an operand row (see ConvIgemmPlan::quads)
 };
 
 // How accumulators become output bytes.  For the reference's  y = sat(rshift_rn((acc + off) * mult, shift) + ozp)
@@ -499,14 +511,15 @@ struct SmemLayout {
 };
 // b_slots: B tiles held in shared memory -- one per pipeline stage, or every k-block of the layer
 // when the weights stay resident.
-__host__ __device__ inline SmemLayout smem_layout(int a_slots, int b_slots, int bk, int bn, int groups, int bn_b = 0)
+// box_bytes: what an A slot takes where that is no tile (MODES 4 and 5).
+__host__ __device__ inline SmemLayout smem_layout(int a_slots, int b_slots, int bk, int bn, int groups, int bn_b = 0, uint32_t box_bytes = 0)
 {
     if (bn_b == 0)
         bn_b = bn;      // rows of a B tile in this CTA's shared memory (half of bn in a CTA pair)
     SmemLayout L;
     uint32_t o = 0;
     L.a = o;
-    o += (uint32_t)a_slots * kTileM * bk;
+    o += (uint32_t)a_slots * (box_bytes ? box_bytes : (uint32_t)kTileM * bk);
     L.b = o;
     uint32_t b_tile = ((uint32_t)bn_b * bk + 1023u) & ~1023u;
     o += (uint32_t)b_slots * b_tile;
@@ -582,11 +595,15 @@ __device__ __forceinline__ void store_ragged(const IgemmArgs &g, uint32_t seg_ou
 // other one, which carries none of that code.
 // MODE 0: tile by tile.  MODE 1: two pipelines, each with its own producer, MMA issuer and half of the stages, take the CTA's
 // tiles in turn: the producer's and the issuer's chains of instructions set the pace of short k-blocks.  MODE 2: the CTA's tiles go in pairs that share every weight k-block: a stage holds the activation
-// tiles of both and ONE weight tile.  MODE 3: CTA pairs.
+// tiles of both and ONE weight tile.  MODE 3: CTA pairs.  MODE 4: one box of activations for all taps, weights resident; MODE 5:
+// the same in two pipelines.  A box per tap brings every pixel r * s times, and the producer's and issuer's chains with it; one box leaves
+// the MMAs (54 cycles at least for 128 pixels by 32 bytes, 61 with 64 channels, wherever a swizzle atom the operand starts) and the epilogue.
+// 3x3 64 -> 64 on 56 x 56: batch 256 49.3 -> 47.0 us, 32 11.2 -> 10.2; 32 -> 64 on 112 x 112, batch 64: 48.7 -> 36.4; with a weight zero
+// point, which has one pipeline with a box per tap, 83 -> 48.7 and 82.9 -> 36.8.
 // RAGGED: the instantiation that can store channel counts the TMA store cannot address (modes 0 and 1 run without it where
 // they need not, which is worth 2 % to the layers their epilogue bounds).
 template <int EPI, bool HAS_RES, bool HAS_WZP, int MODE, bool RAGGED = true>
-__global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ IgemmArgs g)
+__global__ void __launch_bounds__(MODE == 1 || MODE == 5 ? kThreads2 : kThreads, 1) conv_igemm_i8_kernel(const __grid_constant__ IgemmMaps maps, const __grid_constant__ std::conditional_t<MODE == 4 || MODE == 5, IgemmBoxArgs, IgemmArgs> g)
 {
     extern __shared__ uint8_t smem_raw[];
     // the swizzle patterns are functions of the absolute shared address: align the base to 1024
@@ -602,7 +619,11 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
     const bool leader = !PAIR || cta_rank == 0;
     constexpr int kOnes = HAS_WZP ? 16 : 0;      // rows of B, and accumulator columns, behind the tile's channels
     const int bnl = PAIR ? g.bn >> 1 : g.bn + kOnes;     // rows of B this CTA holds
-    const SmemLayout L = smem_layout(MODE == 2 ? 2 * slots : slots, g.b_resident ? kblocks_all : slots, g.bk, g.bn, g.groups, bnl);
+    constexpr bool HALO = MODE == 4 || MODE == 5, RINGS = MODE == 1 || MODE == 5;
+    uint32_t box_bytes = 0;
+    if constexpr (HALO)
+        box_bytes = g.box_bytes;
+    const SmemLayout L = smem_layout(MODE == 2 ? 2 * slots : slots, g.b_resident ? kblocks_all : slots, g.bk, g.bn, g.groups, bnl, box_bytes);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform, and known to be
     const int lane = threadIdx.x & 31;
@@ -689,10 +710,10 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
     };
 
     // this warp's pipeline (MODE 1), its stages and its first tile
-    constexpr int tile_step = MODE == 1 || MODE == 2 ? 2 : 1;
-    const int ring = MODE == 1 && warp >= kRing1Warp ? 1 : 0, ring_stages = MODE == 1 ? g.stages >> 1 : g.stages;
+    constexpr int tile_step = RINGS || MODE == 2 ? 2 : 1;
+    const int ring = RINGS && warp >= kRing1Warp ? 1 : 0, ring_stages = RINGS ? g.stages >> 1 : g.stages;
     const int ring_tile0 = tile0 + ring * tstride, stage0 = ring * ring_stages;
-    if (warp == 0 || (MODE == 1 && warp == kRing1Warp)) {
+    if (warp == 0 || (RINGS && warp == kRing1Warp)) {
         // ================= TMA producer =================
         // The warp walks the k-blocks of this CTA's tiles in order, one elected lane issues: wait for the stage of the next group of k-blocks, post
         // the group's byte count, issue its loads.  The chain of instructions of one k-block bounds the mainloop (its MMAs take
@@ -723,6 +744,49 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                         }
                     }
             }
+            if constexpr (HALO) {
+                const HaloTiles &h = g.halo;
+                const uint32_t bars0 = full_bar(stage0), a_dst0 = base + L.a + (uint32_t)stage0 * g.box_bytes;
+                uint32_t fb = bars0, a_dst = a_dst0, phase = 1;
+                int stage = 0;
+                TileWalker tw;
+                walker_init(tw);
+                if (ring == 1)
+                    tw.advance(g);
+                pdl_wait();
+                bool ok = true;
+                for (int tile = ring_tile0; ok && tile < total_tiles; tile += tile_step * tstride) {
+                    const int x0 = tw.wi(g) << g.tw_sh, y0 = tw.hi(g) << g.th_sh, n0 = tw.ni(g);
+                    for (int c = 0; ok && c < cchunks; ++c)
+                        for (int pl = 0; pl < h.planes; ++pl) {
+                            if (!mbar_wait_warp(fb + 8u * kMaxStages, phase, abort_flag)) {
+                                if (lane == 0)
+                                    atomicCAS(g.status, 0, kErrProducerWait);
+                                *abort_flag = 1;
+                                ok = false;
+                                break;
+                            }
+                            if (elect_one()) {
+                                mbar_expect_tx(fb, (uint32_t)(h.rows[pl] * g.a_pitch));
+                                if (g.quads)
+                                    tma_load_3d(a_dst, &maps.a[pl], fb, (x0 + h.dx[pl]) * 2, y0 + h.dy[pl], n0);
+                                else
+                                    tma_load_4d(a_dst, &maps.a[pl], fb, c * (int)bk, x0 + h.dx[pl], y0 + h.dy[pl], n0);
+                            }
+                            __syncwarp();
+                            fb += 8;
+                            a_dst += g.box_bytes;
+                            if (++stage == ring_stages) {
+                                stage = 0;
+                                fb = bars0;
+                                a_dst = a_dst0;
+                                phase ^= 1;
+                            }
+                        }
+                    for (int i = 0; i < tile_step; ++i)
+                        tw.advance(g);
+                }
+            } else {
             const int groups = kblocks / (int)kgroup;
             const int sh_h = g.stride_h - 1, sh_w = g.stride_w - 1;         // strides are 1 or 2
             const int c_end = cchunks * (int)bk, c_pitch = g.c, taps_w = g.s, pad_w = g.pad_w, pad_h = g.pad_h;
@@ -872,13 +936,14 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                 if (MODE == 2)
                     tw2.advance(g);
             }
+            }
         }
         __syncwarp();
         // every load is on its way: the next launch's blocks may come (a block per SM that waits for longer
         // would keep the SM from the launches of other streams)
         if (ring == 0)
             pdl_trigger();
-    } else if (warp == 1 || (MODE == 1 && warp == kRing1Warp + 1)) {
+    } else if (warp == 1 || (RINGS && warp == kRing1Warp + 1)) {
         // ================= MMA issuer =================
         // The warp walks, one elected lane issues.  Descriptors of one operand differ only in the start-address field, so only their low words are
         // computed.  In a CTA pair the leading CTA's warp issues for both; the peer's has nothing to do.
@@ -917,6 +982,67 @@ __global__ void __launch_bounds__(MODE == 1 ? kThreads2 : kThreads, 1) conv_igem
                 const uint32_t d_tmem = tmem_base + (uint32_t)as * acc_cols;
                 uint32_t accumulate = 0;
                 int chunk = 0;        // k-block of the tap
+                if constexpr (HALO) {
+                    const HaloTiles &h = g.halo;
+                    const uint32_t a_hi = halo_desc_hi(desc_hi, g.box_group, g.a_pitch, g.quads);
+                    const uint32_t a_col = (uint32_t)g.a_pitch >> 4, a_row = (uint32_t)(h.pitch * g.a_pitch) >> 4;
+                    const uint32_t b_tap = (uint32_t)cchunks * b_step, b_col = h.tap_col * b_tap, b_row = h.tap_row * b_tap;
+                    const uint32_t box_step = g.box_bytes >> 4;
+                    for (int c = 0; ok && c < cchunks; ++c) {
+                        const int ksteps = c + 1 == cchunks ? last_steps : ksteps_full;
+                        for (int pl = 0; pl < h.planes; ++pl) {
+                            if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
+                                give_up(kErrMmaFullWait);
+                                break;
+                            }
+                            tc_fence_after();
+                            // the taps of the plane, up to three of a row at a time
+                            uint32_t a0 = (uint32_t)adesc0 + (uint32_t)stage * box_step, b0 = b_lo0 + (uint32_t)c * b_step + h.tap0[pl] * b_tap;
+                            const int th = h.taps_h[pl], tw = h.taps_w[pl];
+                            for (int i = 0; i < th; ++i, a0 += a_row, b0 += b_row) {
+                                uint32_t a = a0, b = b0;
+                                for (int j = 0; j < tw; j += 3, a += 3 * a_col, b += 3 * b_col) {
+                                    auto tap = [&](uint32_t ta, uint32_t tb, uint32_t acc) {
+                                        mma_i8_ab(d_tmem, ta, tb, a_hi, desc_hi, idesc, acc);
+                                        if (ksteps >= 2)
+                                            mma_i8_ab(d_tmem, ta + 2, tb + 2, a_hi, desc_hi, idesc, 1);
+                                        if (ksteps >= 3)
+                                            mma_i8_ab(d_tmem, ta + 4, tb + 4, a_hi, desc_hi, idesc, 1);
+                                        if (ksteps == 4)
+                                            mma_i8_ab(d_tmem, ta + 6, tb + 6, a_hi, desc_hi, idesc, 1);
+                                    };
+                                    if (elect_one()) {
+                                        tap(a, b, accumulate);
+                                        if (j + 1 < tw)
+                                            tap(a + a_col, b + b_col, 1);
+                                        if (j + 2 < tw)
+                                            tap(a + 2 * a_col, b + 2 * b_col, 1);
+                                    }
+                                    __syncwarp();
+                                    accumulate = 1;
+                                }
+                            }
+                            if (elect_one()) {
+                                mma_commit(empty_bar(stage));
+                                if (c + 1 == cchunks && pl + 1 == h.planes)
+                                    mma_commit(tfull_bar(as));
+                            }
+                            __syncwarp();
+                            if (++stage == stage0 + ring_stages) {
+                                stage = stage0;
+                                phase ^= 1;
+                            }
+                        }
+                    }
+                    if (!ok)
+                        break;
+                    as += tile_step;
+                    if (as >= g.acc_stages) {
+                        as -= g.acc_stages;
+                        aphase ^= 1;
+                    }
+                    continue;
+                }
                 if (resident)
                     b_lo = b_lo0;
                 for (int grp = 0; grp < groups; ++grp) {
@@ -1186,6 +1312,9 @@ IgemmKernel igemm_kernel_mode1(int epi);
 IgemmKernel igemm_kernel_ragged(int epi, bool two_pipelines);
 IgemmKernel igemm_kernel_mode2(int epi);
 IgemmKernel igemm_kernel_mode3(int epi);                // none for variants that only short reductions have
+typedef void (*IgemmBoxKernel)(const IgemmMaps, const IgemmBoxArgs);
+IgemmBoxKernel igemm_kernel_mode4(int epi, bool wzp);
+IgemmBoxKernel igemm_kernel_mode5(int epi, bool wzp);
 IgemmKernel igemm_kernel_wzp(int epi);                  // a weight zero point other than 128
 IgemmKernel igemm_kernel_residual(int epi);             // a residual add: none for the Full variants and kEpiAny
 

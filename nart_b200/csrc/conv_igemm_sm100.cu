@@ -177,6 +177,14 @@ struct ConvIgemmPlan {
     // two cluster-wide syncs), so the plan carries both configurations and build_launch picks.
     int pair_ok = 0, pair_want = -1, stages_pair = 0;
     int max_clusters = 0;           // co-resident CTA pairs of that kernel on this device
+    // Pixels of 16 channels of which an operand row holds as many neighbours as the window has columns, rounded up to 2, 4 or 8: the
+    // pixels of a box lie 16 bytes apart and rows of 32 to 128 bytes overlap, which the unswizzled layout can say.  A row of
+    // the window is then one tap (taps_w is 1).
+    int quads = 0, taps_w = 0;
+    // One box of activations for all taps (kernel MODE 4), its tiles and its stages (0: not possible)
+    HaloTiles halo;
+    int stages_halo = 0, box_group = 8;
+    uint32_t box_bytes = 0;
     int n_row_cls = 0, n_col_cls = 0;
     int seg_w[2] = { 0, 0 };        // see epilogue_segments
     int form = kEpiGeneric, variant = kEpiAny, ushift = 0, rnd_hi = 0;      // see EpiForm, EpiVariant
@@ -212,14 +220,17 @@ struct ConvIgemmPlan {
         int *status;
         bool small;                 // the one-tile-per-CTA kernel (conv_small_sm100.cu): smaps, sargs, m_tiles
         int cta_pair;
+        bool halo;
         int m_tiles;
+        bool small_box;             // the small kernel with one box for all taps
         IgemmKernel kernel;
+        IgemmBoxKernel box_kernel;
         dim3 grid;
         size_t smem;
         SmallMaps smaps;
-        SmallArgs sargs;
+        SmallBoxArgs sargs;
         IgemmMaps maps;
-        IgemmArgs args;
+        IgemmBoxArgs args;
     };
     static constexpr size_t kMaxSaved = 8;
     std::vector<Launch> saved;
@@ -306,7 +317,7 @@ static void tap_classes(int out, int in, int kernel, int pad, int stride, std::v
 
 int conv_igemm_create(
     const ConvGeom &g, const std::vector<int8_t> &w_s8, const int32_t *bias, const uint32_t *mult,
-    const int32_t *shift, ConvIgemmPlan **out, bool a_row_swizzled, int window)
+    const int32_t *shift, ConvIgemmPlan **out, bool a_row_swizzled, int window, bool quads)
 {
     if (a_row_swizzled && !(g.c == 32 && g.s == 1 && g.stride_w == 1 && g.pad_w == 0 && g.w == g.ow))
         return fail(B200_ERR_INVALID, "conv(igemm): pre-swizzled rows need 32 channels and an r x 1 kernel");
@@ -341,10 +352,13 @@ int conv_igemm_create(
     }
     p->saved.reserve(ConvIgemmPlan::kMaxSaved);   // launches never grow it: a later run touches no heap
     p->a_wide = a_row_swizzled ? 1 : 0;
+    p->quads = quads ? 1 : 0;
+    p->taps_w = quads ? 1 : g.s;
+    const int mma_taps = g.r * p->taps_w;
     // K of an 8-bit MMA is 32 bytes: the channel count is rounded up to a multiple of 32 in the
     // repacked weights (zero weights); on the activation side the TMA box runs past the tensor's
     // channel extent and reads zeros there
-    p->cpad = (g.c + 31) / 32 * 32;
+    p->cpad = quads ? (g.s <= 2 ? 32 : g.s <= 4 ? 64 : 128) : (g.c + 31) / 32 * 32;
     // The k-block: 32, 64 or 128 channels.  The last block of a tap may run past the channels (TMA zero fill; its empty
     // MMA steps are left out), which costs shared memory but no traffic, and every block costs a barrier round trip:
     // 80 channels are one block of 128, 224 two, 160 and 192 three of 64.
@@ -393,7 +407,7 @@ int conv_igemm_create(
     p->kpad = n_tiles_n * p->bn;
     // pipeline depth from the shared memory left after the staging buffer
     {
-        const int kblocks = g.r * g.s * cchunks;
+        const int kblocks = mma_taps * cchunks;
         // weights resident when there is one channel tile and they leave room for >= 3 A stages
         // four epilogue groups (four tiles in flight behind the mainloop) when the tiles are narrow:
         // their per-tile latency chain, not their arithmetic, sets the epilogue rate
@@ -488,18 +502,60 @@ int conv_igemm_create(
         }
         p->stages = stages;
         p->kgroup = kgroup;
+        // One box for all taps.  Tiles of eight by sixteen pixels, or of whole lines where a power of two holds a line
+        // and its ring: the shapes whose 32-pixel quarters are boxes of the output.
+        const HaloWindow win(g.r, p->taps_w, g.stride_h, g.stride_w, g.pad_h, g.pad_w, quads ? g.s : 0, quads ? p->bk / 16 : 1);
+        const char *e = getenv("B200_IGEMM_HALO");        // tuning aid: 0 never
+        if (win.fits() && !p->a_wide && n_tiles_n == 1 && g.k % 16 == 0 && (quads || !(e && atoi(e) == 0))) {
+            int line = 8;
+            while (line < g.ow + win.ring_w)
+                line *= 2;
+            const long long by_cols = (long long)((g.ow + 7) / 8) * ((g.oh + 15) / 16);
+            const long long by_lines = line <= kTileM ? (g.oh + kTileM / line - 1) / (kTileM / line) : by_cols + 1;
+            for (int form = 0; form < 2 && p->stages_halo == 0; ++form) {      // the one of fewer tiles, or the other if only that fits
+                const bool lines = (by_lines <= by_cols) == (form == 0);
+                if (lines && line > kTileM)
+                    break;
+                HaloTiles &h = p->halo;
+                memset(&h, 0, sizeof(h));
+                h.tw = lines ? line : 8;
+                h.th = kTileM / h.tw;
+                h.pitch = lines ? line : 8 + win.ring_w;
+                p->box_group = lines ? 8 : h.pitch;
+                halo_planes(win, p->box_group, &h);
+                p->box_bytes = ((uint32_t)(h.span * (quads ? 16 : p->bk)) + 1023u) & ~1023u;
+                int st = kMaxStages;
+                while (st > 0 && smem_layout(st, kblocks, p->bk, p->bn, p->groups, p->bn + ones, p->box_bytes).total + 1024 > 227 * 1024)
+                    --st;
+                if (st >= 2)
+                    p->stages_halo = st >= 4 ? st & ~1 : st;       // (two pipelines from four on)
+            }
+        }
     }
-    if (smem_layout((p->pair ? 2 : 1) * p->stages * p->kgroup, p->b_resident ? g.r * g.s * cchunks : p->stages * p->kgroup, p->bk, p->bn, p->groups, p->bn + ones).total + 1024 > 227 * 1024) {
+    if (quads && !p->stages_halo) {         // (there is no other way to read these pixels)
+        delete p;
+        return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no box of this image fits shared memory");
+    }
+    if (!quads && smem_layout((p->pair ? 2 : 1) * p->stages * p->kgroup, p->b_resident ? mma_taps * cchunks : p->stages * p->kgroup, p->bk, p->bn, p->groups, p->bn + ones).total + 1024 > 227 * 1024) {
         delete p;
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): tile does not fit shared memory");
     }
 
     const int taps = g.r * g.s;
     // ---- weights [kpad][r][s][c] ---------------------------------------------------------------
-    std::vector<int8_t> wp((size_t)p->kpad * taps * p->cpad, 0);
+    std::vector<int8_t> wp((size_t)p->kpad * mma_taps * p->cpad, 0);
     std::vector<int32_t> wtap((size_t)g.k * taps);       // sum over channels per (k, tap)
-    for (int k = 0; k < g.k; ++k)
-        weights_tap_major(&w_s8[(size_t)k * g.c * taps], g.c, taps, &wp[(size_t)k * taps * p->cpad], p->cpad, &wtap[(size_t)k * taps]);
+    if (quads) {        // [kpad][r][pixels of a row][16]
+        std::vector<int8_t> row((size_t)taps * 16);
+        for (int k = 0; k < g.k; ++k) {
+            weights_tap_major(&w_s8[(size_t)k * g.c * taps], g.c, taps, row.data(), 16, &wtap[(size_t)k * taps]);
+            for (int rr = 0; rr < g.r; ++rr)
+                memcpy(&wp[((size_t)k * g.r + rr) * p->cpad], &row[(size_t)rr * g.s * 16], (size_t)g.s * 16);
+        }
+    } else {
+        for (int k = 0; k < g.k; ++k)
+            weights_tap_major(&w_s8[(size_t)k * g.c * taps], g.c, taps, &wp[(size_t)k * taps * p->cpad], p->cpad, &wtap[(size_t)k * taps]);
+    }
     // ---- border classes and offsets ---------------------------------------------------------------
     std::vector<uint8_t> row_cls, col_cls;
     std::vector<std::vector<char>> row_valid, col_valid;
@@ -665,16 +721,16 @@ void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
 {
     const ConvIgemmPlan::Launch *l = p->last_launch();      // the tiling depends on the batch of the run
     if (l && l->small) {
-        snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d slots=%d split=%d one tile per %s", l->sargs.bn, p->bk, l->sargs.slots, l->sargs.split,
-                 l->sargs.split > 1 ? "cluster" : "CTA");
+        snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d slots=%d split=%d one tile per %s%s", l->sargs.bn, p->bk, l->sargs.slots, l->sargs.split,
+                 l->sargs.split > 1 ? "cluster" : "CTA", l->small_box ? ", one box for all taps" : "");
         return;
     }
     const bool cta_pair = l && l->cta_pair;
-    const char *mode = cta_pair ? "cta-pair (cta_group::2, M=256)" : p->pair ? "tile pairs on one weight tile"
+    const char *mode = l && l->halo ? "one box for all taps" : cta_pair ? "cta-pair (cta_group::2, M=256)" : p->pair ? "tile pairs on one weight tile"
         : p->pair_ok ? "tile by tile (cta pairs on long launches)"
         : p->rings == 2 ? "two pipelines" : "tile by tile";
     snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d stages=%d kgroup=%d groups=%d acc_stages=%d %s%s%s%s", p->bn, p->bk,
-             cta_pair ? p->stages_pair : p->stages, p->kgroup, p->groups, p->acc_stages, mode, p->b_resident ? ", weights resident" : "",
+             l ? l->args.stages : p->stages, l ? l->args.kgroup : p->kgroup, p->groups, p->acc_stages, mode, (l ? l->args.b_resident : p->b_resident) ? ", weights resident" : "",
              p->form == kEpiFp ? ", fp32 epilogue" : p->form == kEpiInt ? ", uniform-shift epilogue" : ", generic requantize",
              p->rev ? ", reversed" : "");
 }
@@ -759,11 +815,35 @@ static int encode_activations(const ConvIgemmPlan *p, const uint8_t *x, int n, i
     return B200_OK;
 }
 
+// The same for the boxes of HaloTiles, a map per plane.
+static int encode_boxes(const ConvIgemmPlan *p, const uint8_t *x, int n, const HaloTiles &h, CUtensorMap (&maps)[4])
+{
+    const ConvGeom &g = p->g;
+    for (int i = 0; i < h.planes; ++i) {
+        const int ph = h.parity[i] >> 1, pw = h.parity[i] & 1;
+        if (p->quads) {         // whole lines of the image, in 8-byte elements
+            cuuint64_t dims[3] = { (cuuint64_t)g.w * 2, (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
+            cuuint64_t strides[2] = { (cuuint64_t)g.stride_h * g.w * 16, (cuuint64_t)g.h * g.w * 16 };
+            cuuint32_t box[3] = { (cuuint32_t)h.pitch * 2, (cuuint32_t)(h.rows[i] / h.pitch), 1 };
+            B200_TRY(encode(&maps[i], (void *)(x + (size_t)ph * g.w * 16), 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_DATA_TYPE_UINT64));
+            continue;
+        }
+        cuuint64_t dims[4] = { (cuuint64_t)g.c, (cuuint64_t)((g.w - pw + g.stride_w - 1) / g.stride_w),
+                               (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
+        cuuint64_t strides[3] = { (cuuint64_t)g.stride_w * g.c, (cuuint64_t)g.stride_h * g.w * g.c, (cuuint64_t)g.h * g.w * g.c };
+        cuuint32_t box[4] = { (cuuint32_t)p->bk, (cuuint32_t)h.pitch, (cuuint32_t)(h.rows[i] / h.pitch), 1 };
+        B200_TRY(encode(&maps[i], (void *)(x + ((size_t)ph * g.w + pw) * g.c), 4, dims, strides, box, swizzle_for(p->bk)));
+    }
+    for (int i = h.planes; i < 4; ++i)
+        maps[i] = maps[0];
+    return B200_OK;
+}
+
 // Tensor map of [rows][r*s*c] weights in boxes of `box_rows` rows and one k-block.
 // frag: the row order of the fragment epilogue (frag_segment): row 8 j + 2 q + e of every sixteen is channel 4 q + 2 j + e.
 static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int box_rows, CUtensorMap *map, bool frag = false)
 {
-    const int ktot = p->g.r * p->g.s * p->cpad;
+    const int ktot = p->g.r * p->taps_w * p->cpad;
     if (frag) {
         cuuint64_t dims[5] = { (cuuint64_t)ktot, 2, 4, 2, (cuuint64_t)(rows / 16) };
         cuuint64_t strides[4] = { (cuuint64_t)ktot, 4 * (cuuint64_t)ktot, 2 * (cuuint64_t)ktot, 16 * (cuuint64_t)ktot };
@@ -780,7 +860,7 @@ static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int
 static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status, int tw, int th, int tn, const ConvSum *ws, ConvIgemmPlan::Launch &l)
 {
     const ConvGeom &g = p->g;
-    SmallArgs &a = l.sargs;
+    SmallBoxArgs &a = l.sargs;
     memset(&a, 0, sizeof(a));
     a.tiles_w = (g.ow + tw - 1) / tw;
     a.tiles_h = (g.oh + th - 1) / th;
@@ -788,16 +868,44 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.cchunks = (p->cpad + p->bk - 1) / p->bk;
     a.cpad = p->cpad;
     a.last_steps = (p->cpad - (a.cchunks - 1) * p->bk) / 32;
-    a.kblocks = g.r * g.s * a.cchunks;
+    a.kblocks = g.r * p->taps_w * a.cchunks;
     a.bk = p->bk;
+    a.quads = p->quads;
+    a.a_pitch = p->quads ? 16 : p->bk;
+    // One box for all taps only where there is no other way: with a box per tap the k-blocks are on their way while the first ones
+    // are multiplied (3x3 64 -> 64 on 56 x 56: 4.3 us, 4.9 with one box).
+    HaloTiles halo;
+    const char *he = getenv("B200_IGEMM_HALO");       // tuning aid: 1 wherever possible
+    const HaloWindow win(g.r, p->taps_w, g.stride_h, g.stride_w, g.pad_h, g.pad_w, p->quads ? g.s : 0, p->quads ? p->bk / 16 : 1);
+    const bool can_halo = (p->quads || (he && atoi(he) == 1)) && !p->a_wide && halo_tiles(win, g.ow, g.oh, &halo);
+    const int halo_w = can_halo ? (g.ow + halo.tw - 1) / halo.tw : 0, halo_h = can_halo ? (g.oh + halo.th - 1) / halo.th : 0;
+    bool use_halo = false;
     if (p->small_bn && p->small_split <= a.kblocks) {              // tuning aid
         a.bn = p->small_bn;
         a.split = p->small_split;
-    } else if (!conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, &a.bn, &a.split)) {
-        return B200_OK;
+        use_halo = can_halo;
+    } else {
+        double cost = 0.0;
+        bool small = conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, 0, 0, &cost, &a.bn, &a.split) && !p->quads;
+        if (can_halo) {
+            int box_rows = 0;
+            for (int i = 0; i < halo.planes; ++i)
+                box_rows += p->quads ? halo.rows[i] / halo.pitch : halo.rows[i];
+            use_halo = conv_small_pick(halo_w * halo_h * n, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, g.r * p->taps_w, box_rows, &cost, &a.bn, &a.split);
+            small = small || use_halo;
+        }
+        if (!small)
+            return B200_OK;
+    }
+    int tiles = m_tiles;
+    if (use_halo) {
+        a.halo = halo;
+        a.tiles_w = halo_w;
+        a.tiles_h = halo_h;
+        tiles = halo_w * halo_h * n;
     }
     a.n = n; a.oh = g.oh; a.ow = g.ow; a.cout = g.k;
-    a.r = g.r; a.s = g.s; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
+    a.r = g.r; a.s = p->taps_w; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
     for (a.tw_sh = 0; (1 << a.tw_sh) < tw; ++a.tw_sh) {}
     for (a.th_sh = 0; (1 << a.th_sh) < th; ++a.th_sh) {}
     a.tn = tn;
@@ -813,7 +921,7 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.y = y;
     a.status = status;
     a.next_ro = p->next_ro; a.next_ro_bytes = p->next_ro_bytes;
-    if (ws && g.k % 16 == 0 && !g.act_signed) {         // (other channel counts leave through staged rows)
+    if (ws && g.k % 16 == 0 && !g.act_signed && !use_halo) {         // (other channel counts leave through staged rows)
         const int ci = ws->conv_input, other = 1 - ci;
         const EltwiseArgs &e = *ws->elt;
         a.res = ws->res;
@@ -823,16 +931,20 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
         a.r_s0 = e.s0; a.r_ozp = e.ozp; a.r_lo = e.relu_lo;
         l.summed = true;
     }
-    const size_t smem = conv_small_smem(a, g.act_signed != 0);
+    l.small_box = use_halo;
+    const size_t smem = conv_small_smem(a, use_halo, g.act_signed != 0);
     if (smem > 227 * 1024)
         return B200_OK;
-    B200_TRY(encode_activations(p, x, n, tw, th, tn, l.smaps.a));
+    if (use_halo)
+        B200_TRY(encode_boxes(p, x, n, halo, l.smaps.a));
+    else
+        B200_TRY(encode_activations(p, x, n, tw, th, tn, l.smaps.a));
     B200_TRY(encode_weights(p, p->w_dev, p->kpad, a.bn, &l.smaps.b));
     l.smaps.ones = l.smaps.b;
     if (p->ones_dev)
         B200_TRY(encode_weights(p, p->ones_dev, 16, 16, &l.smaps.ones));
     l.smem = smem;
-    l.m_tiles = m_tiles;
+    l.m_tiles = tiles;
     l.small = true;
     return B200_OK;
 }
@@ -846,14 +958,15 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     l.sum_res = ws ? ws->res : nullptr; l.sum = ws ? ws->sum : nullptr; l.summed = false;
     l.small = false;
     l.cta_pair = 0;
-    IgemmArgs &a = l.args;
+    l.halo = false;
+    IgemmBoxArgs &a = l.args;
     memset(&a, 0, sizeof(a));
     if (status_word)
         a.status = status_word;       // caller-provided word (the allocation-free entry point)
     else
         B200_TRY(status_word_ptr(&a.status));
     a.n = n; a.oh = g.oh; a.ow = g.ow; a.cout = g.k;
-    a.r = g.r; a.s = g.s; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
+    a.r = g.r; a.s = p->taps_w; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
     a.c = p->cpad;
     if (p->a_wide)   // whole swizzle atoms (8 pixels) per row segment, at most 256 8-byte elements
         choose_tile(g.ow, g.oh, n, &a.tw, &a.th, &a.tn, 3, 6);
@@ -896,6 +1009,33 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         // 512 -> 512: 34.1 -> 31.1)
         l.cta_pair = (p->pair_want == 1 || pair_tiles >= p->max_clusters) ? 1 : 0;
     }
+    if (p->stages_halo && !res && !l.cta_pair) {
+        const HaloTiles &h = p->halo;
+        const long long boxes = (long long)((g.ow + h.tw - 1) / h.tw) * ((g.oh + h.th - 1) / h.th) * n;
+        // Windows of stride 1, whose taps all share one box.  What the tiles waste beside the image decides: they hold one image's
+        // pixels, and lines end in them.  Up to a fifth the box wins 4 .. 50 % (64 -> 64 on 56 x 56, batch 64: 16.6 -> 15.8 us, 32 -> 64 on 112 x 112:
+        // 48.7 -> 36.6, 96 -> 96 on 40 x 40: 18.3 -> 14.9); with k-blocks of 128 channels up to a third (128 -> 128 on 14 x 14, batch 256:
+        // 12.4 -> 11.5; 64 -> 64 there 8.04 -> 7.84, on 27 x 35 11.7 -> 12.7), and up to a half where a window-sum column leaves one pipeline
+        // to a box per tap (24.6 -> 16.3; on 14 x 14 10.1 -> 8.2).  Tiles of more than 128 channels wait for their epilogue (32 -> 256 on 30 x 30:
+        // 13.8 -> 14.9); with a stride a box holds few taps (64 -> 128, stride 2: 9.8 -> 10.8).
+        const char *e = getenv("B200_IGEMM_HALO");       // tuning aid: 1 wherever possible
+        const long long tiles = (long long)a.tiles_w * a.tiles_h * a.tiles_n;
+        l.halo = p->quads || (e && atoi(e) == 1)
+            || (h.planes == 1 && (p->bn <= 128 || g.wzp_d != 0) && boxes * 100 <= tiles * (g.wzp_d != 0 ? 150 : p->bk == 128 ? 133 : 120));
+        if (l.halo) {
+            a.tw = h.tw; a.th = h.th; a.tn = 1;
+            a.tiles_w = (g.ow + a.tw - 1) / a.tw;
+            a.tiles_h = (g.oh + a.th - 1) / a.th;
+            a.tiles_n = n;
+            a.halo = h;
+            a.box_bytes = p->box_bytes;
+            a.box_group = p->box_group;
+            a.quads = p->quads;
+            a.a_pitch = p->quads ? 16 : p->bk;
+        }
+    }
+    if (p->quads && !l.halo)
+        return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no launch for this image");
     a.bk = p->bk; a.bn = p->bn; a.stages = l.cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
     a.cchunks = (p->cpad + p->bk - 1) / p->bk;
     a.last_steps = (p->cpad - (a.cchunks - 1) * p->bk) / 32;
@@ -930,7 +1070,10 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     a.wzp_d = g.wzp_d;
 
     // ---- tensor maps -------------------------------------------------------------------------------
-    B200_TRY(encode_activations(p, x, n, a.tw, a.th, a.tn, l.maps.a));
+    if (l.halo)
+        B200_TRY(encode_boxes(p, x, n, p->halo, l.maps.a));
+    else
+        B200_TRY(encode_activations(p, x, n, a.tw, a.th, a.tn, l.maps.a));
     const bool frag = !res && !g.wzp_d && p->n_row_cls * p->n_col_cls == 1 && p->variant != kEpiAny;   // as the kernel's `frag`
     B200_TRY(encode_weights(p, p->w_dev, p->kpad, l.cta_pair ? p->bn / 2 : p->bn, &l.maps.b, frag));   // a CTA of a pair loads half the rows
     l.maps.ones = l.maps.b;
@@ -951,18 +1094,26 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     } else {
         l.maps.y[0] = l.maps.y[1] = l.maps.b;
     }
+    if (l.halo) {
+        a.stages = p->stages_halo;
+        a.kgroup = 1;
+        a.b_resident = 1;
+    }
+    l.box_kernel = !l.halo ? nullptr : (a.stages >= 4 ? igemm_kernel_mode5 : igemm_kernel_mode4)(p->variant, g.wzp_d != 0);
     l.kernel = res ? igemm_kernel_residual(p->variant)
         : g.wzp_d ? igemm_kernel_wzp(p->variant)
         : l.cta_pair ? igemm_kernel_mode3(p->variant)
         : p->pair ? igemm_kernel_mode2(p->variant)
         : !a.use_tma_store ? igemm_kernel_ragged(p->variant, p->rings == 2)
         : p->rings == 2 ? igemm_kernel_mode1(p->variant) : igemm_kernel_mode0(p->variant);
-    if (!l.kernel)
+    if (!l.kernel && !l.box_kernel)
         return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no kernel of epilogue variant %d for this launch", p->variant);
     const int total_tiles = a.tiles_w * a.tiles_h * a.tiles_n * a.n_tiles_n;
     l.grid = dim3((unsigned)(total_tiles < sms ? total_tiles : sms));
-    l.smem = smem_layout((p->pair ? 2 : 1) * a.stages * p->kgroup, p->b_resident ? g.r * g.s * a.cchunks : a.stages * p->kgroup, p->bk, p->bn, p->groups,
+    l.smem = smem_layout((p->pair ? 2 : 1) * a.stages * p->kgroup, p->b_resident ? g.r * p->taps_w * a.cchunks : a.stages * p->kgroup, p->bk, p->bn, p->groups,
                          l.cta_pair ? p->bn / 2 : p->bn + ones).total + 1024;
+    if (l.halo)
+        l.smem = smem_layout(a.stages, g.r * p->taps_w * a.cchunks, p->bk, p->bn, p->groups, p->bn + ones, p->box_bytes).total + 1024;
     if (l.cta_pair) {
         // pair tiles (two neighbouring M tiles, one channel tile) over the CTA pairs that fit the device at once
         a.pm_tiles = (a.tiles_w * a.tiles_h * a.tiles_n + 1) / 2;
@@ -1023,9 +1174,11 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
     if (summed)
         *summed = l.small && l.summed;
     if (l.small)
-        return conv_small_launch(l.smaps, l.sargs, l.m_tiles, l.smem, bytes, st);
-    const bool two_rings = !l.cta_pair && !res && p->g.wzp_d == 0 && !p->pair && p->rings == 2;
-    return launch_kernel(l.kernel, l.grid, dim3(two_rings ? kThreads2 : kThreads), l.smem, st, bytes, l.cta_pair ? 2 : 1, l.maps, l.args);
+        return conv_small_launch(l.smaps, l.sargs, l.small_box, l.m_tiles, l.smem, bytes, st);
+    const bool two_rings = l.halo ? l.args.stages >= 4 : !l.cta_pair && !res && p->g.wzp_d == 0 && !p->pair && p->rings == 2;
+    if (l.halo)
+        return launch_kernel(l.box_kernel, l.grid, dim3(two_rings ? kThreads2 : kThreads), l.smem, st, bytes, 1, l.maps, l.args);
+    return launch_kernel(l.kernel, l.grid, dim3(two_rings ? kThreads2 : kThreads), l.smem, st, bytes, l.cta_pair ? 2 : 1, l.maps, static_cast<const IgemmArgs &>(l.args));
 }
 
 // Everything the first launch of any plan would otherwise do once per process or device: the driver
@@ -1047,6 +1200,10 @@ int conv_igemm_warm()
                                igemm_kernel_mode2(epi), igemm_kernel_mode3(epi),
                                igemm_kernel_wzp(epi), igemm_kernel_residual(epi) })
             if (k)
+                B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    for (int epi = 0; epi < kEpiVariants; ++epi)
+        for (bool wzp : { false, true })
+            for (IgemmBoxKernel k : { igemm_kernel_mode4(epi, wzp), igemm_kernel_mode5(epi, wzp) })
                 B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     if (device < 256)
         done[device].store(true, std::memory_order_release);

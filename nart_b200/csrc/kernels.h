@@ -129,7 +129,7 @@ int conv_igemm_supported(const ConvGeom &g, char *why, size_t why_len);
 int conv_igemm_create(
     const ConvGeom &g, const std::vector<int8_t> &w_s8 /* [k][c][r][s] */, const int32_t *bias,
     const uint32_t *mult, const int32_t *shift, ConvIgemmPlan **plan, bool a_row_swizzled = false,
-    int window = 0);
+    int window = 0, bool quads = false);
 // a_row_swizzled: the activation tensor has 32 channels, the kernel is r x 1 with no horizontal
 // stride or padding, and the tensor was written by conv_lower_rows_launch (halves swapped by ow bit 2); window: the
 // pixels of its 8-pixel windows that the original kernel row covers.

@@ -213,6 +213,18 @@ __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint32_t a_lo, uint32_t 
         ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same where the high words differ (the eight-row groups of A lie further apart)
+__device__ __forceinline__ void mma_i8_ab(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t a_hi, uint32_t b_hi, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\t"
+        "mov.b64 db, {%2, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(a_hi), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // The barrier gets one arrival when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar)
 {

@@ -1,0 +1,49 @@
+"""Convs that load a tile's activations once for all taps: against the CUDA-core kernel, which the other tests pin to the CPU
+restatement."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(c, k, r, s, h, w, n, seed, signed=False):
+    import torch
+    rng = np.random.default_rng(seed)
+    wt = rng.integers(-127, 128, (k, c, r, s)).astype(np.int8) if signed else rng.integers(0, 256, (k, c, r, s), dtype=np.uint8)
+    bias = rng.integers(-4096, 4097, k).astype(np.int32)
+    walpha = rng.uniform(0.001, 0.01, k).astype(np.float32)
+    q = dict(ialpha=0.02, walpha=walpha, oalpha=float(np.float32(0.02 * 74 * 0.0055 * 73 * np.sqrt(c * r * s) / (20 if signed else 45))))
+    q.update(dict(obits=7, signed=True) if signed else dict(izp=117, ozp=99))
+    x = torch.from_numpy(rng.integers(0, 256, (n, h, w, c), dtype=np.uint8)).cuda()
+    return wt, bias, x.view(torch.int8) if signed else x, q
+
+
+# (c, k, kernel (r, s), strides, pads, h, w, n): lines that fill a power of two with their ring and not, maps of one pixel more or
+# less than the tiles, planes of a strided window with one and two taps an axis, several channel chunks, an asymmetric window
+BOXES = [(64, 64, (3, 3), (1, 1), (1, 1), 56, 56, 9), (64, 48, (3, 3), (1, 1), (1, 1), 27, 35, 30), (32, 16, (3, 3), (1, 1), (1, 1), 17, 126, 8),
+         (32, 32, (3, 3), (1, 1), (1, 1), 16, 127, 9), (128, 128, (3, 3), (1, 1), (1, 1), 28, 30, 24), (96, 80, (3, 3), (2, 2), (1, 1), 33, 31, 40),
+         (16, 256, (3, 3), (1, 1), (0, 0), 10, 9, 60), (48, 96, (5, 3), (1, 2), (2, 1), 30, 29, 20), (160, 32, (2, 4), (2, 1), (1, 3), 21, 23, 30),
+         (64, 64, (1, 3), (1, 1), (0, 1), 3, 6, 200), (32, 64, (4, 4), (2, 2), (0, 2), 40, 62, 12)]
+
+
+@pytest.mark.parametrize("shape", BOXES)
+@pytest.mark.parametrize("kind", ["plain", "wzp", "signed"])
+@pytest.mark.parametrize("cut", ["0", "16x1", "64x2", "128x4"])
+def test_one_box_for_all_taps(monkeypatch, shape, kind, cut):
+    """The persistent kernel (cut 0) and the one-tile one, whole and split sums."""
+    import torch
+    from nart_b200 import ops
+    c, k, (r, s), st, pad, h, w, n = shape
+    wt, bias, x, q = _inputs(c, k, r, s, h, w, n, c + k + h, kind == "signed")
+    if kind == "wzp":
+        q["wzp"] = 90
+    args = dict(in_hw=(h, w), stride=st, pad=pad, relu=kind == "plain", **q)
+    want = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **args)(x)
+    monkeypatch.setenv("B200_IGEMM_SMALL", cut)
+    monkeypatch.setenv("B200_IGEMM_HALO", "1")
+    conv = ops.Conv2d(wt, bias, algo=ops.ALGO_IGEMM, **args)
+    for part in (x, x[:1]):
+        assert torch.equal(conv(part), want[:part.shape[0]]), conv.describe()
+        assert ops.device_status() == 0
+    assert cut == "0" or "one box for all taps" in conv.describe()
+    assert len(torch.unique(want)) > 16
