@@ -156,9 +156,14 @@ int encode(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims, const c
     if (!fn)
         return fail(B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     cuuint32_t estr[5] = { 1, 1, 1, 1, 1 };
-    CUresult r = fn(m, dtype, (cuuint32_t)rank, base, dims, strides_bytes, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = CUDA_SUCCESS;
+    for (int round = 0; round < 2; ++round) {
+        r = fn(m, dtype, (cuuint32_t)rank, base, dims, strides_bytes, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        int device = 0;
+        if (r != CUDA_ERROR_INVALID_CONTEXT || cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess)
+            break;      // else this is the thread's first call to CUDA: its context is current now
+    }
     if (r != CUDA_SUCCESS)
         return fail(B200_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d (rank %d, dims %llu %llu, box %u %u)",
                     (int)r, rank, (unsigned long long)dims[0], (unsigned long long)dims[1], box[0], box[1]);

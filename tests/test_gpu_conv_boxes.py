@@ -47,3 +47,22 @@ def test_one_box_for_all_taps(monkeypatch, shape, kind, cut):
         assert ops.device_status() == 0
     assert cut == "0" or "one box for all taps" in conv.describe()
     assert len(torch.unique(want)) > 16
+
+
+@pytest.mark.parametrize("c,k,ks", [(64, 64, 3), (24, 144, 1), (4, 64, 7)])
+def test_run_is_the_first_call_of_a_thread(c, k, ks):
+    """A thread that has called nothing of CUDA has no current context."""
+    import threading
+    import torch
+    from nart_b200 import ops
+    wt, bias, x, q = _inputs(c, k, ks, ks, 16, 16, 3, c)
+    args = dict(in_hw=(16, 16), stride=(1 if c > 4 else 2,) * 2, pad=(ks // 2,) * 2, relu=True, **q)
+    want, conv, got = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **args)(x), ops.Conv2d(wt, bias, **args), []
+    torch.cuda.synchronize()
+    y = torch.empty_like(want)
+    stream = torch.cuda.current_stream().cuda_stream
+    t = threading.Thread(target=lambda: got.append(ops.lib.b200_conv2d_run(conv._h, x.data_ptr(), 3, y.data_ptr(), stream)))
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert got == [0] and torch.equal(y, want)
