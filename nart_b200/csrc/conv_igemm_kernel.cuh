@@ -37,7 +37,7 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "conv_small.h"
+#include "conv_boxes.h"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 

@@ -227,13 +227,12 @@ struct ConvIgemmPlan {
         int cta_pair;
         bool halo;
         int m_tiles;
-        bool small_box;             // the small kernel with one box for all taps
         IgemmKernel kernel;
         IgemmBoxKernel box_kernel;
         dim3 grid;
         size_t smem;
         SmallMaps smaps;
-        SmallBoxArgs sargs;
+        SmallArgs sargs;
         IgemmMaps maps;
         IgemmBoxArgs args;
     };
@@ -726,8 +725,8 @@ void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
 {
     const ConvIgemmPlan::Launch *l = p->last_launch();      // the tiling depends on the batch of the run
     if (l && l->small) {
-        snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d slots=%d split=%d one tile per %s%s", l->sargs.bn, p->bk, l->sargs.slots, l->sargs.split,
-                 l->sargs.split > 1 ? "cluster" : "CTA", l->small_box ? ", one box for all taps" : "");
+        snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d slots=%d split=%d one tile per %s", l->sargs.bn, p->bk, l->sargs.slots, l->sargs.split,
+                 l->sargs.split > 1 ? "cluster" : "CTA");
         return;
     }
     const bool cta_pair = l && l->cta_pair;
@@ -820,6 +819,68 @@ static int encode_activations(const ConvIgemmPlan *p, const uint8_t *x, int n, i
     return B200_OK;
 }
 
+// Per axis: the least and the largest offset, in pixels of the parity, of the taps of one parity; false where there is none.
+static bool tap_span(int kernel, int stride, int pad, int parity, int *lo, int *hi)
+{
+    *lo = 1 << 20;
+    *hi = -(1 << 20);
+    for (int t = 0; t < kernel; ++t) {
+        const int d = t - pad, p = d & (stride - 1), o = (d - p) / stride;
+        if (p == parity) {
+            *lo = o < *lo ? o : *lo;
+            *hi = o > *hi ? o : *hi;
+        }
+    }
+    return *lo <= *hi;
+}
+
+HaloWindow::HaloWindow(int r_, int s_, int stride_h_, int stride_w_, int pad_h_, int pad_w_, int row_pixels, int width_)
+    : r(r_), s(s_), stride_h(stride_h_), stride_w(stride_w_), pad_h(pad_h_), pad_w(pad_w_), width(width_)
+{
+    int lo, hi;
+    for (int p = 0; p < stride_w; ++p)
+        if (tap_span(s, stride_w, pad_w, p, &lo, &hi) && hi - lo > ring_w)
+            ring_w = hi - lo;
+    for (int p = 0; p < stride_h; ++p)
+        if (tap_span(r, stride_h, pad_h, p, &lo, &hi) && hi - lo > ring_h)
+            ring_h = hi - lo;
+    if (row_pixels > 0)
+        ring_w = row_pixels - 1;
+}
+
+void halo_planes(const HaloWindow &win, int group, HaloTiles *out)
+{
+    HaloTiles &h = *out;
+    h.planes = 0;
+    h.span = 0;
+    h.tap_row = win.stride_h * win.s;
+    h.tap_col = win.stride_w;
+    // the first tap of a parity along one axis, and how many follow it a stride apart
+    auto first_tap = [](int kernel, int stride, int pad, int parity) {
+        int t = 0;
+        while (t < kernel && ((t - pad) & (stride - 1)) != parity)
+            ++t;
+        return t;
+    };
+    for (int ph = 0; ph < win.stride_h; ++ph)
+        for (int pw = 0; pw < win.stride_w; ++pw) {
+            int y0, y1, x0, x1;
+            if (!tap_span(win.r, win.stride_h, win.pad_h, ph, &y0, &y1) || !tap_span(win.s, win.stride_w, win.pad_w, pw, &x0, &x1))
+                continue;
+            const int pl = h.planes++, r0 = first_tap(win.r, win.stride_h, win.pad_h, ph), s0 = first_tap(win.s, win.stride_w, win.pad_w, pw);
+            h.dx[pl] = x0;
+            h.dy[pl] = y0;
+            h.rows[pl] = h.pitch * (h.th + y1 - y0);
+            h.parity[pl] = (uint8_t)(ph * 2 + pw);
+            h.taps_h[pl] = (win.r - r0 + win.stride_h - 1) / win.stride_h;
+            h.taps_w[pl] = (win.s - s0 + win.stride_w - 1) / win.stride_w;
+            h.tap0[pl] = r0 * win.s + s0;
+            // an operand is sixteen groups of eight rows from its first one on (of `width` pixels each)
+            const int last = (h.taps_h[pl] - 1) * h.pitch + h.taps_w[pl] - 1;
+            h.span = std::max(h.span, std::max(h.rows[pl], last + 15 * group + 8 + win.width - 1));
+        }
+}
+
 // The same for the boxes of HaloTiles, a map per plane.
 static int encode_boxes(const ConvIgemmPlan *p, const uint8_t *x, int n, const HaloTiles &h, CUtensorMap (&maps)[4])
 {
@@ -865,7 +926,7 @@ static int encode_weights(const ConvIgemmPlan *p, const int8_t *w, int rows, int
 static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, int *status, int tw, int th, int tn, const ConvSum *ws, ConvIgemmPlan::Launch &l)
 {
     const ConvGeom &g = p->g;
-    SmallBoxArgs &a = l.sargs;
+    SmallArgs &a = l.sargs;
     memset(&a, 0, sizeof(a));
     a.tiles_w = (g.ow + tw - 1) / tw;
     a.tiles_h = (g.oh + th - 1) / th;
@@ -873,44 +934,16 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.cchunks = (p->cpad + p->bk - 1) / p->bk;
     a.cpad = p->cpad;
     a.last_steps = (p->cpad - (a.cchunks - 1) * p->bk) / 32;
-    a.kblocks = g.r * p->taps_w * a.cchunks;
+    a.kblocks = g.r * g.s * a.cchunks;
     a.bk = p->bk;
-    a.quads = p->quads;
-    a.a_pitch = p->quads ? 16 : p->bk;
-    // One box for all taps only where there is no other way: with a box per tap the k-blocks are on their way while the first ones
-    // are multiplied (3x3 64 -> 64 on 56 x 56: 4.3 us, 4.9 with one box).
-    HaloTiles halo;
-    const char *he = getenv("B200_IGEMM_HALO");       // tuning aid: 1 wherever possible
-    const HaloWindow win(g.r, p->taps_w, g.stride_h, g.stride_w, g.pad_h, g.pad_w, p->quads ? g.s : 0, p->quads ? p->bk / 16 : 1);
-    const bool can_halo = (p->quads || (he && atoi(he) == 1)) && !p->a_wide && halo_tiles(win, g.ow, g.oh, &halo);
-    const int halo_w = can_halo ? (g.ow + halo.tw - 1) / halo.tw : 0, halo_h = can_halo ? (g.oh + halo.th - 1) / halo.th : 0;
-    bool use_halo = false;
     if (p->small_bn && p->small_split <= a.kblocks) {              // tuning aid
         a.bn = p->small_bn;
         a.split = p->small_split;
-        use_halo = can_halo;
-    } else {
-        double cost = 0.0;
-        bool small = conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, 0, 0, &cost, &a.bn, &a.split) && !p->quads;
-        if (can_halo) {
-            int box_rows = 0;
-            for (int i = 0; i < halo.planes; ++i)
-                box_rows += p->quads ? halo.rows[i] / halo.pitch : halo.rows[i];
-            use_halo = conv_small_pick(halo_w * halo_h * n, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, g.r * p->taps_w, box_rows, &cost, &a.bn, &a.split);
-            small = small || use_halo;
-        }
-        if (!small)
-            return B200_OK;
-    }
-    int tiles = m_tiles;
-    if (use_halo) {
-        a.halo = halo;
-        a.tiles_w = halo_w;
-        a.tiles_h = halo_h;
-        tiles = halo_w * halo_h * n;
+    } else if (!conv_small_pick(m_tiles, g.k, a.kblocks, a.bk, g.wzp_d != 0, p->bn, &a.bn, &a.split)) {
+        return B200_OK;
     }
     a.n = n; a.oh = g.oh; a.ow = g.ow; a.cout = g.k;
-    a.r = g.r; a.s = p->taps_w; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
+    a.r = g.r; a.s = g.s; a.pad_h = g.pad_h; a.pad_w = g.pad_w; a.stride_h = g.stride_h; a.stride_w = g.stride_w;
     for (a.tw_sh = 0; (1 << a.tw_sh) < tw; ++a.tw_sh) {}
     for (a.th_sh = 0; (1 << a.th_sh) < th; ++a.th_sh) {}
     a.tn = tn;
@@ -926,7 +959,7 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.y = y;
     a.status = status;
     a.next_ro = p->next_ro; a.next_ro_bytes = p->next_ro_bytes;
-    if (ws && g.k % 16 == 0 && !g.act_signed && !use_halo) {         // (other channel counts leave through staged rows)
+    if (ws && g.k % 16 == 0 && !g.act_signed) {         // (other channel counts leave through staged rows)
         const int ci = ws->conv_input, other = 1 - ci;
         const EltwiseArgs &e = *ws->elt;
         a.res = ws->res;
@@ -936,20 +969,16 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
         a.r_s0 = e.s0; a.r_ozp = e.ozp; a.r_lo = e.relu_lo;
         l.summed = true;
     }
-    l.small_box = use_halo;
-    const size_t smem = conv_small_smem(a, use_halo, g.act_signed != 0);
+    const size_t smem = conv_small_smem(a, g.act_signed != 0);
     if (smem > 227 * 1024)
         return B200_OK;
-    if (use_halo)
-        B200_TRY(encode_boxes(p, x, n, halo, l.smaps.a));
-    else
-        B200_TRY(encode_activations(p, x, n, tw, th, tn, l.smaps.a));
+    B200_TRY(encode_activations(p, x, n, tw, th, tn, l.smaps.a));
     B200_TRY(encode_weights(p, p->w_dev, p->kpad, a.bn, &l.smaps.b));
     l.smaps.ones = l.smaps.b;
     if (p->ones_dev)
         B200_TRY(encode_weights(p, p->ones_dev, 16, 16, &l.smaps.ones));
     l.smem = smem;
-    l.m_tiles = tiles;
+    l.m_tiles = m_tiles;
     l.small = true;
     return B200_OK;
 }
@@ -986,7 +1015,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         B200_TRY(conv_igemm_warm());
         p->attr_set = true;
     }
-    if (!res && p->small_ok && !(p->pair_ok && p->pair_want == 1)) {
+    if (!res && p->small_ok && !p->quads && !(p->pair_ok && p->pair_want == 1)) {
         B200_TRY(build_small(p, x, n, y, a.status, a.tw, a.th, a.tn, ws, l));
         if (l.small)
             return B200_OK;
@@ -1179,7 +1208,7 @@ int conv_igemm_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, cud
     if (summed)
         *summed = l.small && l.summed;
     if (l.small)
-        return conv_small_launch(l.smaps, l.sargs, l.small_box, l.m_tiles, l.smem, bytes, st);
+        return conv_small_launch(l.smaps, l.sargs, l.m_tiles, l.smem, bytes, st);
     const bool two_rings = l.halo ? l.args.stages >= 4 : !l.cta_pair && !res && p->g.wzp_d == 0 && !p->pair && p->rings == 2;
     if (l.halo)
         return launch_kernel(l.box_kernel, l.grid, dim3(two_rings ? kThreads2 : kThreads), l.smem, st, bytes, 1, l.maps, l.args);

@@ -15,10 +15,6 @@
 // epilogue is the persistent kernel's arithmetic (EpiForm); requantizing channel by channel with a shift each, as this kernel
 // first did, took 0.9 us per 16 channels of a tile, most of a 64-channel launch's time.
 #include <stdlib.h>
-#include <string.h>
-
-#include <algorithm>
-#include <type_traits>
 
 #include "common.cuh"
 #include "conv_igemm_kernel.cuh"
@@ -34,7 +30,6 @@ constexpr int kSmallEpiThreads = 256;
 constexpr int kSmallThreads = 64 + kSmallEpiThreads;
 constexpr int kSmallM = 128;            // pixels per tile
 constexpr int kSmallSlots = 16;
-constexpr int kSmallBoxes = 8;          // boxes of activations in flight (HaloTiles)
 constexpr int kSmallClsCols = 4096;     // border classes x channels that are staged in shared memory; more are read in place
 
 constexpr int kErrSmallProducer = 0x201, kErrSmallFull = 0x202, kErrSmallEpilogue = 0x203;
@@ -42,14 +37,10 @@ constexpr int kErrSmallProducer = 0x201, kErrSmallFull = 0x202, kErrSmallEpilogu
 struct SmallLayout {
     uint32_t b, b_tile, red, xred, mult, shift, off, stage, stage_pitch, bars, tmem_slot, abort_flag, total;
 };
-template <typename Args>
-__host__ __device__ inline SmallLayout small_layout(const Args &g)
+__host__ __device__ inline SmallLayout small_layout(const SmallArgs &g)
 {
-    constexpr bool box = std::is_same<Args, SmallBoxArgs>::value;
     SmallLayout L;
     uint32_t o = (uint32_t)g.slots * kSmallM * g.bk;
-    if constexpr (box)
-        o = (uint32_t)g.a_slots * g.a_slot_bytes;
     L.b = o;
     L.b_tile = ((uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk + 1023u) & ~1023u;
     o += g.slots * L.b_tile;
@@ -69,8 +60,8 @@ __host__ __device__ inline SmallLayout small_layout(const Args &g)
     L.stage = o;
     L.stage_pitch = (uint32_t)(g.bn / g.split) + 16;
     o += g.cout % 16 != 0 ? kSmallM * L.stage_pitch : 0;
-    L.bars = o;                                             // full[slots], empty[slots], accumulator, empty boxes
-    o += (2 * kSmallSlots + 1 + (box ? kSmallBoxes : 0)) * 8;
+    L.bars = o;                                             // full[slots], empty[slots], accumulator
+    o += (2 * kSmallSlots + 1) * 8;
     L.tmem_slot = o;
     o += 8;
     L.abort_flag = o;
@@ -87,43 +78,6 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v)
 {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-
-// A walk over the k-blocks of HaloTiles: chunk by chunk, plane by plane, tap by tap; by counters, as every role walks it in step
-// with uniform registers.
-struct HaloWalk {
-    int chunk, pl, i, j, tap, pixel;        // pixel: of the box, where the tap's operand begins
-    __device__ __forceinline__ void open(const HaloTiles &h, int plane)
-    {
-        pl = plane;
-        i = j = pixel = 0;
-        tap = h.tap0[plane];
-    }
-    __device__ __forceinline__ bool next(const HaloTiles &h)        // true: the next k-block is another box's
-    {
-        if (++j < h.taps_w[pl]) {
-            tap += h.tap_col;
-            ++pixel;
-            return false;
-        }
-        j = 0;
-        if (++i < h.taps_h[pl]) {
-            tap = h.tap0[pl] + i * h.tap_row;
-            pixel = i * h.pitch;
-            return false;
-        }
-        const bool last = pl + 1 == h.planes;
-        chunk += last ? 1 : 0;
-        open(h, last ? 0 : pl + 1);
-        return true;
-    }
-    __device__ __forceinline__ void start(const HaloTiles &h, int kb, int taps)
-    {
-        chunk = kb / taps;
-        open(h, 0);
-        for (kb -= chunk * taps; kb > 0; --kb)
-            next(h);
-    }
-};
 
 // Where a CTA's tables lie (shared addresses), and this thread's border class's offsets.
 struct SmallTables {
@@ -184,9 +138,9 @@ __device__ __forceinline__ void store_channels(const uint32_t (&acc)[N], const S
     }
 }
 
-// SUM: the instantiation that also forms a residual add (ConvSum); BOX: the one for HaloTiles.  The others carry none of that code.
-template <bool SUM, bool BOX>
-__global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_constant__ SmallMaps maps, const __grid_constant__ std::conditional_t<BOX, SmallBoxArgs, SmallArgs> g)
+// SUM: the instantiation that also forms a residual add (ConvSum); the other one carries none of that code.
+template <bool SUM>
+__global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_constant__ SmallMaps maps, const __grid_constant__ SmallArgs g)
 {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
@@ -198,7 +152,6 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
     auto full_bar = [&](int s) { return bars + 8u * s; };
     auto empty_bar = [&](int s) { return bars + 8u * (kSmallSlots + s); };
     const uint32_t acc_bar = bars + 8u * (2 * kSmallSlots);
-    auto box_bar = [&](int s) { return acc_bar + 8u + 8u * s; };       // the box's MMAs are done
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem + L.tmem_slot);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.abort_flag);
 
@@ -219,9 +172,6 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
             mbar_init(empty_bar(s), 1);
         }
         mbar_init(acc_bar, 1);
-        if constexpr (BOX)
-            for (int s = 0; s < g.a_slots; ++s)
-                mbar_init(box_bar(s), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -243,73 +193,6 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
 
     if (warp == 0) {
         // ================= TMA =================
-        if constexpr (BOX) {
-            const uint32_t b_bytes = (uint32_t)(g.bn + (g.wzp_d ? 16 : 0)) * g.bk;
-            // the k-blocks chunk by chunk, and of a chunk its taps plane by plane; the bytes of a box are counted on the first of
-            // its k-blocks
-            const HaloTiles &h = g.halo;
-            HaloWalk first;
-            first.start(h, kb0, g.r * g.s);
-            auto load_b = [&](int slot, const HaloWalk &w, bool opens) {
-                const uint32_t b_dst = base + L.b + slot * L.b_tile;
-                const int kc = w.tap * g.cpad + w.chunk * g.bk;
-                const uint32_t tx = b_bytes + (opens ? (uint32_t)(h.rows[w.pl] * g.a_pitch) : 0u);
-                if (elect_one()) {
-                    mbar_expect_tx(full_bar(slot), tx);
-                    tma_load_2d(b_dst, &maps.b, full_bar(slot), kc, k0);
-                    if (g.wzp_d)
-                        tma_load_2d(b_dst + g.bn * g.bk, &maps.ones, full_bar(slot), kc, 0);
-                }
-                __syncwarp();
-            };
-            HaloWalk w = first;
-            bool opens = true;
-            for (int kb = kb0, slot = 0; slot < g.slots && kb < kb1; ++kb, ++slot) {
-                load_b(slot, w, opens);
-                opens = w.next(h);
-            }
-            pdl_wait();
-            w = first;
-            opens = true;
-            int slot = 0, box = 0, boxes = 0;
-            uint32_t phase = 1, box_phase = 1;
-            bool ok = true;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                if (kb >= kb0 + g.slots) {
-                    ok = mbar_wait_warp(empty_bar(slot), phase, abort_flag);
-                    if (ok)
-                        load_b(slot, w, opens);
-                }
-                if (opens && boxes >= g.a_slots)
-                    ok = ok && mbar_wait_warp(box_bar(box), box_phase, abort_flag);
-                if (!ok) {
-                    if (lane == 0)
-                        atomicCAS(g.status, 0, kErrSmallProducer);
-                    *abort_flag = 1;
-                    break;
-                }
-                if (opens) {
-                    const int x0 = twi * h.tw + h.dx[w.pl], y0 = thi * h.th + h.dy[w.pl];
-                    if (elect_one()) {
-                        if (g.quads)
-                            tma_load_3d(base + (uint32_t)box * g.a_slot_bytes, &maps.a[w.pl], full_bar(slot), x0 * 2, y0, tni);
-                        else
-                            tma_load_4d(base + (uint32_t)box * g.a_slot_bytes, &maps.a[w.pl], full_bar(slot), w.chunk * g.bk, x0, y0, tni);
-                    }
-                    __syncwarp();
-                    ++boxes;
-                    if (++box == g.a_slots) {
-                        box = 0;
-                        box_phase ^= 1;
-                    }
-                }
-                opens = w.next(h);
-                if (++slot == g.slots) {
-                    slot = 0;
-                    phase ^= 1;
-                }
-            }
-        } else {
         // in order: the weights of the first `slots` k-blocks (constant, the launch before this one does not matter to them),
         // and behind its wait the k-blocks one by one; uniform loops around elect_one(), see there
         {
@@ -373,20 +256,13 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 }
             }
         }
-        }
         __syncwarp();
         pdl_trigger();
     } else if (warp == 1) {
         // ================= MMA =================
         const uint64_t adesc0 = make_smem_desc(base, g.bk), bdesc0 = make_smem_desc(base + L.b, g.bk);
         const uint32_t desc_hi = (uint32_t)(adesc0 >> 32);
-        HaloWalk w;
-        uint32_t a_hi = desc_hi;
-        if constexpr (BOX) {
-            w.start(g.halo, kb0, g.r * g.s);
-            a_hi = halo_desc_hi(desc_hi, 8, g.a_pitch, g.quads);
-        }
-        int slot = 0, chunk = kb0 % g.cchunks, box = 0;
+        int slot = 0, chunk = kb0 % g.cchunks;
         uint32_t phase = 0, accumulate = 0;
         bool ok = true;
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -398,42 +274,22 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 break;
             }
             tc_fence_after();
-            uint32_t a_lo = (uint32_t)adesc0 + slot * (a_tile >> 4);
-            const uint32_t b_lo = (uint32_t)bdesc0 + slot * (L.b_tile >> 4);
-            bool box_done = false;
-            int at = chunk;
-            if constexpr (BOX) {
-                a_lo = (uint32_t)adesc0 + (((uint32_t)box * g.a_slot_bytes + (uint32_t)(w.pixel * g.a_pitch)) >> 4);
-                at = w.chunk;
-                box_done = w.next(g.halo);
-            }
-            const int ksteps = at == g.cchunks - 1 ? g.last_steps : g.bk / 32;
+            const uint32_t a_lo = (uint32_t)adesc0 + slot * (a_tile >> 4), b_lo = (uint32_t)bdesc0 + slot * (L.b_tile >> 4);
+            const int ksteps = chunk == g.cchunks - 1 ? g.last_steps : g.bk / 32;
             chunk = chunk == g.cchunks - 1 ? 0 : chunk + 1;
             if (elect_one()) {
-                auto mma = [&](int k, uint32_t acc) {
-                    if constexpr (BOX)
-                        mma_i8_ab(tmem_base, a_lo + 2 * k, b_lo + 2 * k, a_hi, desc_hi, g.idesc, acc);
-                    else
-                        mma_i8(tmem_base, a_lo + 2 * k, b_lo + 2 * k, desc_hi, g.idesc, acc);
-                };
-                mma(0, accumulate);
+                mma_i8(tmem_base, a_lo, b_lo, desc_hi, g.idesc, accumulate);
                 if (ksteps >= 2)
-                    mma(1, 1);
+                    mma_i8(tmem_base, a_lo + 2, b_lo + 2, desc_hi, g.idesc, 1);
                 if (ksteps >= 3)
-                    mma(2, 1);
+                    mma_i8(tmem_base, a_lo + 4, b_lo + 4, desc_hi, g.idesc, 1);
                 if (ksteps == 4)
-                    mma(3, 1);
+                    mma_i8(tmem_base, a_lo + 6, b_lo + 6, desc_hi, g.idesc, 1);
                 if (kb + g.slots < kb1)
                     mma_commit(empty_bar(slot));
-                if (BOX && box_done)
-                    mma_commit(box_bar(box));
             }
             __syncwarp();
             accumulate = 1;
-            if constexpr (BOX) {
-                if (box_done)
-                    box = box + 1 == g.a_slots ? 0 : box + 1;
-            }
             if (++slot == g.slots) {
                 slot = 0;
                 phase ^= 1;
@@ -449,23 +305,9 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
     const int row = quarter * 32 + lane;
     const int bnl = g.bn / split;                       // channels this CTA finishes
     const bool off_staged = g.n_cls * g.bn <= kSmallClsCols;
-    // output pixel of an accumulator row
-    auto pixel = [&](int prow, int &px, int &py, int &pn) {
-        if constexpr (BOX) {
-            const int lh = prow / g.halo.pitch, lw = prow - lh * g.halo.pitch;
-            px = twi * g.halo.tw + lw;
-            py = thi * g.halo.th + lh;
-            pn = tni;
-            return lw < g.halo.tw && lh < g.halo.th && px < g.ow && py < g.oh;
-        } else {
-            px = (twi << g.tw_sh) + (prow & ((1 << g.tw_sh) - 1));
-            py = (thi << g.th_sh) + ((prow >> g.tw_sh) & ((1 << g.th_sh) - 1));
-            pn = tni * g.tn + (prow >> (g.tw_sh + g.th_sh));
-            return px < g.ow && py < g.oh && pn < g.n;
-        }
-    };
-    int ow, oh, img;
-    const bool pix_valid = pixel(row, ow, oh, img);
+    const int lw = row & ((1 << g.tw_sh) - 1), lh = (row >> g.tw_sh) & ((1 << g.th_sh) - 1), ln = row >> (g.tw_sh + g.th_sh);
+    const int ow = (twi << g.tw_sh) + lw, oh = (thi << g.th_sh) + lh, img = tni * g.tn + ln;
+    const bool pix_valid = ow < g.ow && oh < g.oh && img < g.n;
     const size_t at = (((size_t)img * g.oh + oh) * g.ow + ow) * g.cout + k0;
     const EpiConsts ec = { g.ozp, g.qmax, g.relu_lo, g.ushift, g.rnd_hi, (float)g.ozp + 0.5f, g.out_flip,
                            g.r_m[0], g.r_add[0], g.r_b[0], g.r_m[1], g.r_add[1], g.r_b[1], g.r_s0, g.r_ozp, g.r_lo };
@@ -580,9 +422,8 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
                 if (!((valid >> pr) & 1))
                     continue;
                 const int prow = quarter * 32 + pr;
-                int px, py, pn;
-                pixel(prow, px, py, pn);
-                uint8_t *dst = g.y + (((size_t)pn * g.oh + py) * g.ow + px) * g.cout + k0 + c1;
+                const int plw = prow & ((1 << g.tw_sh) - 1), plh = (prow >> g.tw_sh) & ((1 << g.th_sh) - 1), pln = prow >> (g.tw_sh + g.th_sh);
+                uint8_t *dst = g.y + (((size_t)(tni * g.tn + pln) * g.oh + (thi << g.th_sh) + plh) * g.ow + (twi << g.tw_sh) + plw) * g.cout + k0 + c1;
                 const uint32_t src = base + L.stage + (uint32_t)prow * L.stage_pitch;
                 copy_row(dst, n, lane & (lanes - 1), lanes, [&](int off) { return lds1(src + off); });
             }
@@ -598,102 +439,15 @@ __global__ void __launch_bounds__(kSmallThreads) conv_small_kernel(const __grid_
 
 }  // namespace
 
-// Per axis: the least and the largest offset, in pixels of the parity, of the taps of one parity; false where there is none.
-static bool tap_span(int kernel, int stride, int pad, int parity, int *lo, int *hi)
-{
-    *lo = 1 << 20;
-    *hi = -(1 << 20);
-    for (int t = 0; t < kernel; ++t) {
-        const int d = t - pad, p = d & (stride - 1), o = (d - p) / stride;
-        if (p == parity) {
-            *lo = o < *lo ? o : *lo;
-            *hi = o > *hi ? o : *hi;
-        }
-    }
-    return *lo <= *hi;
-}
-
-HaloWindow::HaloWindow(int r_, int s_, int stride_h_, int stride_w_, int pad_h_, int pad_w_, int row_pixels, int width_)
-    : r(r_), s(s_), stride_h(stride_h_), stride_w(stride_w_), pad_h(pad_h_), pad_w(pad_w_), width(width_)
-{
-    int lo, hi;
-    for (int p = 0; p < stride_w; ++p)
-        if (tap_span(s, stride_w, pad_w, p, &lo, &hi) && hi - lo > ring_w)
-            ring_w = hi - lo;
-    for (int p = 0; p < stride_h; ++p)
-        if (tap_span(r, stride_h, pad_h, p, &lo, &hi) && hi - lo > ring_h)
-            ring_h = hi - lo;
-    if (row_pixels > 0)
-        ring_w = row_pixels - 1;
-}
-
-void halo_planes(const HaloWindow &win, int group, HaloTiles *out)
-{
-    HaloTiles &h = *out;
-    h.planes = 0;
-    h.span = 0;
-    h.tap_row = win.stride_h * win.s;
-    h.tap_col = win.stride_w;
-    // the first tap of a parity along one axis, and how many follow it a stride apart
-    auto first_tap = [](int kernel, int stride, int pad, int parity) {
-        int t = 0;
-        while (t < kernel && ((t - pad) & (stride - 1)) != parity)
-            ++t;
-        return t;
-    };
-    for (int ph = 0; ph < win.stride_h; ++ph)
-        for (int pw = 0; pw < win.stride_w; ++pw) {
-            int y0, y1, x0, x1;
-            if (!tap_span(win.r, win.stride_h, win.pad_h, ph, &y0, &y1) || !tap_span(win.s, win.stride_w, win.pad_w, pw, &x0, &x1))
-                continue;
-            const int pl = h.planes++, r0 = first_tap(win.r, win.stride_h, win.pad_h, ph), s0 = first_tap(win.s, win.stride_w, win.pad_w, pw);
-            h.dx[pl] = x0;
-            h.dy[pl] = y0;
-            h.rows[pl] = h.pitch * (h.th + y1 - y0);
-            h.parity[pl] = (uint8_t)(ph * 2 + pw);
-            h.taps_h[pl] = (win.r - r0 + win.stride_h - 1) / win.stride_h;
-            h.taps_w[pl] = (win.s - s0 + win.stride_w - 1) / win.stride_w;
-            h.tap0[pl] = r0 * win.s + s0;
-            // an operand is sixteen groups of eight rows from its first one on (of `width` pixels each)
-            const int last = (h.taps_h[pl] - 1) * h.pitch + h.taps_w[pl] - 1;
-            h.span = std::max(h.span, std::max(h.rows[pl], last + 15 * group + 8 + win.width - 1));
-        }
-}
-
-bool halo_tiles(const HaloWindow &win, int ow, int oh, HaloTiles *out)
-{
-    HaloTiles &h = *out;
-    memset(&h, 0, sizeof(h));
-    if (!win.fits())
-        return false;
-    // the fewest tiles, and of those the fewest pixels to load
-    long long best = -1;
-    for (int tw = 1; tw <= ow && tw <= kSmallM; ++tw) {
-        const int pitch = tw + win.ring_w, th_max = (kSmallM - tw) / pitch + 1, cols = (ow + tw - 1) / tw;
-        const int th0 = th_max < oh ? th_max : oh, lines = (oh + th0 - 1) / th0, th = (oh + lines - 1) / lines;
-        const long long tiles = (long long)cols * lines, cost = tiles * 100000 + pitch * (th + win.ring_h);
-        if (pitch <= 128 && (best < 0 || cost < best)) {
-            best = cost;
-            h.tw = tw;
-            h.th = th;
-            h.pitch = pitch;
-        }
-    }
-    if (best < 0)
-        return false;
-    halo_planes(win, 8, &h);
-    return true;
-}
-
-bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int bn_p, int taps, int box_rows, double *cost_out, int *bn_out, int *split_out)
+bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int bn_p, int *bn_out, int *split_out)
 {
     // Microseconds on this GPU, fitted to sweeps over both kernels' tilings of ResNet-50's and MobileNetV2's layers at
     // batches 1 to 32.  What counts: a k-block's rows through the SM's TMA unit (0.25 us for 128 rows of 64 bytes, 0.37 of
     // 128), the epilogue behind the last MMA, and the cluster's exchange of partial sums.
     const int sms = sm_count(), extra = wzp ? 16 : 0, k16 = (k + 15) / 16 * 16;
     const double row = 0.13 + 0.0019 * bk;
-    double best = *cost_out;
-    if (best == 0.0) {   // the persistent kernel: a round's loads and the epilogue of the round before it overlap
+    double best;
+    {   // the persistent kernel: a round's loads and the epilogue of the round before it overlap
         const int rounds = (m_tiles * ((k + bn_p - 1) / bn_p) + sms - 1) / sms;
         const double load = kblocks * row * (bn_p > 128 ? 1.4 : 1.1), epi = 0.008 * bn_p;
         best = 3.4 + rounds * (load > epi ? load : epi) + (load > epi ? epi : load);
@@ -707,11 +461,10 @@ bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int bn_p
             const int ctas = tiles * split, kb = (kblocks + split - 1) / split;
             // two CTAs share an SM where both fit its shared memory; clusters of four and eight leave SMs of a GPC over
             const int slots = kb < 4 ? kb : 4;
-            const bool two = split == 1 && (size_t)slots * (kSmallM + bn + extra) * bk <= 104 * 1024;
+            const bool two = split == 1 && slots * (kSmallM + bn + extra) * bk <= 104 * 1024;
             if (ctas > (split == 8 ? sms * 2 / 3 : split == 4 ? sms * 7 / 8 : two ? 2 * sms : sms))
                 continue;
-            const double load = box_rows == 0 ? kb * (row + 0.0003 * (bn + extra))
-                : (kb + taps - 1) / taps * box_rows * row / kSmallM + kb * (0.06 + 0.0003 * (bn + extra));
+            const double load = kb * (row + 0.0003 * (bn + extra));
             const double epi = split > 1 ? 0.6 + 0.012 * bn + 0.7 * ctas / sms + (split == 8 ? 0.5 : 0.0) : bn > 32 ? 0.0125 * (bn - 32) : 0.0;
             const double cost = ctas > sms ? 3.2 + (load + epi) * ctas / sms : 2.3 + load + epi;
             if (cost < best) {
@@ -722,21 +475,10 @@ bool conv_small_pick(int m_tiles, int k, int kblocks, int bk, bool wzp, int bn_p
             }
         }
     }
-    *cost_out = best;
     return small;
 }
 
-template <typename Args>
-static size_t fit_slots(Args &a)
-{
-    while (a.slots > 4 && small_layout(a).total > 110 * 1024)       // two CTAs per SM: this launch's and the next one's
-        --a.slots;
-    while (a.slots > 1 && small_layout(a).total > 227 * 1024)
-        --a.slots;
-    return small_layout(a).total;
-}
-
-size_t conv_small_smem(SmallBoxArgs &a, bool box, bool act_signed)
+size_t conv_small_smem(SmallArgs &a, bool act_signed)
 {
     const int kb = (a.kblocks + a.split - 1) / a.split, n = a.bn + (a.wzp_d ? 16 : 0);
     a.idesc = (2u << 4) | ((act_signed ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
@@ -744,34 +486,26 @@ size_t conv_small_smem(SmallBoxArgs &a, bool box, bool act_signed)
     while (a.tmem_cols < (uint32_t)n)
         a.tmem_cols <<= 1;
     a.slots = kb < kSmallSlots ? kb : kSmallSlots;
-    if (box) {
-        const int taps = a.r * a.s, units = (kb + taps - 1) / taps * a.halo.planes + 1;
-        a.a_slot_bytes = ((uint32_t)(a.halo.span * a.a_pitch) + 1023u) & ~1023u;
-        a.a_slots = units < kSmallBoxes ? units : kSmallBoxes;
-        while (a.a_slots > 2 && (uint32_t)a.a_slots * a.a_slot_bytes > 64 * 1024)
-            --a.a_slots;
-    }
+    while (a.slots > 4 && small_layout(a).total > 110 * 1024)       // two CTAs per SM: this launch's and the next one's
+        --a.slots;
+    while (a.slots > 1 && small_layout(a).total > 227 * 1024)
+        --a.slots;
     // A CTA waits for tensor memory (512 columns an SM) while its cluster waits for it, so CTAs of clusters must never fill an
     // SM's columns against each other: two clusters could each hold what the other's peer waits for.  Three CTAs fit an
     // SM's registers, and 128 columns each fit.  Those of 256 (a window-sum column beside 128 channels) ask for more than half
     // of the shared memory, so that an SM holds one of them at most.  (CTAs without a cluster give theirs back by themselves.)
-    const size_t total = box ? fit_slots(a) : fit_slots(static_cast<SmallArgs &>(a)), half_sm = 116 * 1024;
+    const size_t total = small_layout(a).total, half_sm = 116 * 1024;
     return a.split > 1 && a.tmem_cols > 128 && total < half_sm ? half_sm : total;
 }
 
-int conv_small_launch(const SmallMaps &maps, const SmallBoxArgs &a, bool box, int m_tiles, size_t smem, size_t bytes, cudaStream_t st)
+int conv_small_launch(const SmallMaps &maps, const SmallArgs &a, int m_tiles, size_t smem, size_t bytes, cudaStream_t st)
 {
-    const dim3 grid((unsigned)(m_tiles * a.n_tiles_n * a.split));
-    if (box)
-        return launch_kernel(conv_small_kernel<false, true>, grid, dim3(kSmallThreads), smem, st, bytes, a.split, maps, a);
-    return launch_kernel(a.res ? conv_small_kernel<true, false> : conv_small_kernel<false, false>, grid, dim3(kSmallThreads), smem, st, bytes, a.split, maps,
-                         static_cast<const SmallArgs &>(a));
+    return launch_kernel(a.res ? conv_small_kernel<true> : conv_small_kernel<false>, dim3((unsigned)(m_tiles * a.n_tiles_n * a.split)), dim3(kSmallThreads), smem, st, bytes, a.split, maps, a);
 }
 
 int conv_small_warm()
 {
-    B200_CUDA_TRY(cudaFuncSetAttribute(conv_small_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    for (auto k : { conv_small_kernel<false, false>, conv_small_kernel<true, false> })
+    for (auto k : { conv_small_kernel<false>, conv_small_kernel<true> })
         B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     return B200_OK;
 }
