@@ -542,7 +542,9 @@ int b200_case_prepare(b200_case_t *cs, int32_t max_batch)
                     rev = zigzag ? 1 : 0;
                 if (op.conv->igemm)
                     conv_igemm_set_reverse(op.conv->igemm, rev);
-                else
+                if (op.conv->grouped)
+                    conv_igemm_set_reverse(op.conv->grouped, rev);
+                if (!op.conv->igemm)
                     rev = 0;
             } else if (op.kind != OpKind::Eltwise) {
                 rev = 0;
@@ -557,7 +559,12 @@ int b200_case_prepare(b200_case_t *cs, int32_t max_batch)
     {
         const char *e = getenv("B200_CASE_PREFETCH");
         const bool on = !(e && atoi(e) == 0);
-        ConvIgemmPlan *prev = nullptr;
+        const b200_conv *prev = nullptr;
+        auto set_next = [&](const uint8_t *w, size_t bytes) {
+            conv_igemm_set_next_readonly(prev->igemm, w, bytes);
+            if (prev->grouped)
+                conv_igemm_set_next_readonly(prev->grouped, w, bytes);
+        };
         for (auto &op : cs->ops) {
             if (op.skipped || op.kind != OpKind::Conv || !op.conv->igemm)
                 continue;
@@ -565,13 +572,13 @@ int b200_case_prepare(b200_case_t *cs, int32_t max_batch)
                 const uint8_t *w = nullptr;
                 size_t bytes = 0;
                 if (on)
-                    conv_igemm_weights(op.conv->igemm, &w, &bytes);
-                conv_igemm_set_next_readonly(prev, w, bytes);
+                    conv_igemm_weights(conv_runs_grouped(op.conv, nullptr, cs->max_batch) ? op.conv->grouped : op.conv->igemm, &w, &bytes);
+                set_next(w, bytes);
             }
-            prev = op.conv->igemm;
+            prev = op.conv;
         }
         if (prev)
-            conv_igemm_set_next_readonly(prev, nullptr, 0);
+            set_next(nullptr, 0);
     }
     cs->prepared = true;
     return B200_OK;
@@ -1147,9 +1154,10 @@ int b200_case_launch_count(const b200_case_t *cs, int32_t *launches)
         return fail(B200_ERR_INVALID, "case_launch_count: NULL argument");
     int n = (int)(cs->inputs.size() + cs->ops.size() + cs->outputs.size());
     for (const auto &op : cs->ops) {
-        if (op.conv && op.conv->lowered)
+        const bool grouped = op.conv && conv_runs_grouped(op.conv, nullptr, cs->max_batch);
+        if (op.conv && op.conv->lowered && !grouped)
             ++n;   // the row-lowering kernel runs ahead of the convolution kernel
-        if (op.conv && op.conv->pad_c)
+        if (op.conv && op.conv->pad_c && (op.conv->lowered || !grouped))
             ++n;   // and the copy into a padded tensor ahead of both
         if (op.skipped)
             --n;   // an eltwise op that runs inside a conv's epilogue

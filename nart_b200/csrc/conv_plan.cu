@@ -110,6 +110,8 @@ void destroy_conv(b200_conv *cv)
     cudaFree(cv->direct.shift_dev);
     if (cv->igemm)
         conv_igemm_destroy(cv->igemm);
+    if (cv->grouped)
+        conv_igemm_destroy(cv->grouped);
     scratch_free(cv->scratch, cv->device);
     scratch_free(cv->padded, cv->device);
     scratch_free(cv->home, cv->device);
@@ -133,6 +135,8 @@ int conv_run_igemm(b200_conv *cv, const uint8_t *x, int32_t n, uint8_t *y, uint8
         B200_TRY(conv_pad_channels_launch(x, padded, (size_t)n * g.h * g.w, cv->g.c, cv->pad_c, (uint8_t)g.izp, st));
         x = padded;
     }
+    if (cv->lowered && conv_runs_grouped(cv, x, n))
+        return conv_igemm_launch(cv->grouped, x, n, y, st);
     if (cv->lowered) {
         B200_TRY(conv_lower_rows_launch(g, x, n, lowered, st));
         x = lowered;
@@ -177,8 +181,59 @@ int conv_run_padded(b200_conv *cv, const uint8_t *x, int32_t n, uint8_t *y, cuda
     return conv_run_igemm(cv, x, n, y, cv->home, cv->home + need.lowered_at(), st);
 }
 
-// Scratch tensors that serve every run of the plan, for n images
-int reserve_owned(b200_conv *conv, int32_t n)
+// A conv as one on groups of m neighbouring pixels, where the lines of the image are whole groups of a multiple of 16 bytes: its
+// output pixel is the m / stride neighbouring output pixels whose windows start in one group, side by side as they lie in
+// memory, its window the groups that theirs reach.  Part of the weights is zero (7x7 on 4 channels, stride 2: 128 output
+// channels and 7 x 3 groups of 16 for 64 and 7 x 7 pixels of 4), but the image is read as it is.  flat: 1x1, all of an image is one line.
+int create_grouped(const ConvGeom &g, int m, bool flat, const std::vector<int8_t> &w, const int32_t *bias, const std::vector<uint32_t> &mult,
+                   const std::vector<int32_t> &shift, ConvIgemmPlan **out)
+{
+    *out = nullptr;
+    ConvGeom q = g;
+    if (flat) {
+        q.w = q.ow = g.h * g.w;
+        q.h = q.oh = 1;
+    }
+    if (q.w % m != 0 || m % g.stride_w != 0 || g.wzp_d != 0 || g.act_signed)
+        return B200_ERR_UNSUPPORTED;
+    const int per = m / g.stride_w;
+    auto group = [m](int px) { return (px >= 0 ? px : px - (m - 1)) / m; };
+    const int first = group(-g.pad_w), last = group((per - 1) * g.stride_w + g.s - 1 - g.pad_w);
+    const bool quads = m * g.c == 16;
+    if (q.ow % per != 0 || (long long)per * g.k * m * g.c * g.r * (last - first + 1) > (1 << 20))      // (mostly zeros by then)
+        return B200_ERR_UNSUPPORTED;
+    q.c = m * g.c; q.w /= m; q.ow /= per; q.k = per * g.k; q.s = last - first + 1; q.pad_w = -first; q.stride_w = 1;
+    if (quads && q.s > 8)
+        return B200_ERR_UNSUPPORTED;
+    std::vector<int8_t> wq((size_t)q.k * q.c * q.r * q.s, 0);       // [k][c][r][s]
+    std::vector<int32_t> bq(bias ? q.k : 0), sq(q.k);
+    std::vector<uint32_t> mq(q.k);
+    for (int o = 0; o < per; ++o)
+        for (int k = 0; k < g.k; ++k) {
+            const int kq = o * g.k + k;
+            if (bias)
+                bq[kq] = bias[k];
+            mq[kq] = mult[k];
+            sq[kq] = shift[k];
+            for (int c = 0; c < g.c; ++c)
+                for (int rr = 0; rr < g.r; ++rr)
+                    for (int ss = 0; ss < g.s; ++ss) {
+                        const int px = o * g.stride_w + ss - g.pad_w - first * m;      // from the window's first pixel on
+                        wq[(((size_t)kq * q.c + px % m * g.c + c) * q.r + rr) * q.s + px / m] = w[(((size_t)k * g.c + c) * g.r + rr) * g.s + ss];
+                    }
+        }
+    return conv_igemm_create(q, wq, bias ? bq.data() : nullptr, mq.data(), sq.data(), out, false, 0, quads);
+}
+
+// The images from which on a launch has a tile of groups of m pixels for every SM
+int tile_an_sm(const ConvGeom &g, int m)
+{
+    const int per = m / g.stride_w;
+    return (int)(((size_t)sm_count() * 128 * per + (size_t)g.oh * g.ow - 1) / ((size_t)g.oh * g.ow));
+}
+
+// Scratch tensors that serve every run of the plan, for n images, and the rows of a lowered one for n_lowered
+int reserve_owned(b200_conv *conv, int32_t n, int32_t n_lowered)
 {
     const PaddedBytes need(conv, n);
     auto grow = [conv](uint8_t *&buf, size_t &have, size_t need) -> int {
@@ -193,13 +248,18 @@ int reserve_owned(b200_conv *conv, int32_t n)
         return B200_OK;
     };
     if (conv->lowered)
-        B200_TRY(grow(conv->scratch, conv->scratch_bytes, need.lowered));
+        B200_TRY(grow(conv->scratch, conv->scratch_bytes, PaddedBytes(conv, n_lowered).lowered));
     if (conv->pad_c)
         B200_TRY(grow(conv->padded, conv->padded_bytes, need.padded));
     return B200_OK;
 }
 
 }  // namespace
+
+bool b200::conv_runs_grouped(const b200_conv *cv, const uint8_t *x, int32_t n)
+{
+    return cv->grouped && cv->algo == B200_CONV_ALGO_IGEMM && ((uintptr_t)x & 15) == 0 && (cv->pad_c && !cv->lowered ? 2.5 + n * cv->grouped_gain > 0.0 : n >= cv->grouped_from);
+}
 
 extern "C" {
 
@@ -440,6 +500,12 @@ int b200_conv2d_create(
         if (rc == B200_OK) {
             cv->lowered = true;
             cv->g_low = gl;
+            // The image in groups of four pixels instead, on launches of a tile of groups an SM: 7x7, 64 channels, 224 x 224,
+            // batch 256: 175 -> 104 us, batch 8: 12.1 -> 8.3.  Smaller launches lower: alone they are faster on groups too (batch 1 5.0 against
+            // 6.0 us), but not behind the other kernels of a network (ResNet-18, batch 1: 100.7 us, 102.2 on groups; batch 2: 111.2, 111.7;
+            // batch 4: 121.7, 120.6).
+            create_grouped(gt, 4, false, *wt, bias, mult, shift, &cv->grouped);     // (declined: all are lowered)
+            cv->grouped_from = tile_an_sm(gt, 4);
             // for callers of b200_conv2d_run_static_scratch: everything that entry point would otherwise do
             // once per device (kernel set-up, the static array's address) happens here, where allocation is
             // allowed; a failure only matters to that entry point, which reports it itself
@@ -450,6 +516,18 @@ int b200_conv2d_create(
         rc = conv_igemm_create(gt, *wt, bias, mult.data(), shift.data(), &cv->igemm);
     } else if (p->algo == B200_CONV_ALGO_IGEMM) {
         rc = fail(B200_ERR_UNSUPPORTED, "conv: implicit-GEMM path declined: %s", why);
+    }
+    const bool flat = taps == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0;
+    if (rc == B200_OK && cv->pad_c > 4) {
+        // Without the copy: groups of two or four pixels whose channels are a multiple of 16.  The zero weights cost `factor`
+        // times the multiply-adds (2 PFLOP/s), the copy three passes over the activations and a launch (2.5 us).
+        const int m = g.c % 8 == 0 && !(flat && g.c == 8) ? 2 : g.c % 4 == 0 ? 4 : 0;
+        if (m != 0) {
+            create_grouped(g, m, flat, w_s8, bias, mult, shift, &cv->grouped);
+            const double factor = flat ? m : m * ((g.s - 1 + m - 1) / m + 1.0) / g.s;
+            const double pixels = (double)g.oh * g.ow;
+            cv->grouped_gain = (double)g.h * g.w * (g.c + 2 * cv->pad_c) / 5e6 - pixels * 2.0 * (factor - 1.0) * g.c * taps * g.k / 2e9;
+        }
     }
     if (rc == B200_OK) {
         cv->algo = B200_CONV_ALGO_IGEMM;
@@ -516,12 +594,16 @@ int b200_conv2d_describe(const b200_conv_t *conv, char *buf, size_t len)
     if (!conv || !buf || len == 0)
         return fail(B200_ERR_INVALID, "conv(describe): bad argument");
     if (conv->algo == B200_CONV_ALGO_IGEMM && conv->igemm) {
-        conv_igemm_describe(conv->igemm, buf, len);
+        const bool grouped = conv->ran_grouped;
+        conv_igemm_describe(grouped ? conv->grouped : conv->igemm, buf, len);
         if (conv->lowered) {
             size_t used = strlen(buf);
-            snprintf(buf + used, len - used, ", on the row-lowered image");
+            snprintf(buf + used, len - used, grouped ? ", on four-pixel groups of the image" : ", on the row-lowered image");
         }
-        if (conv->pad_c) {
+        if (grouped && !conv->lowered) {
+            size_t used = strlen(buf);
+            snprintf(buf + used, len - used, ", on groups of pixels");
+        } else if (conv->pad_c) {
             size_t used = strlen(buf);
             snprintf(buf + used, len - used, ", channels padded to %d", conv->pad_c);
         }
@@ -547,11 +629,14 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
     if (conv->pad_c && (((uintptr_t)y & 15) != 0 || !conv_pad_channels_fits((size_t)n * conv->g.h * conv->g.w, conv->pad_c)))
         return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st);
     std::lock_guard<std::mutex> lock(conv->mu);
+    conv->ran_grouped = conv_runs_grouped(conv, conv->pad_c && conv->lowered ? nullptr : x, n);     // (a padded copy is aligned)
+    if (conv->ran_grouped && !(conv->pad_c && conv->lowered))
+        return conv_igemm_launch(conv->grouped, x, n, y, st);
     if (conv->pad_c && !conv->one_owner) {
         const int rc = conv_run_padded(conv, x, n, y, st);
         return rc == B200_ERR_NOMEM ? conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st) : rc;
     }
-    B200_TRY(reserve_owned(conv, n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
+    B200_TRY(reserve_owned(conv, n, conv->ran_grouped ? 0 : n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
     return conv_run_igemm(conv, x, n, y, conv->padded, conv->scratch, st);
 }
 
@@ -561,7 +646,8 @@ int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
         return fail(B200_ERR_INVALID, "conv(reserve): bad argument");
     std::lock_guard<std::mutex> lock(conv->mu);
     if (!conv->pad_c || conv->one_owner) {
-        const int rc = reserve_owned(conv, n);
+        // (a case's tensors are aligned: its larger launches run on groups)
+        const int rc = reserve_owned(conv, n, conv->one_owner && conv->grouped ? std::min(n, conv->grouped_from - 1) : n);
         if (rc != B200_ERR_NOMEM || !conv->pad_c)
             return rc;
         conv->algo = B200_CONV_ALGO_DIRECT;         // needs no scratch

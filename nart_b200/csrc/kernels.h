@@ -191,6 +191,13 @@ struct b200_conv {
     int pad_c = 0;
     b200::ConvGeom g_pad;
     uint8_t *padded = nullptr;      // [n][h][w][pad_c]
+    // The same conv on groups of neighbouring pixels (create_grouped), for aligned activations.  Where that leaves out the padded copy: what
+    // a run gains by it per image, in microseconds (below zero: it loses) beside the copy's launch; else the images from which on it
+    // is the faster.
+    b200::ConvIgemmPlan *grouped = nullptr;
+    double grouped_gain = 0.0;
+    int grouped_from = 0;
+    bool ran_grouped = false;       // the last run did
     size_t padded_bytes = 0;
     // One owner orders all runs of the plan, on whatever streams, and keeps it longer than the graphs it captures (the case
     // runner): `scratch` and `padded` serve every run.  Else a padded plan may be run by several streams and threads at
@@ -204,3 +211,9 @@ struct b200_conv {
     float oalpha = 0.f;             // output scale, kept for b200_conv2d_fuse_residual_add
     bool fused_residual = false;    // the plan computes eltwise_sum(conv(x), res)
 };
+
+namespace b200 {
+// Whether a run takes the plan on groups of pixels.
+bool conv_runs_grouped(const b200_conv *conv, const uint8_t *x, int32_t n);
+}  // namespace b200
+

@@ -46,6 +46,37 @@ def test_one_box_for_all_taps(monkeypatch, shape, kind):
     assert len(torch.unique(want)) > 16
 
 
+# (c, k, kernel, strides, pads, h, w): images of four channels and of three, ragged channel counts
+GROUPS = [(4, 64, (7, 7), (2, 2), (3, 3), 30, 32), (4, 32, (3, 3), (2, 2), (1, 1), 31, 36), (4, 16, (3, 5), (1, 1), (1, 2), 9, 8), (4, 48, (8, 2), (1, 4), (0, 0), 12, 20),
+          (3, 64, (7, 7), (2, 2), (3, 3), 33, 64), (4, 64, (7, 7), (2, 2), (3, 3), 30, 226), (24, 144, (1, 1), (1, 1), (0, 0), 9, 8), (20, 33, (1, 1), (1, 1), (0, 0), 6, 6),
+          (24, 40, (3, 3), (1, 1), (1, 1), 11, 14), (12, 18, (3, 3), (2, 2), (1, 1), 9, 16), (40, 20, (3, 3), (2, 2), (1, 1), 13, 10), (100, 150, (1, 1), (1, 1), (0, 0), 20, 10)]
+
+
+@pytest.mark.parametrize("shape", GROUPS)
+@pytest.mark.parametrize("size", ["small", "large"])
+def test_groups_of_pixels(shape, size):
+    """Aligned activations, and a view that only the copy or the lowering takes; both behind one plan, in either order."""
+    import torch
+    from nart_b200 import ops
+    c, k, (r, s), st, pad, h, w = shape
+    oh, ow = (h + 2 * pad[0] - r) // st[0] + 1, (w + 2 * pad[1] - s) // st[1] + 1
+    n = 1 if size == "small" else -(-148 * 128 * 4 // (oh * ow)) + 1        # four pixels or fewer a group, a tile an SM
+    wt, bias, x, q = _inputs(c, k, r, s, h, w, n, c + k + (n > 1))
+    args = dict(in_hw=(h, w), stride=st, pad=pad, relu=True, **q)
+    want = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **args)(x)
+    shifted = torch.empty(x.numel() + 4, device="cuda", dtype=torch.uint8)[4:].copy_(x.view(-1)).view(x.shape)
+    conv, said = ops.Conv2d(wt, bias, **args), []
+    for part in (x, shifted, x):
+        assert torch.equal(conv(part), want)
+        said.append(conv.describe())
+    assert ops.device_status() == 0 and conv.algo == ops.ALGO_IGEMM
+    if c <= 4:
+        groups = size == "large" and w % 4 == 0
+        assert ["four-pixel groups" in d for d in said] == [groups, groups and c == 3, groups], said        # (a padded copy is aligned)
+    if c == 24 and r == 1:
+        assert "groups of pixels" in said[0] and "groups of pixels" not in said[1] and said[2] == said[0]
+
+
 @pytest.mark.parametrize("c,k,ks", [(64, 64, 3), (24, 144, 1), (4, 64, 7)])
 def test_run_is_the_first_call_of_a_thread(c, k, ks):
     """A thread that has called nothing of CUDA has no current context."""
