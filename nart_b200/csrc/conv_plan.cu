@@ -518,6 +518,28 @@ int b200_conv2d_create(
         rc = fail(B200_ERR_UNSUPPORTED, "conv: implicit-GEMM path declined: %s", why);
     }
     const bool flat = taps == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0;
+    if (rc == B200_OK && !cv->pad_c && !cv->lowered && g.stride_w == 1 && g.stride_h == 1) {
+        // Few output channels: what a tile costs beside its outputs -- an MMA takes 54 cycles for 128 pixels by 32 bytes whether it has 16
+        // or 32 channels, 61 for 64, and an epilogue its waits -- is shared by the m pixels of a group.  1x1: up to four pixels and 128
+        // columns (32 -> 16 on 112 x 112, batch 256: 60.2 -> 26.6 us; 64 -> 64 on 56 x 56: 24.3 -> 19.2; with 256 columns 20.5; 144 -> 32: 44.0 -> 24.8;
+        // 256 -> 64, batch 64: 11.9 -> 12.4, too many zeros), 192 for 16 channels, which leave half of an operand row empty (16 -> 96 on
+        // 112 x 112, batch 64: 30.8 -> 28.6).  Larger windows: pairs, up to 64 columns (16 -> 32, 3x3, 112 x 112, batch 128: 54.3 -> 32.6; 64 -> 64 on
+        // 56 x 56: 47.3 -> 52.9), 128 up to 32 channels (32 -> 64 on 112 x 112: 36.6 -> 35.4).  On launches of a tile of groups an SM.
+        const bool one = taps == 1;
+        auto worth = [&](int m) {
+            const int columns = m * g.k, depth = m * g.c;
+            if ((flat ? g.h * g.w : g.w) % m != 0 || (!flat && g.ow % m != 0))
+                return false;
+            if (one)
+                return columns <= (g.c == 16 ? 192 : 128) && depth <= (columns <= 64 ? 512 : 384);
+            return m == 2 && columns <= (g.c <= 32 ? 128 : 64) && depth <= 128;
+        };
+        const int m = worth(4) ? 4 : worth(2) ? 2 : 0;
+        if (m != 0) {
+            create_grouped(g, m, flat, w_s8, bias, mult, shift, &cv->grouped);
+            cv->grouped_from = tile_an_sm(g, m);
+        }
+    }
     if (rc == B200_OK && cv->pad_c > 4) {
         // Without the copy: groups of two or four pixels whose channels are a multiple of 16.  The zero weights cost `factor`
         // times the multiply-adds (2 PFLOP/s), the copy three passes over the activations and a launch (2.5 us).

@@ -77,6 +77,27 @@ def test_groups_of_pixels(shape, size):
         assert "groups of pixels" in said[0] and "groups of pixels" not in said[1] and said[2] == said[0]
 
 
+# (c, k, kernel, pad, h, w): one group more or less than a tile, lines of one group, the largest and smallest widths the rule takes
+NARROW = [(32, 16, 1, 0, 28, 28), (64, 64, 1, 0, 13, 26), (48, 17, 1, 0, 6, 10), (16, 96, 1, 0, 9, 14), (256, 32, 1, 0, 7, 4), (96, 32, 1, 0, 16, 8),
+          (16, 32, 3, 1, 28, 30), (64, 32, 3, 1, 15, 14), (32, 64, 3, 1, 20, 2), (48, 20, 3, 0, 12, 18), (16, 31, 5, 2, 9, 22)]
+
+
+@pytest.mark.parametrize("shape", NARROW)
+def test_few_output_channels_on_groups_of_pixels(shape):
+    """Launches that fill the device and launches that don't, and a view that groups can't read."""
+    import torch
+    from nart_b200 import ops
+    c, k, ks, pad, h, w = shape
+    n = -(-148 * 128 * 4 // (h * w)) + 3
+    wt, bias, x, q = _inputs(c, k, ks, ks, h, w, n, c + k)
+    args = dict(in_hw=(h, w), stride=(1, 1), pad=(pad, pad), relu=False, **q)
+    want = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **args)(x)
+    conv = ops.Conv2d(wt, bias, **args)
+    assert torch.equal(conv(x), want) and "groups of pixels" in conv.describe(), conv.describe()
+    assert torch.equal(conv(x[:2]), want[:2]) and "groups of pixels" not in conv.describe()
+    assert torch.equal(conv(x), want) and ops.device_status() == 0
+
+
 @pytest.mark.parametrize("c,k,ks", [(64, 64, 3), (24, 144, 1), (4, 64, 7)])
 def test_run_is_the_first_call_of_a_thread(c, k, ks):
     """A thread that has called nothing of CUDA has no current context."""
