@@ -483,6 +483,8 @@ int b200_case_output_f32(b200_case_t *cs, int32_t tensor, float ialpha, uint8_t 
     return B200_OK;
 }
 
+static size_t head_ops(const b200_case_t *cs, int32_t batch);
+
 int b200_case_prepare(b200_case_t *cs, int32_t max_batch)
 {
     B200_TRY(check_building(cs, "case_prepare"));
@@ -579,6 +581,10 @@ int b200_case_prepare(b200_case_t *cs, int32_t max_batch)
         }
         if (prev)
             set_next(nullptr, 0);
+    }
+    if (head_ops(cs, max_batch) > 1 && !cs->part_event) {
+        B200_CUDA_TRY(cudaStreamCreateWithFlags(&cs->part_stream, cudaStreamNonBlocking));
+        B200_CUDA_TRY(cudaEventCreateWithFlags(&cs->part_event, cudaEventDisableTiming));
     }
     cs->prepared = true;
     return B200_OK;
@@ -1014,10 +1020,6 @@ struct DirectBuffers {
 static int split_host_run(b200_case_t *cs, int32_t batch, const void *const *inputs, b200_stream_t stream)
 {
     cudaStream_t cst = as_stream(stream);
-    if (!cs->part_stream)
-        B200_CUDA_TRY(cudaStreamCreateWithFlags(&cs->part_stream, cudaStreamNonBlocking));
-    if (!cs->part_event)
-        B200_CUDA_TRY(cudaEventCreateWithFlags(&cs->part_event, cudaEventDisableTiming));
     B200_CUDA_TRY(cudaEventRecord(cs->part_event, cst));
     B200_CUDA_TRY(cudaStreamWaitEvent(cs->part_stream, cs->part_event, 0));
     const int32_t n1 = first_part(batch);
@@ -1041,7 +1043,7 @@ static int split_host_run(b200_case_t *cs, int32_t batch, const void *const *inp
 static int run_on_host_buffers(b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs, b200_stream_t stream)
 {
     DirectBuffers buffers{ cs, as_stream(stream) };
-    bool split = cs->use_graph && !cs->profiling && stream != nullptr && head_ops(cs, batch) > 1;
+    bool split = cs->use_graph && !cs->profiling && stream != nullptr && cs->part_event && head_ops(cs, batch) > 1;
     for (size_t i = 0; i < cs->inputs.size(); ++i) {
         CaseIO &io = cs->inputs[i];
         if (batch > 0 && !inputs[i])
