@@ -731,7 +731,9 @@ static int run_batch(b200_case_t *cs, int32_t batch, b200_stream_t stream)
 
 // A host run whose images take long to copy: the first part of them goes through the first ops of the case while the others are
 // on their way (ResNet-18, 64 images: 185 us of copy).  Parts of a multiple of 16 images, so that every tensor of the second one is
-// aligned; the ops whose time on the first part the copy of the second covers.
+// aligned; the ops whose time on the first part the copy of the second covers.  The second graph, and the first ops' second launches,
+// cost about 35 us: ResNet-18 of 224 x 224, with 48 us of work in the first part (44 images) 427 -> 414 us, with 28 (32 images)
+// 344 -> 342; MobileNetV2 with 65 (64 images) 661 -> 629, with 41 (44 images) 527 -> 534; ResNet-50 of 130 x 130 with 16 (64 images) 638 -> 645.
 static int32_t first_part(int32_t batch) { return batch / 32 * 16; }
 static size_t head_ops(const b200_case_t *cs, int32_t batch)
 {
@@ -739,11 +741,13 @@ static size_t head_ops(const b200_case_t *cs, int32_t batch)
     double copy = 0.0;                                      // us, of the second part
     for (const auto &io : cs->inputs)
         copy += (double)io.bytes_per_image * (batch - n1) / 52e3;
-    if (n1 == 0 || copy < 20.0)
+    if (n1 == 0)
         return 0;
     size_t n = 0, whole = 0;
+    double work = 0.0, whole_work = 0.0;        // of the first part, beside the launches
     for (double t = 0.0; n < cs->ops.size(); ) {
         const CaseOp &op = cs->ops[n];
+        double us = 0.0;
         if (!op.skipped) {
             double bytes = (double)cs->tensors[op.out].bytes_per_image(), macs = 0.0;
             for (int in : op.ins)
@@ -752,19 +756,23 @@ static size_t head_ops(const b200_case_t *cs, int32_t batch)
                 const ConvGeom &g = op.conv->g;
                 macs = (double)g.oh * g.ow * g.k * (g.c / g.group) * g.r * g.s;
             }
-            t += 2.5 + n1 * (bytes / 4e6 + macs / 0.6e9);
+            us = n1 * (bytes / 4e6 + macs / 0.6e9);
+            t += 2.5 + us;
         }
         if (t > copy)
             break;
         ++n;
+        work += us;
         // (a conv and the SUM that its launch may form stay together)
         bool pair = false;
         for (size_t i = 0; i < n; ++i)
             pair = pair || cs->ops[i].sum_op >= (int)n;
-        if (!pair)
+        if (!pair) {
             whole = n;
+            whole_work = work;
+        }
     }
-    return whole;
+    return whole_work < 45.0 ? 0 : whole;
 }
 
 // The ops in graph mode: the first run at a batch size is eager (plans build their tensor maps and scratch

@@ -180,11 +180,11 @@ class _Buffer:
         self.__cuda_array_interface__ = dict(data=(ptr, False), shape=shape, typestr=typestr, version=3)
 
 
-@pytest.mark.parametrize("net,hw,batch", [("resnet18", 128, 48), ("mobilenet_v2", 160, 33), ("resnet50", 112, 70)])
+@pytest.mark.parametrize("net,hw,batch", [("resnet18", 224, 96), ("mobilenet_v2", 224, 65), ("resnet50", 176, 134)])
 @pytest.mark.parametrize("pinned", [True, False])
 def test_images_that_are_copied_in_two_parts(net, hw, batch, pinned):
-    """Graph mode, images of some megabytes: eager, captured and replayed runs with other images each time, against runs on
-    images that are on the device already; smaller batches of the same case, and a run without a graph, in between."""
+    """Graph mode, batches whose first part has 45 us of work and more: eager, captured and replayed runs with other images each time,
+    against runs on images that are on the device already; smaller batches of the same case, and a run without a graph, in between."""
     from nart_b200 import nets
     spec = nets.mobilenet_v2(seed=3, hw=hw, spread=True) if net == "mobilenet_v2" else nets.resnet(int(net[6:]), seed=3, hw=hw, spread=True, width_div=2)
     cs, _ = nets.to_case(spec, batch)
