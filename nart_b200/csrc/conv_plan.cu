@@ -254,6 +254,20 @@ int reserve_owned(b200_conv *conv, int32_t n, int32_t n_lowered)
     return B200_OK;
 }
 
+// A run on groups needs no rows, but the plan's scratch grows with the batch whatever route a run takes: after it, a smaller batch
+// or an unaligned view of as many images neither allocates (it may be under capture) nor moves the rows that a captured graph knows.
+int reserve_beside_groups(b200_conv *conv, int32_t n, cudaStream_t st)
+{
+    if (PaddedBytes(conv, n).lowered <= conv->scratch_bytes)
+        return B200_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    B200_CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    if (capture != cudaStreamCaptureStatusNone)
+        return B200_OK;
+    const int rc = reserve_owned(conv, n, n);
+    return rc == B200_ERR_NOMEM ? B200_OK : rc;
+}
+
 }  // namespace
 
 bool b200::conv_runs_grouped(const b200_conv *cv, const uint8_t *x, int32_t n)
@@ -654,8 +668,11 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
         return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st);
     std::lock_guard<std::mutex> lock(conv->mu);
     conv->ran_grouped = conv_runs_grouped(conv, conv->pad_c && conv->lowered ? nullptr : x, n);     // (a padded copy is aligned)
-    if (conv->ran_grouped && !(conv->pad_c && conv->lowered))
+    if (conv->ran_grouped && !(conv->pad_c && conv->lowered)) {
+        if (conv->lowered && !conv->one_owner)
+            B200_TRY(reserve_beside_groups(conv, n, st));
         return conv_igemm_launch(conv->grouped, x, n, y, st);
+    }
     if (conv->pad_c && !conv->one_owner) {
         const int rc = conv_run_padded(conv, x, n, y, st);
         return rc == B200_ERR_NOMEM ? conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st) : rc;

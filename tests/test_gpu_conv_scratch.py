@@ -114,6 +114,28 @@ def test_first_run_under_capture_and_replays_beside_growth(c, k, hw, n):
         assert all(torch.equal(e, want_big[:n * (seed + 1)]) for e in eager)
 
 
+def test_captures_behind_a_large_run_of_a_four_channel_image():
+    """A run on groups of pixels uses no scratch, but sizes it: smaller batches and views that groups can't read are captured behind it
+    without an allocation, and the graph's scratch stays where it is."""
+    c, k, hw, n = 4, 32, 56, 64
+    plan, direct = _plan(c, k, hw), _direct(c, k, hw)
+    big = torch.randint(0, 256, (n, hw, hw, c), device="cuda", dtype=torch.uint8)
+    shifted = torch.empty(big.numel() + 4, device="cuda", dtype=torch.uint8)[4:].view(big.shape).copy_(big)
+    want = direct(big)
+    assert torch.equal(plan(big), want) and "four-pixel groups" in plan.describe()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        one = plan(big[:1])
+        views = plan(shifted)
+    for m in (3, 24, n):            # (none of them moves the scratch)
+        assert torch.equal(plan(big[:m]), want[:m]) and torch.equal(plan(shifted[:m]), want[:m])
+        one.zero_(), views.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(one, want[:1]) and torch.equal(views, want)
+
+
 def test_first_run_of_a_process_under_capture():
     """Nothing that a capture forbids is left to the first run."""
     import os
