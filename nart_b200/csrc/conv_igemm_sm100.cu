@@ -470,7 +470,7 @@ int conv_igemm_create(
         // (3x3 128-channel layer 0.047 -> 0.043 ms.  256-wide tiles lose: their two accumulators fill the
         // tensor memory, so the next pair's mainloop cannot overlap this pair's epilogue: 0.039 -> 0.044 ms.)
         const bool pair_off = getenv("B200_IGEMM_PAIR") && atoi(getenv("B200_IGEMM_PAIR")) == 0;   // tuning aid
-        if (!pair_off && !ones && !p->b_resident && kgroup == 1 && !p->a_wide && n_tiles_n == 1 && p->bn <= 128) {
+        if (!pair_off && !ones && !p->b_resident && kgroup == 1 && !p->a_wide && !quads && n_tiles_n == 1 && p->bn <= 128) {
             int st = kMaxStages;
             auto fits2 = [&](int n) { return smem_layout(2 * n, n, p->bk, p->bn, p->groups).total + 1024 <= 227 * 1024; };
             while (st > 2 && !fits2(st))
@@ -489,7 +489,7 @@ int conv_igemm_create(
         {
             const char *e = getenv("B200_IGEMM_CTA_PAIR");     // tuning aid: 0 never, 1 wherever possible
             p->pair_want = e ? atoi(e) : -1;
-            const bool can = !p->b_resident && !p->a_wide && !p->pair && p->bn % 32 == 0 && p->bn >= 64 && g.wzp_d == 0;
+            const bool can = !p->b_resident && !p->a_wide && !quads && !p->pair && p->bn % 32 == 0 && p->bn >= 64 && g.wzp_d == 0;
             const bool automatic = p->bn == 256 && kblocks * p->bk >= 1024;
             if (can && (p->pair_want == 1 || (p->pair_want == -1 && automatic))) {
                 auto fits_p = [&](int st, int kg) {
@@ -1068,8 +1068,6 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
             a.a_pitch = p->quads ? 16 : p->bk;
         }
     }
-    if (p->quads && !l.halo)
-        return fail(B200_ERR_UNSUPPORTED, "conv(igemm): no launch for this image");
     a.bk = p->bk; a.bn = p->bn; a.stages = l.cta_pair ? p->stages_pair : p->stages; a.kgroup = p->kgroup; a.groups = p->groups; a.acc_stages = p->acc_stages;
     a.cchunks = (p->cpad + p->bk - 1) / p->bk;
     a.last_steps = (p->cpad - (a.cchunks - 1) * p->bk) / 32;

@@ -77,6 +77,22 @@ def test_groups_of_pixels(shape, size):
         assert "groups of pixels" in said[0] and "groups of pixels" not in said[1] and said[2] == said[0]
 
 
+@pytest.mark.parametrize("pair", ["0", "1"])
+def test_pixel_groups_beside_the_cta_pair_switch(monkeypatch, pair):
+    """Weights that don't fit beside three ordinary tiles, which is when CTA pairs are considered, but do beside boxes of four-channel
+    pixels, which pairs can't read."""
+    import torch
+    from nart_b200 import ops
+    h, w, n = 30, 64, 90
+    wt, bias, x, q = _inputs(4, 128, 9, 7, h, w, n, 5)
+    args = dict(in_hw=(h, w), stride=(2, 2), pad=(4, 3), relu=True, **q)
+    want = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **args)(x)
+    monkeypatch.setenv("B200_IGEMM_CTA_PAIR", pair)
+    conv = ops.Conv2d(wt, bias, **args)
+    assert torch.equal(conv(x), want) and "four-pixel groups" in conv.describe(), conv.describe()
+    assert torch.equal(conv(x[:1]), want[:1]) and ops.device_status() == 0
+
+
 # (c, k, kernel, pad, h, w): one group more or less than a tile, lines of one group, the largest and smallest widths the rule takes
 NARROW = [(32, 16, 1, 0, 28, 28), (64, 64, 1, 0, 13, 26), (48, 17, 1, 0, 6, 10), (16, 96, 1, 0, 9, 14), (256, 32, 1, 0, 7, 4), (96, 32, 1, 0, 16, 8),
           (16, 32, 3, 1, 28, 30), (64, 32, 3, 1, 15, 14), (32, 64, 3, 1, 20, 2), (48, 20, 3, 0, 12, 18), (16, 31, 5, 2, 9, 22)]
