@@ -126,7 +126,7 @@ B200_API void b200_get_quant_scale(float x, int bits, uint32_t *mult, int8_t *sh
  *   B200_IGEMM_CTA_PAIR=<0|1>                never / wherever possible run on CTA pairs (tcgen05 cta_group::2)
  *   B200_IGEMM_SMALL=<0|BNxS>                never one tile per CTA or cluster (launches that leave SMs without a tile), or
  *                                            always, with BN channels per tile and S CTAs
- *   B200_IGEMM_HALO=1                        one box of activations for all taps of a window wherever possible
+ *   B200_IGEMM_HALO=<0|1>                    never / wherever possible one box of activations for all taps of a window
  *   B200_IGEMM_EPI=<1|2>                     1: no fp32 requantize in the epilogue, 2: nor one shift for all channels
  * and by b200_case_prepare:
  *   B200_CASE_ZIGZAG=0                       every op walks its tiles first to last (default: each op walks against the

@@ -188,7 +188,7 @@ struct ConvIgemmPlan {
     int quads = 0, taps_w = 0;
     // One box of activations for all taps (kernel MODE 4), its tiles and its stages (0: not possible)
     HaloTiles halo;
-    int stages_halo = 0, box_group = 8;
+    int stages_halo = 0, box_group = 8, halo_want = -1;
     uint32_t box_bytes = 0;
     int n_row_cls = 0, n_col_cls = 0;
     int seg_w[2] = { 0, 0 };        // see epilogue_segments
@@ -509,8 +509,9 @@ int conv_igemm_create(
         // One box for all taps.  Tiles of eight by sixteen pixels, or of whole lines where a power of two holds a line
         // and its ring: the shapes whose 32-pixel quarters are boxes of the output.
         const HaloWindow win(g.r, p->taps_w, g.stride_h, g.stride_w, g.pad_h, g.pad_w, quads ? g.s : 0, quads ? p->bk / 16 : 1);
-        const char *e = getenv("B200_IGEMM_HALO");        // tuning aid: 0 never
-        if (win.fits() && !p->a_wide && n_tiles_n == 1 && g.k % 16 == 0 && (quads || !(e && atoi(e) == 0))) {
+        if (const char *e = getenv("B200_IGEMM_HALO"))      // tuning aid: 0 never, 1 wherever possible
+            p->halo_want = atoi(e);
+        if (win.fits() && !p->a_wide && n_tiles_n == 1 && g.k % 16 == 0 && (quads || p->halo_want != 0)) {
             int line = 8;
             while (line < g.ow + win.ring_w)
                 line *= 2;
@@ -1052,9 +1053,8 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
         // 12.4 -> 11.5; 64 -> 64 there 8.04 -> 7.84, on 27 x 35 11.7 -> 12.7), and up to a half where a window-sum column leaves one pipeline
         // to a box per tap (24.6 -> 16.3; on 14 x 14 10.1 -> 8.2).  Tiles of more than 128 channels wait for their epilogue (32 -> 256 on 30 x 30:
         // 13.8 -> 14.9); with a stride a box holds few taps (64 -> 128, stride 2: 9.8 -> 10.8).
-        const char *e = getenv("B200_IGEMM_HALO");       // tuning aid: 1 wherever possible
         const long long tiles = (long long)a.tiles_w * a.tiles_h * a.tiles_n;
-        l.halo = p->quads || (e && atoi(e) == 1)
+        l.halo = p->quads || p->halo_want == 1
             || (h.planes == 1 && (p->bn <= 128 || g.wzp_d != 0) && boxes * 100 <= tiles * (g.wzp_d != 0 ? 150 : p->bk == 128 ? 133 : 120));
         if (l.halo) {
             a.tw = h.tw; a.th = h.th; a.tn = 1;

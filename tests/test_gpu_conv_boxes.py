@@ -46,6 +46,22 @@ def test_one_box_for_all_taps(monkeypatch, shape, kind):
     assert len(torch.unique(want)) > 16
 
 
+def test_the_box_switch_is_read_at_creation(monkeypatch):
+    """As the header says of all switches: what the environment holds later changes no plan."""
+    import torch
+    from nart_b200 import ops
+    wt, bias, x, q = _inputs(64, 64, 3, 3, 27, 35, 60, 1)       # a map whose boxes waste too much to be taken by themselves
+    args = dict(in_hw=(27, 35), stride=(1, 1), pad=(1, 1), relu=True, **q)
+    want = ops.Conv2d(wt, bias, algo=ops.ALGO_DIRECT, **args)(x)
+    for value in ("1", "0"):
+        plain = ops.Conv2d(wt, bias, **args)
+        monkeypatch.setenv("B200_IGEMM_HALO", value)
+        switched = ops.Conv2d(wt, bias, **args)
+        assert torch.equal(plain(x), want) and "one box" not in plain.describe()
+        monkeypatch.delenv("B200_IGEMM_HALO")
+        assert torch.equal(switched(x), want) and ("one box" in switched.describe()) == (value == "1")
+
+
 # (c, k, kernel, strides, pads, h, w): images of four channels and of three, ragged channel counts
 GROUPS = [(4, 64, (7, 7), (2, 2), (3, 3), 30, 32), (4, 32, (3, 3), (2, 2), (1, 1), 31, 36), (4, 16, (3, 5), (1, 1), (1, 2), 9, 8), (4, 48, (8, 2), (1, 4), (0, 0), 12, 20),
           (3, 64, (7, 7), (2, 2), (3, 3), 33, 64), (4, 64, (7, 7), (2, 2), (3, 3), 30, 226), (24, 144, (1, 1), (1, 1), (0, 0), 9, 8), (20, 33, (1, 1), (1, 1), (0, 0), 6, 6),
