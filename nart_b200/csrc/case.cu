@@ -886,6 +886,7 @@ static int run_eager(b200_case_t *cs, int32_t batch, b200_stream_t stream, int p
                 B200_TRY(b200_conv2d_run_residual(op.conv, x, batch, at(op.residual), y, stream));
             else if (op.sum_op >= 0 && !prof && !conv_runs_grouped(op.conv, x, batch)) {
                 CaseOp &add = cs->ops[op.sum_op];
+                op.conv->ran_grouped = false;
                 const ConvSum ws = { at(add.ins[1 - op.sum_input]), at(add.out), &add.elt, op.sum_input };
                 B200_TRY(conv_igemm_launch(op.conv->igemm, x, batch, y, as_stream(stream), nullptr, nullptr, &ws, &add.summed));
             } else {

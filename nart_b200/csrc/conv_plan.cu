@@ -667,8 +667,9 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
     if (conv->pad_c && (((uintptr_t)y & 15) != 0 || !conv_pad_channels_fits((size_t)n * conv->g.h * conv->g.w, conv->pad_c)))
         return conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st);
     std::lock_guard<std::mutex> lock(conv->mu);
-    conv->ran_grouped = conv_runs_grouped(conv, conv->pad_c && conv->lowered ? nullptr : x, n);     // (a padded copy is aligned)
-    if (conv->ran_grouped && !(conv->pad_c && conv->lowered)) {
+    const bool grouped = conv_runs_grouped(conv, conv->pad_c && conv->lowered ? nullptr : x, n);     // (a padded copy is aligned)
+    conv->ran_grouped = grouped;
+    if (grouped && !(conv->pad_c && conv->lowered)) {
         if (conv->lowered && !conv->one_owner)
             B200_TRY(reserve_beside_groups(conv, n, st));
         return conv_igemm_launch(conv->grouped, x, n, y, st);
@@ -677,7 +678,7 @@ int b200_conv2d_run(b200_conv_t *conv, const uint8_t *x, int32_t n, uint8_t *y, 
         const int rc = conv_run_padded(conv, x, n, y, st);
         return rc == B200_ERR_NOMEM ? conv_direct_launch(conv->g, conv->direct, x, n, y, nullptr, st) : rc;
     }
-    B200_TRY(reserve_owned(conv, n, conv->ran_grouped ? 0 : n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
+    B200_TRY(reserve_owned(conv, n, grouped ? 0 : n));   // grow-only scratch: the first call at a larger batch allocates (and synchronizes)
     return conv_run_igemm(conv, x, n, y, conv->padded, conv->scratch, st);
 }
 
@@ -746,6 +747,7 @@ int b200_conv2d_run_residual(
         return fail(B200_ERR_INVALID, "conv(residual): the plan has no residual add (b200_conv2d_fuse_residual_add)");
     if (n == 0)
         return B200_OK;
+    conv->ran_grouped = false;
     return conv_igemm_launch(conv->igemm, x, n, y, as_stream(stream), nullptr, res);
 }
 

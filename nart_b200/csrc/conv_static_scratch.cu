@@ -108,6 +108,7 @@ extern "C" int b200_conv2d_run_static_scratch(
     // word is not cleared here: a code left by an earlier call stays until b200_static_scratch_status
     // has reported it.
     uint8_t *lowered = base + kHeaderBytes;
+    conv->ran_grouped = false;
     B200_TRY(conv_lower_rows_launch(g, x, n, lowered, st));
     return conv_igemm_launch(conv->igemm, lowered, n, y, st, reinterpret_cast<int *>(base));
 }

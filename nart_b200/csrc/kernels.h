@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -197,7 +198,7 @@ struct b200_conv {
     b200::ConvIgemmPlan *grouped = nullptr;
     double grouped_gain = 0.0;
     int grouped_from = 0;
-    bool ran_grouped = false;       // the last run did
+    std::atomic<bool> ran_grouped{ false };     // the last run did (b200_conv2d_describe)
     size_t padded_bytes = 0;
     // One owner orders all runs of the plan, on whatever streams, and keeps it longer than the graphs it captures (the case
     // runner): `scratch` and `padded` serve every run.  Else a padded plan may be run by several streams and threads at

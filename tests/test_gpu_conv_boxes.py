@@ -130,6 +130,28 @@ def test_few_output_channels_on_groups_of_pixels(shape):
     assert torch.equal(conv(x), want) and ops.device_status() == 0
 
 
+def test_describe_names_what_the_last_run_took():
+    """Entry points that never run on groups, after a run that did."""
+    import torch
+    from nart_b200 import ops
+    n = 200
+    wt, bias, x, q = _inputs(64, 64, 1, 1, 28, 28, n, 3)
+    conv = ops.Conv2d(wt, bias, in_hw=(28, 28), relu=False, **q)
+    y = conv(x)
+    assert "on groups of pixels" in conv.describe()
+    zp = (q["ozp"], 90)
+    conv.fuse_residual_add(0, (q["oalpha"], 0.03), zp, 0.05, 120)
+    assert torch.equal(conv.run_residual(x, y), ops.add(y, y, (q["oalpha"], 0.03), zp, 0.05, 120))
+    assert "groups of pixels" not in conv.describe()
+    wt, bias, x, q = _inputs(4, 64, 7, 7, 28, 28, n, 4)
+    conv = ops.Conv2d(wt, bias, in_hw=(28, 28), stride=(2, 2), pad=(3, 3), relu=False, **q)
+    y = conv(x)
+    assert "four-pixel groups" in conv.describe()
+    z = torch.empty_like(y)
+    assert ops.lib.b200_conv2d_run_static_scratch(conv._h, x.data_ptr(), n, z.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(y, z) and "row-lowered" in conv.describe()
+
+
 @pytest.mark.parametrize("c,k,ks", [(64, 64, 3), (24, 144, 1), (4, 64, 7)])
 def test_run_is_the_first_call_of_a_thread(c, k, ks):
     """A thread that has called nothing of CUDA has no current context."""
