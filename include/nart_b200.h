@@ -395,7 +395,9 @@ B200_API int b200_case_run_host(
 B200_API int b200_case_submit_host(
     b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs);
 B200_API int b200_case_wait(b200_case_t *cs);
-/* Number of kernels one b200_case_run_device launches.  (A residual add that a small conv launch forms itself still counts.) */
+/* A line of text per op, as b200_conv2d_describe has it for convolutions: what the last launch of each was. */
+B200_API int b200_case_describe(const b200_case_t *cs, char *buf, size_t len);
+/* Number of kernels one b200_case_run_device of max_batch images launches.  (A residual add that a small conv launch forms itself still counts.) */
 B200_API int b200_case_launch_count(const b200_case_t *cs, int32_t *launches);
 /* Folds residual adds into the convs that feed them (default: off; call before b200_case_prepare).
  * Off by default: ResNet-50 at batch 256 runs 2.80 ms per step fused against 2.67 ms with the adds as kernels of

@@ -106,6 +106,7 @@ SIGNATURES = {
     "b200_case_run_host": (C.c_int, [vp, i32, C.POINTER(vp), C.POINTER(vp), vp]),
     "b200_case_submit_host": (C.c_int, [vp, i32, C.POINTER(vp), C.POINTER(vp)]),
     "b200_case_wait": (C.c_int, [vp]),
+    "b200_case_describe": (C.c_int, [vp, C.c_char_p, sz]),
     "b200_case_launch_count": (C.c_int, [vp, pi32]),
     "b200_case_use_graph": (C.c_int, [vp, i32]),
     "b200_case_set_fusion": (C.c_int, [vp, i32]),

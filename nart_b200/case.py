@@ -120,6 +120,12 @@ class Case:
         check(lib.b200_case_launch_count(self._h, C.byref(v)))
         return v.value
 
+    def describe(self):
+        """A line per op: the kernel variant of its last launch (b200_case_describe)."""
+        buf = C.create_string_buffer(1 << 16)
+        check(lib.b200_case_describe(self._h, buf, len(buf)))
+        return buf.value.decode().splitlines()
+
     def use_graph(self, enable: bool = True):
         """Replay run_device as one CUDA graph per batch size (see b200_case_use_graph)."""
         check(lib.b200_case_use_graph(self._h, int(enable)))

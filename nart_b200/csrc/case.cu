@@ -562,25 +562,20 @@ int b200_case_prepare(b200_case_t *cs, int32_t max_batch)
         const char *e = getenv("B200_CASE_PREFETCH");
         const bool on = !(e && atoi(e) == 0);
         const b200_conv *prev = nullptr;
-        auto set_next = [&](const uint8_t *w, size_t bytes) {
-            conv_igemm_set_next_readonly(prev->igemm, w, bytes);
+        auto set_next = [&](const NextRead &next) {
+            conv_igemm_set_next_readonly(prev->igemm, next);
             if (prev->grouped)
-                conv_igemm_set_next_readonly(prev->grouped, w, bytes);
+                conv_igemm_set_next_readonly(prev->grouped, next);
         };
         for (auto &op : cs->ops) {
             if (op.skipped || op.kind != OpKind::Conv || !op.conv->igemm)
                 continue;
-            if (prev) {
-                const uint8_t *w = nullptr;
-                size_t bytes = 0;
-                if (on)
-                    conv_igemm_weights(conv_runs_grouped(op.conv, nullptr, cs->max_batch) ? op.conv->grouped : op.conv->igemm, &w, &bytes);
-                set_next(w, bytes);
-            }
+            if (prev)
+                set_next(on ? conv_weights_read(op.conv) : NextRead());
             prev = op.conv;
         }
         if (prev)
-            set_next(nullptr, 0);
+            set_next(NextRead());
     }
     if (head_ops(cs, max_batch) > 1 && !cs->part_event) {
         B200_CUDA_TRY(cudaStreamCreateWithFlags(&cs->part_stream, cudaStreamNonBlocking));
@@ -1159,6 +1154,23 @@ int b200_case_wait(b200_case_t *cs)
     B200_TRY(b200_device_status(reinterpret_cast<b200_stream_t>(cs->comp_stream), &word));
     if (word != 0)
         return fail(B200_ERR_DEVICE_WAIT, "case_wait: a device-side wait ran out (code 0x%x)", word);
+    return B200_OK;
+}
+
+int b200_case_describe(const b200_case_t *cs, char *buf, size_t len)
+{
+    if (!cs || !buf || len == 0)
+        return fail(B200_ERR_INVALID, "case_describe: bad argument");
+    buf[0] = 0;
+    size_t used = 0;
+    for (const auto &op : cs->ops) {
+        static const char *const names[] = { "conv", "eltwise", "relu", "pool" };
+        char text[320] = "";
+        if (op.conv)
+            B200_TRY(b200_conv2d_describe(op.conv, text, sizeof(text)));
+        const int n = snprintf(buf + used, len - used, "%s%s%s%s\n", names[(int)op.kind], text[0] ? ": " : "", text, op.skipped ? ", inside a conv" : "");
+        used += n < 0 || (size_t)n >= len - used ? len - used - 1 : (size_t)n;
+    }
     return B200_OK;
 }
 

@@ -201,8 +201,7 @@ struct ConvIgemmPlan {
     int32_t *shift_dev = nullptr;   // [kpad]
     uint8_t *row_cls_dev = nullptr, *col_cls_dev = nullptr;
     int rev = 0;                    // reversed tile traversal (conv_igemm_set_reverse)
-    const uint8_t *next_ro = nullptr;   // what the next launch reads first (conv_igemm_set_next_readonly)
-    uint32_t next_ro_bytes = 0;
+    NextRead next;                  // what the next launch reads first (conv_igemm_set_next_readonly)
     size_t w_bytes = 0;             // size of w_dev
     // fused residual add (conv_igemm_set_residual)
     bool has_res = false;
@@ -725,9 +724,15 @@ static void choose_tile(int ow, int oh, int n, int *tw, int *th, int *tn, int mi
 void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
 {
     const ConvIgemmPlan::Launch *l = p->last_launch();      // the tiling depends on the batch of the run
+    auto prefetch = [&](uint32_t bytes) {
+        const size_t used = strlen(buf);
+        if (bytes != 0)
+            snprintf(buf + used, len - used, ", prefetches %u bytes", bytes);
+    };
     if (l && l->small) {
         snprintf(buf, len, "tcgen05 igemm: bn=%d bk=%d slots=%d split=%d one tile per %s", l->sargs.bn, p->bk, l->sargs.slots, l->sargs.split,
                  l->sargs.split > 1 ? "cluster" : "CTA");
+        prefetch(l->sargs.next_ro_bytes);
         return;
     }
     const bool cta_pair = l && l->cta_pair;
@@ -738,6 +743,8 @@ void conv_igemm_describe(const ConvIgemmPlan *p, char *buf, size_t len)
              l ? l->args.stages : p->stages, l ? l->args.kgroup : p->kgroup, p->groups, p->acc_stages, mode, (l ? l->args.b_resident : p->b_resident) ? ", weights resident" : "",
              p->form == kEpiFp ? ", fp32 epilogue" : p->form == kEpiInt ? ", uniform-shift epilogue" : ", generic requantize",
              p->rev ? ", reversed" : "");
+    if (l)
+        prefetch(l->args.next_ro_bytes);
 }
 
 void conv_igemm_set_reverse(ConvIgemmPlan *p, int reverse)
@@ -754,17 +761,21 @@ void conv_igemm_weights(const ConvIgemmPlan *p, const uint8_t **ptr, size_t *byt
     *bytes = p->w_bytes;
 }
 
-void conv_igemm_set_next_readonly(ConvIgemmPlan *p, const uint8_t *ptr, size_t bytes)
+void conv_igemm_set_next_readonly(ConvIgemmPlan *p, const NextRead &next)
 {
-    // 16-byte granules (the bulk prefetch's unit); anything beyond 64 MiB would only evict what the layers between need
-    if (((uintptr_t)ptr & 15) != 0 || bytes > (64u << 20))
-        ptr = nullptr;
-    const uint32_t b = ptr ? (uint32_t)(bytes & ~(size_t)15) : 0u;
-    if (p->next_ro != ptr || p->next_ro_bytes != b) {
-        p->next_ro = ptr;
-        p->next_ro_bytes = b;
-        p->saved.clear();
-    }
+    p->next = next;
+    p->saved.clear();
+}
+
+// The bulk prefetch of a launch of n images, in its unit of 16 bytes; more than 64 MiB would only evict what the layers between need.
+static void next_read(const ConvIgemmPlan *p, int n, const uint8_t **ptr, uint32_t *bytes)
+{
+    const bool grouped = n >= p->next.from && n <= p->next.to;
+    const uint8_t *w = grouped ? p->next.grouped : p->next.plain;
+    const size_t size = grouped ? p->next.grouped_bytes : p->next.plain_bytes;
+    const bool fits = w && ((uintptr_t)w & 15) == 0 && size <= (64u << 20);
+    *ptr = fits ? w : nullptr;
+    *bytes = fits ? (uint32_t)(size & ~(size_t)15) : 0u;
 }
 
 int conv_igemm_set_residual(ConvIgemmPlan *p, const EltwiseArgs &e, int conv_input)
@@ -959,7 +970,7 @@ static int build_small(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, in
     a.wzp_d = g.wzp_d;
     a.y = y;
     a.status = status;
-    a.next_ro = p->next_ro; a.next_ro_bytes = p->next_ro_bytes;
+    next_read(p, n, &a.next_ro, &a.next_ro_bytes);
     if (ws && g.k % 16 == 0 && !g.act_signed) {         // (other channel counts leave through staged rows)
         const int ci = ws->conv_input, other = 1 - ci;
         const EltwiseArgs &e = *ws->elt;
@@ -1091,7 +1102,7 @@ static int build_launch(ConvIgemmPlan *p, const uint8_t *x, int n, uint8_t *y, i
     a.ozp = g.ozp; a.qmax = g.qmax; a.relu_lo = g.relu_lo;
     a.out_flip = g.act_signed ? 0x80808080u : 0u;
     a.rev = p->rev;
-    a.next_ro = p->next_ro; a.next_ro_bytes = p->next_ro_bytes;
+    next_read(p, n, &a.next_ro, &a.next_ro_bytes);
     a.use_tma_store = (g.k % 16 == 0) ? 1 : 0;
     a.y = y;
     a.res = res;

@@ -272,7 +272,20 @@ int reserve_beside_groups(b200_conv *conv, int32_t n, cudaStream_t st)
 
 bool b200::conv_runs_grouped(const b200_conv *cv, const uint8_t *x, int32_t n)
 {
-    return cv->grouped && cv->algo == B200_CONV_ALGO_IGEMM && ((uintptr_t)x & 15) == 0 && (cv->pad_c && !cv->lowered ? 2.5 + n * cv->grouped_gain > 0.0 : n >= cv->grouped_from);
+    return cv->grouped && cv->algo == B200_CONV_ALGO_IGEMM && !cv->fused_residual && ((uintptr_t)x & 15) == 0 && n >= cv->grouped_from && n <= cv->grouped_to;
+}
+
+NextRead b200::conv_weights_read(const b200_conv *cv)
+{
+    NextRead r;
+    if (cv->algo == B200_CONV_ALGO_IGEMM)
+        conv_igemm_weights(cv->igemm, &r.plain, &r.plain_bytes);
+    if (cv->grouped && cv->algo == B200_CONV_ALGO_IGEMM && !cv->fused_residual) {
+        conv_igemm_weights(cv->grouped, &r.grouped, &r.grouped_bytes);
+        r.from = cv->grouped_from;
+        r.to = cv->grouped_to;
+    }
+    return r;
 }
 
 extern "C" {
@@ -564,7 +577,9 @@ int b200_conv2d_create(
             create_grouped(g, m, flat, w_s8, bias, mult, shift, &cv->grouped);
             const double factor = flat ? m : m * ((g.s - 1 + m - 1) / m + 1.0) / g.s;
             const double pixels = (double)g.oh * g.ow;
-            cv->grouped_gain = (double)g.h * g.w * (g.c + 2 * cv->pad_c) / 5e6 - pixels * 2.0 * (factor - 1.0) * g.c * taps * g.k / 1e9;
+            const double gain = (double)g.h * g.w * (g.c + 2 * cv->pad_c) / 5e6 - pixels * 2.0 * (factor - 1.0) * g.c * taps * g.k / 1e9;    // us an image
+            if (gain < 0.0)
+                cv->grouped_to = (int)std::min(std::ceil(2.5 / -gain) - 1.0, (double)INT32_MAX);
         }
     }
     if (rc == B200_OK) {

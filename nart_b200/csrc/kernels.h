@@ -156,9 +156,15 @@ void conv_igemm_destroy(ConvIgemmPlan *plan);
 // depend on it; a consumer that walks against its producer's direction starts on data still in L2.
 void conv_igemm_set_reverse(ConvIgemmPlan *plan, int reverse);
 // The repacked weights of a plan (device pointer, bytes), and the read-only operand of the launch that follows this
-// plan's: the kernel asks for it to be brought into L2 while it runs (nullptr: none).
+// plan's: the kernel asks for it to be brought into L2 while it runs.  Launches of from .. to images ask for `grouped`, all
+// others for `plain` (nullptr: nothing).
+struct NextRead {
+    const uint8_t *plain = nullptr, *grouped = nullptr;
+    size_t plain_bytes = 0, grouped_bytes = 0;
+    int from = 1, to = 0;
+};
 void conv_igemm_weights(const ConvIgemmPlan *plan, const uint8_t **ptr, size_t *bytes);
-void conv_igemm_set_next_readonly(ConvIgemmPlan *plan, const uint8_t *ptr, size_t bytes);
+void conv_igemm_set_next_readonly(ConvIgemmPlan *plan, const NextRead &next);
 // One line of text naming the plan's tiling and kernel variant.
 void conv_igemm_describe(const ConvIgemmPlan *plan, char *buf, size_t len);
 // Per-process / per-device set-up of the tensor-core kernels (driver entry point, shared-memory
@@ -192,12 +198,9 @@ struct b200_conv {
     int pad_c = 0;
     b200::ConvGeom g_pad;
     uint8_t *padded = nullptr;      // [n][h][w][pad_c]
-    // The same conv on groups of neighbouring pixels (create_grouped), for aligned activations.  Where that leaves out the padded copy: what
-    // a run gains by it per image, in microseconds (below zero: it loses) beside the copy's launch; else the images from which on it
-    // is the faster.
+    // The same conv on groups of neighbouring pixels (create_grouped), for aligned activations of grouped_from .. grouped_to images.
     b200::ConvIgemmPlan *grouped = nullptr;
-    double grouped_gain = 0.0;
-    int grouped_from = 0;
+    int grouped_from = 0, grouped_to = INT32_MAX;
     std::atomic<bool> ran_grouped{ false };     // the last run did (b200_conv2d_describe)
     size_t padded_bytes = 0;
     // One owner orders all runs of the plan, on whatever streams, and keeps it longer than the graphs it captures (the case
@@ -216,5 +219,7 @@ struct b200_conv {
 namespace b200 {
 // Whether a run takes the plan on groups of pixels.
 bool conv_runs_grouped(const b200_conv *conv, const uint8_t *x, int32_t n);
+// The weights that runs of the plan read, on aligned activations.
+NextRead conv_weights_read(const b200_conv *conv);
 }  // namespace b200
 

@@ -130,6 +130,29 @@ def test_few_output_channels_on_groups_of_pixels(shape):
     assert torch.equal(conv(x), want) and ops.device_status() == 0
 
 
+@pytest.mark.parametrize("fused", [False, True])
+def test_the_prefetched_weights_are_those_that_are_read(fused):
+    """In a case a conv asks for the next one's weights: on groups of pixels from a tile an SM on (twice the columns and twice the
+    depth here), and never where that conv has taken over a residual add."""
+    from nart_b200.case import Case
+    n = 200
+    wt, bias, x, q = _inputs(64, 64, 1, 1, 28, 28, n, 6)
+    x = x.cpu().numpy().transpose(0, 3, 1, 2).copy()
+    cs = Case()
+    cs.set_fusion(fused)
+    image = cs.input_u8(64, 28, 28)
+    a = cs.conv2d(image, wt, bias, **q)
+    b = cs.conv2d(a, wt, bias, **q)
+    cs.output_u8(cs.eltwise_sum([b, a], (q["oalpha"],) * 2, (q["ozp"],) * 2, 0.05, 120))
+    cs.prepare(n)
+    for batch, on_groups in ((n, not fused), (1, False), (n, not fused)):
+        cs.run_host([x[:batch]], [(np.uint8, (64, 28, 28))])
+        first, second = cs.describe()[:2]
+        assert ("groups of pixels" in second) == on_groups, second
+        assert "prefetches %d bytes" % (64 * 64 * (4 if on_groups else 1)) in first, (batch, first)
+    cs.close()
+
+
 def test_describe_names_what_the_last_run_took():
     """Entry points that never run on groups, after a run that did."""
     import torch
