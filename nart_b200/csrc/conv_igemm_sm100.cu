@@ -255,22 +255,15 @@ static void epilogue_segments(int bn, int warps_per_quarter, int (&w)[2])
     w[1] = (t - a) * 16;
 }
 
-// One filter's weights [c][taps] to [taps][pitch], with the sum of each tap.
-void weights_tap_major(const int8_t *w, int c, int taps, int8_t *dst, int pitch, int32_t *sums)
+// One filter's weights [taps][c] to [taps][pitch], with the sum of each tap.
+void weights_to_pitch(const int8_t *w, int c, int taps, int8_t *dst, int pitch, int32_t *sums)
 {
     for (int t = 0; t < taps; ++t) {
-        int8_t *row = dst + (size_t)t * pitch;
+        const int8_t *src = w + (size_t)t * c;
+        memcpy(dst + (size_t)t * pitch, src, c);
         int32_t sum = 0;
-        if (taps == 1) {
-            memcpy(row, w, c);
-            for (int i = 0; i < c; ++i)
-                sum += w[i];
-        } else {
-            for (int i = 0; i < c; ++i) {
-                row[i] = w[(size_t)i * taps + t];
-                sum += row[i];
-            }
-        }
+        for (int i = 0; i < c; ++i)
+            sum += src[i];
         sums[t] = sum;
     }
 }
@@ -292,29 +285,34 @@ int conv_igemm_supported(const ConvGeom &g, char *why, size_t why_len)
 }
 
 // Distinct sets of in-image taps along one axis: cls[o] = class of output coordinate o, and
-// valid[class] = bit mask of taps that fall inside the image.
+// valid[class][t] = whether tap t falls inside the image.  The taps of a coordinate that do are neighbours: two numbers a class.
 static void tap_classes(int out, int in, int kernel, int pad, int stride, std::vector<uint8_t> &cls,
                         std::vector<std::vector<char>> &valid)
 {
     cls.resize(out);
     valid.clear();
+    std::vector<std::pair<int, int>> spans;         // [first, end) of the taps inside, per class
+    size_t id = 0;
     for (int o = 0; o < out; ++o) {
-        std::vector<char> v(kernel);
-        for (int t = 0; t < kernel; ++t) {
-            int i = o * stride + t - pad;
-            v[t] = (i >= 0 && i < in) ? 1 : 0;
-        }
-        int id = -1;
-        for (size_t j = 0; j < valid.size(); ++j)
-            if (valid[j] == v) {
-                id = (int)j;
-                break;
+        const long long at = (long long)o * stride - pad;
+        std::pair<int, int> span((int)std::max(0ll, -at), (int)std::min((long long)kernel, in - at));
+        if (span.first >= span.second)
+            span = { 0, 0 };
+        if (id >= spans.size() || spans[id] != span) {
+            id = 0;
+            while (id < spans.size() && spans[id] != span)
+                ++id;
+            if (id == spans.size()) {
+                spans.push_back(span);
+                valid.emplace_back(kernel, 0);
+                std::fill(valid[id].begin() + span.first, valid[id].begin() + span.second, 1);
             }
-        if (id < 0) {
-            valid.push_back(v);
-            id = (int)valid.size() - 1;
         }
-        cls[o] = (uint8_t)id;
+        int last = o;
+        if (span.first == 0 && span.second == kernel)       // all up to the other border
+            last = (int)std::min((long long)out - 1, ((long long)in - kernel + pad) / stride);
+        std::fill(cls.begin() + o, cls.begin() + last + 1, (uint8_t)id);
+        o = last;
     }
 }
 
@@ -552,13 +550,13 @@ int conv_igemm_create(
     if (quads) {        // [kpad][r][pixels of a row][16]
         std::vector<int8_t> row((size_t)taps * 16);
         for (int k = 0; k < g.k; ++k) {
-            weights_tap_major(&w_s8[(size_t)k * g.c * taps], g.c, taps, row.data(), 16, &wtap[(size_t)k * taps]);
+            weights_to_pitch(&w_s8[(size_t)k * g.c * taps], g.c, taps, row.data(), 16, &wtap[(size_t)k * taps]);
             for (int rr = 0; rr < g.r; ++rr)
                 memcpy(&wp[((size_t)k * g.r + rr) * p->cpad], &row[(size_t)rr * g.s * 16], (size_t)g.s * 16);
         }
     } else {
         for (int k = 0; k < g.k; ++k)
-            weights_tap_major(&w_s8[(size_t)k * g.c * taps], g.c, taps, &wp[(size_t)k * taps * p->cpad], p->cpad, &wtap[(size_t)k * taps]);
+            weights_to_pitch(&w_s8[(size_t)k * g.c * taps], g.c, taps, &wp[(size_t)k * taps * p->cpad], p->cpad, &wtap[(size_t)k * taps]);
     }
     // ---- border classes and offsets ---------------------------------------------------------------
     std::vector<uint8_t> row_cls, col_cls;
@@ -663,27 +661,32 @@ int conv_igemm_create(
         { row_cls.data(), row_cls.size(), (void **)&p->row_cls_dev },
         { col_cls.data(), col_cls.size(), (void **)&p->col_cls_dev },
     };
-    size_t small = 0;       // what goes behind the weights, copied together
+    size_t small = 0;       // what goes behind the weights
     for (auto &q : parts)
         small += q.src == wp.data() ? 0 : (q.bytes + 255) / 256 * 256;
     const size_t behind = (wp.size() + 255) / 256 * 256;
-    std::vector<uint8_t> tables(small);
+    // copied together, small weights with them: a copy costs what moving 50 KB on the host does
+    const size_t lead = wp.size() <= (64u << 10) ? behind : 0;
+    std::vector<uint8_t> tables(lead + small);
     auto upload_all = [&]() -> int {
         B200_CUDA_TRY(cudaMalloc((void **)&p->block_dev, behind + small));
         size_t at = 0;
         for (auto &q : parts) {
             if (q.src == wp.data()) {
                 *q.dst = p->block_dev;
+                if (lead != 0)
+                    memcpy(tables.data(), wp.data(), wp.size());
                 continue;
             }
             if (q.bytes == 0)
                 continue;
-            memcpy(&tables[at], q.src, q.bytes);
+            memcpy(&tables[lead + at], q.src, q.bytes);
             *q.dst = p->block_dev + behind + at;
             at += (q.bytes + 255) / 256 * 256;
         }
-        B200_CUDA_TRY(cudaMemcpy(p->block_dev, wp.data(), wp.size(), cudaMemcpyHostToDevice));
-        B200_CUDA_TRY(cudaMemcpy(p->block_dev + behind, tables.data(), at, cudaMemcpyHostToDevice));
+        if (lead == 0)
+            B200_CUDA_TRY(cudaMemcpy(p->block_dev, wp.data(), wp.size(), cudaMemcpyHostToDevice));
+        B200_CUDA_TRY(cudaMemcpy(p->block_dev + behind - lead, tables.data(), lead + at, cudaMemcpyHostToDevice));
         return B200_OK;
     };
     const int rc = upload_all();

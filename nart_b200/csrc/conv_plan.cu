@@ -28,6 +28,29 @@ int upload(const std::vector<T> &v, T **dev)
     return B200_OK;
 }
 
+// The weights and tables of the CUDA-core kernel: one block that w_dev owns, one copy, or two where the weights are large (an allocation
+// and a copy cost 8 us, moving 64 KB on the host 5).
+int upload_direct(const std::vector<int8_t> &w, const std::vector<int32_t> &bias, const std::vector<uint32_t> &mult, const std::vector<int32_t> &shift, ConvDirectPlan *d)
+{
+    const size_t each = (bias.size() * 4 + 255) / 256 * 256, behind = (w.size() + 255) / 256 * 256, lead = w.size() <= (64u << 10) ? behind : 0;
+    std::vector<uint8_t> image(lead + 3 * each);
+    if (lead != 0)
+        memcpy(image.data(), w.data(), w.size());
+    memcpy(&image[lead], bias.data(), bias.size() * 4);
+    memcpy(&image[lead + each], mult.data(), mult.size() * 4);
+    memcpy(&image[lead + 2 * each], shift.data(), shift.size() * 4);
+    uint8_t *block = nullptr;
+    B200_CUDA_TRY(cudaMalloc((void **)&block, behind + 3 * each));
+    d->w_dev = reinterpret_cast<int8_t *>(block);
+    d->bias_fold_dev = reinterpret_cast<int32_t *>(block + behind);
+    d->mult_dev = reinterpret_cast<uint32_t *>(block + behind + each);
+    d->shift_dev = reinterpret_cast<int32_t *>(block + behind + 2 * each);
+    if (lead == 0)
+        B200_CUDA_TRY(cudaMemcpy(block, w.data(), w.size(), cudaMemcpyHostToDevice));
+    B200_CUDA_TRY(cudaMemcpy(block + behind - lead, image.data(), image.size(), cudaMemcpyHostToDevice));
+    return B200_OK;
+}
+
 // A plan's scratch tensors (they grow with the batch, so the first run allocates them).  Small ones come from a pool per device
 // that keeps up to 64 MB of what was given back: mapping fresh device memory costs 0.3 .. 2.6 ms, taking it from the pool
 // some 10 us.
@@ -105,9 +128,6 @@ void destroy_conv(b200_conv *cv)
     cudaFree(cv->direct.w_dw3p_dev);
     cudaFree(cv->direct.q_dw3_dev);
     cudaFree(cv->direct.q_dw3p_dev);
-    cudaFree(cv->direct.bias_fold_dev);
-    cudaFree(cv->direct.mult_dev);
-    cudaFree(cv->direct.shift_dev);
     if (cv->igemm)
         conv_igemm_destroy(cv->igemm);
     if (cv->grouped)
@@ -205,23 +225,21 @@ int create_grouped(const ConvGeom &g, int m, bool flat, const std::vector<int8_t
     q.c = m * g.c; q.w /= m; q.ow /= per; q.k = per * g.k; q.s = last - first + 1; q.pad_w = -first; q.stride_w = 1;
     if (quads && q.s > 8)
         return B200_ERR_UNSUPPORTED;
-    std::vector<int8_t> wq((size_t)q.k * q.c * q.r * q.s, 0);       // [k][c][r][s]
+    std::vector<int8_t> wq((size_t)q.k * q.c * q.r * q.s, 0);
     std::vector<int32_t> bq(bias ? q.k : 0), sq(q.k);
     std::vector<uint32_t> mq(q.k);
-    for (int o = 0; o < per; ++o)
-        for (int k = 0; k < g.k; ++k) {
+    for (int k = 0; k < g.k; ++k) {
+        for (int o = 0; o < per; ++o) {
             const int kq = o * g.k + k;
             if (bias)
                 bq[kq] = bias[k];
             mq[kq] = mult[k];
             sq[kq] = shift[k];
-            for (int c = 0; c < g.c; ++c)
-                for (int rr = 0; rr < g.r; ++rr)
-                    for (int ss = 0; ss < g.s; ++ss) {
-                        const int px = o * g.stride_w + ss - g.pad_w - first * m;      // from the window's first pixel on
-                        wq[(((size_t)kq * q.c + px % m * g.c + c) * q.r + rr) * q.s + px / m] = w[(((size_t)k * g.c + c) * g.r + rr) * g.s + ss];
-                    }
+            for (int rr = 0; rr < g.r; ++rr)        // a row of the window lies in the groups as it does in the image
+                memcpy(&wq[((size_t)kq * q.r + rr) * q.s * q.c + (size_t)(o * g.stride_w - g.pad_w - first * m) * g.c],
+                       &w[((size_t)k * g.r + rr) * g.s * g.c], (size_t)g.s * g.c);
         }
+    }
     return conv_igemm_create(q, wq, bias ? bq.data() : nullptr, mq.data(), sq.data(), out, false, 0, quads);
 }
 
@@ -352,9 +370,20 @@ int b200_conv2d_create(
     // (gemm/default/gemm.c:306-355), so no bound on the reduction length is needed.
     // Any stored byte minus 128 is an int8; a weight zero point other than 128 is carried as
     // wzp_d = wzp - 128 and applied through the sum of the activations (ConvGeom::wzp_d).
-    std::vector<int8_t> w_s8(wcount);   // [k][cg][r][s], value = stored - 128
-    for (size_t i = 0; i < wcount; ++i)
-        w_s8[i] = s8 ? (int8_t)weights[i] : (int8_t)((int)weights[i] - 128);
+    std::vector<int8_t> w_s8(wcount);   // [k][r][s][cg], value = stored - 128
+    const int minus = s8 ? 0 : 128;
+    for (int k = 0; k < g.k; ++k) {
+        const uint8_t *src = weights + (size_t)k * cg * taps;
+        int8_t *dst = &w_s8[(size_t)k * cg * taps];
+        if (taps == 1 || cg == 1) {
+            for (int i = 0; i < cg * taps; ++i)
+                dst[i] = (int8_t)(src[i] - minus);
+            continue;
+        }
+        for (int t = 0; t < taps; ++t)
+            for (int c = 0; c < cg; ++c)
+                dst[(size_t)t * cg + c] = (int8_t)(src[(size_t)c * taps + t] - minus);
+    }
 
     std::vector<uint32_t> mult(g.k);
     std::vector<int32_t> shift(g.k);
@@ -382,7 +411,7 @@ int b200_conv2d_create(
     std::vector<int8_t> w_pack((size_t)g.k * taps * cg4, 0);
     std::vector<int32_t> bias_fold(g.k), tap_sum(taps);
     for (int k = 0; k < g.k; ++k) {
-        weights_tap_major(&w_s8[(size_t)k * cg * taps], cg, taps, &w_pack[(size_t)k * taps * cg4], cg4, tap_sum.data());
+        weights_to_pitch(&w_s8[(size_t)k * cg * taps], cg, taps, &w_pack[(size_t)k * taps * cg4], cg4, tap_sum.data());
         long long wsum = 0;
         for (int t = 0; t < taps; ++t)
             wsum += tap_sum[t];
@@ -390,10 +419,7 @@ int b200_conv2d_create(
         bias_fold[k] = (int32_t)(uint32_t)(unsigned long long)bf;   // modulo 2^32
     }
     cv->direct.cg4 = cg4;
-    int rc = upload(w_pack, &cv->direct.w_dev);
-    if (rc == B200_OK) rc = upload(bias_fold, &cv->direct.bias_fold_dev);
-    if (rc == B200_OK) rc = upload(mult, &cv->direct.mult_dev);
-    if (rc == B200_OK) rc = upload(shift, &cv->direct.shift_dev);
+    int rc = upload_direct(w_pack, bias_fold, mult, shift, &cv->direct);
     if (rc == B200_OK && g.group == g.c && g.group == g.k && g.c % 16 == 0) {
         std::vector<int8_t> w_dw((size_t)taps * g.c);
         for (int c = 0; c < g.c; ++c)
@@ -497,8 +523,8 @@ int b200_conv2d_create(
             cv->pad_c = gt.c;
             cv->g_pad = gt;
             w_pad.assign((size_t)g.k * gt.c * taps, 0);
-            for (int k = 0; k < g.k; ++k)
-                memcpy(&w_pad[(size_t)k * gt.c * taps], &w_s8[(size_t)k * g.c * taps], (size_t)g.c * taps);
+            for (size_t i = 0; i < (size_t)g.k * taps; ++i)
+                memcpy(&w_pad[i * gt.c], &w_s8[i * g.c], g.c);
             wt = &w_pad;
         }
     }
@@ -517,12 +543,9 @@ int b200_conv2d_create(
         gl.s = 1;
         gl.pad_w = 0;
         gl.stride_w = 1;
-        std::vector<int8_t> w_low((size_t)g.k * gl.c * g.r, 0);   // [k][32][r][1]
-        for (int k = 0; k < g.k; ++k)
-            for (int c = 0; c < 4; ++c)
-                for (int rr = 0; rr < g.r; ++rr)
-                    for (int j = 0; j < g.s; ++j)
-                        w_low[((size_t)k * gl.c + j * 4 + c) * g.r + rr] = (*wt)[(((size_t)k * 4 + c) * g.r + rr) * g.s + j];
+        std::vector<int8_t> w_low((size_t)g.k * gl.c * g.r, 0);   // [k][r][1][32]
+        for (size_t i = 0; i < (size_t)g.k * g.r; ++i)
+            memcpy(&w_low[i * gl.c], &(*wt)[i * g.s * 4], (size_t)g.s * 4);
         rc = conv_igemm_create(gl, w_low, bias, mult.data(), shift.data(), &cv->igemm, true, g.s);
         if (rc == B200_OK) {
             cv->lowered = true;

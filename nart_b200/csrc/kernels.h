@@ -90,7 +90,7 @@ struct ConvGeom {
 // zero filled), bias_fold[k] = bias[k] - izp * sum(w[k]) so that out-of-image taps, read as izp,
 // contribute nothing.
 struct ConvDirectPlan {
-    int8_t *w_dev = nullptr;
+    int8_t *w_dev = nullptr;      // and behind it, in one block, bias_fold_dev, mult_dev and shift_dev
     int8_t *w_dw_dev = nullptr;   // depthwise only: [r][s][c] int8
     // depthwise 3x3 with every requantize shift >= 33 and 8-bit output: weights as dp4a words
     // [c/4][3 tap groups][4 channels] (taps 0-3, 4-7, 8 of one channel per word) and per channel
@@ -125,10 +125,10 @@ int conv_pad_channels_launch(const uint8_t *x, uint8_t *y, size_t pixels, int c,
 
 // Implicit-GEMM (tcgen05) convolution plan; defined in conv_igemm_sm100.cu.
 struct ConvIgemmPlan;
-void weights_tap_major(const int8_t *w, int c, int taps, int8_t *dst, int pitch, int32_t *sums);
+void weights_to_pitch(const int8_t *w, int c, int taps, int8_t *dst, int pitch, int32_t *sums);
 int conv_igemm_supported(const ConvGeom &g, char *why, size_t why_len);
 int conv_igemm_create(
-    const ConvGeom &g, const std::vector<int8_t> &w_s8 /* [k][c][r][s] */, const int32_t *bias,
+    const ConvGeom &g, const std::vector<int8_t> &w_s8 /* [k][r][s][c] */, const int32_t *bias,
     const uint32_t *mult, const int32_t *shift, ConvIgemmPlan **plan, bool a_row_swizzled = false,
     int window = 0, bool quads = false);
 // a_row_swizzled: the activation tensor has 32 channels, the kernel is r x 1 with no horizontal

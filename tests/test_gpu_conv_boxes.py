@@ -130,6 +130,19 @@ def test_few_output_channels_on_groups_of_pixels(shape):
     assert torch.equal(conv(x), want) and ops.device_status() == 0
 
 
+def test_preparation_does_not_grow_with_the_map():
+    """All pixels of a 1x1 conv's image are one line of groups: 4 million of them here, of one kind (66 ms when each was looked at)."""
+    import time
+    from nart_b200 import ops
+    wt, bias, _, q = _inputs(16, 16, 1, 1, 8, 8, 1, 2)
+    took = []
+    for _ in range(5):
+        start = time.perf_counter()
+        ops.Conv2d(wt, bias, in_hw=(4096, 4096), relu=True, **q)
+        took.append(time.perf_counter() - start)
+    assert min(took) < 0.015, took
+
+
 @pytest.mark.parametrize("fused", [False, True])
 def test_the_prefetched_weights_are_those_that_are_read(fused):
     """In a case a conv asks for the next one's weights: on groups of pixels from a tile an SM on (twice the columns and twice the
