@@ -211,6 +211,8 @@ int create_grouped(const ConvGeom &g, int m, bool flat, const std::vector<int8_t
     *out = nullptr;
     ConvGeom q = g;
     if (flat) {
+        if ((long long)g.h * g.w > INT32_MAX)
+            return B200_ERR_UNSUPPORTED;
         q.w = q.ow = g.h * g.w;
         q.h = q.oh = 1;
     }
@@ -578,7 +580,7 @@ int b200_conv2d_create(
         const bool one = taps == 1;
         auto worth = [&](int m) {
             const int columns = m * g.k, depth = m * g.c;
-            if ((flat ? g.h * g.w : g.w) % m != 0 || (!flat && g.ow % m != 0))
+            if ((flat ? (long long)g.h * g.w : g.w) % m != 0 || (!flat && g.ow % m != 0))
                 return false;
             if (one)
                 return columns <= (g.c == 16 ? 192 : 128) && depth <= (columns <= 64 ? 512 : 384);

@@ -143,6 +143,14 @@ def test_preparation_does_not_grow_with_the_map():
     assert min(took) < 0.015, took
 
 
+def test_plans_of_maps_of_more_than_two_billion_pixels():
+    """Too long a line for groups (its pixels are counted in 31 bits): the plan is made without."""
+    from nart_b200 import ops
+    wt, bias, _, q = _inputs(16, 16, 1, 1, 8, 8, 1, 2)
+    conv = ops.Conv2d(wt, bias, in_hw=(46344, 46344), relu=True, **q)
+    assert conv.algo == ops.ALGO_IGEMM
+
+
 @pytest.mark.parametrize("fused", [False, True])
 def test_the_prefetched_weights_are_those_that_are_read(fused):
     """In a case a conv asks for the next one's weights: on groups of pixels from a tile an SM on (twice the columns and twice the
