@@ -252,10 +252,9 @@ int tile_an_sm(const ConvGeom &g, int m)
     return (int)(((size_t)sm_count() * 128 * per + (size_t)g.oh * g.ow - 1) / ((size_t)g.oh * g.ow));
 }
 
-// Scratch tensors that serve every run of the plan, for n images, and the rows of a lowered one for n_lowered
-int reserve_owned(b200_conv *conv, int32_t n, int32_t n_lowered)
+// Scratch tensors that serve every run of the plan: a copy with padded channels for n_padded images, a lowered one's rows for n_lowered
+int reserve_owned(b200_conv *conv, int32_t n_padded, int32_t n_lowered)
 {
-    const PaddedBytes need(conv, n);
     auto grow = [conv](uint8_t *&buf, size_t &have, size_t need) -> int {
         if (need <= have)
             return B200_OK;
@@ -270,7 +269,7 @@ int reserve_owned(b200_conv *conv, int32_t n, int32_t n_lowered)
     if (conv->lowered)
         B200_TRY(grow(conv->scratch, conv->scratch_bytes, PaddedBytes(conv, n_lowered).lowered));
     if (conv->pad_c)
-        B200_TRY(grow(conv->padded, conv->padded_bytes, need.padded));
+        B200_TRY(grow(conv->padded, conv->padded_bytes, PaddedBytes(conv, n_padded).padded));
     return B200_OK;
 }
 
@@ -728,8 +727,9 @@ int b200_conv2d_reserve(b200_conv_t *conv, int32_t n)
         return fail(B200_ERR_INVALID, "conv(reserve): bad argument");
     std::lock_guard<std::mutex> lock(conv->mu);
     if (!conv->pad_c || conv->one_owner) {
-        // (a case's tensors are aligned: its larger launches run on groups)
-        const int rc = reserve_owned(conv, n, conv->one_owner && conv->grouped ? std::min(n, conv->grouped_from - 1) : n);
+        // a case's tensors are aligned: launches on groups need neither the rows nor (their pixels are the conv's own) the copy
+        const bool groups = conv->one_owner && conv->grouped;
+        const int rc = reserve_owned(conv, groups && !conv->lowered && n <= conv->grouped_to ? 0 : n, groups ? std::min(n, conv->grouped_from - 1) : n);
         if (rc != B200_ERR_NOMEM || !conv->pad_c)
             return rc;
         conv->algo = B200_CONV_ALGO_DIRECT;         // needs no scratch

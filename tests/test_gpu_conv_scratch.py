@@ -192,3 +192,27 @@ def test_case_counts_the_copy_into_the_padded_tensor(port):
     (got,) = cs.run_host([x], [(np.uint8, (32, 9, 9))])
     cs.close()
     assert np.array_equal(got, port.conv2d_u8(x, wt, np.zeros(32, np.int32), (1, 1), (1, 1), 1, 0.02, 120, q["walpha"], 128, 0.5, 99))
+
+
+def test_case_keeps_no_copy_for_a_conv_that_runs_on_groups():
+    """24 channels on pairs of pixels at every batch: the case holds its tensors and staging buffers, and no padded tensor beside them."""
+    from nart_b200.case import Case
+    rng = np.random.default_rng(6)
+    n, hw = 200, 112
+    wt = rng.integers(0, 256, (32, 24, 1, 1), dtype=np.uint8)
+    cs = Case()
+    cs.output_u8(cs.conv2d(cs.input_u8(24, hw, hw), wt, None, ialpha=0.02, izp=120, walpha=np.float32([0.005]), oalpha=0.5, ozp=99))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    cs.prepare(n)
+    held = before - torch.cuda.mem_get_info()[0]
+    pixels = n * hw * hw
+    assert held < 2 * pixels * (24 + 32) + (32 << 20), held         # (with the copy 32 bytes a pixel more, 80 MB)
+    assert cs.launch_count() == 3
+    x = rng.integers(0, 256, (n, 24, hw, hw), dtype=np.uint8)
+    (got,) = cs.run_host([x], [(np.uint8, (32, hw, hw))])
+    cs.close()
+    from nart_b200 import ops
+    plan = ops.Conv2d(wt, None, in_hw=(hw, hw), algo=ops.ALGO_DIRECT, ialpha=0.02, izp=120, walpha=np.float32([0.005]), oalpha=0.5, ozp=99)
+    want = plan(torch.from_numpy(x).cuda().permute(0, 2, 3, 1).contiguous())
+    assert torch.equal(torch.from_numpy(got).cuda().view(n, 32, hw, hw).permute(0, 2, 3, 1), want)
