@@ -395,7 +395,8 @@ B200_API int b200_case_run_host(
 B200_API int b200_case_submit_host(
     b200_case_t *cs, int32_t batch, const void *const *inputs, void *const *outputs);
 B200_API int b200_case_wait(b200_case_t *cs);
-/* A line of text per op, as b200_conv2d_describe has it for convolutions: what the last launch of each was. */
+/* A line of text per op, as b200_conv2d_describe has it for convolutions: what the last launch of each was.  Behind them, after
+ * b200_case_run_host, whether the last one took its images in two parts. */
 B200_API int b200_case_describe(const b200_case_t *cs, char *buf, size_t len);
 /* Number of kernels one b200_case_run_device of max_batch images launches.  (A residual add that a small conv launch forms itself still counts.) */
 B200_API int b200_case_launch_count(const b200_case_t *cs, int32_t *launches);

@@ -121,7 +121,7 @@ class Case:
         return v.value
 
     def describe(self):
-        """A line per op: the kernel variant of its last launch (b200_case_describe)."""
+        """A line per op, the kernel variant of its last launch, and one on the last host run (b200_case_describe)."""
         buf = C.create_string_buffer(1 << 16)
         check(lib.b200_case_describe(self._h, buf, len(buf)))
         return buf.value.decode().splitlines()

@@ -118,6 +118,7 @@ struct b200_case {
     int *status_host = nullptr;        // pinned: the device status word as the end of a run found it
     int *publish_to = nullptr;         // a host run wants it there: the last output's kernel does it where it can (published)
     bool published = false;
+    int host_parts[2] = { 0, 0 };      // images in the parts of the last host run
 };
 
 namespace {
@@ -1066,6 +1067,8 @@ static int run_on_host_buffers(b200_case_t *cs, int32_t batch, const void *const
             cs->outputs[i].direct = direct_view(outputs[i], cs->outputs[i].bytes_per_image * batch);
     cs->publish_to = cs->status_host;
     cs->published = false;
+    cs->host_parts[0] = split ? first_part(batch) : batch;
+    cs->host_parts[1] = batch - cs->host_parts[0];
     if (split)
         B200_TRY(split_host_run(cs, batch, inputs, stream));
     else
@@ -1163,14 +1166,18 @@ int b200_case_describe(const b200_case_t *cs, char *buf, size_t len)
         return fail(B200_ERR_INVALID, "case_describe: bad argument");
     buf[0] = 0;
     size_t used = 0;
+    auto add = [&](int n) { used += n < 0 || (size_t)n >= len - used ? len - used - 1 : (size_t)n; };
     for (const auto &op : cs->ops) {
         static const char *const names[] = { "conv", "eltwise", "relu", "pool" };
         char text[320] = "";
         if (op.conv)
             B200_TRY(b200_conv2d_describe(op.conv, text, sizeof(text)));
-        const int n = snprintf(buf + used, len - used, "%s%s%s%s\n", names[(int)op.kind], text[0] ? ": " : "", text, op.skipped ? ", inside a conv" : "");
-        used += n < 0 || (size_t)n >= len - used ? len - used - 1 : (size_t)n;
+        add(snprintf(buf + used, len - used, "%s%s%s%s\n", names[(int)op.kind], text[0] ? ": " : "", text, op.skipped ? ", inside a conv" : ""));
     }
+    if (cs->host_parts[1] != 0)
+        add(snprintf(buf + used, len - used, "host run: in parts of %d and %d images\n", cs->host_parts[0], cs->host_parts[1]));
+    else if (cs->host_parts[0] != 0)
+        add(snprintf(buf + used, len - used, "host run: %d images\n", cs->host_parts[0]));
     return B200_OK;
 }
 

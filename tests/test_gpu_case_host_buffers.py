@@ -205,5 +205,48 @@ def test_images_that_are_copied_in_two_parts(net, hw, batch, pinned):
         ref.run_device(n, 0)
         torch.cuda.synchronize()
         assert torch.equal(y[:n], y_dev[:n].cpu()), i
+        assert ("in parts of %d and" % (n // 32 * 16) in cs.describe()[-1]) == (n == batch and i != 4), (i, cs.describe()[-1])
+    cs.close()
+    ref.close()
+
+
+def _two_branches(batch):
+    """A float and a byte image, each through a stem and a 3x3 conv, and their sum: bytes and, pooled, floats."""
+    from nart_b200.case import Case
+    rng = np.random.default_rng(8)
+    q = dict(ialpha=0.02, izp=117, oalpha=0.4, ozp=99, walpha=np.float32([0.004]))
+    cs = Case()
+    ends = []
+    for image in (cs.input_f32(3, 96, 128, 0.02, 117), cs.input_u8(4, 96, 128)):
+        stem = cs.conv2d(image, rng.integers(0, 256, (64, cs.dims(image)[0], 7, 7), dtype=np.uint8), None, stride=(2, 2), pad=(3, 3), **q)
+        ends.append(cs.conv2d(stem, rng.integers(0, 256, (64, 64, 3, 3), dtype=np.uint8), None, pad=(1, 1), **dict(q, ialpha=0.4, izp=99, oalpha=11.0)))
+    total = cs.eltwise_sum(ends, (11.0, 11.0), (99, 99), 14.0, 120)
+    pooled = cs.pool(total, 0, (8, 8), (0, 0), (8, 8), False, 14.0, 120, 14.0, 120)
+    cs.output_u8(pooled)
+    cs.output_f32(total, 14.0, 120)
+    cs.prepare(batch)
+    return cs
+
+
+def test_two_inputs_that_are_copied_in_two_parts():
+    batch = 187
+    cs, ref = _two_branches(batch), _two_branches(batch)
+    cs.use_graph(True)
+    stream = torch.cuda.Stream()
+    shapes = [((batch, 3, 96, 128), "<f4"), ((batch, 4, 96, 128), "|u1"), ((batch, 64, 6, 8), "|u1"), ((batch, 64, 48, 64), "<f4")]
+    dev = [torch.as_tensor(_Buffer(ref.io_device_ptr(i > 1, i % 2), *shapes[i]), device="cuda") for i in range(4)]
+    host = [torch.empty(s, dtype=torch.uint8 if t == "|u1" else torch.float32).pin_memory() for s, t in shapes]
+    for i, n in enumerate([batch, batch, batch, 40, batch]):
+        host[0].normal_(0, 1.5)
+        host[1].random_(0, 256)
+        cs.run_host_ptrs(n, [h.data_ptr() for h in host[:2]], [h.data_ptr() for h in host[2:]], stream.cuda_stream)
+        for d, h in zip(dev, host[:2]):
+            d.copy_(h)
+        torch.cuda.synchronize()
+        ref.run_device(n, 0)
+        torch.cuda.synchronize()
+        for d, h in zip(dev[2:], host[2:]):
+            assert torch.equal(h[:n], d[:n].cpu()) and len(torch.unique(d[:n])) > 8, i
+        assert ("in parts of 80 and 107" in cs.describe()[-1]) == (n == batch), (i, cs.describe()[-1])
     cs.close()
     ref.close()

@@ -65,7 +65,8 @@ def test_the_box_switch_is_read_at_creation(monkeypatch):
 # (c, k, kernel, strides, pads, h, w): images of four channels and of three, ragged channel counts
 GROUPS = [(4, 64, (7, 7), (2, 2), (3, 3), 30, 32), (4, 32, (3, 3), (2, 2), (1, 1), 31, 36), (4, 16, (3, 5), (1, 1), (1, 2), 9, 8), (4, 48, (8, 2), (1, 4), (0, 0), 12, 20),
           (3, 64, (7, 7), (2, 2), (3, 3), 33, 64), (4, 64, (7, 7), (2, 2), (3, 3), 30, 226), (24, 144, (1, 1), (1, 1), (0, 0), 9, 8), (20, 33, (1, 1), (1, 1), (0, 0), 6, 6),
-          (24, 40, (3, 3), (1, 1), (1, 1), 11, 14), (12, 18, (3, 3), (2, 2), (1, 1), 9, 16), (40, 20, (3, 3), (2, 2), (1, 1), 13, 10), (100, 150, (1, 1), (1, 1), (0, 0), 20, 10)]
+          (24, 40, (3, 3), (1, 1), (1, 1), 11, 14), (8, 48, (3, 3), (1, 1), (1, 1), 10, 12), (8, 33, (1, 5), (1, 1), (0, 2), 7, 6), (8, 64, (3, 3), (2, 2), (1, 1), 15, 18),
+          (12, 18, (3, 3), (2, 2), (1, 1), 9, 16), (40, 20, (3, 3), (2, 2), (1, 1), 13, 10), (100, 150, (1, 1), (1, 1), (0, 0), 20, 10)]
 
 
 @pytest.mark.parametrize("shape", GROUPS)
@@ -89,6 +90,8 @@ def test_groups_of_pixels(shape, size):
     if c <= 4:
         groups = size == "large" and w % 4 == 0
         assert ["four-pixel groups" in d for d in said] == [groups, groups and c == 3, groups], said        # (a padded copy is aligned)
+    if c == 8 and k % 16 == 0:      # two pixels are the sixteen channels of a box's
+        assert ["on groups of pixels" in d for d in said] == [True, False, True], said
     if c == 24 and r == 1:
         assert "groups of pixels" in said[0] and "groups of pixels" not in said[1] and said[2] == said[0]
 
