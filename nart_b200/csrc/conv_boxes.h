@@ -8,15 +8,16 @@ namespace b200 {
 
 // Tiles whose activations are loaded once for all taps.  One TMA box holds the tile's pixels and the ring around them that the
 // window reaches, `pitch` pixels a row, and a tap's operand is the same box from a later row on: the descriptor's start address
-// moves, the swizzle being a function of the absolute address.  A strided conv has one box per parity plane.
-constexpr int kHaloTaps = 16;
+// moves, the swizzle being a function of the absolute address.  With a vertical stride there is a box per parity of the rows; columns
+// lie side by side (a horizontal stride only with windows of one column).
 struct HaloTiles {
-    int planes;                        // parity planes with a tap, 1 to 4
+    int planes;                        // row parities with a tap, 1 or 2
     int tw, th, pitch;                 // output pixels a tile (one image)
-    int tap_row, tap_col;              // between the numbers of taps that are neighbours in a plane, along its rows and columns
-    int taps_h[4], taps_w[4], tap0[4]; // per plane: its taps, rows and columns, and the first one's number
-    int dx[4], dy[4], rows[4];         // the box's first pixel against the tile's, its pixels (pitch * lines)
-    uint8_t parity[4];                 // row parity * 2 + column parity
+    int tap_row;                       // between the numbers of taps that are neighbours in a plane, along its columns
+    int taps_w, dx;                    // taps a row; the box's first column against the tile's
+    int taps_h[2], tap0[2];            // per plane: rows of taps, the first tap's number
+    int dy[2], rows[2];                // the box's first line against the tile's, its pixels (pitch * lines)
+    uint8_t row_parity[2], col_parity;
     int span;                          // pixels that the operands of a box reach over
 };
 // What the boxes depend on: the window.  row_pixels: the columns of the window that one operand row holds, 0 for one.
@@ -25,7 +26,8 @@ struct HaloWindow {
     int width;                         // pixels an operand row holds; 1, or (ConvIgemmPlan::quads) all those of a window's row: s is 1 then
     int ring_w = 0, ring_h = 0;        // pixels beside the tile's, along each axis
     HaloWindow(int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int row_pixels = 0, int width = 1);
-    bool fits() const { return r * s <= kHaloTaps && (r * s >= 2 || width > 1) && ring_h <= 64; }
+    // (up to sixteen taps and 64 lines of ring: nothing in the kernel asks for it, larger windows have not been measured)
+    bool fits() const { return (stride_w == 1 || s == 1) && r * s <= 16 && (r * s >= 2 || width > 1) && ring_h <= 64; }
 };
 // Planes and taps from h.tw, h.th and h.pitch; the eight-row groups of an operand lie `group` pixels apart.
 void halo_planes(const HaloWindow &win, int group, HaloTiles *h);

@@ -769,9 +769,9 @@ __global__ void __launch_bounds__(MODE == 1 || MODE == 5 ? kThreads2 : kThreads,
                             if (elect_one()) {
                                 mbar_expect_tx(fb, (uint32_t)(h.rows[pl] * g.a_pitch));
                                 if (g.quads)
-                                    tma_load_3d(a_dst, &maps.a[pl], fb, (x0 + h.dx[pl]) * 2, y0 + h.dy[pl], n0);
+                                    tma_load_3d(a_dst, &maps.a[pl], fb, (x0 + h.dx) * 2, y0 + h.dy[pl], n0);
                                 else
-                                    tma_load_4d(a_dst, &maps.a[pl], fb, c * (int)bk, x0 + h.dx[pl], y0 + h.dy[pl], n0);
+                                    tma_load_4d(a_dst, &maps.a[pl], fb, c * (int)bk, x0 + h.dx, y0 + h.dy[pl], n0);
                             }
                             __syncwarp();
                             fb += 8;
@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(MODE == 1 || MODE == 5 ? kThreads2 : kThreads,
                     const HaloTiles &h = g.halo;
                     const uint32_t a_hi = halo_desc_hi(desc_hi, g.box_group, g.a_pitch, g.quads);
                     const uint32_t a_col = (uint32_t)g.a_pitch >> 4, a_row = (uint32_t)(h.pitch * g.a_pitch) >> 4;
-                    const uint32_t b_tap = (uint32_t)cchunks * b_step, b_col = h.tap_col * b_tap, b_row = h.tap_row * b_tap;
+                    const uint32_t b_tap = (uint32_t)cchunks * b_step, b_row = h.tap_row * b_tap;
                     const uint32_t box_step = g.box_bytes >> 4;
                     for (int c = 0; ok && c < cchunks; ++c) {
                         const int ksteps = c + 1 == cchunks ? last_steps : ksteps_full;
@@ -998,10 +998,10 @@ __global__ void __launch_bounds__(MODE == 1 || MODE == 5 ? kThreads2 : kThreads,
                             tc_fence_after();
                             // the taps of the plane, up to three of a row at a time
                             uint32_t a0 = (uint32_t)adesc0 + (uint32_t)stage * box_step, b0 = b_lo0 + (uint32_t)c * b_step + h.tap0[pl] * b_tap;
-                            const int th = h.taps_h[pl], tw = h.taps_w[pl];
+                            const int th = h.taps_h[pl], tw = h.taps_w;
                             for (int i = 0; i < th; ++i, a0 += a_row, b0 += b_row) {
                                 uint32_t a = a0, b = b0;
-                                for (int j = 0; j < tw; j += 3, a += 3 * a_col, b += 3 * b_col) {
+                                for (int j = 0; j < tw; j += 3, a += 3 * a_col, b += 3 * b_tap) {
                                     auto tap = [&](uint32_t ta, uint32_t tb, uint32_t acc) {
                                         mma_i8_ab(d_tmem, ta, tb, a_hi, desc_hi, idesc, acc);
                                         if (ksteps >= 2)
@@ -1014,9 +1014,9 @@ __global__ void __launch_bounds__(MODE == 1 || MODE == 5 ? kThreads2 : kThreads,
                                     if (elect_one()) {
                                         tap(a, b, accumulate);
                                         if (j + 1 < tw)
-                                            tap(a + a_col, b + b_col, 1);
+                                            tap(a + a_col, b + b_tap, 1);
                                         if (j + 2 < tw)
-                                            tap(a + 2 * a_col, b + 2 * b_col, 1);
+                                            tap(a + 2 * a_col, b + 2 * b_tap, 1);
                                     }
                                     __syncwarp();
                                     accumulate = 1;

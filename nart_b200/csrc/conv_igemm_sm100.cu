@@ -853,14 +853,10 @@ HaloWindow::HaloWindow(int r_, int s_, int stride_h_, int stride_w_, int pad_h_,
     : r(r_), s(s_), stride_h(stride_h_), stride_w(stride_w_), pad_h(pad_h_), pad_w(pad_w_), width(width_)
 {
     int lo, hi;
-    for (int p = 0; p < stride_w; ++p)
-        if (tap_span(s, stride_w, pad_w, p, &lo, &hi) && hi - lo > ring_w)
-            ring_w = hi - lo;
     for (int p = 0; p < stride_h; ++p)
         if (tap_span(r, stride_h, pad_h, p, &lo, &hi) && hi - lo > ring_h)
             ring_h = hi - lo;
-    if (row_pixels > 0)
-        ring_w = row_pixels - 1;
+    ring_w = row_pixels > 0 ? row_pixels - 1 : s - 1;
 }
 
 void halo_planes(const HaloWindow &win, int group, HaloTiles *out)
@@ -869,31 +865,26 @@ void halo_planes(const HaloWindow &win, int group, HaloTiles *out)
     h.planes = 0;
     h.span = 0;
     h.tap_row = win.stride_h * win.s;
-    h.tap_col = win.stride_w;
-    // the first tap of a parity along one axis, and how many follow it a stride apart
-    auto first_tap = [](int kernel, int stride, int pad, int parity) {
-        int t = 0;
-        while (t < kernel && ((t - pad) & (stride - 1)) != parity)
-            ++t;
-        return t;
-    };
-    for (int ph = 0; ph < win.stride_h; ++ph)
-        for (int pw = 0; pw < win.stride_w; ++pw) {
-            int y0, y1, x0, x1;
-            if (!tap_span(win.r, win.stride_h, win.pad_h, ph, &y0, &y1) || !tap_span(win.s, win.stride_w, win.pad_w, pw, &x0, &x1))
-                continue;
-            const int pl = h.planes++, r0 = first_tap(win.r, win.stride_h, win.pad_h, ph), s0 = first_tap(win.s, win.stride_w, win.pad_w, pw);
-            h.dx[pl] = x0;
-            h.dy[pl] = y0;
-            h.rows[pl] = h.pitch * (h.th + y1 - y0);
-            h.parity[pl] = (uint8_t)(ph * 2 + pw);
-            h.taps_h[pl] = (win.r - r0 + win.stride_h - 1) / win.stride_h;
-            h.taps_w[pl] = (win.s - s0 + win.stride_w - 1) / win.stride_w;
-            h.tap0[pl] = r0 * win.s + s0;
-            // an operand is sixteen groups of eight rows from its first one on (of `width` pixels each)
-            const int last = (h.taps_h[pl] - 1) * h.pitch + h.taps_w[pl] - 1;
-            h.span = std::max(h.span, std::max(h.rows[pl], last + 15 * group + 8 + win.width - 1));
-        }
+    h.taps_w = win.s;
+    h.col_parity = (uint8_t)(win.pad_w & (win.stride_w - 1));
+    int x1;
+    tap_span(win.s, win.stride_w, win.pad_w, h.col_parity, &h.dx, &x1);
+    for (int ph = 0; ph < win.stride_h; ++ph) {
+        int y0, y1, r0 = 0;
+        if (!tap_span(win.r, win.stride_h, win.pad_h, ph, &y0, &y1))
+            continue;
+        while (((r0 - win.pad_h) & (win.stride_h - 1)) != ph)       // the first tap of this parity; the others follow a stride apart
+            ++r0;
+        const int pl = h.planes++;
+        h.dy[pl] = y0;
+        h.rows[pl] = h.pitch * (h.th + y1 - y0);
+        h.row_parity[pl] = (uint8_t)ph;
+        h.taps_h[pl] = (win.r - r0 + win.stride_h - 1) / win.stride_h;
+        h.tap0[pl] = r0 * win.s;
+        // an operand is sixteen groups of eight rows from its first one on (of `width` pixels each)
+        const int last = (h.taps_h[pl] - 1) * h.pitch + h.taps_w - 1;
+        h.span = std::max(h.span, std::max(h.rows[pl], last + 15 * group + 8 + win.width - 1));
+    }
 }
 
 // The same for the boxes of HaloTiles, a map per plane.
@@ -901,7 +892,7 @@ static int encode_boxes(const ConvIgemmPlan *p, const uint8_t *x, int n, const H
 {
     const ConvGeom &g = p->g;
     for (int i = 0; i < h.planes; ++i) {
-        const int ph = h.parity[i] >> 1, pw = h.parity[i] & 1;
+        const int ph = h.row_parity[i], pw = h.col_parity;
         if (p->quads) {         // whole lines of the image, in 8-byte elements
             cuuint64_t dims[3] = { (cuuint64_t)g.w * 2, (cuuint64_t)((g.h - ph + g.stride_h - 1) / g.stride_h), (cuuint64_t)n };
             cuuint64_t strides[2] = { (cuuint64_t)g.stride_h * g.w * 16, (cuuint64_t)g.h * g.w * 16 };

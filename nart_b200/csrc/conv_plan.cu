@@ -205,6 +205,8 @@ int conv_run_padded(b200_conv *cv, const uint8_t *x, int32_t n, uint8_t *y, cuda
 // output pixel is the m / stride neighbouring output pixels whose windows start in one group, side by side as they lie in
 // memory, its window the groups that theirs reach.  Part of the weights is zero (7x7 on 4 channels, stride 2: 128 output
 // channels and 7 x 3 groups of 16 for 64 and 7 x 7 pixels of 4), but the image is read as it is.  flat: 1x1, all of an image is one line.
+// Left out: lines of no whole number of groups, as a group would hold pixels of two lines; weight zero points, as the window-sum column
+// would sum the pixels of all the group's windows; and signed activations, for which nothing has been measured.
 int create_grouped(const ConvGeom &g, int m, bool flat, const std::vector<int8_t> &w, const int32_t *bias, const std::vector<uint32_t> &mult,
                    const std::vector<int32_t> &shift, ConvIgemmPlan **out)
 {

@@ -19,11 +19,13 @@ def _inputs(c, k, r, s, h, w, n, seed, signed=False):
 
 
 # (c, k, kernel (r, s), strides, pads, h, w, n): lines that fill a power of two with their ring and not, maps of one pixel more or
-# less than the tiles, planes of a strided window with one and two taps an axis, several channel chunks, an asymmetric window
+# less than the tiles, planes of a strided window with one and two taps an axis, several channel chunks, an asymmetric window, windows
+# of one column with a horizontal stride (the others of those keep a box per tap)
 BOXES = [(64, 64, (3, 3), (1, 1), (1, 1), 56, 56, 9), (64, 48, (3, 3), (1, 1), (1, 1), 27, 35, 30), (32, 16, (3, 3), (1, 1), (1, 1), 17, 126, 8),
          (32, 32, (3, 3), (1, 1), (1, 1), 16, 127, 9), (128, 128, (3, 3), (1, 1), (1, 1), 28, 30, 24), (96, 80, (3, 3), (2, 2), (1, 1), 33, 31, 40),
          (16, 256, (3, 3), (1, 1), (0, 0), 10, 9, 60), (48, 96, (5, 3), (1, 2), (2, 1), 30, 29, 20), (160, 32, (2, 4), (2, 1), (1, 3), 21, 23, 30),
-         (64, 64, (1, 3), (1, 1), (0, 1), 3, 6, 200), (32, 64, (4, 4), (2, 2), (0, 2), 40, 62, 12)]
+         (64, 64, (1, 3), (1, 1), (0, 1), 3, 6, 200), (32, 64, (4, 4), (2, 2), (0, 2), 40, 62, 12),
+         (64, 48, (3, 1), (1, 2), (1, 1), 20, 21, 60), (32, 16, (4, 1), (2, 2), (1, 0), 21, 24, 40)]
 
 
 @pytest.mark.parametrize("shape", BOXES)
