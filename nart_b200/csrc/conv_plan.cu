@@ -277,16 +277,29 @@ int reserve_owned(b200_conv *conv, int32_t n_padded, int32_t n_lowered)
 
 // A run on groups needs no rows, but the plan's scratch grows with the batch whatever route a run takes: after it, a smaller batch
 // or an unaligned view of as many images neither allocates (it may be under capture) nor moves the rows that a captured graph knows.
+// Without memory for more rows the plan keeps those it has and does not ask again.
 int reserve_beside_groups(b200_conv *conv, int32_t n, cudaStream_t st)
 {
-    if (PaddedBytes(conv, n).lowered <= conv->scratch_bytes)
+    const size_t need = PaddedBytes(conv, n).lowered;
+    if (need <= conv->scratch_bytes || need >= conv->scratch_declined)
         return B200_OK;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     B200_CUDA_TRY(cudaStreamIsCapturing(st, &capture));
     if (capture != cudaStreamCaptureStatusNone)
         return B200_OK;
-    const int rc = reserve_owned(conv, n, n);
-    return rc == B200_ERR_NOMEM ? B200_OK : rc;
+    const DeviceGuard on(conv->device);
+    uint8_t *rows = nullptr;
+    const int rc = scratch_alloc(&rows, need);
+    if (rc == B200_ERR_NOMEM) {
+        conv->scratch_declined = need;
+        return B200_OK;
+    }
+    B200_TRY(rc);
+    const cudaError_t e = scratch_free(conv->scratch, conv->device);
+    conv->scratch = rows;
+    conv->scratch_bytes = need;
+    B200_CUDA_TRY(e);
+    return B200_OK;
 }
 
 }  // namespace

@@ -193,6 +193,7 @@ struct b200_conv {
     b200::ConvGeom g_low;
     uint8_t *scratch = nullptr;     // [n][h][ow][32]
     size_t scratch_bytes = 0;
+    size_t scratch_declined = SIZE_MAX;     // there was no memory for this much beside a run on groups
     // Channel counts the tensor-core path does not take (no multiple of 16): every run copies the activations into
     // a scratch tensor of pad_c channels, and the igemm plan (g_pad, or g_low on it) has zero weights there.
     int pad_c = 0;

@@ -136,6 +136,37 @@ def test_captures_behind_a_large_run_of_a_four_channel_image():
         assert torch.equal(one, want[:1]) and torch.equal(views, want)
 
 
+def test_a_large_run_without_memory_for_rows_leaves_those_there_are():
+    """A run on groups needs no rows itself: it goes on, and what an earlier graph reads stays."""
+    from nart_b200._lib import lib
+    c, k, hw, n = 4, 32, 56, 2000           # 200 MB of rows
+    plan, direct = _plan(c, k, hw), _direct(c, k, hw)
+    x = torch.randint(0, 256, (n, hw, hw, c), device="cuda", dtype=torch.uint8)
+    y = torch.zeros((n, hw, hw, k), device="cuda", dtype=torch.uint8)
+    want = direct(x)
+    assert torch.equal(plan(x[:20]), want[:20]) and "row-lowered" in plan.describe()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        one = plan(x[:1])
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    filler = torch.empty(free - (120 << 20), device="cuda", dtype=torch.uint8)
+    for _ in range(2):
+        y.zero_()
+        assert lib.b200_conv2d_run(plan._h, x.data_ptr(), n, y.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert "four-pixel groups" in plan.describe()
+    del filler
+    torch.cuda.empty_cache()
+    one.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(one, want[:1])
+    assert torch.equal(plan(x[:20]), want[:20])
+
+
 def test_first_run_of_a_process_under_capture():
     """Nothing that a capture forbids is left to the first run."""
     import os
