@@ -314,16 +314,16 @@ __global__ void __launch_bounds__(256) conv_depthwise3x3_kernel(
 // the fifth word against w2 placed at the channel's own byte (no extraction).  Neighbouring output rows
 // share 3 - S of their input rows.
 //
-// Instruction issue bounds it, and the dp4a pipe (one per two cycles): with 2 x 2 outputs per thread, 64-bit
+// Its instructions bound it, most of them on the integer pipe (63 % of issue slots at 22 % of the warps): with 2 x 2 outputs per thread, 64-bit
 // divisions and a wide integer requantize it took 24 instructions per output byte (144 channels of 56 x 56,
 // batch 64: 35.7 us, 1.6 TB/s).  So weights and constants are read once for ROWS rows, indices are divided by
 // multiplication, and the requantize is fp32, exactly, two values per instruction: the accumulator starts at
 // bits(1.5 * 2^23) + bias, which makes its bits the float 1.5 * 2^23 + acc (|acc| < 2^22, checked when the table
-// is built); mult * 2^-shift is a float m (24 significant bits); acc * m + (zero point + 1/2) is formed by one
+// is built); mult * 2^-shift is a float m (24 significant bits); acc * m + (zero point less floor + 1/2) is formed by one
 // multiply-add rounded toward zero, which never crosses an integer, and 2^23 is added, again toward zero: the low
-// bits are then floor(acc * m + 1/2) + zero point for every result of 0 or more, and for every negative one the
+// bits are then floor(acc * m + 1/2) + zero point less floor for every result of 0 or more, and for every negative one the
 // low 16 bits are a negative 16-bit number (below 2^23 a float's last bit is a half: results stay within -2^14 .. 2^15,
-// checked as well).  Floor and ceiling run on pairs of those.
+// checked as well).  Both bounds run on pairs of those, and the floor goes back onto the packed bytes.
 // (A thread that walks whole columns, every input row loaded and transposed once, is no faster: its accumulators in
 // flight and weights leave 16 to 20 warps per SM, and its row loop's bookkeeping costs what the shared rows save.)
 // Weight table: [c/4][3 kernel rows][2 + (S == 2)][4 channels] words.  Requantize table: [c/4] 4 start values, 4 floats.
